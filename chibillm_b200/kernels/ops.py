@@ -873,6 +873,19 @@ class CudaKernels:
                                 page_size, scale, window, max_q_len, max_ctx_len, min_q_len, seq_rows, cap, r1, r2,
                                 chunk, sink)
             return
+        if not special and q.dtype == torch.float32 and k_cache.dtype == torch.float32 and v_cache.dtype == torch.float32 \
+                and d in (64, 128):
+            # the 32-bit path's usual head sizes (tiles of query rows for prompts, ranges of keys for single tokens)
+            status = self.lib.chibi_attention_f32(
+                _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0), _ptr(q_start),
+                _ptr(ctx_len), _ptr(seq_rows), ctx_len.numel(), nq, nkv, d, page_size, k_cache.shape[0], float(scale),
+                int(window or 0), chunk, int(max_q_len), int(min_q_len), int(max_ctx_len), cap, _ptr(r1), _ptr(r2),
+                _ptr(sink), _ptr(self.error), self._stream())
+            if status == 0:
+                self.launches += (1 if max_q_len > 1 else 0) + (1 if max_q_len == 1 or min_q_len <= 1 else 0)
+                return
+            if status != -2:
+                _check(status, "attention (32-bit)")
         self.launches += 1
         _check(self.lib.chibi_attention_generic_shared(
             _ptr(q), _code(q), _ptr(k_cache), _ptr(v_cache), _code(k_cache), _ptr(out), _code(out),

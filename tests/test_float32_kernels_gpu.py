@@ -49,3 +49,94 @@ def test_linear_float32_keeps_infinities_to_their_rows(k):
         k.linear(x[:rows], w, out)
         bad = ~torch.isfinite(out)
         assert bad[3].all() and bad[:, 50].all() and int(bad.sum()) == 100 + rows - 1
+
+
+def exact_attention(q, keys, values, table, q_lens, ctx, nq, nkv, d, page, scale, window, chunk, softcap, bias, sink):
+    out, at, G = [], 0, nq // nkv
+    for s, (n, c) in enumerate(zip(q_lens, ctx)):
+        pages = table[s, :-(-c // page)].long()
+        k = keys[pages].transpose(1, 2).reshape(-1, nkv, d)[:c].double().repeat_interleave(G, 1)
+        v = values[pages].transpose(1, 2).reshape(-1, nkv, d)[:c].double().repeat_interleave(G, 1)
+        x = torch.einsum("thd,khd->htk", q[at:at + n].view(n, nq, d).double(), k) * scale
+        if softcap:
+            x = softcap * torch.tanh(x / softcap)
+        i, j = torch.arange(c - n, c, device="cuda")[:, None], torch.arange(c, device="cuda")[None]
+        if bias is not None:
+            r1, r2 = (None if r is None else r.double()[:, None, None] for r in bias)
+            x = x - (r1 * (i - j).double() if r2 is None else r1 * torch.log1p(r2 * (i - j).clamp(min=0).double()))
+        hidden = j > i
+        if window:
+            hidden = hidden | (j <= i - window)
+        if chunk:
+            hidden = hidden | (j < i - i % chunk)
+        x = x.masked_fill(hidden, float("-inf"))
+        if sink is not None:
+            x = torch.cat([x, sink.double()[:, None, None].expand(nq, n, 1)], -1)
+            v = torch.cat([v, torch.zeros_like(v[:1])])
+        out.append(torch.einsum("htk,khd->thd", torch.softmax(x, -1), v).reshape(n, nq * d))
+        at += n
+    return torch.cat(out)
+
+
+# lengths: single tokens with 1 key, a range's edge (64 keys), eight ranges and more; portions that begin inside a tile
+# of 32 keys; row tiles cut inside a token's group (5 heads) and by the sequence's end; steps of both kinds
+@pytest.mark.parametrize("d,nq,nkv,page,q_lens,ctx,options", [
+    (128, 4, 2, 16, [1, 1, 1, 1], [1, 64, 65, 1500], {}),
+    (64, 5, 1, 8, [1, 1, 1], [33, 512, 513], {"softcap": 20.0, "sink": True}),
+    (64, 16, 2, 16, [1, 1], [300, 700], {"window": 100, "bias": "linear"}),
+    (64, 4, 4, 32, [1, 1], [300, 40], {"chunk": 64, "bias": "log"}),
+    (128, 4, 2, 16, [2, 33, 130], [2, 40, 330], {}),
+    (64, 5, 1, 8, [100, 13], [100, 77], {"softcap": 20.0, "sink": True}),
+    (64, 16, 2, 16, [70, 1, 5], [300, 90, 5], {"window": 50, "bias": "linear"}),
+    (128, 4, 4, 32, [150, 1], [200, 1], {"chunk": 64, "bias": "log"}),
+])
+def test_attention_float32(k, d, nq, nkv, page, q_lens, ctx, options):
+    T, S = sum(q_lens), len(q_lens)
+    pages = [-(-c // page) for c in ctx]
+    order = torch.randperm(sum(pages) + 3, generator=torch.Generator().manual_seed(1)).to(torch.int32)
+    table = torch.zeros(S, max(pages) + 1, dtype=torch.int32)
+    at = 0
+    for s, n in enumerate(pages):
+        table[s, :n] = order[at:at + n]
+        at += n
+    table = table.cuda()
+    keys, values = rnd(sum(pages) + 3, nkv, page, d, seed=1), rnd(sum(pages) + 3, nkv, page, d, seed=2)
+    q = rnd(T, nq * d, seed=3)
+    # what nobody may read: places past a sequence's end in its last page, and pages of nobody
+    used = torch.zeros(keys.shape[0], page, dtype=torch.bool, device="cuda")
+    for s, c in enumerate(ctx):
+        for u in range(c):
+            used[table[s, u // page].long(), u % page] = True
+    keys.masked_fill_(~used[:, None, :, None], float("nan"))
+    values.masked_fill_(~used[:, None, :, None], float("nan"))
+    starts = [0]
+    for n in q_lens:
+        starts.append(starts[-1] + n)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    bias = {None: None, "linear": (rnd(nq, seed=4).abs() * 0.1, None),
+            "log": (rnd(nq, seed=4).abs(), rnd(nq, seed=5).abs())}[options.get("bias")]
+    sink = rnd(nq, seed=6) if options.get("sink") else None
+    out = torch.full((T, nq * d), float("nan"), device="cuda")
+    k.attention(q, keys, values, out, table, ints(starts), ints(ctx), ints([i for i, n in enumerate(q_lens) for _ in range(n)]),
+                ints([c - n + j for n, c in zip(q_lens, ctx) for j in range(n)]), nq, nkv, d, page, d ** -0.5,
+                options.get("window"), max(q_lens), max(ctx), min_q_len=min(q_lens), softcap=options.get("softcap"),
+                distance_bias=bias, chunk=options.get("chunk"), sink=sink)
+    k.check_error_word()
+    exact = exact_attention(q, keys.nan_to_num(), values.nan_to_num(), table, q_lens, ctx, nq, nkv, d, page, d ** -0.5,
+                            options.get("window"), options.get("chunk"), options.get("softcap"), bias, sink)
+    # a score is off by at most (d / 4 + 8) roundings of sums of magnitude |q| |k| / sqrt(d) < 16, its exponential by
+    # as much relatively, and the weighted mean of values below 6 by twice that
+    assert torch.isfinite(out).all()
+    assert float((out.double() - exact).abs().max()) <= 2 * 6 * 16 * (d / 4 + 16) * UNIT
+
+
+def test_attention_float32_hides_later_values(k):
+    """A value that is not a number reaches only the tokens that see its key."""
+    d, T = 64, 40
+    keys, values, q = rnd(3, 1, 16, d, seed=1), rnd(3, 1, 16, d, seed=2), rnd(T, d, seed=3)
+    values[1, 0, 4] = float("nan")                       # position 20
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    out = torch.empty(T, d, device="cuda")
+    k.attention(q, keys, values, out, ints([[0, 1, 2]]), ints([0, T]), ints([T]), ints([0] * T), ints(list(range(T))), 1, 1, d, 16,
+                d ** -0.5, None, T, T, min_q_len=T)
+    assert torch.isfinite(out[:20]).all() and torch.isnan(out[20:]).all()
