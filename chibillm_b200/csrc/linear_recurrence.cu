@@ -3,7 +3,10 @@
 // * the gated delta rule with a decay per key channel (DELTA):
 //     S <- diag(g_t) S,   u_t = b_t (v_t - S^T k_t),   S <- S + k_t u_t^T,   o_t = S^T q_t
 //   with unit keys and queries and g_t = exp(-exp(A) softplus(z_t + bias)) made here;
-// * linear attention with a constant decay per head: S <- decay S + k_t v_t^T, o_t = S^T q_t.
+// * linear attention with a constant decay per head: S <- decay S + k_t v_t^T, o_t = S^T q_t;
+// * the generalised delta rule, whose removal looks at the state before the decay (GENERAL):
+//     S <- diag(g_t) S - (a_t x_t)(x_t^T S) + k_t v_t^T, o_t = S^T r_t
+//   with unit keys x_t, rates a_t per channel and g_t = exp(-c sigmoid(z_t + bias)) made here.
 //
 // Prompt portions go in chunks of 16 tokens (RC).  With G_t = g_1 .. g_t (row-wise products from the chunk's
 // start) and S_0 the state before the chunk, the u_t of a chunk solve a lower triangular system,
@@ -13,7 +16,13 @@
 //     O = (G q) S_0 + B U = B M V + Q S_0,   Q = (G q) - B W,
 //     S_end = diag(G_end) S_0 + sum_s (g_{s+1} .. g_end k_s) u_s^T.
 // All decays appear as products of factors from 0 to 1 (no quotients), so nothing overflows however strong
-// they are.  Without the delta rule U = V, Q = G q and O = B V + Q S_0.  A first kernel makes, for every chunk
+// they are.  Without the delta rule U = V, Q = G q and O = B V + Q S_0.  The generalised rule has two writes a
+// token: with A^y_ts = sum_c x_t[c] y_s[c] (g_{s+1} .. g_{t-1})[c] and B^y_ts = sum_c r_t[c] y_s[c] (g_{s+1} .. g_t)[c],
+// y = a x or k, M = (I + A^{ax})^-1 and U = -(what the tokens' removals find),
+//     U = -M A^k V + W S_0,          W = -M (G_{t-1} x),
+//     O = (B^k - B^{ax} M A^k) V + Q S_0,   Q = (G r) + B^{ax} W,
+//     S_end = diag(G_end) S_0 + sum_s (g_{s+1} .. g_end a_s x_s) u_s^T + sum_s (g_{s+1} .. g_end k_s) v_s^T.
+// A first kernel makes, for every chunk
 // and head at once, the rows W, Q, g_{s+1..end} k, the row G_end and the matrices M, B M; a second kernel walks
 // over a sequence's chunks with a piece of S (all d rows of some columns) in registers: two small products
 // with S_0 and V, then one into S.  A chunk that is not full has zero rows for the tokens it lacks.
@@ -27,11 +36,14 @@ namespace chibi {
 
 constexpr int RC = 16;                                  // tokens of a chunk
 
+constexpr int LINEAR = 0, DELTA = 1, GENERAL = 2;       // the three recurrences
+
 // A chunk's block in the scratch array, in floats (d padded to DP): KE [RC][DP] | GE [DP] | Q [RC][DP] |
-// B M or B [RC][RC] and, with the delta rule, | -W [RC][DP] | M [RC][RC].
-__host__ __device__ constexpr int rc_block(int DP, bool delta)
+// B M or B [RC][RC] and, with the delta rules, | -W [RC][DP] | M [RC][RC]; with the generalised one its W, -M A^k and
+// B^k - B^{ax} M A^k stand in those places, KE holds the removals' rows and | the keys' [RC][DP] follow.
+__host__ __device__ constexpr int rc_block(int DP, int rule)
 {
-    return (delta ? 3 : 2) * RC * DP + DP + (delta ? 2 : 1) * RC * RC;
+    return (rule + 2) * RC * DP + DP + (rule != LINEAR ? 2 : 1) * RC * RC;
 }
 
 // silu, and the decay exp(rate * softplus(z)).  Beside bfloat16 activations CUDA's faster exponential and logarithm
@@ -66,6 +78,10 @@ struct RecurrenceParams {
     float key_eps, q_scale;
     // linear attention
     const float* decay;        // [heads]
+    // generalised delta rule (q: r; logits: z; dt_bias: its bias)
+    const void* removal;       // [T, stride]: heads * d columns
+    const float* removal_bias; // [heads * d]
+    float decay_scale;
     float* state;              // [slots, heads, d, e]
     float* o;                  // [T, heads * e]
     float* scratch;
@@ -79,7 +95,7 @@ struct RecurrenceParams {
 // sources s and four targets t, lanes along the channels.  Off the diagonal the sources are decayed to the
 // targets' first token and the targets from there, so that a tile is a plain product; on it the sources are
 // decayed token by token.  A tile's 32 sums over the lanes are folded together.
-template <int DP, bool DELTA, typename TX>
+template <int DP, int RULE, typename TX>
 __global__ void __launch_bounds__(256)
 recurrence_prepare_kernel(const RecurrenceParams p)
 {
@@ -111,13 +127,13 @@ recurrence_prepare_kernel(const RecurrenceParams p)
     const int d = p.d, kh = h / (p.heads / p.qk_heads);
     const TX* q = static_cast<const TX*>(p.q) + (size_t)(row0 + base) * p.stride + kh * d;
     const TX* k = static_cast<const TX*>(p.k) + (size_t)(row0 + base) * p.stride + kh * d;
-    float* KE = p.scratch + ((size_t)((row0 / RC) + seq + blockIdx.x) * p.heads + h) * rc_block(DP, DELTA);
+    float* KE = p.scratch + ((size_t)((row0 / RC) + seq + blockIdx.x) * p.heads + h) * rc_block(DP, RULE);
     float* GE = KE + RC * DP;
     float* Qo = GE + DP;
     float* No = Qo + RC * DP;                           // B M, or B
     float* Wo = No + RC * RC;
     float* Mo = Wo + RC * DP;
-    const float rate = DELTA ? -expf(p.a_log[h]) : 0.f;
+    const float rate = RULE == DELTA ? -expf(p.a_log[h]) : 0.f;
 
     // ---- the chunk's keys, queries and decays
     {
@@ -132,7 +148,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
             if (t < n && c < d) {
                 kr[u] = k[(size_t)t * p.stride + c];
                 qr[u] = q[(size_t)t * p.stride + c];
-                if (DELTA)
+                if (RULE == DELTA)
                     zr[u] = p.logits[(size_t)(row0 + base + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
             }
         }
@@ -144,12 +160,12 @@ recurrence_prepare_kernel(const RecurrenceParams p)
                 kv = lr_silu<TX>(kv), qv = lr_silu<TX>(qv);     // (silu(0) is 0)
             ks[i] = kv;
             qs[i] = qv;
-            if (DELTA)
+            if (RULE == DELTA)
                 gs[i] = t < n && c < d ? lr_decay<TX>(rate, zr[u]) : 1.f;
         }
     }
     if (tid < RC) {
-        if (DELTA) {
+        if (RULE == DELTA) {
             bs[tid] = tid < n ? 1.f / (1.f + expf(-to_f32(static_cast<const TX*>(p.beta)[(size_t)(row0 + base + tid)
                                                                                         * p.beta_stride + h]))) : 0.f;
         } else {
@@ -167,7 +183,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
         reinterpret_cast<float4*>(&Ms[0][0])[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __syncthreads();
-    if (DELTA) {
+    if (RULE == DELTA) {
         // unit keys and queries: two tokens to a warp
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -210,7 +226,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
 #pragma unroll
             for (int s = 0; s < 4; ++s)
                 w[s] = ks[(4 * J + s) * DP + c];
-            if (!DELTA) {
+            if (RULE != DELTA) {
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                     const float qv = qs[(4 * I + t) * DP + c];
@@ -268,14 +284,14 @@ recurrence_prepare_kernel(const RecurrenceParams p)
         }
         const int t = 4 * I + ((lane >> 2) & 3), s = 4 * J + (lane & 3);
         if (lane < 16) {
-            if (DELTA)
+            if (RULE == DELTA)
                 As[t][s] = acc[0];
         } else if (t >= s) {
-            Bs[t][s] = DELTA ? acc[0] : acc[0] * power[t - s];
+            Bs[t][s] = RULE == DELTA ? acc[0] : acc[0] * power[t - s];
         }
     }
     __syncthreads();
-    if (!DELTA) {
+    if (RULE != DELTA) {
         No[tid] = Bs[tid / RC][tid % RC];               // (256 threads, 16 x 16 values)
         for (int c = tid; c < DP; c += 256) {
 #pragma unroll
@@ -367,6 +383,262 @@ recurrence_prepare_kernel(const RecurrenceParams p)
     }
 }
 
+// The same for the generalised delta rule; the inner products' tiles take two kinds of sources (removals, keys) at
+// a time, 64 sums.
+template <int DP, typename TX>
+__global__ void __launch_bounds__(256)
+general_prepare_kernel(const RecurrenceParams p)
+{
+#ifdef CHIBI_TIMELINE
+    pdl_enter();
+#else
+    pdl_wait();                                         // (no trigger: as above)
+#endif
+    constexpr int R = DP / 32;
+    extern __shared__ __align__(16) float sm[];
+    float* ks = sm;                                     // [RC][DP] keys
+    float* xs = ks + RC * DP;                           // unit keys
+    float* as = xs + RC * DP;                           // rate * unit key
+    float* rs = as + RC * DP;                           // receptances
+    float* gs = rs + RC * DP;                           // decays
+    float* gg = gs + RC * DP;                           // [4][DP]: the decays' products over four tokens each
+    __shared__ __align__(16) float Aa[RC][RC], Ak[RC][RC], Ba[RC][RC], Bk[RC][RC], Ms[RC][RC], Ns[RC][RC];
+    const int h = blockIdx.y, seq = blockIdx.z;
+    const int row0 = p.q_start[seq];
+    const int base = blockIdx.x * RC;
+    const int n = min(RC, p.q_start[seq + 1] - row0 - base);
+    if (n <= 0)
+        return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int d = p.d;
+    const size_t at0 = (size_t)(row0 + base) * p.stride + h * d;
+    const TX* r = static_cast<const TX*>(p.q) + at0;
+    const TX* k = static_cast<const TX*>(p.k) + at0;
+    const TX* a = static_cast<const TX*>(p.removal) + at0;
+    float* KE = p.scratch + ((size_t)((row0 / RC) + seq + blockIdx.x) * p.heads + h) * rc_block(DP, GENERAL);
+    float* GE = KE + RC * DP;
+    float* Qo = GE + DP;
+    float* No = Qo + RC * DP;
+    float* Wo = No + RC * RC;
+    float* Mo = Wo + RC * DP;
+    float* KV = Mo + RC * RC;
+
+    {
+        constexpr int PER = RC * DP / 256;
+        TX kr[PER], rr[PER], ar[PER];
+        float zr[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int i = tid + 256 * u, t = i / DP, c = i - t * DP;
+            kr[u] = rr[u] = ar[u] = from_f32<TX>(0.f);
+            zr[u] = 0.f;
+            if (t < n && c < d) {
+                kr[u] = k[(size_t)t * p.stride + c];
+                rr[u] = r[(size_t)t * p.stride + c];
+                ar[u] = a[(size_t)t * p.stride + c];
+                zr[u] = p.logits[(size_t)(row0 + base + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int i = tid + 256 * u, t = i / DP, c = i - t * DP;
+            const bool there = t < n && c < d;
+            ks[i] = to_f32(kr[u]);
+            rs[i] = to_f32(rr[u]);
+            as[i] = there ? 1.f / (1.f + expf(-(to_f32(ar[u]) + p.removal_bias[h * d + c]))) : 0.f;     // the rate
+            gs[i] = there ? expf(-p.decay_scale / (1.f + expf(-zr[u]))) : 1.f;
+        }
+    }
+    if (tid < RC * RC / 4) {                            // (what lies above the diagonal)
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        reinterpret_cast<float4*>(&Aa[0][0])[tid] = zero;
+        reinterpret_cast<float4*>(&Ak[0][0])[tid] = zero;
+        reinterpret_cast<float4*>(&Ba[0][0])[tid] = zero;
+        reinterpret_cast<float4*>(&Bk[0][0])[tid] = zero;
+        reinterpret_cast<float4*>(&Ms[0][0])[tid] = zero;
+    }
+    __syncthreads();
+    // unit keys: two tokens to a warp
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int t = warp + 8 * u;
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float v = ks[t * DP + lane + 32 * i];
+            sum = fmaf(v, v, sum);
+        }
+        const float inv = 1.f / sqrtf(warp_sum(sum) + p.key_eps);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int c = t * DP + lane + 32 * i;
+            const float x = ks[c] * inv;
+            xs[c] = x;
+            as[c] *= x;
+        }
+    }
+    for (int i = tid; i < 4 * DP; i += 256) {
+        const int b = i / DP, c = i - b * DP;
+        const float* g = gs + 4 * b * DP + c;
+        gg[i] = g[0] * g[DP] * (g[2 * DP] * g[3 * DP]);
+    }
+    __syncthreads();
+    // ---- tiles of inner products: (block of targets, block of sources); warps 6 and 7 take two on the diagonal
+#pragma unroll 1
+    for (int item = warp; item < 10; item = item < 6 ? 10 : item + 2) {
+        const int I = item < 6 ? (item == 0 ? 1 : item < 3 ? 2 : 3) : item - 6;
+        const int J = item < 6 ? (item == 0 ? 0 : item < 3 ? item - 1 : item - 3) : item - 6;
+        float acc[2][32];                               // [removals, keys][4 t + s]: A, then B
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            acc[0][i] = acc[1][i] = 0.f;
+#pragma unroll 1
+        for (int q = 0; q < R; ++q) {
+            const int c = lane + 32 * q;
+            float wa[4], wk[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                wa[s] = as[(4 * J + s) * DP + c];
+                wk[s] = ks[(4 * J + s) * DP + c];
+            }
+            if (item < 6) {
+                float f = 1.f;                          // from the end of the sources' block to the targets' first token
+                for (int b = J + 1; b < I; ++b)
+                    f *= gg[b * DP + c];
+#pragma unroll
+                for (int s = 3; s >= 0; --s) {
+                    wa[s] *= f;
+                    wk[s] *= f;
+                    if (s > 0)
+                        f *= gs[(4 * J + s) * DP + c];
+                }
+                f = 1.f;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int at = (4 * I + t) * DP + c;
+                    const float xv = xs[at] * f;        // (a removal looks at the state before its token's decay)
+                    f *= gs[at];
+                    const float rv = rs[at] * f;
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        acc[0][4 * t + s] = fmaf(xv, wa[s], acc[0][4 * t + s]);
+                        acc[1][4 * t + s] = fmaf(xv, wk[s], acc[1][4 * t + s]);
+                        acc[0][16 + 4 * t + s] = fmaf(rv, wa[s], acc[0][16 + 4 * t + s]);
+                        acc[1][16 + 4 * t + s] = fmaf(rv, wk[s], acc[1][16 + 4 * t + s]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    const int at = (4 * I + t) * DP + c;
+                    const float xv = xs[at], rv = rs[at], g = gs[at];
+#pragma unroll
+                    for (int s = 0; s < t; ++s) {
+                        acc[0][4 * t + s] = fmaf(xv, wa[s], acc[0][4 * t + s]);
+                        acc[1][4 * t + s] = fmaf(xv, wk[s], acc[1][4 * t + s]);
+                        wa[s] *= g;
+                        wk[s] *= g;
+                        acc[0][16 + 4 * t + s] = fmaf(rv, wa[s], acc[0][16 + 4 * t + s]);
+                        acc[1][16 + 4 * t + s] = fmaf(rv, wk[s], acc[1][16 + 4 * t + s]);
+                    }
+                    acc[0][16 + 4 * t + t] = fmaf(rv, wa[t], acc[0][16 + 4 * t + t]);
+                    acc[1][16 + 4 * t + t] = fmaf(rv, wk[t], acc[1][16 + 4 * t + t]);
+                }
+            }
+        }
+        // fold: after the steps 16, 8, 4, 2, 1 lane l holds the sum over all lanes of value l
+#pragma unroll
+        for (int half = 16, o = 16; half >= 1; half >>= 1, o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < half; ++i)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const float send = upper ? acc[y][i] : acc[y][i + half];
+                    const float keep = upper ? acc[y][i + half] : acc[y][i];
+                    acc[y][i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        }
+        const int t = 4 * I + ((lane >> 2) & 3), s = 4 * J + (lane & 3);
+        if (lane < 16) {
+            Aa[t][s] = acc[0][0];                       // (on and above the diagonal: sums of nothing)
+            Ak[t][s] = acc[1][0];
+        } else if (t >= s) {
+            Ba[t][s] = acc[0][0];
+            Bk[t][s] = acc[1][0];
+        }
+    }
+    __syncthreads();
+    // ---- M: a column to a thread, forward substitution; meanwhile the other warps decay the writes to the chunk's end
+    if (tid < RC) {
+        float m[RC];
+#pragma unroll
+        for (int t = 0; t < RC; ++t) {
+            float v0 = t == tid ? 1.f : 0.f, v1 = 0.f;
+#pragma unroll
+            for (int s = 0; s < t; ++s) {
+                if (s & 1)
+                    v1 = fmaf(-Aa[t][s], m[s], v1);
+                else
+                    v0 = fmaf(-Aa[t][s], m[s], v0);
+            }
+            m[t] = v0 + v1;
+            Ms[t][tid] = m[t];
+        }
+    } else if (tid >= 32) {
+        for (int c = tid - 32; c < DP; c += 224) {
+            float f = 1.f;
+#pragma unroll
+            for (int t = RC - 1; t >= 0; --t) {
+                KE[t * DP + c] = as[t * DP + c] * f;
+                KV[t * DP + c] = ks[t * DP + c] * f;
+                f *= gs[t * DP + c];
+            }
+            GE[c] = f;
+        }
+    }
+    __syncthreads();
+    {
+        const int t = tid / RC, j = tid % RC;
+        float v = 0.f;
+#pragma unroll
+        for (int s = 0; s < RC; ++s)
+            v = fmaf(-Ms[t][s], Ak[s][j], v);
+        Ns[t][j] = v;
+        Mo[tid] = v;
+    }
+    __syncthreads();
+    {
+        const int t = tid / RC, j = tid % RC;
+        float v = Bk[t][j];
+#pragma unroll
+        for (int s = 0; s < RC; ++s)
+            v = fmaf(Ba[t][s], Ns[s][j], v);
+        No[tid] = v;
+    }
+    // ---- W and Q, a channel to a thread
+    for (int c = tid; c < DP; c += 256) {
+        float w[RC], x[RC];
+        float f = 1.f;
+#pragma unroll
+        for (int t = 0; t < RC; ++t) {
+            x[t] = xs[t * DP + c] * f;
+            f *= gs[t * DP + c];
+            float v = 0.f;
+#pragma unroll
+            for (int s = 0; s <= t; ++s)
+                v = fmaf(-Ms[t][s], x[s], v);
+            w[t] = v;
+            Wo[t * DP + c] = v;
+            float o = rs[t * DP + c] * f;
+#pragma unroll
+            for (int s = 0; s <= t; ++s)
+                o = fmaf(Ba[t][s], w[s], o);
+            Qo[t * DP + c] = o;
+        }
+    }
+}
+
 // ---------------------------------------------------------------- over a sequence's chunks
 __device__ __forceinline__ void rc_copy16(float* dst, const float* src)
 {
@@ -406,12 +678,12 @@ __device__ __forceinline__ uint64_t rc_mul2(uint64_t a, uint64_t b)
 // chunk's rows come from shared memory.  The sums over the rows are spread over those threads and folded at the end of a product, all of its
 // values together.  Small pieces of S and many threads: a sequence's chunks come one after the other, so the
 // time of a chunk counts, and with a few columns a block every SM has one.
-template <int DP, int RT, int CT, int COLS, bool DELTA, typename TX>
+template <int DP, int RT, int CT, int COLS, int RULE, typename TX>
 __global__ void __launch_bounds__((DP / RT) * (COLS / CT))
 chunk_recurrence_kernel(const RecurrenceParams p)
 {
     constexpr int L = DP / RT;                          // threads along the rows
-    constexpr int NT = L * (COLS / CT), BLOCK = rc_block(DP, DELTA), CP = COLS + 4;
+    constexpr int NT = L * (COLS / CT), BLOCK = rc_block(DP, RULE), CP = COLS + 4;
     constexpr int VR = L >= RC ? 1 : RC / L;            // rows of V (tokens) that a thread owns for the products
     constexpr int SUMS = RC * CT, OWN = SUMS / L;       // a product's values, and those that a thread is left with
     constexpr int RUNS = RT / 4, RUN_STEP = DP / RUNS;  // its rows: runs r0 + RUN_STEP i .. + 3
@@ -422,6 +694,7 @@ chunk_recurrence_kernel(const RecurrenceParams p)
     extern __shared__ __align__(16) float sm[];
     float* bufs = sm;                                   // two chunks
     float* Us = bufs + 2 * BLOCK;                       // [RC][CP]
+    float* Vs = Us + RC * CP;                           // the same (generalised rule)
     const int h = blockIdx.y, seq = blockIdx.z, tid = threadIdx.x;
     const int d = p.d, e = p.e;
     const int row0 = p.q_start[seq];
@@ -431,6 +704,7 @@ chunk_recurrence_kernel(const RecurrenceParams p)
     const int lr = tid % L, c0 = CT * (tid / L), r0 = 4 * lr;
     const int col = blockIdx.x * COLS + c0;             // the thread's first column
     float* st = p.state + ((size_t)p.slots[seq] * p.heads + h) * d * e;
+    auto place = [&](int r, int c) { return RULE == GENERAL ? (size_t)c * d + r : (size_t)r * e + c; };
     uint64_t S[RT / 2][CT];
     // (the state is what an earlier step left: fetched before the kernel ahead is through)
 #pragma unroll
@@ -438,8 +712,8 @@ chunk_recurrence_kernel(const RecurrenceParams p)
         const int r = r0 + RUN_STEP * (i / 2) + 2 * (i % 2);
 #pragma unroll
         for (int j = 0; j < CT; ++j)
-            S[i][j] = rc_pair((r < d && col + j < e) ? st[(size_t)r * e + col + j] : 0.f,
-                              (r + 1 < d && col + j < e) ? st[(size_t)(r + 1) * e + col + j] : 0.f);
+            S[i][j] = rc_pair((r < d && col + j < e) ? st[place(r, col + j)] : 0.f,
+                              (r + 1 < d && col + j < e) ? st[place(r + 1, col + j)] : 0.f);
     }
 #ifndef CHIBI_TIMELINE
     pdl_wait();
@@ -478,6 +752,7 @@ chunk_recurrence_kernel(const RecurrenceParams p)
         const float* NO = Q + RC * DP;
         const float* W = NO + RC * RC;
         const float* M = W + RC * DP;
+        const float* KV = M + RC * RC;
         const int base = c * RC;
         float vt[VR][CT];
 #pragma unroll
@@ -532,7 +807,7 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                 }
             }
         };
-        if (DELTA) {
+        if (RULE != LINEAR) {
             float acc[SUMS];
             product(W, M, acc);
 #pragma unroll
@@ -545,6 +820,14 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                 for (int j = 0; j < CT; ++j)
                     if (lr + L * i < RC)
                         Us[(lr + L * i) * CP + c0 + j] = vt[i][j];
+        }
+        if (RULE == GENERAL) {
+#pragma unroll
+            for (int i = 0; i < VR; ++i)
+#pragma unroll
+                for (int j = 0; j < CT; ++j)
+                    if (lr + L * i < RC)
+                        Vs[(lr + L * i) * CP + c0 + j] = vt[i][j];
         }
         __syncthreads();
         {
@@ -567,29 +850,34 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                 S[2 * u + 1][j] = rc_mul2(S[2 * u + 1][j], g.y);
             }
         }
+        auto write = [&](const float* rows, const float* columns) {
 #pragma unroll
-        for (int s = 0; s < RC; ++s) {
-            float uv[CT];
-            if constexpr (CT == 4) {
-                const float4 u4 = *reinterpret_cast<const float4*>(Us + s * CP + c0);
-                uv[0] = u4.x, uv[1] = u4.y, uv[2] = u4.z, uv[3] = u4.w;
-            } else if constexpr (CT == 2) {
-                const float2 u2 = *reinterpret_cast<const float2*>(Us + s * CP + c0);
-                uv[0] = u2.x, uv[1] = u2.y;
-            } else {
-                uv[0] = Us[s * CP + c0];
-            }
+            for (int s = 0; s < RC; ++s) {
+                float uv[CT];
+                if constexpr (CT == 4) {
+                    const float4 u4 = *reinterpret_cast<const float4*>(columns + s * CP + c0);
+                    uv[0] = u4.x, uv[1] = u4.y, uv[2] = u4.z, uv[3] = u4.w;
+                } else if constexpr (CT == 2) {
+                    const float2 u2 = *reinterpret_cast<const float2*>(columns + s * CP + c0);
+                    uv[0] = u2.x, uv[1] = u2.y;
+                } else {
+                    uv[0] = columns[s * CP + c0];
+                }
 #pragma unroll
-            for (int u = 0; u < RUNS; ++u) {
-                const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(KE + s * DP + r0 + RUN_STEP * u);
+                for (int u = 0; u < RUNS; ++u) {
+                    const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(rows + s * DP + r0 + RUN_STEP * u);
 #pragma unroll
-                for (int j = 0; j < CT; ++j) {
-                    const uint64_t both = rc_pair(uv[j], uv[j]);
-                    S[2 * u][j] = rc_fma2(k.x, both, S[2 * u][j]);
-                    S[2 * u + 1][j] = rc_fma2(k.y, both, S[2 * u + 1][j]);
+                    for (int j = 0; j < CT; ++j) {
+                        const uint64_t both = rc_pair(uv[j], uv[j]);
+                        S[2 * u][j] = rc_fma2(k.x, both, S[2 * u][j]);
+                        S[2 * u + 1][j] = rc_fma2(k.y, both, S[2 * u + 1][j]);
+                    }
                 }
             }
-        }
+        };
+        write(KE, Us);
+        if (RULE == GENERAL)
+            write(KV, Vs);
     }
 #pragma unroll
     for (int i = 0; i < RT / 2; ++i) {
@@ -598,9 +886,9 @@ chunk_recurrence_kernel(const RecurrenceParams p)
         for (int j = 0; j < CT; ++j) {
             const float2 halves = rc_halves(S[i][j]);
             if (r < d && col + j < e)
-                st[(size_t)r * e + col + j] = halves.x;
+                st[place(r, col + j)] = halves.x;
             if (r + 1 < d && col + j < e)
-                st[(size_t)(r + 1) * e + col + j] = halves.y;
+                st[place(r + 1, col + j)] = halves.y;
         }
     }
 }
@@ -610,7 +898,7 @@ chunk_recurrence_kernel(const RecurrenceParams p)
 // registers.  Per token a warp makes its rows' key, query and decay, the block adds up what the warps find in
 // the old state, and one barrier later everyone knows u: with S' = diag(g) S,
 // o = S'^T q + (k . q) u, so the read-out needs no second barrier.
-template <int W, int R, bool DELTA, typename TX>
+template <int W, int R, int RULE, typename TX>
 __global__ void __launch_bounds__(32 * W)
 recurrence_tokens_kernel(const RecurrenceParams p)
 {
@@ -635,8 +923,8 @@ recurrence_tokens_kernel(const RecurrenceParams p)
 #pragma unroll
     for (int i = 0; i < R; ++i)
         S[i] = (col < e && r0 + i < d) ? st[(size_t)(r0 + i) * e + col] : 0.f;
-    const float rate = DELTA ? -expf(p.a_log[h]) : 0.f;
-    const float decay = DELTA ? 1.f : p.decay[h];
+    const float rate = RULE == DELTA ? -expf(p.a_log[h]) : 0.f;
+    const float decay = RULE == DELTA ? 1.f : p.decay[h];
 #ifndef CHIBI_TIMELINE
     pdl_wait();
 #endif
@@ -648,7 +936,7 @@ recurrence_tokens_kernel(const RecurrenceParams p)
         if (p.activate)
             v = lr_silu<TX>(v);
         float beta = 1.f, ik = 1.f, iq = 1.f;
-        if (DELTA) {
+        if (RULE == DELTA) {
             beta = 1.f / (1.f + expf(-to_f32(static_cast<const TX*>(p.beta)[row * p.beta_stride + h])));
             float sk = 0.f, sq = 0.f;
             for (int c = lane; c < d; c += 32) {
@@ -670,7 +958,7 @@ recurrence_tokens_kernel(const RecurrenceParams p)
                     kv = lr_silu<TX>(kv), qv = lr_silu<TX>(qv);
                 kv *= ik;
                 qv *= iq;
-                g = DELTA ? lr_decay<TX>(rate, p.logits[row * p.logit_stride + h * d + c] + p.dt_bias[h * d + c]) : decay;
+                g = RULE == DELTA ? lr_decay<TX>(rate, p.logits[row * p.logit_stride + h * d + c] + p.dt_bias[h * d + c]) : decay;
             }
             vec[warp][0][i] = kv;
             vec[warp][1][i] = qv;
@@ -682,13 +970,13 @@ recurrence_tokens_kernel(const RecurrenceParams p)
         for (int i = 0; i < R; ++i) {
             const float kv = vec[warp][0][i], qv = vec[warp][1][i];
             S[i] *= vec[warp][2][i];
-            if (DELTA)
+            if (RULE == DELTA)
                 sk = fmaf(S[i], kv, sk);
             sq = fmaf(S[i], qv, sq);
             kq = fmaf(kv, qv, kq);
         }
         const int turn = t & 1;
-        if (DELTA)
+        if (RULE == DELTA)
             part[turn][0][warp][lane] = sk;
         part[turn][1][warp][lane] = sq;
         part[turn][2][warp][lane] = kq;
@@ -696,12 +984,12 @@ recurrence_tokens_kernel(const RecurrenceParams p)
         sk = sq = kq = 0.f;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-            if (DELTA)
+            if (RULE == DELTA)
                 sk += part[turn][0][w][lane];
             sq += part[turn][1][w][lane];
             kq += part[turn][2][w][lane];
         }
-        const float u = DELTA ? beta * (v - sk) : v;
+        const float u = RULE == DELTA ? beta * (v - sk) : v;
 #pragma unroll
         for (int i = 0; i < R; ++i)
             S[i] = fmaf(vec[warp][0][i], u, S[i]);
@@ -728,22 +1016,22 @@ static inline int recurrence_sm_count()
     return sms;
 }
 
-template <int DP, int RT, int CT, int COLS, bool DELTA, typename TX>
+template <int DP, int RT, int CT, int COLS, int RULE, typename TX>
 static void launch_chunks(const RecurrenceParams& p, int seqs, cudaStream_t stream)
 {
-    const size_t smem = (size_t)(2 * rc_block(DP, DELTA) + RC * (COLS + 4)) * sizeof(float);
-    auto kernel = chunk_recurrence_kernel<DP, RT, CT, COLS, DELTA, TX>;
+    const size_t smem = (size_t)(2 * rc_block(DP, RULE) + (RULE == GENERAL ? 2 : 1) * RC * (COLS + 4)) * sizeof(float);
+    auto kernel = chunk_recurrence_kernel<DP, RT, CT, COLS, RULE, TX>;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch(kernel, dim3((unsigned)((p.e + COLS - 1) / COLS), (unsigned)p.heads, (unsigned)seqs),
            dim3((DP / RT) * (COLS / CT)), smem, stream, p);
 }
 
-template <int DP, bool DELTA, typename TX>
+template <int DP, int RULE, typename TX>
 static void launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cudaStream_t stream)
 {
-    const size_t smem = (size_t)(DELTA ? 3 * RC + 4 : 2 * RC) * DP * sizeof(float);
-    auto prepare = recurrence_prepare_kernel<DP, DELTA, TX>;
+    const size_t smem = (size_t)(RULE == GENERAL ? 5 * RC + 4 : RULE == DELTA ? 3 * RC + 4 : 2 * RC) * DP * sizeof(float);
+    auto prepare = RULE == GENERAL ? general_prepare_kernel<DP, TX> : recurrence_prepare_kernel<DP, RULE == GENERAL ? DELTA : RULE, TX>;
     if (smem > 44 * 1024)
         cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch(prepare, dim3((unsigned)((max_q_len + RC - 1) / RC), (unsigned)p.heads, (unsigned)seqs), dim3(256), smem, stream, p);
@@ -751,30 +1039,30 @@ static void launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cu
     constexpr int RT = DP >= 128 ? 8 : 4;
     const long long per_head = (long long)p.heads * seqs, sms = recurrence_sm_count();
     if (((p.e + 7) / 8) * per_head <= sms)
-        launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, DELTA, TX>(p, seqs, stream);
+        launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, RULE, TX>(p, seqs, stream);
     else if (((p.e + 15) / 16) * per_head <= sms)
-        launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, DELTA, TX>(p, seqs, stream);
+        launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, RULE, TX>(p, seqs, stream);
     else
-        launch_chunks<DP, RT, 4, 32, DELTA, TX>(p, seqs, stream);
+        launch_chunks<DP, RT, 4, 32, RULE, TX>(p, seqs, stream);
 }
 
-template <bool DELTA, typename TX>
+template <int RULE, typename TX>
 static void launch_tokens(const RecurrenceParams& p, int seqs, cudaStream_t stream)
 {
     const dim3 grid((unsigned)((p.e + 31) / 32), (unsigned)p.heads, (unsigned)seqs);
     if (p.d <= 32)
-        launch(recurrence_tokens_kernel<8, 4, DELTA, TX>, grid, dim3(256), 0, stream, p);
+        launch(recurrence_tokens_kernel<8, 4, RULE, TX>, grid, dim3(256), 0, stream, p);
     else if (p.d <= 64)
-        launch(recurrence_tokens_kernel<8, 8, DELTA, TX>, grid, dim3(256), 0, stream, p);
+        launch(recurrence_tokens_kernel<8, 8, RULE, TX>, grid, dim3(256), 0, stream, p);
     else if (p.d <= 128)
-        launch(recurrence_tokens_kernel<8, 16, DELTA, TX>, grid, dim3(256), 0, stream, p);
+        launch(recurrence_tokens_kernel<8, 16, RULE, TX>, grid, dim3(256), 0, stream, p);
     else if (p.d <= 256)
-        launch(recurrence_tokens_kernel<16, 16, DELTA, TX>, grid, dim3(512), 0, stream, p);
+        launch(recurrence_tokens_kernel<16, 16, RULE, TX>, grid, dim3(512), 0, stream, p);
     else
-        launch(recurrence_tokens_kernel<16, 32, DELTA, TX>, grid, dim3(512), 0, stream, p);
+        launch(recurrence_tokens_kernel<16, 32, RULE, TX>, grid, dim3(512), 0, stream, p);
 }
 
-template <bool DELTA>
+template <int RULE>
 static int launch_recurrence(const RecurrenceParams& p, int x_type, long long scratch_floats, long long tokens, int seqs,
                              int max_q_len, int few, cudaStream_t stream)
 {
@@ -782,21 +1070,24 @@ static int launch_recurrence(const RecurrenceParams& p, int x_type, long long sc
         return CHIBI_ERR_UNSUPPORTED;
     const int DP = padded_rows(p.d);
     if (max_q_len <= few || DP == 0) {
-        CHIBI_DISPATCH_TYPE(x_type, TX, { launch_tokens<DELTA, TX>(p, seqs, stream); });
+        if constexpr (RULE == GENERAL)
+            return CHIBI_ERR_UNSUPPORTED;               // (a kernel of sequence_ops.cu)
+        else
+            CHIBI_DISPATCH_TYPE(x_type, TX, { launch_tokens<RULE, TX>(p, seqs, stream); });
         return launch_status();
     }
     if (!p.scratch || (reinterpret_cast<uintptr_t>(p.scratch) & 15)
-        || scratch_floats < (tokens / RC + seqs) * (long long)p.heads * rc_block(DP, DELTA))
+        || scratch_floats < (tokens / RC + seqs) * (long long)p.heads * rc_block(DP, RULE))
         return CHIBI_ERR_ARGUMENT;
     CHIBI_DISPATCH_TYPE(x_type, TX, {
         if (DP == 32)
-            launch_prompt<32, DELTA, TX>(p, seqs, max_q_len, stream);
+            launch_prompt<32, RULE, TX>(p, seqs, max_q_len, stream);
         else if (DP == 64)
-            launch_prompt<64, DELTA, TX>(p, seqs, max_q_len, stream);
+            launch_prompt<64, RULE, TX>(p, seqs, max_q_len, stream);
         else if (DP == 128)
-            launch_prompt<128, DELTA, TX>(p, seqs, max_q_len, stream);
+            launch_prompt<128, RULE, TX>(p, seqs, max_q_len, stream);
         else
-            launch_prompt<256, DELTA, TX>(p, seqs, max_q_len, stream);
+            launch_prompt<256, RULE, TX>(p, seqs, max_q_len, stream);
     });
     return launch_status();
 }
@@ -806,13 +1097,15 @@ static int launch_recurrence(const RecurrenceParams& p, int x_type, long long sc
 using namespace chibi;
 
 // Floats of scratch that a step of so many tokens and sequences needs where a sequence brings more tokens
-// than the token-by-token kernel is used for; a sequence's chunks start at slot q_start / 16 + sequence.
-CHIBI_API int chibi_recurrence_scratch(long long tokens, int seqs, int heads, int d, int delta, long long* floats)
+// than the token-by-token kernel is used for (rule: 0 linear attention, 1 delta rule, 2 generalised delta rule); a
+// sequence's chunks start at slot q_start / 16 + sequence.
+CHIBI_API int chibi_recurrence_scratch(long long tokens, int seqs, int heads, int d, int rule, long long* floats)
 {
     const int DP = padded_rows(d);
-    if (!floats || tokens < 0 || seqs < 0 || heads <= 0 || d <= 0)
+    if (!floats || tokens < 0 || seqs < 0 || heads <= 0 || d <= 0
+        || rule < LINEAR || rule > GENERAL)
         return CHIBI_ERR_ARGUMENT;
-    *floats = DP == 0 ? 0 : (tokens / RC + seqs) * (long long)heads * rc_block(DP, delta != 0);
+    *floats = DP == 0 ? 0 : (tokens / RC + seqs) * (long long)heads * rc_block(DP, rule);
     return CHIBI_OK;
 }
 
@@ -853,7 +1146,7 @@ CHIBI_API int chibi_channel_delta(const void* qkv, int x_type, long long stride,
     p.qk_heads = qk_heads;
     p.d = d;
     p.e = e;
-    return launch_recurrence<true>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
+    return launch_recurrence<DELTA>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
 }
 
 CHIBI_API int chibi_decayed_attention(const void* qkv, int x_type, long long stride, int activate, const float* decay,
@@ -882,5 +1175,42 @@ CHIBI_API int chibi_decayed_attention(const void* qkv, int x_type, long long str
     p.qk_heads = heads;
     p.d = d;
     p.e = e;
-    return launch_recurrence<false>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
+    return launch_recurrence<LINEAR>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
+}
+
+// The generalised delta rule over prompt portions.  A row of proj holds r | k | v | gate | removal | low, heads * d columns
+// each but the last; logits [T, heads * d]; state [slots, heads, d (value), d (key)].
+CHIBI_API int chibi_delta_rule_chunks(const void* proj, int x_type, long long stride, const float* logits,
+                                      const float* decay_bias, const float* removal_bias, float* state, float* o,
+                                      float* scratch, long long scratch_floats, const int* q_start, const int* slots,
+                                      long long tokens, int seqs, int max_q_len, int heads, int d, float decay_scale,
+                                      float key_eps, cudaStream_t stream)
+{
+    if (seqs <= 0 || tokens <= 0 || max_q_len <= 0)
+        return CHIBI_OK;
+    if (!proj || !logits || !decay_bias || !removal_bias || !state || !o || heads <= 0 || d <= 0)
+        return CHIBI_ERR_ARGUMENT;
+    const size_t part = (size_t)heads * d * (x_type == CHIBI_BF16 ? 2 : 4);
+    RecurrenceParams p = {};
+    p.q = proj;
+    p.k = static_cast<const char*>(proj) + part;
+    p.v = static_cast<const char*>(proj) + 2 * part;
+    p.removal = static_cast<const char*>(proj) + 4 * part;
+    p.stride = stride;
+    p.logits = logits;
+    p.logit_stride = (long long)heads * d;
+    p.dt_bias = decay_bias;
+    p.removal_bias = removal_bias;
+    p.decay_scale = decay_scale;
+    p.key_eps = key_eps;
+    p.state = state;
+    p.o = o;
+    p.scratch = scratch;
+    p.q_start = q_start;
+    p.slots = slots;
+    p.heads = heads;
+    p.qk_heads = heads;
+    p.d = d;
+    p.e = d;
+    return launch_recurrence<GENERAL>(p, x_type, scratch_floats, tokens, seqs, max_q_len, 0, stream);
 }

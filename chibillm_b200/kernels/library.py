@@ -101,6 +101,7 @@ _SIGNATURES = {
         "chibi_norm_then_gate": [P, P, I, L, P, F, P, L, I, P],
         "chibi_bias_xielu": [P, I, I, P, P, I, L, I, F, F, P],
         "chibi_recurrence_scratch": [L, I, I, I, I, P],
+        "chibi_delta_rule_chunks": [P, I, L, P, P, P, P, P, P, L, P, P, L, I, I, I, I, F, F, P],
         "chibi_channel_delta": [P, I, L, P, L, P, L, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, F, F, I, P],
         "chibi_decayed_attention": [P, I, L, I, P, P, P, P, L, P, P, L, I, I, I, I, I, I, P],
     },

@@ -1162,6 +1162,16 @@ class CudaKernels:
         if proj.shape[1] != 5 * W + rank or state.dtype != torch.float32 or not state.is_contiguous() \
                 or tuple(state.shape[1:]) != (heads, d, d):
             raise KernelError("delta_rule: proj [T, 5 * heads * d + rank] and state float32 [slots, heads, d, d]")
+        if max_q_len > self.RECURRENCE_FEW_TOKENS and d <= 256:
+            # prompt portions, in chunks of tokens (a first kernel prepares all chunks, a second walks over them)
+            seqs = state_slots.numel()
+            scratch = self._recurrence_scratch(T, seqs, heads, d, 2, max_q_len)
+            self.launches += 2
+            _check(self.lib.chibi_delta_rule_chunks(
+                _ptr(proj), _code(proj), proj.stride(0), _ptr(decay_logits), _ptr(decay_bias), _ptr(removal_bias), _ptr(state),
+                _ptr(o), _ptr(scratch), scratch.numel(), _ptr(q_start), _ptr(state_slots), T, seqs, int(max_q_len), heads, d,
+                float(decay_scale), float(key_eps), self._stream()), "delta_rule (chunks)")
+            return
         self.launches += 1
         _check(self.lib.chibi_delta_rule(_ptr(proj), _code(proj), proj.stride(0), _ptr(decay_logits),
                                          _ptr(decay_bias), _ptr(removal_bias), _ptr(state), _ptr(o), _ptr(q_start),
@@ -2097,11 +2107,11 @@ class CudaKernels:
     # chunks of 16 tokens
     RECURRENCE_FEW_TOKENS = 4
 
-    def _recurrence_scratch(self, tokens: int, seqs: int, heads: int, d: int, delta: bool, max_q_len: int):
+    def _recurrence_scratch(self, tokens: int, seqs: int, heads: int, d: int, rule: int, max_q_len: int):
         if max_q_len <= self.RECURRENCE_FEW_TOKENS:
             return None
         floats = ctypes.c_longlong(0)
-        _check(self.lib.chibi_recurrence_scratch(tokens, seqs, heads, d, 1 if delta else 0, ctypes.addressof(floats)),
+        _check(self.lib.chibi_recurrence_scratch(tokens, seqs, heads, d, rule, ctypes.addressof(floats)),
                "recurrence scratch")
         return self._scratch(floats.value)
 
@@ -2127,7 +2137,7 @@ class CudaKernels:
             if t.dtype != torch.float32 or t.numel() != size or not t.is_contiguous():
                 raise KernelError("channel_delta: a_log [heads] and dt_bias [heads d] are contiguous float32")
         seqs = state_slots.numel()
-        scratch = self._recurrence_scratch(T, seqs, heads, d, True, max_q_len)
+        scratch = self._recurrence_scratch(T, seqs, heads, d, 1, max_q_len)
         self.launches += 2 if scratch is not None and d <= 256 else 1
         _check(self.lib.chibi_channel_delta(
             _ptr(qkv), _code(qkv), qkv.stride(0), _ptr(logits), logits.stride(0), _ptr(beta), beta.stride(0), _ptr(a_log),
@@ -2149,7 +2159,7 @@ class CudaKernels:
                 or o.dtype != torch.float32 or o.shape != (T, heads * e) or not o.is_contiguous():
             raise KernelError("decayed_attention: shapes or types")
         seqs = state_slots.numel()
-        scratch = self._recurrence_scratch(T, seqs, heads, d, False, max_q_len)
+        scratch = self._recurrence_scratch(T, seqs, heads, d, 0, max_q_len)
         self.launches += 2 if scratch is not None and d <= 256 else 1
         _check(self.lib.chibi_decayed_attention(
             _ptr(qkv), _code(qkv), qkv.stride(0), 1 if activate else 0, _ptr(decay), _ptr(state), _ptr(o), _ptr(scratch),
