@@ -264,6 +264,7 @@ differential_combine_kernel(const float* __restrict__ att, const TX* __restrict_
 // shared-memory loads of one another.
 constexpr int SSM_CHUNK = 16;
 constexpr int SSM_CW = 2;                               // columns of a warp
+constexpr int SSM_FEW = 4;                              // tokens a sequence, on average, up to which they go one by one
 
 // The state row that lane l holds as its i-th: runs of four rows to a lane where a lane has four or more
 // (one 16-byte load of B and of C serves four multiply-adds), else row 32 i + l.
@@ -437,6 +438,107 @@ state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const 
                 S[(size_t)(col + w) * N + r] = s[w][i];
         }
     }
+}
+
+// The same for steps of about one token a sequence: bound by the state's way from memory and back, so a warp holds
+// 8 columns (4 of states above 128 rows, 2 above 256) of state rows in 16-byte pieces and nothing goes
+// through shared memory: a lane reads its own rows of a token's B and C, and the columns' sums over the lanes are folded
+// together.  64 sequences of 32 heads of 64 x 128: 77 us with the kernel above (whose block stages a chunk of
+// 16 tokens, of which there is one, behind two barriers).
+template <typename TX, int R>
+__global__ void __launch_bounds__(64)
+state_space_token_kernel(const TX* __restrict__ xbc, long long xbc_stride, const TX* __restrict__ dt_raw,
+                         long long dt_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                         const float* __restrict__ skip, float* state, float* __restrict__ y,
+                         const int* __restrict__ q_start, const int* __restrict__ slots, int heads, int groups, int e,
+                         int N)
+{
+    pdl_enter();
+    constexpr int CW = R <= 4 ? 8 : R == 8 ? 4 : 2;     // columns of a warp
+    const int h = blockIdx.y, seq = blockIdx.z, l = threadIdx.x & 31;
+    const int g = h / (heads / groups), inner = heads * e;
+    const int col = (blockIdx.x * 2 + (threadIdx.x >> 5)) * CW;
+    const int row0 = q_start[seq], row1 = q_start[seq + 1];
+    if (row1 <= row0 || col >= e)
+        return;
+    float* const S = state + (((size_t)slots[seq] * heads + h) * e + col) * N;
+    const bool wide = R >= 4 && N % 4 == 0;             // a lane's runs of four rows are whole and aligned
+    float s[CW][R];
+#pragma unroll
+    for (int w = 0; w < CW; ++w)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = ssm_row<R>(i, l);
+            const bool there = col + w < e && r < N;
+            if (wide) {
+                if (i % 4 == 0) {
+                    const float4 v = there ? *reinterpret_cast<const float4*>(S + (size_t)w * N + r)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+                    s[w][i] = v.x;
+                    if constexpr (R >= 4)
+                        s[w][i + 1] = v.y, s[w][i + 2] = v.z, s[w][i + 3] = v.w;
+                }
+            } else {
+                s[w][i] = there ? S[(size_t)w * N + r] : 0.f;
+            }
+        }
+    const float A = -expf(a_log[h]), bias = dt_bias[h], D = skip[h];
+    for (int t = row0; t < row1; ++t) {
+        const TX* row = xbc + (size_t)t * xbc_stride;
+        const float dt = softplus_f(to_f32(dt_raw[(size_t)t * dt_stride + h]) + bias), a = expf(A * dt);
+        float b[R], c[R], acc[CW];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = ssm_row<R>(i, l);
+            const TX* src = row + inner + g * N + r;
+            b[i] = r < N ? to_f32(src[0]) : 0.f;
+            c[i] = r < N ? to_f32(src[(size_t)groups * N]) : 0.f;
+        }
+#pragma unroll
+        for (int w = 0; w < CW; ++w) {
+            const float bx = dt * (col + w < e ? to_f32(row[h * e + col + w]) : 0.f);
+            acc[w] = 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                s[w][i] = fmaf(a, s[w][i], bx * b[i]);
+                acc[w] = fmaf(s[w][i], c[i], acc[w]);
+            }
+        }
+        // fold: halves of the columns until a lane has one, its number in the lane's upper bits, then plain sums
+        int o = 16;
+#pragma unroll
+        for (int half = CW / 2; half >= 1; half >>= 1, o >>= 1) {
+            const bool upper = (l & o) != 0;
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+                const float send = upper ? acc[i] : acc[i + half];
+                const float keep = upper ? acc[i + half] : acc[i];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+#pragma unroll
+        for (; o >= 1; o >>= 1)
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+        const int w = l / (32 / CW);
+        if (l % (32 / CW) == 0 && col + w < e)
+            y[(size_t)t * inner + h * e + col + w] = fmaf(D, to_f32(row[h * e + col + w]), acc[0]);
+    }
+#pragma unroll
+    for (int w = 0; w < CW; ++w)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int r = ssm_row<R>(i, l);
+            if (col + w < e && r < N) {
+                if (wide) {
+                    if constexpr (R >= 4)
+                        if (i % 4 == 0)
+                            *reinterpret_cast<float4*>(S + (size_t)w * N + r) =
+                                make_float4(s[w][i], s[w][i + 1], s[w][i + 2], s[w][i + 3]);
+                } else {
+                    S[(size_t)w * N + r] = s[w][i];
+                }
+            }
+        }
 }
 
 // grid (tokens, parts), out = v / rms(v over the part) * weight with v = y * silu(z).  A part of up to
@@ -800,10 +902,22 @@ static void launch_scan(int seqs, cudaStream_t stream, const void* xbc, long lon
            xbc_stride, (const TX*)dt_raw, dt_stride, dt_bias, a_log, skip, state, y, q_start, slots, heads, groups, e, N);
 }
 
+template <typename TX, int R>
+static void launch_scan_tokens(int seqs, cudaStream_t stream, const void* xbc, long long xbc_stride, const void* dt_raw,
+                               long long dt_stride, const float* dt_bias, const float* a_log, const float* skip,
+                               float* state, float* y, const int* q_start, const int* slots, int heads, int groups, int e,
+                               int N)
+{
+    constexpr int COLS = 2 * (R <= 4 ? 8 : R == 8 ? 4 : 2);
+    launch(state_space_token_kernel<TX, R>, dim3((unsigned)((e + COLS - 1) / COLS), (unsigned)heads, (unsigned)seqs), dim3(64),
+           0, stream, (const TX*)xbc, xbc_stride, (const TX*)dt_raw, dt_stride, dt_bias, a_log, skip, state, y, q_start,
+           slots, heads, groups, e, N);
+}
+
 CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_stride, const void* dt_raw,
                                      long long dt_stride, const float* dt_bias, const float* a_log, const float* skip,
-                                     float* state, float* y, const int* q_start, const int* slots, int seqs, int heads,
-                                     int groups, int e, int N, cudaStream_t stream)
+                                     float* state, float* y, const int* q_start, const int* slots, long long tokens,
+                                     int seqs, int heads, int groups, int e, int N, cudaStream_t stream)
 {
     if (seqs <= 0)
         return CHIBI_OK;
@@ -812,6 +926,22 @@ CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_
         return CHIBI_ERR_ARGUMENT;
     if (N > 16 * 32 || heads > 65535 || seqs > 65535)      // (two buffers of a chunk's B and C must fit shared memory)
         return CHIBI_ERR_UNSUPPORTED;
+    // (16-byte pieces of state rows; the state is an array of its own)
+    if (tokens <= SSM_FEW * (long long)seqs && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
+        const int rows = (N + 31) / 32;
+#define CHIBI_SCAN_TOKENS(RR)                                                                                        \
+    CHIBI_DISPATCH_TYPE(x_type, TX, {                                                                                \
+        launch_scan_tokens<TX, RR>(seqs, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip, state, y, \
+                                   q_start, slots, heads, groups, e, N);                                             \
+    })
+        if (rows <= 1) CHIBI_SCAN_TOKENS(1);
+        else if (rows <= 2) CHIBI_SCAN_TOKENS(2);
+        else if (rows <= 4) CHIBI_SCAN_TOKENS(4);
+        else if (rows <= 8) CHIBI_SCAN_TOKENS(8);
+        else CHIBI_SCAN_TOKENS(16);
+#undef CHIBI_SCAN_TOKENS
+        return launch_status();
+    }
     // blocks of 16 columns, or of 8 where those would leave SMs without a block
     static int sms = 0;
     if (sms == 0) {

@@ -2026,8 +2026,8 @@ class CudaKernels:
         self.launches += 1
         _check(self.lib.chibi_state_space_scan(_ptr(xbc), _code(xbc), xbc.stride(0), _ptr(dt), dt.stride(0),
                                                _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state), _ptr(y),
-                                               _ptr(q_start), _ptr(state_slots), state_slots.numel(), heads, groups,
-                                               e, n, self._stream()), "state_space_scan")
+                                               _ptr(q_start), _ptr(state_slots), T, state_slots.numel(), heads,
+                                               groups, e, n, self._stream()), "state_space_scan")
 
     def gated_group_rms(self, y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps: float, parts: int,
                         out: torch.Tensor) -> None:
