@@ -27,7 +27,7 @@
 // over a sequence's chunks with a piece of S (all d rows of some columns) in registers: two small products
 // with S_0 and V, then one into S.  A chunk that is not full has zero rows for the tokens it lacks.
 //
-// Few tokens a sequence (decode steps) run token by token in a kernel of their own.
+// Few tokens a sequence (decode steps) run token by token in kernels of their own.
 #define CHIBI_UNIT linear_recurrence
 #define CHIBI_UNIT_ID 14
 #include "common.cuh"
@@ -1002,6 +1002,273 @@ recurrence_tokens_kernel(const RecurrenceParams p)
             st[(size_t)(r0 + i) * e + col] = S[i];
 }
 
+// The same for heads of at most 128 key rows, where a lane can hold its column's rows by itself: a warp owns 32
+// value columns, nothing is added up across lanes or warps and there is no block barrier.  Bound by the state's way
+// from memory and back, R lines of 128 bytes of a warp in flight together (64 sequences of 16 heads of
+// 128 x 128: 31.2 us, 47.6 with the kernel above, whose eight warps of 16 rows wait for one another at every token).
+template <int R, int RULE, typename TX>
+__global__ void __launch_bounds__(32)
+recurrence_columns_kernel(const RecurrenceParams p)
+{
+#ifdef CHIBI_TIMELINE
+    pdl_enter();
+#else
+    pdl_trigger();
+#endif
+    __shared__ __align__(16) float vec[3][R];           // the token's k, q, g
+    const int h = blockIdx.y, seq = blockIdx.z, lane = threadIdx.x;
+    const int d = p.d, e = p.e, kh = h / (p.heads / p.qk_heads);
+    const int row0 = p.q_start[seq];
+    const int len = p.q_start[seq + 1] - row0;
+    if (len <= 0)
+        return;
+    const int col = blockIdx.x * 32 + lane;
+    float* st = p.state + ((size_t)p.slots[seq] * p.heads + h) * d * e;
+#ifndef CHIBI_TIMELINE
+    for (int r = lane; r < d; r += 32)                  // (only asked for: who wrote it last may be the kernel ahead)
+        prefetch_l2(st + (size_t)r * e + blockIdx.x * 32);
+    pdl_wait();
+#endif
+    float S[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        S[r] = (col < e && r < d) ? st[(size_t)r * e + col] : 0.f;
+    const float rate = RULE == DELTA ? -expf(p.a_log[h]) : 0.f;
+    const float decay = RULE == DELTA ? 1.f : p.decay[h];
+    for (int t = 0; t < len; ++t) {
+        const size_t row = (size_t)(row0 + t);
+        const TX* q = static_cast<const TX*>(p.q) + row * p.stride + kh * d;
+        const TX* k = static_cast<const TX*>(p.k) + row * p.stride + kh * d;
+        float v = col < e ? to_f32(static_cast<const TX*>(p.v)[row * p.stride + (size_t)h * e + col]) : 0.f;
+        float kv[R / 32], qv[R / 32], g[R / 32];
+#pragma unroll
+        for (int i = 0; i < R / 32; ++i) {
+            const int c = lane + 32 * i;
+            kv[i] = qv[i] = g[i] = 0.f;
+            if (c < d) {
+                kv[i] = to_f32(k[c]);
+                qv[i] = to_f32(q[c]);
+                g[i] = RULE == DELTA ? p.logits[row * p.logit_stride + h * d + c] + p.dt_bias[h * d + c] : decay;
+            }
+        }
+        if (p.activate) {
+            v = lr_silu<TX>(v);
+#pragma unroll
+            for (int i = 0; i < R / 32; ++i)
+                kv[i] = lr_silu<TX>(kv[i]), qv[i] = lr_silu<TX>(qv[i]);
+        }
+        float beta = 1.f, kq = 0.f;
+        if (RULE == DELTA) {
+            beta = 1.f / (1.f + expf(-to_f32(static_cast<const TX*>(p.beta)[row * p.beta_stride + h])));
+            float sk = 0.f, sq = 0.f;
+#pragma unroll
+            for (int i = 0; i < R / 32; ++i) {
+                sk = fmaf(kv[i], kv[i], sk);
+                sq = fmaf(qv[i], qv[i], sq);
+            }
+            const float ik = 1.f / sqrtf(warp_sum(sk) + p.key_eps);
+            const float iq = p.q_scale / sqrtf(warp_sum(sq) + p.key_eps);
+#pragma unroll
+            for (int i = 0; i < R / 32; ++i) {
+                kv[i] *= ik;
+                qv[i] *= iq;
+                g[i] = lane + 32 * i < d ? lr_decay<TX>(rate, g[i]) : 0.f;
+            }
+        }
+        __syncwarp();                                   // (the token before is through)
+#pragma unroll
+        for (int i = 0; i < R / 32; ++i) {
+            vec[0][lane + 32 * i] = kv[i];
+            vec[1][lane + 32 * i] = qv[i];
+            vec[2][lane + 32 * i] = g[i];
+            kq = fmaf(kv[i], qv[i], kq);
+        }
+        kq = warp_sum(kq);
+        __syncwarp();
+        // S' = diag(g) S, u = b (v - S'^T k), S = S' + k u^T, o = S'^T q + (k . q) u
+        float sk[4] = { 0.f, 0.f, 0.f, 0.f }, sq[4] = { 0.f, 0.f, 0.f, 0.f };
+#pragma unroll
+        for (int r = 0; r < R; r += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(&vec[0][r]);
+            const float4 q4 = *reinterpret_cast<const float4*>(&vec[1][r]);
+            const float4 g4 = *reinterpret_cast<const float4*>(&vec[2][r]);
+            const float kk[4] = { k4.x, k4.y, k4.z, k4.w }, qq[4] = { q4.x, q4.y, q4.z, q4.w },
+                        gg[4] = { g4.x, g4.y, g4.z, g4.w };
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                S[r + x] *= gg[x];
+                if (RULE == DELTA)
+                    sk[x] = fmaf(S[r + x], kk[x], sk[x]);
+                sq[x] = fmaf(S[r + x], qq[x], sq[x]);
+            }
+        }
+        asm volatile("" ::: "memory");                  // (the keys are read again, not kept beside the state)
+        const float u = RULE == DELTA ? beta * (v - ((sk[0] + sk[1]) + (sk[2] + sk[3]))) : v;
+#pragma unroll
+        for (int r = 0; r < R; r += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(&vec[0][r]);
+            S[r] = fmaf(k4.x, u, S[r]);
+            S[r + 1] = fmaf(k4.y, u, S[r + 1]);
+            S[r + 2] = fmaf(k4.z, u, S[r + 2]);
+            S[r + 3] = fmaf(k4.w, u, S[r + 3]);
+        }
+        if (col < e)
+            p.o[row * p.heads * e + (size_t)h * e + col] = fmaf(kq, u, (sq[0] + sq[1]) + (sq[2] + sq[3]));
+    }
+    int step = e;
+    asm volatile("" : "+r"(step), "+l"(st));            // (addresses are made again, not kept)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (col < e && r < d)
+            st[(size_t)r * step + col] = S[r];
+}
+
+// The generalised delta rule, whose state lies value column first: a warp owns CW neighbouring columns, a lane R key
+// rows of each (runs of up to four), and a token's sums over the rows are folded over the lanes for all columns
+// together.  With the removals' p = x^T S, o = r^T (g S) - (r . a x) p + (r . k) v needs no second fold.  Two warps to a
+// block, no shared memory: bound by the state's way from memory and back (64 sequences of 32 heads of 64 x 64
+// 14.6 us; 118 before, in a kernel whose eight producer warps and chunk buffers served one token).
+template <int R, int CW, typename TX>
+__global__ void __launch_bounds__(64)
+general_tokens_kernel(const RecurrenceParams p)
+{
+#ifdef CHIBI_TIMELINE
+    pdl_enter();
+#else
+    pdl_trigger();
+#endif
+    constexpr int RUN = R < 4 ? R : 4;                  // rows of a lane that lie side by side
+    const int h = blockIdx.y, seq = blockIdx.z, lane = threadIdx.x & 31;
+    const int d = p.d;
+    const int col = (blockIdx.x * 2 + (threadIdx.x >> 5)) * CW;
+    const int row0 = p.q_start[seq];
+    const int len = p.q_start[seq + 1] - row0;
+    if (len <= 0 || col >= d)
+        return;
+    float* st = p.state + (((size_t)p.slots[seq] * p.heads + h) * d + col) * d;
+#ifndef CHIBI_TIMELINE
+    for (int i = lane * 32; i < min(CW, d - col) * d; i += 1024)
+        prefetch_l2(st + i);                            // (only asked for: who wrote it last may be the kernel ahead)
+    pdl_wait();
+#endif
+    auto row_of = [&](int i) { return (i / RUN) * 32 * RUN + RUN * lane + i % RUN; };
+    const bool wide = RUN > 1 && d % RUN == 0 && (reinterpret_cast<uintptr_t>(p.state) & 15) == 0;
+    float S[CW][R];
+#pragma unroll
+    for (int j = 0; j < CW; ++j)
+#pragma unroll
+        for (int i = 0; i < R; i += RUN) {
+            const int r = row_of(i);
+            const float* src = st + (size_t)j * d + r;
+            if (wide) {
+                const bool there = col + j < d && r < d;
+                if constexpr (RUN == 4) {
+                    const float4 v = there ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    S[j][i] = v.x, S[j][i + 1] = v.y, S[j][i + 2] = v.z, S[j][i + 3] = v.w;
+                } else if constexpr (RUN == 2) {
+                    const float2 v = there ? *reinterpret_cast<const float2*>(src) : make_float2(0.f, 0.f);
+                    S[j][i] = v.x, S[j][i + 1] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int x = 0; x < RUN; ++x)
+                    S[j][i + x] = (col + j < d && r + x < d) ? src[x] : 0.f;
+            }
+        }
+    for (int t = 0; t < len; ++t) {
+        const size_t row = (size_t)(row0 + t);
+        const TX* r_ = static_cast<const TX*>(p.q) + row * p.stride + h * d;
+        const TX* k_ = static_cast<const TX*>(p.k) + row * p.stride + h * d;
+        const TX* a_ = static_cast<const TX*>(p.removal) + row * p.stride + h * d;
+        const TX* v_ = static_cast<const TX*>(p.v) + row * p.stride + h * d + col;
+        float k[R], x[R], ax[R], rw[R], w[R];
+        float kk = 0.f, rk = 0.f, rax = 0.f;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int c = row_of(i);
+            k[i] = rw[i] = ax[i] = w[i] = 0.f;
+            if (c < d) {
+                k[i] = to_f32(k_[c]);
+                rw[i] = to_f32(r_[c]);
+                ax[i] = 1.f / (1.f + expf(-(to_f32(a_[c]) + p.removal_bias[h * d + c])));
+                w[i] = expf(-p.decay_scale / (1.f + expf(-(p.logits[row * p.logit_stride + h * d + c] + p.dt_bias[h * d + c]))));
+            }
+            kk = fmaf(k[i], k[i], kk);
+        }
+        const float inv = 1.f / sqrtf(warp_sum(kk) + p.key_eps);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            x[i] = k[i] * inv;
+            ax[i] *= x[i];
+            rk = fmaf(rw[i], k[i], rk);
+            rax = fmaf(rw[i], ax[i], rax);
+            rw[i] *= w[i];
+        }
+        rk = warp_sum(rk);
+        rax = warp_sum(rax);
+        float sums[2 * CW];                             // x^T S, then r^T (g S), of every column
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+            sums[j] = sums[CW + j] = 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                sums[j] = fmaf(x[i], S[j][i], sums[j]);
+                sums[CW + j] = fmaf(rw[i], S[j][i], sums[CW + j]);
+            }
+        }
+        // fold: halves of the sums until a lane has one, its number in the lane's upper bits; then plain sums
+        int o = 16;
+#pragma unroll
+        for (int half = CW; half >= 1; half >>= 1, o >>= 1) {
+            const bool upper = (lane & o) != 0;
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+                const float send = upper ? sums[i] : sums[i + half];
+                const float keep = upper ? sums[i + half] : sums[i];
+                sums[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+#pragma unroll
+        for (; o >= 1; o >>= 1)
+            sums[0] += __shfl_xor_sync(0xffffffffu, sums[0], o);
+        constexpr int STEP = 32 / (2 * CW);             // lanes with the same sum
+        const float mine = sums[0];
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+            const float found = __shfl_sync(0xffffffffu, mine, j * STEP);
+            const float v = col + j < d ? to_f32(v_[j]) : 0.f;
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+                S[j][i] = fmaf(k[i], v, fmaf(w[i], S[j][i], -ax[i] * found));
+        }
+        // lane (CW + j) STEP has column j's r^T (g S), lane j STEP its removal
+        const int j = lane / STEP - CW;
+        const float found = __shfl_sync(0xffffffffu, mine, (lane / STEP % CW) * STEP);
+        if (j >= 0 && lane % STEP == 0 && col + j < d)
+            p.o[row * p.heads * d + (size_t)h * d + col + j] = fmaf(rk, to_f32(v_[j]), fmaf(-rax, found, mine));
+    }
+#pragma unroll
+    for (int j = 0; j < CW; ++j)
+#pragma unroll
+        for (int i = 0; i < R; i += RUN) {
+            const int r = row_of(i);
+            float* dst = st + (size_t)j * d + r;
+            if (wide) {
+                if (col + j < d && r < d) {
+                    if constexpr (RUN == 4)
+                        *reinterpret_cast<float4*>(dst) = make_float4(S[j][i], S[j][i + 1], S[j][i + 2], S[j][i + 3]);
+                    else if constexpr (RUN == 2)
+                        *reinterpret_cast<float2*>(dst) = make_float2(S[j][i], S[j][i + 1]);
+                }
+            } else {
+#pragma unroll
+                for (int x = 0; x < RUN; ++x)
+                    if (col + j < d && r + x < d)
+                        dst[x] = S[j][i + x];
+            }
+        }
+}
+
 // ---------------------------------------------------------------- launches
 static inline int padded_rows(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : d <= 128 ? 128 : d <= 256 ? 256 : 0; }
 
@@ -1049,8 +1316,30 @@ static void launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cu
 template <int RULE, typename TX>
 static void launch_tokens(const RecurrenceParams& p, int seqs, cudaStream_t stream)
 {
+    if constexpr (RULE == GENERAL) {
+        auto grid = [&](int columns) { return dim3((unsigned)((p.d + 2 * columns - 1) / (2 * columns)), (unsigned)p.heads, (unsigned)seqs); };
+        if (p.d <= 32)
+            launch(general_tokens_kernel<1, 16, TX>, grid(16), dim3(64), 0, stream, p);
+        else if (p.d <= 64)
+            launch(general_tokens_kernel<2, 16, TX>, grid(16), dim3(64), 0, stream, p);
+        else if (p.d <= 128)
+            launch(general_tokens_kernel<4, 8, TX>, grid(8), dim3(64), 0, stream, p);
+        else
+            launch(general_tokens_kernel<8, 4, TX>, grid(4), dim3(64), 0, stream, p);
+        return;
+    } else {
     const dim3 grid((unsigned)((p.e + 31) / 32), (unsigned)p.heads, (unsigned)seqs);
-    if (p.d <= 32)
+    // Whole columns to a lane where that fills the SMs with four warps each; with fewer, eight warps share the rows (one
+    // token of a sequence, heads of 128: 1 sequence of 16 heads 2.9 us and 6.9 with whole columns, 8 sequences
+    // of 16 heads, 512 warps, 7.2 and 8.0, of 32 heads 12.6 and 8.5, 64 of 16 heads 47.6 and 31.2).
+    const bool whole = (long long)grid.x * grid.y * grid.z >= 4LL * recurrence_sm_count();
+    if (whole && p.d <= 32)
+        launch(recurrence_columns_kernel<32, RULE, TX>, grid, dim3(32), 0, stream, p);
+    else if (whole && p.d <= 64)
+        launch(recurrence_columns_kernel<64, RULE, TX>, grid, dim3(32), 0, stream, p);
+    else if (whole && p.d <= 128)
+        launch(recurrence_columns_kernel<128, RULE, TX>, grid, dim3(32), 0, stream, p);
+    else if (p.d <= 32)
         launch(recurrence_tokens_kernel<8, 4, RULE, TX>, grid, dim3(256), 0, stream, p);
     else if (p.d <= 64)
         launch(recurrence_tokens_kernel<8, 8, RULE, TX>, grid, dim3(256), 0, stream, p);
@@ -1060,20 +1349,18 @@ static void launch_tokens(const RecurrenceParams& p, int seqs, cudaStream_t stre
         launch(recurrence_tokens_kernel<16, 16, RULE, TX>, grid, dim3(512), 0, stream, p);
     else
         launch(recurrence_tokens_kernel<16, 32, RULE, TX>, grid, dim3(512), 0, stream, p);
+    }
 }
 
 template <int RULE>
 static int launch_recurrence(const RecurrenceParams& p, int x_type, long long scratch_floats, long long tokens, int seqs,
                              int max_q_len, int few, cudaStream_t stream)
 {
-    if (p.d > 512 || p.heads > 65535 || seqs > 65535)
+    if (p.d > (RULE == GENERAL ? 256 : 512) || p.heads > 65535 || seqs > 65535)
         return CHIBI_ERR_UNSUPPORTED;
     const int DP = padded_rows(p.d);
     if (max_q_len <= few || DP == 0) {
-        if constexpr (RULE == GENERAL)
-            return CHIBI_ERR_UNSUPPORTED;               // (a kernel of sequence_ops.cu)
-        else
-            CHIBI_DISPATCH_TYPE(x_type, TX, { launch_tokens<RULE, TX>(p, seqs, stream); });
+        CHIBI_DISPATCH_TYPE(x_type, TX, { launch_tokens<RULE, TX>(p, seqs, stream); });
         return launch_status();
     }
     if (!p.scratch || (reinterpret_cast<uintptr_t>(p.scratch) & 15)
@@ -1178,13 +1465,13 @@ CHIBI_API int chibi_decayed_attention(const void* qkv, int x_type, long long str
     return launch_recurrence<LINEAR>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
 }
 
-// The generalised delta rule over prompt portions.  A row of proj holds r | k | v | gate | removal | low, heads * d columns
+// A row of proj holds r | k | v | gate | removal | low, heads * d columns
 // each but the last; logits [T, heads * d]; state [slots, heads, d (value), d (key)].
-CHIBI_API int chibi_delta_rule_chunks(const void* proj, int x_type, long long stride, const float* logits,
-                                      const float* decay_bias, const float* removal_bias, float* state, float* o,
-                                      float* scratch, long long scratch_floats, const int* q_start, const int* slots,
-                                      long long tokens, int seqs, int max_q_len, int heads, int d, float decay_scale,
-                                      float key_eps, cudaStream_t stream)
+CHIBI_API int chibi_delta_rule(const void* proj, int x_type, long long stride, const float* logits,
+                               const float* decay_bias, const float* removal_bias, float* state, float* o,
+                               float* scratch, long long scratch_floats, const int* q_start, const int* slots,
+                               long long tokens, int seqs, int max_q_len, int heads, int d, float decay_scale,
+                               float key_eps, int few, cudaStream_t stream)
 {
     if (seqs <= 0 || tokens <= 0 || max_q_len <= 0)
         return CHIBI_OK;
@@ -1212,5 +1499,5 @@ CHIBI_API int chibi_delta_rule_chunks(const void* proj, int x_type, long long st
     p.qk_heads = heads;
     p.d = d;
     p.e = d;
-    return launch_recurrence<GENERAL>(p, x_type, scratch_floats, tokens, seqs, max_q_len, 0, stream);
+    return launch_recurrence<GENERAL>(p, x_type, scratch_floats, tokens, seqs, max_q_len, few, stream);
 }

@@ -47,7 +47,6 @@ _SIGNATURES = {
                                               I, I, F, F, I, P, P],
         "chibi_attention_generic": [P, I, P, P, I, P, P, I, P, P, P, P, P, L, I, I, I, I, I, I, F, I, I, F, P, P, P, P, P],
         "chibi_short_conv": [P, I, L, P, P, P, P, L, P, P, I, I, I, I, P],
-        "chibi_delta_rule": [P, I, L, P, P, P, P, P, P, P, I, I, I, I, I, F, F, P],
         "chibi_decay_logits": [P, I, L, P, P, L, I, I, P],
         "chibi_gated_group_norm": [P, P, I, L, P, P, I, L, I, I, F, P],
         "chibi_scale": [P, F, L, P],
@@ -101,7 +100,7 @@ _SIGNATURES = {
         "chibi_norm_then_gate": [P, P, I, L, P, F, P, L, I, P],
         "chibi_bias_xielu": [P, I, I, P, P, I, L, I, F, F, P],
         "chibi_recurrence_scratch": [L, I, I, I, I, P],
-        "chibi_delta_rule_chunks": [P, I, L, P, P, P, P, P, P, L, P, P, L, I, I, I, I, F, F, P],
+        "chibi_delta_rule": [P, I, L, P, P, P, P, P, P, L, P, P, L, I, I, I, I, F, F, I, P],
         "chibi_channel_delta": [P, I, L, P, L, P, L, P, P, P, P, P, L, P, P, L, I, I, I, I, I, I, F, F, I, P],
         "chibi_decayed_attention": [P, I, L, I, P, P, P, P, L, P, P, L, I, I, I, I, I, I, P],
     },

@@ -1162,21 +1162,14 @@ class CudaKernels:
         if proj.shape[1] != 5 * W + rank or state.dtype != torch.float32 or not state.is_contiguous() \
                 or tuple(state.shape[1:]) != (heads, d, d):
             raise KernelError("delta_rule: proj [T, 5 * heads * d + rank] and state float32 [slots, heads, d, d]")
-        if max_q_len > self.RECURRENCE_FEW_TOKENS and d <= 256:
-            # prompt portions, in chunks of tokens (a first kernel prepares all chunks, a second walks over them)
-            seqs = state_slots.numel()
-            scratch = self._recurrence_scratch(T, seqs, heads, d, 2, max_q_len)
-            self.launches += 2
-            _check(self.lib.chibi_delta_rule_chunks(
-                _ptr(proj), _code(proj), proj.stride(0), _ptr(decay_logits), _ptr(decay_bias), _ptr(removal_bias), _ptr(state),
-                _ptr(o), _ptr(scratch), scratch.numel(), _ptr(q_start), _ptr(state_slots), T, seqs, int(max_q_len), heads, d,
-                float(decay_scale), float(key_eps), self._stream()), "delta_rule (chunks)")
-            return
-        self.launches += 1
-        _check(self.lib.chibi_delta_rule(_ptr(proj), _code(proj), proj.stride(0), _ptr(decay_logits),
-                                         _ptr(decay_bias), _ptr(removal_bias), _ptr(state), _ptr(o), _ptr(q_start),
-                                         _ptr(state_slots), state_slots.numel(), int(max_q_len), heads, d, rank,
-                                         float(decay_scale), float(key_eps), self._stream()), "delta_rule")
+        seqs = state_slots.numel()
+        scratch = self._recurrence_scratch(T, seqs, heads, d, 2, max_q_len)
+        self.launches += 2 if scratch is not None and d <= 256 else 1
+        _check(self.lib.chibi_delta_rule(
+            _ptr(proj), _code(proj), proj.stride(0), _ptr(decay_logits), _ptr(decay_bias), _ptr(removal_bias), _ptr(state),
+            _ptr(o), _ptr(scratch), scratch.numel() if scratch is not None else 0, _ptr(q_start), _ptr(state_slots), T, seqs,
+            int(max_q_len), heads, d, float(decay_scale), float(key_eps), self.RECURRENCE_FEW_TOKENS, self._stream()),
+            "delta_rule")
 
     def gated_group_norm(self, x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: float, group: int,
                          out: torch.Tensor) -> None:

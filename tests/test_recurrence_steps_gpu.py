@@ -1,0 +1,59 @@
+"""Steps of few tokens of many sequences: the recurrences' kernels for full servers against the ones for few sequences."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def k():
+    from chibillm_b200.kernels.ops import CudaKernels
+    return CudaKernels(torch.device(DEV))
+
+
+def ints(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+# heads x columns of 32 x sequences reach four warps an SM (592) in one call and stay below it sequence by sequence; key
+# rows and value columns that fill no whole 32, 64 or 128
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,d,e", [(4, 20, 40), (4, 64, 64), (6, 50, 33), (3, 128, 72), (4, 100, 128)])
+@pytest.mark.parametrize("rule", ["delta", "decayed"])
+def test_many_sequences_equal_single_ones(k, rule, dtype, heads, d, e):
+    g = torch.Generator(device=DEV).manual_seed(d)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    seqs = 100
+    lens = [1 + (i * 7) % 4 for i in range(seqs)]
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    T = starts[-1]
+    qkv = rnd(T, heads * (2 * d + e)).to(dtype)
+    logits, beta, a_log, bias = rnd(T, heads * d), rnd(T, heads).to(dtype), rnd(heads), rnd(heads * d)
+    decay = torch.rand(heads, generator=g, device=DEV)
+    first = rnd(seqs + 1, heads, d, e)
+
+    def run(state, o, a, b, slots, longest):
+        q_start = ints([s - starts[a] for s in starts[a:b + 1]])
+        rows = slice(starts[a], starts[b])
+        if rule == "delta":
+            k.channel_delta(qkv[rows], logits[rows], beta[rows], a_log, bias, state, o[rows], q_start, ints(slots), heads, heads,
+                            d, e, 1e-6, d ** -0.5, longest)
+        else:
+            k.decayed_attention(qkv[rows], decay, state, o[rows], q_start, ints(slots), heads, d, e, longest, activate=True)
+
+    assert heads * -(-e // 32) * seqs >= 592 > heads * -(-e // 32)
+    slots = [(i * 37) % seqs for i in range(seqs)]
+    one, many = first.clone(), first.clone()
+    o1, o2 = torch.full((T, heads * e), float("nan"), device=DEV), torch.full((T, heads * e), float("nan"), device=DEV)
+    run(many, o2, 0, seqs, slots, 4)
+    for i in range(seqs):
+        run(one, o1, i, i + 1, slots[i:i + 1], lens[i])
+    # the same multiply-adds with the sums over the d rows in another order: d / 2 roundings of sums of magnitude
+    # sqrt(d) max|S| at most (unit keys and queries of the delta rule; plain ones of the other)
+    scale = float(o1.abs().max())
+    assert float((o1 - o2).abs().max()) <= (d / 2 + 16) * 2.0 ** -24 * 4 * scale
+    assert float((one - many).abs().max()) <= (d / 2 + 16) * 2.0 ** -24 * 4 * float(one.abs().max())
+    assert torch.equal(many[seqs], first[seqs])
