@@ -73,7 +73,7 @@ _SIGNATURES = {
         "chibi_softcap": [P, F, L, P],
         "chibi_zero": [P, L, P],
         "chibi_expert_tile_rows": [],
-        "chibi_expert_rows_tc": [P, P, P, L, P, L, I, I, I, I, I, P, P, P],
+        "chibi_expert_rows_tc": [P, P, P, L, P, L, L, I, I, I, I, I, P, P, P],
         "chibi_expert_tile_rows_tensor_cores": [],
         "chibi_attention_f32": [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, F, I, I, I, I, I, F, P, P, P, P, P],
         "chibi_attention_generic_shared": [P, I, P, P, I, P, I, P, I, P, P, P, P, P, L, I, I, I, I, I, I, F, I, I, F, P, P,

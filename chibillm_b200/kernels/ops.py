@@ -1401,10 +1401,10 @@ class CudaKernels:
             max_tiles = (pairs + tile - 1) // tile + E
             rows = route[E + 1 + 2 * pairs + 2 * max_tiles:E + 1 + 3 * pairs + 2 * max_tiles]
             self.gather_rows(x, rows, sorted_x)
-            s1 = self.lib.chibi_expert_rows_tc(_ptr(sorted_x), _ptr(gate_up), _ptr(act), F, _ptr(route), pairs, E,
+            s1 = self.lib.chibi_expert_rows_tc(_ptr(sorted_x), _ptr(gate_up), _ptr(act), F, _ptr(route), pairs, T, E,
                                                2 * F, D, 1, self.ACTIVATIONS[kind], None, _ptr(self.error), stream)
             if s1 == 0:
-                _check(self.lib.chibi_expert_rows_tc(_ptr(act), _ptr(down), _ptr(y), D, _ptr(route), pairs, E, D, F, 0,
+                _check(self.lib.chibi_expert_rows_tc(_ptr(act), _ptr(down), _ptr(y), D, _ptr(route), pairs, T, E, D, F, 0,
                                                      0, None, _ptr(self.error), stream), "routed_experts (down, tcgen05)")
                 _check(self.lib.chibi_combine_experts(_ptr(y), _ptr(route), _ptr(acc), acc.stride(0), T, D, top, E,
                                                       float(weight), None, stream), "routed_experts (combine)")
@@ -1698,10 +1698,10 @@ class CudaKernels:
             max_tiles = (pairs + tile - 1) // tile + E
             rows = route[E + 1 + 2 * pairs + 2 * max_tiles:E + 1 + 3 * pairs + 2 * max_tiles]
             self.gather_rows(x, rows, sorted_x)
-            s1 = self.lib.chibi_expert_rows_tc(_ptr(sorted_x), _ptr(up), _ptr(act), F, _ptr(route), pairs, E, rows_up, D,
+            s1 = self.lib.chibi_expert_rows_tc(_ptr(sorted_x), _ptr(up), _ptr(act), F, _ptr(route), pairs, T, E, rows_up, D,
                                                first, code, row_weight, _ptr(self.error), stream)
             if s1 == 0:
-                _check(self.lib.chibi_expert_rows_tc(_ptr(act), _ptr(down), _ptr(y), D, _ptr(route), pairs, E, D, F, 0,
+                _check(self.lib.chibi_expert_rows_tc(_ptr(act), _ptr(down), _ptr(y), D, _ptr(route), pairs, T, E, D, F, 0,
                                                      0, None, _ptr(self.error), stream), "chosen_experts (down, tcgen05)")
                 combine()
                 self.tensor_core_calls += 2
