@@ -62,6 +62,31 @@ __device__ __forceinline__ void af_copy16(float* dst, const float* src, int byte
 __device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+__device__ __forceinline__ void af_cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// What lies at the same place of the shared memory of CTA `rank` of this cluster.
+__device__ __forceinline__ uint32_t af_peer_address(const float* local, int rank)
+{
+    uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local)), b;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+    return b;
+}
+__device__ __forceinline__ float af_peer(const float* local, int rank)
+{
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(af_peer_address(local, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 af_peer4(const float* local, int rank)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(af_peer_address(local, rank)) : "memory");
+    return v;
+}
+
 // What becomes of a dot product; `distance`: query position - key position.
 __device__ __forceinline__ float af_score(const AttentionF32& p, float dot, float r1, float r2, int distance)
 {
@@ -76,15 +101,18 @@ __device__ __forceinline__ float af_score(const AttentionF32& p, float dot, floa
 __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -INFINITY ? 0.f : expf(m - m_new); }
 
 // ---------------------------------------------------------------- sequences that bring several tokens
-// grid (row tiles, kv heads, sequences), 128 threads.  A tile is 64 rows, the group's heads of neighbouring tokens, and
-// walks over its keys 32 at a time, from a multiple of 32 on.  A thread owns rows ty + 16 i; of the scores
+// grid (4 CTAs for each row tile, kv heads, sequences), 128 threads.  A tile is 64 rows, the group's heads of
+// neighbouring tokens; the keys are taken 32 at a time, from a multiple of 32 on, and blocks of 64 keys (counted from the
+// sequence's start) go to the four CTAs of a cluster in turn, which add up what they found at the end: a causal
+// tile's keys spread evenly, and few rows make four times the CTAs (three prompts of up to 400 tokens of 16 heads:
+// 137 us with one CTA a tile).  A thread owns rows ty + 16 i; of the scores
 // the keys tx + 8 j, of the output the columns 4 tx + 32 j .. + 3, so a row's eight threads sit side by side in a warp:
 // its maximum and sum are three shuffles, and its probabilities reach them through shared memory without a block
 // barrier.  The next keys are fetched while the values are used and the other way round.  Scores take two
 // neighbouring features at a time (fma.rn.f32x2), the output two neighbouring columns.  Bound by the reads of
 // shared memory beside the multiply-adds (8 reads of 16 bytes, 32 cycles, to 16 cycles of multiply-adds for the
 // scores; 80 to 64 for the output); 76 KB a CTA, three to an SM.
-constexpr int AF_ROWS = 64, AF_KEYS = 32, AF_P = AF_KEYS + 4;
+constexpr int AF_ROWS = 64, AF_KEYS = 32, AF_P = AF_KEYS + 4, AF_RANKS = 4, AF_BLOCK = 64;
 
 template <int D> constexpr size_t af_shared()
 {
@@ -111,11 +139,23 @@ attention_f32_prompt_kernel(const AttentionF32 p)
     const int pos0 = p.ctx_len[seq] - q_len;            // the first token's position
     const int* const table = p.block_table + (size_t)(p.seq_rows ? p.seq_rows[seq] : seq) * p.table_stride;
 
+    const int rank = blockIdx.x % AF_RANKS;
+    float* const ml = P;                                // at the end: [AF_ROWS] maxima, [AF_ROWS] sums
+    float* const part = K;                              // and, over keys and values, [AF_ROWS][D] sums
+
     // the tiles with the most keys first
-    for (int tile = tiles - 1 - (int)blockIdx.x; tile >= 0; tile -= gridDim.x) {
+    for (int tile = tiles - 1 - (int)blockIdx.x / AF_RANKS; tile >= 0; tile -= gridDim.x / AF_RANKS) {
         const int first_row = tile * AF_ROWS, last_row = min(first_row + AF_ROWS, all_rows) - 1;
         const int last_pos = pos0 + last_row / G;
-        const int begin = first_visible_key(pos0 + first_row / G, p.window, p.chunk) & ~(AF_KEYS - 1);
+        const int oldest = first_visible_key(pos0 + first_row / G, p.window, p.chunk);      // (older pages may be gone)
+        const int visible = oldest & ~(AF_KEYS - 1);
+        // this CTA's blocks: those whose number is rank modulo AF_RANKS
+        const int block = visible / AF_BLOCK, mine = block + (rank + AF_RANKS - block % AF_RANKS) % AF_RANKS;
+        const int begin = mine == block ? visible : mine * AF_BLOCK;
+        auto after = [&](int base) {
+            const int next = base + AF_KEYS;
+            return next % AF_BLOCK ? next : next + (AF_RANKS - 1) * AF_BLOCK;
+        };
         __syncthreads();                                // (the tile before is through)
         for (int c = tid; c < AF_ROWS * QUADS; c += 128) {
             const int r = c / QUADS, at = 4 * (c % QUADS), row = first_row + r;
@@ -128,7 +168,7 @@ attention_f32_prompt_kernel(const AttentionF32 p)
         auto fetch = [&](const float* cache, float* dst, int stride, int base) {
             const int u = base + lane;
             long long at = -1;
-            if (u <= last_pos) {
+            if (u >= oldest && u <= last_pos) {
                 const int page = table[u / p.page_size];
                 if (page < 0 || page >= p.num_pages) {
                     if (p.error)
@@ -156,14 +196,14 @@ attention_f32_prompt_kernel(const AttentionF32 p)
             pos[i] = pos0 + row / G;
             r1[i] = p.bias_r1 ? p.bias_r1[h] : 0.f;
             r2[i] = p.bias_r2 ? p.bias_r2[h] : 0.f;
-            m[i] = p.sink ? p.sink[h] : -INFINITY;
-            l[i] = p.sink ? 1.f : 0.f;
+            m[i] = -INFINITY;
+            l[i] = 0.f;
 #pragma unroll
             for (int j = 0; j < CJ; ++j)
                 O[i][j][0] = O[i][j][1] = 0;
         }
         usable = fetch(p.k_cache, K, DS, begin);        // (one group with the queries)
-        for (int base = begin; base <= last_pos; base += AF_KEYS) {
+        for (int base = begin; base <= last_pos; base = after(base)) {
             const unsigned keys = usable;
             af_wait<0>();
             __syncthreads();                            // the keys are there; everyone is through with the values before
@@ -234,8 +274,8 @@ attention_f32_prompt_kernel(const AttentionF32 p)
             }
             af_wait<0>();
             __syncthreads();                            // the values are there (and the row's probabilities)
-            if (base + AF_KEYS <= last_pos)
-                usable = fetch(p.k_cache, K, DS, base + AF_KEYS);
+            if (after(base) <= last_pos)
+                usable = fetch(p.k_cache, K, DS, after(base));
             auto values = [&](bool all) {
 #pragma unroll 2
                 for (int kk = 0; kk < AF_KEYS; kk += 4) {
@@ -270,19 +310,56 @@ attention_f32_prompt_kernel(const AttentionF32 p)
             else
                 values(false);
         }
+        af_wait<0>();
+        __syncthreads();                                // keys and values are through: their place takes the sums
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int row = first_row + ty + 16 * i;
-            if (row < all_rows) {
-                const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
-                float* o = p.out + ((size_t)(row0 + row / G) * p.nq + kv_head * G + row % G) * D + 4 * tx;
+            const int r = ty + 16 * i;
 #pragma unroll
-                for (int j = 0; j < CJ; ++j) {
-                    const float2 a = af_halves(O[i][j][0]), b = af_halves(O[i][j][1]);
-                    *reinterpret_cast<float4*>(o + 32 * j) = make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
-                }
+            for (int j = 0; j < CJ; ++j)
+                *reinterpret_cast<ulonglong2*>(part + r * D + 4 * tx + 32 * j) = make_ulonglong2(O[i][j][0], O[i][j][1]);
+            if (tx == 0) {
+                ml[r] = m[i];
+                ml[AF_ROWS + r] = l[i];
             }
         }
+        af_cluster_sync();
+        // each CTA finishes a quarter of the rows
+        constexpr int OWN = AF_ROWS / AF_RANKS;
+        for (int c = tid; c < OWN * QUADS; c += 128) {
+            const int r = rank * OWN + c / QUADS, at = 4 * (c % QUADS), row = first_row + r;
+            if (row >= all_rows)
+                continue;
+            float pm[AF_RANKS], pl[AF_RANKS];
+            float4 po[AF_RANKS];
+#pragma unroll
+            for (int x = 0; x < AF_RANKS; ++x) {
+                pm[x] = af_peer(ml + r, x);
+                pl[x] = af_peer(ml + AF_ROWS + r, x);
+                po[x] = af_peer4(part + r * D + at, x);
+            }
+            const int h = kv_head * G + row % G;
+            const float sink = p.sink ? p.sink[h] : -INFINITY;
+            float top = sink;
+#pragma unroll
+            for (int x = 0; x < AF_RANKS; ++x)
+                top = fmaxf(top, pm[x]);
+            float sum = p.sink ? af_keep(sink, top) : 0.f;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int x = 0; x < AF_RANKS; ++x) {
+                const float keep = af_keep(pm[x], top);
+                sum = fmaf(pl[x], keep, sum);           // (a CTA without a key for the row has zeros)
+                v.x = fmaf(po[x].x, keep, v.x);
+                v.y = fmaf(po[x].y, keep, v.y);
+                v.z = fmaf(po[x].z, keep, v.z);
+                v.w = fmaf(po[x].w, keep, v.w);
+            }
+            const float inv = sum > 0.f ? 1.f / sum : 0.f;
+            *reinterpret_cast<float4*>(p.out + ((size_t)(row0 + row / G) * p.nq + h) * D + at) =
+                make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+        }
+        af_cluster_sync();                              // nobody goes on while its sums are read
     }
 }
 
@@ -445,16 +522,9 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
     }
     auto sync = [&]() {
         if (ranks > 1)
-            asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+            af_cluster_sync();
         else
             __syncthreads();
-    };
-    auto peer = [&](const float* local, int from) {
-        uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local)), b;
-        float v;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(from));
-        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(b) : "memory");
-        return v;
     };
     sync();
     for (int i = rank * 128 + tid; i < heads * D; i += ranks * 128) {
@@ -465,9 +535,9 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
             pm[r] = -INFINITY;
             pl[r] = po[r] = 0.f;
             if (r < ranks) {
-                pm[r] = peer(&range_m[g], r);
-                pl[r] = peer(&range_l[g], r);
-                po[r] = peer(&range_o[g][c], r);
+                pm[r] = af_peer(&range_m[g], r);
+                pl[r] = af_peer(&range_l[g], r);
+                po[r] = af_peer(&range_o[g][c], r);
             }
         }
         float top = p.sink ? p.sink[h0 + g] : -INFINITY;
@@ -502,7 +572,10 @@ static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min
             configured = true;
         }
         const long long tiles = ((long long)max_q_len * G + AF_ROWS - 1) / AF_ROWS;
-        launch(attention_f32_prompt_kernel<D>, dim3((unsigned)tiles, p.nkv, seqs), dim3(128), af_shared<D>(), stream, p);
+        if (tiles * AF_RANKS > 2147483647LL)
+            return CHIBI_ERR_UNSUPPORTED;
+        launch_cluster_x(attention_f32_prompt_kernel<D>, dim3((unsigned)tiles * AF_RANKS, p.nkv, seqs), dim3(128), af_shared<D>(),
+                         stream, AF_RANKS, p);
         if (const int status = launch_status())
             return status;
     }

@@ -464,6 +464,7 @@ class CudaKernels:
                     31: "a wait that ran out (experts' product: loader)",
                     32: "a wait that ran out (experts' product: tensor-core issuer)",
                     33: "a wait that ran out (experts' product: epilogue)",
+                    34: "a wait that ran out (experts' product: accumulator hand-over)",
                     **{c: f"a wait that ran out (tcgen05 attention, point {c})" for c in range(21, 30)}}.get(code, f"code {code}")
             raise KernelError(f"a kernel refused {what}")
 

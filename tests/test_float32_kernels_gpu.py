@@ -54,7 +54,7 @@ def test_linear_float32_keeps_infinities_to_their_rows(k):
 def exact_attention(q, keys, values, table, q_lens, ctx, nq, nkv, d, page, scale, window, chunk, softcap, bias, sink):
     out, at, G = [], 0, nq // nkv
     for s, (n, c) in enumerate(zip(q_lens, ctx)):
-        pages = table[s, :-(-c // page)].long()
+        pages = table[s, :-(-c // page)].long().clamp(min=0)
         k = keys[pages].transpose(1, 2).reshape(-1, nkv, d)[:c].double().repeat_interleave(G, 1)
         v = values[pages].transpose(1, 2).reshape(-1, nkv, d)[:c].double().repeat_interleave(G, 1)
         x = torch.einsum("thd,khd->htk", q[at:at + n].view(n, nq, d).double(), k) * scale
@@ -99,6 +99,12 @@ def test_attention_float32(k, d, nq, nkv, page, q_lens, ctx, options):
     for s, n in enumerate(pages):
         table[s, :n] = order[at:at + n]
         at += n
+    # pages that every query's window or block has left behind are gone
+    for s, (n, c) in enumerate(zip(q_lens, ctx)):
+        i = c - n
+        oldest = max(i - options["window"] + 1 if options.get("window") else 0,
+                     i - i % options["chunk"] if options.get("chunk") else 0, 0)
+        table[s, :oldest // page] = -1
     table = table.cuda()
     keys, values = rnd(sum(pages) + 3, nkv, page, d, seed=1), rnd(sum(pages) + 3, nkv, page, d, seed=2)
     q = rnd(T, nq * d, seed=3)
@@ -106,7 +112,8 @@ def test_attention_float32(k, d, nq, nkv, page, q_lens, ctx, options):
     used = torch.zeros(keys.shape[0], page, dtype=torch.bool, device="cuda")
     for s, c in enumerate(ctx):
         for u in range(c):
-            used[table[s, u // page].long(), u % page] = True
+            if table[s, u // page] >= 0:
+                used[table[s, u // page].long(), u % page] = True
     keys.masked_fill_(~used[:, None, :, None], float("nan"))
     values.masked_fill_(~used[:, None, :, None], float("nan"))
     starts = [0]
