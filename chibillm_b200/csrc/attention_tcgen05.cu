@@ -50,8 +50,42 @@ constexpr size_t ATC_SMEM = SMEM_TILES + NUM_BARS * 8 + 16 + 1024;
 constexpr uint32_t TMEM_S0 = 0, TMEM_S1 = 128, TMEM_O = 256;
 
 // Options of the score, compiled in: 0 none; 1 any of them (a soft cap, a bias of either kind); 2 a bias linear in
-// the distance and nothing else, which costs a multiply-add or two a score.
-constexpr int OPT_NONE = 0, OPT_ANY = 1, OPT_LINEAR = 2;
+// the distance and nothing else, which costs a multiply-add or two a score; 3 a soft cap and nothing else.
+constexpr int OPT_NONE = 0, OPT_ANY = 1, OPT_LINEAR = 2, OPT_CAP = 3;
+
+// v[i] = (cap log2 e) tanh(v[i] scale / cap): capped scores in units of log2.  The two special-function operations of
+// 1 - 2 / (exp(2 x) + 1) beside the softmax's one bound the kernel (an SM does 16 a cycle), so where all of a warp's
+// arguments are below 0.4 in magnitude, scores below 12 with a cap of 30, the odd Taylor polynomial of tanh to x^11 takes
+// their place (its next term is below 6e-8 of the result there).
+template <int N>
+__device__ __forceinline__ void cap_scores(uint32_t (&v)[N], float inv_cap, float cap_log2)
+{
+    float most = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float x = __uint_as_float(v[i]) * inv_cap;
+        v[i] = __float_as_uint(x);
+        most = fmaxf(most, fabsf(x));
+    }
+    if (__any_sync(0xffffffffu, !(most < 0.4f))) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float x = __uint_as_float(v[i]);
+            v[i] = __float_as_uint(cap_log2 * (1.f - __fdividef(2.f, fast_exp2(x * 2.8853900817779268f) + 1.f)));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float x = __uint_as_float(v[i]), t = x * x;
+            float y = fmaf(t, -1382.f / 155925.f, 62.f / 2835.f);
+            y = fmaf(y, t, -17.f / 315.f);
+            y = fmaf(y, t, 2.f / 15.f);
+            y = fmaf(y, t, -1.f / 3.f);
+            y = fmaf(y, t, 1.f);
+            v[i] = __float_as_uint(y * (x * cap_log2));
+        }
+    }
+}
 
 template <int OPT>
 __global__ void __launch_bounds__(ATC_THREADS)
@@ -252,12 +286,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
         // with options the scores are brought to their final form (in units of log2) right after
         // they are read, and the scale below is 1
-        constexpr bool options = OPT == OPT_ANY;
+        constexpr bool options = OPT == OPT_ANY || OPT == OPT_CAP;
         const float sl2 = OPT != OPT_NONE ? 1.f : p.scale_log2;
         const int bias_head = kv_head * p.group + (live ? r - tok * p.group : 0);
         const float r1 = p.bias_r1 ? p.bias_r1[bias_head] : 0.f, r2 = p.bias_r2 ? p.bias_r2[bias_head] : 0.f;
         const bool linear_bias = p.bias_r1 && !p.bias_r2;       // r1 * distance instead of r1 * ln(1 + r2 * distance)
         const float two_over_cap_log2 = p.softcap > 0.f ? 2.f * 1.4426950408889634f / p.softcap : 0.f;
+        const float inv_cap = OPT == OPT_CAP ? p.scale / p.softcap : 0.f, cap_log2 = p.softcap * 1.4426950408889634f;
         // The output accumulates in TMEM over all tiles.  `m` is the maximum that the exponents are
         // taken against; it follows the true maximum only when that has grown by more than 2^8
         // (then the output so far is rescaled in TMEM, a rare event after the first tiles), so
@@ -277,7 +312,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             tmem_load_wait();
             tcgen05_fence_before();
             mbar_arrive(&s_free[st]);                        // the MMA thread may fill this buffer again
-            if (options) {
+            if (OPT == OPT_CAP) {
+                cap_scores(sv, inv_cap, cap_log2);
+            } else if (options) {
 #pragma unroll
                 for (int i = 0; i < KEYS; ++i) {
                     float v = __uint_as_float(sv[i]) * p.scale;
@@ -675,12 +712,13 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         float m = -INFINITY, l = 0.f;
         // options of the score: both passes over the row bring their piece to its final form (in
         // units of log2) right after it is read, and the scale below is 1
-        constexpr bool options = OPT == OPT_ANY;
+        constexpr bool options = OPT == OPT_ANY || OPT == OPT_CAP;
         const float sl2 = OPT != OPT_NONE ? 1.f : p.scale_log2;
         const int bias_head = kv_head * p.group + (live ? r - tok * p.group : 0);
         const float r1 = p.bias_r1 ? p.bias_r1[bias_head] : 0.f, r2 = p.bias_r2 ? p.bias_r2[bias_head] : 0.f;
         const bool linear_bias = p.bias_r1 && !p.bias_r2;       // r1 * distance instead of r1 * ln(1 + r2 * distance)
         const float two_over_cap_log2 = p.softcap > 0.f ? 2.f * 1.4426950408889634f / p.softcap : 0.f;
+        const float inv_cap = OPT == OPT_CAP ? p.scale / p.softcap : 0.f, cap_log2 = p.softcap * 1.4426950408889634f;
         for (int j = 0; j < my_tiles; ++j) {
             const int st = j & 1;
             const int key0 = key_begin + j * KEYS;
@@ -705,7 +743,9 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                     for (int i = 0; i < 32; ++i)
                         v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), p.scale_log2, fmaf((float)(c0 + i), slope, at0 - off)));
                 }
-                if (options) {
+                if (OPT == OPT_CAP) {
+                    cap_scores(v, inv_cap, cap_log2);
+                } else if (options) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         float x = __uint_as_float(v[i]) * p.scale;
@@ -900,19 +940,20 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
     p.bias_r1 = bias_r1;
     p.bias_r2 = bias_r2;
     p.sink = sink;
-    const int options = softcap > 0.f || bias_r2 ? OPT_ANY : (bias_r1 ? OPT_LINEAR : OPT_NONE);
+    const int options = bias_r2 || (softcap > 0.f && bias_r1) ? OPT_ANY
+        : softcap > 0.f ? OPT_CAP : (bias_r1 ? OPT_LINEAR : OPT_NONE);
     CUtensorMap mk, mv;
     if (!tensor_map_2d(k_cache, p.cache_rows, D, D, page_size, &mk)
         || !tensor_map_2d(v_cache, p.cache_rows, D, D, page_size, &mv))
         return CHIBI_ERR_UNSUPPORTED;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const AttnTcParams);
-    static const Kernel one_tile[3] = { attn_prefill_tc_kernel<OPT_NONE>, attn_prefill_tc_kernel<OPT_ANY>,
-                                        attn_prefill_tc_kernel<OPT_LINEAR> };
-    static const Kernel two_tiles[3] = { attn_prefill_tc2_kernel<OPT_NONE>, attn_prefill_tc2_kernel<OPT_ANY>,
-                                         attn_prefill_tc2_kernel<OPT_LINEAR> };
+    static const Kernel one_tile[4] = { attn_prefill_tc_kernel<OPT_NONE>, attn_prefill_tc_kernel<OPT_ANY>,
+                                        attn_prefill_tc_kernel<OPT_LINEAR>, attn_prefill_tc_kernel<OPT_CAP> };
+    static const Kernel two_tiles[4] = { attn_prefill_tc2_kernel<OPT_NONE>, attn_prefill_tc2_kernel<OPT_ANY>,
+                                         attn_prefill_tc2_kernel<OPT_LINEAR>, attn_prefill_tc2_kernel<OPT_CAP> };
     static bool configured = false;
     if (!configured) {
-        for (int i = 0; i < 3; ++i) {
+        for (int i = 0; i < 4; ++i) {
             cudaError_t e = cudaFuncSetAttribute(one_tile[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC_SMEM);
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(two_tiles[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC2_SMEM);
