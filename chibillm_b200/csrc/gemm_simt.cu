@@ -203,14 +203,12 @@ gemm_f32_tile_kernel(const F32Params p)
         fetch(s);
 
     uint64_t acc[TM][8];
-    float group[TM][8];
+    float kept[TM][8];                                  // the group's sum
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 8; ++j)
             acc[i][j] = 0;
-            group[i][j] = 0.f;
-        }
     const int part_blocks = p.part / F32_KB;
     int in_part = 0, part = 0;
     for (int kb = 0; kb < blocks; ++kb) {
@@ -239,25 +237,24 @@ gemm_f32_tile_kernel(const F32Params p)
         if (++in_part == part_blocks || kb + 1 == blocks) {
             in_part = 0;
             const bool opens = part % F32_GROUP == 0;
+            ++part;
+            const bool closes = part % F32_GROUP == 0 || kb + 1 == blocks;
+            const int g = (part - 1) / F32_GROUP;
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float s = f32_halves_sum(acc[i][j]);
+                    float s = f32_halves_sum(acc[i][j]);
                     acc[i][j] = 0;
-                    group[i][j] = opens ? s : group[i][j] + s;
-                }
-            ++part;
-            if (part % F32_GROUP == 0 || kb + 1 == blocks) {
-                const int g = (part - 1) / F32_GROUP;
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
+                    if (!opens)
+                        s = kept[i][j] + s;
+                    if (!closes) {
+                        kept[i][j] = s;
+                    } else {
                         float* const t = sums + ((ranks > 1 ? g * BM : 0) + ty + TY * i) * 64 + tx + 8 * j;
-                        *t = ranks > 1 || g == 0 ? group[i][j] : *t + group[i][j];
+                        *t = ranks > 1 || g == 0 ? s : *t + s;
                     }
-            }
+                }
         }
     }
     if (ranks > 1)
@@ -519,13 +516,15 @@ static int f32_few(F32Params p, cudaStream_t stream)
 
 static int f32_tiles(F32Params p, cudaStream_t stream)
 {
-    // How many CTAs share a tile: what the busiest SM has to do, in groups of parts, with an eighth of one for a CTA's
-    // start and end.
+    // How many CTAs share a tile.  An SM holds two CTAs (the registers; with bounds for three the sums spill, 128 rows of
+    // 1,024 x 2,048 38 -> 50 us), and one alone takes 0.8 of the time of two (512 rows of 1,024 x 2,048, 128 tiles: 134 us
+    // whole, 76 shared).  The busiest SM's time in groups of parts, with an eighth of one for a CTA's start and end.
     const long long tiles = (long long)((p.N + 63) / 64) * ((p.M + 63) / 64);
     const int groups = (p.parts + F32_GROUP - 1) / F32_GROUP;
     double least = 0.0;
     for (int ranks = 1; ranks <= groups; ranks *= 2) {
-        const double cost = (double)((tiles * ranks + F32_SMS - 1) / F32_SMS) * ((groups + ranks - 1) / ranks + 0.125);
+        const long long ctas = (tiles * ranks + F32_SMS - 1) / F32_SMS;
+        const double cost = ((double)(ctas / 2) + (ctas % 2 ? 0.8 : 0.0)) * ((groups + ranks - 1) / ranks + 0.125);
         if (ranks == 1 || cost < least) {
             p.ranks = ranks;
             least = cost;
@@ -544,9 +543,9 @@ static int gemm_f32(const float* x, const float* w, float* out, const float* res
     p.part = (sixteenth + F32_KB - 1) / F32_KB * F32_KB;
     p.part = p.part < 128 ? 128 : p.part;
     p.parts = (K + p.part - 1) / p.part;
-    // Few rows to 48 (blocks of 16 above 8): 4,096 x 1,024 / 1,024 x 3,072 take 6.6, 7.7 us with 4 rows, 16, 15 us with
-    // 32, 30, 26 us with 48 and 39, 49 us in tiles of 64 rows (the kernel for all before this: 150, 180 us from one row to
-    // 64).  From 5 rows on, where the weights'
+    // Few rows to 48 (blocks of 16 above 8), to 128 where N is small: 4,096 x 1,024 / 1,024 x 3,072 take 6.6, 7.7 us with
+    // 4 rows, 30, 26 us with 48 (50 in tiles of 64 rows), 30, 26 with 64 (37, 43), 58, 44 with 128 (39, 53); the
+    // kernel for all before this 150, 180 us from one row to 64.  From 5 rows on, where the weights'
     // tiles fill the SMs (N >= 64 x 148), a lane takes two of their rows (151,936 x 1,024: 8 rows 155 -> 125 us, 16 rows
     // 246 -> 173; with fewer tiles two rows a lane leave SMs idle, 4,096 x 1,024: 7.9 -> 10.9).
     if (M <= 1)
@@ -558,7 +557,7 @@ static int gemm_f32(const float* x, const float* w, float* out, const float* res
     const bool wide = N >= 64 * F32_SMS;
     if (M <= 8)
         return wide ? f32_few<8, 2, 2>(p, stream) : f32_few<8, 1, 4>(p, stream);
-    if (M <= 48)
+    if (M <= 48 || (M <= 128 && (long long)((N + 31) / 32) * ((M + 15) / 16) <= 512))
         return wide ? f32_few<16, 2, 2>(p, stream) : f32_few<16, 1, 3>(p, stream);
     return f32_tiles(p, stream);
 }
