@@ -559,7 +559,7 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
 }
 
 template <int D>
-static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min_q_len, int max_ctx_len, cudaStream_t stream)
+static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min_q_len, int ranks, cudaStream_t stream)
 {
     const int G = p.nq / p.nkv;
     if (max_q_len > 1) {
@@ -580,10 +580,6 @@ static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min
             return status;
     }
     if (max_q_len == 1 || min_q_len <= 1) {
-        // one CTA for every 64 keys up to eight (which longer contexts share in eighths)
-        int ranks = 1;
-        while (ranks < 8 && 64 * ranks < max_ctx_len)
-            ranks *= 2;
         const int blocks = G <= 1 ? 1 : G <= 2 ? 1 : (G + 3) / 4;
         const dim3 grid(ranks, p.nkv * blocks, seqs);
         if (G <= 1)
@@ -601,11 +597,12 @@ static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min
 using namespace chibi;
 
 // Which of its two kernels run: one for sequences of several tokens if max_q_len > 1, one for single tokens if
-// min_q_len <= 1 (0: not known).
+// min_q_len <= 1 (0: not known).  ranks (1, 2, 4 or 8): CTAs that share a single token's keys; fewer than its ranges take
+// several each.
 CHIBI_API int chibi_attention_f32(const float* q, const float* k_cache, const float* v_cache, float* out,
                                   const int* block_table, int table_stride, const int* q_start, const int* ctx_len,
                                   const int* seq_rows, int seqs, int nq, int nkv, int d, int page_size, int num_pages,
-                                  float scale, int window, int chunk, int max_q_len, int min_q_len, int max_ctx_len,
+                                  float scale, int window, int chunk, int max_q_len, int min_q_len, int ranks,
                                   float softcap, const float* bias_r1, const float* bias_r2, const float* sink, int* error,
                                   cudaStream_t stream)
 {
@@ -613,11 +610,11 @@ CHIBI_API int chibi_attention_f32(const float* q, const float* k_cache, const fl
         return CHIBI_OK;
     // (pieces of 16 bytes; the grid's limits)
     if ((d != 64 && d != 128) || nkv <= 0 || nq % nkv != 0 || window < 0 || chunk < 0 || softcap < 0.f || page_size <= 0
-        || (bias_r2 != nullptr && bias_r1 == nullptr) || seqs > 65535 || nq > 65535
+        || (bias_r2 != nullptr && bias_r1 == nullptr) || seqs > 65535 || (ranks != 1 && ranks != 2 && ranks != 4 && ranks != 8) || nq > 65535
         || ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) % 16 != 0)
         return CHIBI_ERR_UNSUPPORTED;
     const AttentionF32 p = { q, k_cache, v_cache, out, block_table, table_stride, q_start, ctx_len, seq_rows, nq, nkv,
                              page_size, num_pages, scale, window, chunk, softcap, bias_r1, bias_r2, sink, error };
-    return d == 64 ? attention_f32<64>(p, seqs, max_q_len, min_q_len, max_ctx_len, stream)
-                   : attention_f32<128>(p, seqs, max_q_len, min_q_len, max_ctx_len, stream);
+    return d == 64 ? attention_f32<64>(p, seqs, max_q_len, min_q_len, ranks, stream)
+                   : attention_f32<128>(p, seqs, max_q_len, min_q_len, ranks, stream);
 }

@@ -1,8 +1,9 @@
 // Causal grouped-query attention over the paged cache, any head size up to
 // 1,024, any group size, optional window; element types are template parameters.
 //
-// This is the attention of the true 32-bit path and the fall-back of the
-// bfloat16 path for head sizes the tensor-core kernels do not cover.  One warp
+// This is the attention of the true 32-bit path for head sizes other than 64 and 128
+// (attention_f32.cu), and the fall-back of the bfloat16 path for what the tensor-core
+// kernels do not cover.  One warp
 // owns one (token, query head).  Keys are visited in position order in chunks
 // of 32: lane l scores key base+l (dot product over d in 32-bit, scaled after
 // the sum), the chunk joins the running softmax (m, l, acc rescaled by

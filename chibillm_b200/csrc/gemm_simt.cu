@@ -2,9 +2,10 @@
 //
 // This is the matrix product of the true 32-bit path (no tensor-core mode, so
 // no reduced-precision inputs or accumulators) and the fall-back of the
-// bfloat16 path for shapes the tensor-core kernel refuses.  Every output
-// element is one thread's sequential sum over k = 0..K-1, so the result of a
-// row does not depend on how many rows the call has.
+// bfloat16 path for shapes the tensor-core kernel refuses.  Operands that are all
+// 32-bit, with rows on 16-byte boundaries, run the two kernels further down; the first one
+// takes the rest: every output element is one thread's sequential sum over k = 0..K-1.  In
+// both the result of a row does not depend on how many rows the call has.
 #define CHIBI_UNIT gemm_simt
 #define CHIBI_UNIT_ID 2
 #include "common.cuh"

@@ -810,8 +810,9 @@ class CudaKernels:
                   sink: Optional[torch.Tensor] = None, kv_share: int = 1) -> None:
         """Causal attention of every token over its sequence's pages.  bfloat16
         with a head size that is a multiple of 16 runs on the tensor cores (one
-        library per head size, compiled when first needed); everything else, the
-        32-bit path included, runs the plain kernel.  ``softcap`` c: a scaled score
+        library per head size, compiled when first needed); 32-bit operands with head
+        sizes 64 and 128 run kernels of their own (32-bit arithmetic throughout);
+        everything else runs the plain kernel.  ``softcap`` c: a scaled score
         s becomes c * tanh(s / c).  ``distance_bias`` (r1, r2), float32 [nq] each:
         r1[h] * ln(1 + r2[h] * (i - j)) is taken off the score of query i and key j.
         ``v_cache`` may be ``k_cache`` itself (values tied to the keys).  ``chunk`` C: a
@@ -880,7 +881,7 @@ class CudaKernels:
             status = self.lib.chibi_attention_f32(
                 _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0), _ptr(q_start),
                 _ptr(ctx_len), _ptr(seq_rows), ctx_len.numel(), nq, nkv, d, page_size, k_cache.shape[0], float(scale),
-                int(window or 0), chunk, int(max_q_len), int(min_q_len), int(max_ctx_len), cap, _ptr(r1), _ptr(r2),
+                int(window or 0), chunk, int(max_q_len), int(min_q_len), self.float32_token_ranks(max_ctx_len), cap, _ptr(r1), _ptr(r2),
                 _ptr(sink), _ptr(self.error), self._stream())
             if status == 0:
                 self.launches += (1 if max_q_len > 1 else 0) + (1 if max_q_len == 1 or min_q_len <= 1 else 0)
@@ -913,6 +914,12 @@ class CudaKernels:
             nq, nkv, int(kv_share), page_size, k_cache.shape[0], float(scale), int(window or 0), int(chunk),
             int(max_q_len), float(softcap), _ptr(bias_r1), _ptr(bias_r2), _ptr(sink), _ptr(self.error),
             self._stream()), "attention (tensor cores, prompt)")
+
+    @staticmethod
+    def float32_token_ranks(max_ctx_len: int) -> int:
+        """CTAs that share the keys of a single token in the 32-bit attention kernel: one for every
+        64 keys up to eight (longer contexts are shared in eighths).  A captured step depends on it."""
+        return 1 if max_ctx_len <= 64 else 2 if max_ctx_len <= 128 else 4 if max_ctx_len <= 256 else 8
 
     def decode_attention_splits(self, seqs: int, nq: int, nkv: int, max_ctx_len: int) -> int:
         """Key ranges per sequence of the decode attention kernel: as many CTAs as

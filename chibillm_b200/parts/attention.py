@@ -249,7 +249,7 @@ class PagedAttention(Mixer):
         if splits is None:
             return None
         s = self.spec
-        return (splits(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),)
+        return (splits(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) + self.runtime.float32_launch_key(ctx)
 
     # ---- run
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, overwrite: bool = False, hold: bool = False):

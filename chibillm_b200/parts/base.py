@@ -30,6 +30,11 @@ class Runtime:
     def is_float32(self) -> bool:
         return self.dtype == torch.float32
 
+    def float32_launch_key(self, ctx) -> tuple:
+        """What a captured step of the 32-bit attention kernels depends on besides its data."""
+        ranks = getattr(self.kernels, "float32_token_ranks", None)
+        return (ranks(ctx.max_ctx_len),) if self.is_float32 and ranks is not None else ()
+
 
 # ------------------------------------------------------------------ tensors
 @dataclass(frozen=True)

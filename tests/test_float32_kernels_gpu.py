@@ -147,3 +147,17 @@ def test_attention_float32_hides_later_values(k):
     k.attention(q, keys, values, out, ints([[0, 1, 2]]), ints([0, T]), ints([T]), ints([0] * T), ints(list(range(T))), 1, 1, d, 16,
                 d ** -0.5, None, T, T, min_q_len=T)
     assert torch.isfinite(out[:20]).all() and torch.isnan(out[20:]).all()
+
+
+@pytest.mark.parametrize("ranks", [1, 2, 4])
+def test_single_tokens_with_fewer_ranges_than_keys(k, ranks, monkeypatch):
+    """A step captured while contexts were short runs on: its CTAs then take several ranges each."""
+    d, c = 64, 900
+    keys, values, q = rnd(60, 2, 16, d, seed=1), rnd(60, 2, 16, d, seed=2), rnd(1, 4 * d, seed=3)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    table, out = ints([list(range(57))]), torch.full((1, 4 * d), float("nan"), device="cuda")
+    monkeypatch.setattr(type(k), "float32_token_ranks", staticmethod(lambda n: ranks))
+    k.attention(q, keys, values, out, table, ints([0, 1]), ints([c]), ints([0]), ints([c - 1]), 4, 2, d, 16, d ** -0.5, None, 1, c,
+                min_q_len=1)
+    exact = exact_attention(q, keys, values, table, [1], [c], 4, 2, d, 16, d ** -0.5, None, None, None, None, None)
+    assert float((out.double() - exact).abs().max()) <= 2 * 6 * 16 * (d / 4 + 16) * UNIT
