@@ -886,6 +886,41 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     }
 }
 
+// Whether the kernel with one query tile per CTA finishes a plain causal step before the one with two, although that
+// would give every SM a CTA: with hardly more CTAs than SMs, the time is that of the CTA with the most keys, and a
+// CTA with two tiles takes 1.76 (heads of 64) or 1.5 (128) times as long for a key tile as one with one.  In units of one tile's
+// time for 128 keys, 1.5 for a CTA's start and end: the longer of the longest CTA and of all work spread over the SMs,
+// the columns of CTAs taken as so many of the longest sequence as the step has tokens for.  Two tiles' time over one
+// tile's, measured (estimated), 152 CTAs with two tiles: heads of 64, one prompt 1.63 (1.48), after 1,500 tokens 1.28
+// (1.17); of 128 1.40 (1.27) and 1.05 (1.00), four heads to a key head 1.16 (1.19) and 0.91 (0.89); 256 CTAs of the
+// first: 1.20 (0.93).  The estimate has to be 1.08.
+static bool one_tile_is_faster(long long rows, int group, int max_q_len, int max_ctx_len, long long tokens, int nkv,
+                               int window, int chunk, int sms)
+{
+    const double pair_cost = D == 64 ? 1.76 : 1.5, start = 1.5;
+    const long long tiles1 = (rows + ROWS - 1) / ROWS, tiles2 = (rows + 2 * ROWS - 1) / (2 * ROWS);
+    const double columns = (double)nkv * (tokens > 0 ? (double)tokens / max_q_len : 1.0);
+    int most = max_ctx_len;                       // keys that a row can see
+    if (window > 0 && window + ROWS / group < most)
+        most = window + ROWS / group;
+    if (chunk > 0 && chunk < most)
+        most = chunk;
+    auto keys = [&](long long rows_before) {      // key tiles of a CTA whose last row is number rows_before - 1
+        const long long seen = max_ctx_len - max_q_len + (rows_before < rows ? rows_before : rows) / group;
+        return (double)(((seen < most ? seen : most) + KEYS - 1) / KEYS);
+    };
+    const double longest = keys(rows);
+    if (longest < 4.0)
+        return false;                             // (four prompts of up to 300 tokens, four heads to a key head: 21.3 and 20.0 us)
+    double all1 = 0.0, all2 = 0.0;
+    for (long long i = 1; i <= tiles1; ++i)
+        all1 += keys(i * ROWS) + start;
+    for (long long i = 1; i <= tiles2; ++i)
+        all2 += keys(i * 2 * ROWS) * pair_cost + start;
+    const double t1 = fmax(longest + start, all1 * columns / sms), t2 = fmax(longest * pair_cost + start, all2 * columns / sms);
+    return t2 > 1.08 * t1;
+}
+
 } // namespace chibi
 
 using namespace chibi;
@@ -900,7 +935,7 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
                                          const int* block_table, int table_stride, const int* seq_rows,
                                          const int* q_start, const int* ctx_len, int seqs, int nq, int nkv,
                                          int page_size, int num_pages, float scale, int window, int chunk,
-                                         int skip_single, int max_q_len, int variant, int kv_splits,
+                                         int skip_single, int max_q_len, int max_ctx_len, int variant, int kv_splits,
                                          float* scratch, long long scratch_floats, long long tokens,
                                          float softcap, const float* bias_r1, const float* bias_r2,
                                          const float* sink, int* error, cudaStream_t stream)
@@ -969,7 +1004,11 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
     int sms = 148, device = 0;
     if (cudaGetDevice(&device) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (variant == 2 || (variant == 0 && ctas2 >= sms)) {
+    // (with max_ctx_len 0, not known, that is all the rule)
+    const bool two = ctas2 >= sms
+        && !(options == OPT_NONE && max_ctx_len > 0 && ctas2 < 2 * sms
+             && one_tile_is_faster(rows, p.group, max_q_len, max_ctx_len, tokens, nkv, window, chunk, sms));
+    if (variant == 2 || (variant == 0 && two)) {
         const dim3 grid2((unsigned)((rows + 2 * ROWS - 1) / (2 * ROWS)), nkv, seqs);
         launch(two_tiles[options], grid2, dim3(ATC2_THREADS), ATC2_SMEM, stream, mk, mv, p);
         return launch_status();

@@ -986,7 +986,7 @@ class CudaKernels:
             status = tc.chibi_attention_prefill_tc(
                 _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0),
                 _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv, page_size, k_cache.shape[0],
-                float(scale), int(window or 0), int(chunk), 1 if mode & 1 else 0, int(max_q_len),
+                float(scale), int(window or 0), int(chunk), 1 if mode & 1 else 0, int(max_q_len), int(max_ctx_len),
                 int(self.tcgen05_attention_variant), kv_splits, _ptr(part),
                 part.numel() if part is not None else 0, q.shape[0], float(softcap), _ptr(bias_r1), _ptr(bias_r2),
                 _ptr(sink), _ptr(self.error), self._stream())
