@@ -298,6 +298,30 @@ def test_attention_with_cap_bias_and_tied_values(kernels, dtype, H, G, d):
         close(cut_up, ref, tol, f"attention portions and single tokens cap {softcap} bias {bias}")
 
 
+@pytest.mark.parametrize("scores", ["far below the cap", "at the cap", "row by row"])
+@pytest.mark.parametrize("variant", [1, 2])
+@pytest.mark.parametrize("H,G,d", [(2, 2, 64), (4, 2, 128)])
+def test_a_cap_alone_gives_the_bits_of_a_cap_with_a_bias_of_zeros(kernels, H, G, d, variant, scores):
+    """Prompt attention on tcgen05 has an instantiation for a cap alone: the same operations, a bias of nothing left out."""
+    g = torch.Generator().manual_seed(d)
+    T, page_size, cap = 300, 16, 30.0
+    q, k = torch.randn(T, H, d, generator=g), torch.randn(T, G, d, generator=g).bfloat16()
+    q = q * {"far below the cap": torch.ones(T, 1, 1), "at the cap": torch.full((T, 1, 1), 25.0),
+             "row by row": torch.where(torch.arange(T) % 3 == 0, 25.0, 1.0)[:, None, None]}[scores]
+    q = q.bfloat16()
+    zeros = torch.zeros(H)
+    kernels.tcgen05_attention_variant = variant
+    try:
+        alone = run_attention(kernels, q, k, None, None, d ** -0.5, cap, "bfloat16", page_size, [(0, T)])
+        beside = run_attention(kernels, q, k, zeros, zeros, d ** -0.5, cap, "bfloat16", page_size, [(0, T)])
+    finally:
+        kernels.tcgen05_attention_variant = 0
+    assert torch.equal(alone, beside)
+    ref = plain.capped_distance_scores(q.double(), k.double(), zeros.double(), zeros.double(), d ** -0.5, cap)
+    # probabilities and outputs are rounded to bfloat16 (2^-9 of a value each, against values of a few units)
+    close(alone, ref, 2e-2, f"cap alone, scores {scores}")
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_attention_finds_a_far_key(kernels, dtype):
     """One key, hundreds of positions back and next to a page border, is made to stand
