@@ -708,7 +708,8 @@ chunk_recurrence_kernel(const RecurrenceParams p)
     float* st = p.state + ((size_t)p.slots[seq] * p.heads + h) * d * e;
     auto place = [&](int r, int c) { return RULE == GENERAL ? (size_t)c * d + r : (size_t)r * e + c; };
     uint64_t S[RT / 2][CT];
-    // (the state is what an earlier step left: fetched before the kernel ahead is through)
+    // (before the wait: the kernel ahead is this call's preparing kernel, which does not write the state and does not let
+    // this one in before its own end, when all that ran before it has ended too)
 #pragma unroll
     for (int i = 0; i < RT / 2; ++i) {
         const int r = r0 + RUN_STEP * (i / 2) + 2 * (i % 2);
@@ -920,16 +921,17 @@ recurrence_tokens_kernel(const RecurrenceParams p)
         return;
     const int col = blockIdx.x * 32 + lane, r0 = warp * R;
     float* st = p.state + ((size_t)p.slots[seq] * p.heads + h) * d * e;
+#ifndef CHIBI_TIMELINE
+    if (lane < R && r0 + lane < d)                      // (only asked for: who wrote it last may be the kernel ahead)
+        prefetch_l2(st + (size_t)(r0 + lane) * e + blockIdx.x * 32);
+    pdl_wait();
+#endif
     float S[R];
-    // (the state is what an earlier step left: fetched before the kernel ahead is through)
 #pragma unroll
     for (int i = 0; i < R; ++i)
         S[i] = (col < e && r0 + i < d) ? st[(size_t)(r0 + i) * e + col] : 0.f;
     const float rate = RULE == DELTA ? -expf(p.a_log[h]) : 0.f;
     const float decay = RULE == DELTA ? 1.f : p.decay[h];
-#ifndef CHIBI_TIMELINE
-    pdl_wait();
-#endif
     for (int t = 0; t < len; ++t) {
         const size_t row = (size_t)(row0 + t);
         const TX* q = static_cast<const TX*>(p.q) + row * p.stride + kh * d;
@@ -1007,7 +1009,8 @@ recurrence_tokens_kernel(const RecurrenceParams p)
 // The same for heads of at most 128 key rows, where a lane can hold its column's rows by itself: a warp owns 32
 // value columns, nothing is added up across lanes or warps and there is no block barrier.  Bound by the state's way
 // from memory and back, R lines of 128 bytes of a warp in flight together (64 sequences of 16 heads of
-// 128 x 128: 31.2 us, 47.6 with the kernel above, whose eight warps of 16 rows wait for one another at every token).
+// 128 x 128, states that L2 does not hold: 37.5 us, 57.4 with the kernel above, whose eight warps of 16 rows wait for one
+// another at every token).
 template <int R, int RULE, typename TX>
 __global__ void __launch_bounds__(32)
 recurrence_columns_kernel(const RecurrenceParams p)
@@ -1128,8 +1131,9 @@ recurrence_columns_kernel(const RecurrenceParams p)
 // The generalised delta rule, whose state lies value column first: a warp owns CW neighbouring columns, a lane R key
 // rows of each (runs of up to four), and a token's sums over the rows are folded over the lanes for all columns
 // together.  With the removals' p = x^T S, o = r^T (g S) - (r . a x) p + (r . k) v needs no second fold.  Two warps to a
-// block, no shared memory: bound by the state's way from memory and back (64 sequences of 32 heads of 64 x 64
-// 14.6 us; 118 before, in a kernel whose eight producer warps and chunk buffers served one token).
+// block, no shared memory: bound by the state's way from memory and back (64 sequences of 32 heads of 64 x 64,
+// states that L2 does not hold: 19.6 us; 119.8 before, in a kernel whose eight producer warps and chunk buffers served one
+// token).
 template <int R, int CW, typename TX>
 __global__ void __launch_bounds__(64)
 general_tokens_kernel(const RecurrenceParams p)
@@ -1332,8 +1336,8 @@ static void launch_tokens(const RecurrenceParams& p, int seqs, cudaStream_t stre
     } else {
     const dim3 grid((unsigned)((p.e + 31) / 32), (unsigned)p.heads, (unsigned)seqs);
     // Whole columns to a lane where that fills the SMs with four warps each; with fewer, eight warps share the rows (one
-    // token of a sequence, heads of 128: 1 sequence of 16 heads 2.9 us and 6.9 with whole columns, 8 sequences
-    // of 16 heads, 512 warps, 7.2 and 8.0, of 32 heads 12.6 and 8.5, 64 of 16 heads 47.6 and 31.2).
+    // token of a sequence, heads of 128: 1 sequence of 16 heads 3.1 us and 6.6 with whole columns, 8 sequences
+    // of 16 heads, 512 warps, 6.7 and 7.8, of 32 heads 12.3 and 8.2, 64 of 16 heads 57.4 and 37.5).
     const bool whole = (long long)grid.x * grid.y * grid.z >= 4LL * recurrence_sm_count();
     if (whole && p.d <= 32)
         launch(recurrence_columns_kernel<32, RULE, TX>, grid, dim3(32), 0, stream, p);

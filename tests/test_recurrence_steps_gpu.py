@@ -57,3 +57,43 @@ def test_many_sequences_equal_single_ones(k, rule, dtype, heads, d, e):
     assert float((o1 - o2).abs().max()) <= (d / 2 + 16) * 2.0 ** -24 * 4 * scale
     assert float((one - many).abs().max()) <= (d / 2 + 16) * 2.0 ** -24 * 4 * float(one.abs().max())
     assert torch.equal(many[seqs], first[seqs])
+
+
+# heads: whole columns to a lane from 592 warps on, rows over warps below; d 200 has rows beyond 128
+@pytest.mark.parametrize("seqs,d", [(1, 64), (1, 128), (1, 200), (8, 64), (8, 128), (8, 200), (200, 64)])
+@pytest.mark.parametrize("rule", ["delta", "decayed", "general", "state space"])
+def test_steps_without_a_wait_between_them_go_on_from_each_other(k, rule, seqs, d):
+    """Each call finds the state that the one before it left, though the kernels start before that one has ended."""
+    heads, steps = 2, 24
+    g = torch.Generator(device=DEV).manual_seed(seqs + d)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x, logits, beta = rnd(steps, seqs, 5 * heads * d + 8), rnd(steps, seqs, heads * d), rnd(steps, seqs, heads)
+    a_log, bias, removal = rnd(heads), rnd(heads * d), rnd(heads * d)
+    decay = torch.rand(heads, generator=g, device=DEV)
+    starts, slots = ints(list(range(seqs + 1))), ints(list(range(seqs)))
+    first = rnd(seqs, heads, d, d)
+
+    def run(wait):
+        state, out = first.clone(), torch.full((steps, seqs, heads * d), float("nan"), device=DEV)
+        torch.cuda.synchronize()
+        for t in range(steps):
+            if rule == "delta":
+                k.channel_delta(x[t][:, :3 * heads * d], logits[t], beta[t], a_log, bias, state, out[t], starts, slots, heads,
+                                heads, d, d, 1e-6, d ** -0.5, 1)
+            elif rule == "decayed":
+                k.decayed_attention(x[t][:, :3 * heads * d], decay, state, out[t], starts, slots, heads, d, d, 1)
+            elif rule == "general":
+                k.delta_rule(x[t], logits[t], bias, removal, state, out[t], starts, slots, heads, d, 8, 0.6, 1e-6, 1)
+            else:
+                k.state_space_scan(x[t][:, :3 * heads * d], beta[t], a_log, a_log, a_log, state, out[t], starts, slots, heads,
+                                   heads, d, d)
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return state, out
+
+    state, out = run(True)
+    assert torch.isfinite(out).all()
+    for _ in range(3):
+        again = run(False)
+        assert torch.equal(again[0], state) and torch.equal(again[1], out)
