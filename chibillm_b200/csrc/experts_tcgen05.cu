@@ -163,7 +163,7 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         for (int it = 0; tile_at(it, expert, row0, n0); ++it) {
             const uint32_t buf = it & 1, use = it >> 1;
-            if (!mbar_wait(&tmem_full_bar[buf], use & 1, p.error, 33))
+            if (!mbar_wait_warp(&tmem_full_bar[buf], use & 1, p.error, 33))
                 break;
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + buf * XT_N + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -333,7 +333,7 @@ expert_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
     } else {
         const int quarter = warp & 3, n = n0 + quarter * 32 + lane;
-        const bool ok = mbar_wait(tmem_full_bar, 0, p.error, 33);
+        const bool ok = mbar_wait_warp(tmem_full_bar, 0, p.error, 33);
         tcgen05_fence_after();
 #pragma unroll 1
         for (int c0 = 0; ok && c0 < row_end - row0; c0 += 16) {

@@ -233,7 +233,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
         bool ok = true;
         pdl_wait();        // before this warp reads or writes global memory
         if (kb_count > 0)
-            ok = mbar_wait(tmem_full_bar, 0, p.error, 13);
+            ok = mbar_wait_warp(tmem_full_bar, 0, p.error, 13);
         tcgen05_fence_after();
         timeline_mark(0);              // the accumulator is complete
         constexpr int CHUNK = BN < 32 ? 16 : 32;
@@ -898,7 +898,7 @@ __device__ __forceinline__ void collect_partial_tiles(const GemmParams& p, uint3
                 fetch(i + 2);
             }
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(&bars[i % 3], (i / 3) & 1, p.error, 16)))
+        if (!mbar_wait_warp(&bars[i % 3], (i / 3) & 1, p.error, 16))
             return;                              // (the whole warp: what follows is warp-wide)
         const float4* src = reinterpret_cast<const float4*>(buffers + (i % 3) * BYTES) + lane;
         const uint32_t col0 = (i & 1) * 128;
@@ -1219,7 +1219,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             int tile_a, tile_b;
             tile_of<TILE_BAND / 2>(t, tiles_m, tiles_total, tile_a, tile_b);   // bands of 2,048 rows here too
             const uint32_t buf = lt & 1, use = lt >> 1;
-            if (!mbar_wait(&tmem_full_bar[buf], use & 1, p.error, 19))
+            if (!mbar_wait_warp(&tmem_full_bar[buf], use & 1, p.error, 19))
                 break;
             tcgen05_fence_after();
             const uint32_t taddr = tmem_base + buf * BN + (static_cast<uint32_t>(quarter * 32) << 16);

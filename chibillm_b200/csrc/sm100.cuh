@@ -92,6 +92,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
     return true;
 }
 
+// The same for a whole warp whose lanes decide by the outcome: every lane counts its own clock, so near the limit some
+// lanes may see the phase end and others give up.  One lane that gave up counts for all; the warp goes on, or leaves,
+// together, and what follows may be warp-wide (tcgen05.ld, shuffles).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* error, int code)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, error, code));
+}
+
 // ------------------------------------------------------------------ clusters
 __device__ __forceinline__ uint32_t cluster_cta_rank()
 {
