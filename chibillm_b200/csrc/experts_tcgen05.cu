@@ -15,15 +15,17 @@
 // issues tcgen05.mma (128 x 256 x 16) into one of two TMEM accumulators, and eight warps
 // read the other back with tcgen05.ld.  Bound by what an SM can take in (48 KB to 128 x 256 x 64
 // multiply-adds) and by the epilogue: a CTA a tile of 128 x 128, which this replaces, wanted 64 KB for as many
-// and began and ended each tile by itself, and with four epilogue warps the gate bounds the tiles (2,048 tokens, two
-// of eight experts of 2,048 x 3,072, the whole feed-forward: 232 us before, 221 with four warps, 173 now; of
-// 4,096 x 6,144 882 -> 704).  Rows past the expert's last row are computed (they are the next expert's rows,
+// and began and ended each tile by itself, and with four epilogue warps the gate bounds the tiles (the whole
+// feed-forward, two of eight experts a token, three sets of weights in turn, more than L2 holds: 2,048 tokens of
+// 2,048 x 3,072 231 us before, 176 now, of 4,096 x 6,144 770 -> 650; with weights that L2 holds 232 before, 221 with four
+// warps, 176 with eight).  The gate is made with CUDA's exact exponential and division, 1.6 % of the first of these.
+// Rows past the expert's last row are computed (they are the next expert's rows,
 // or zeros past the array's end) and not written.
 //
 // Few tokens: an expert has few rows and the weights' way from memory bounds the products.  The
 // operands are swapped: a CTA takes 128 weight rows as the instruction's rows and the tile's rows, 16, 32 or
 // 64 at a time, as its columns, so that beside 16 KB of weights a stage brings 2 to 8 KB of rows
-// instead of 16 (8 tokens, the same experts: 121 -> 60.5 us).
+// instead of 16 (8 tokens, the same experts: 109 -> 58.4 us).
 //
 // Warp roles: warp 0 loads, warp 1 owns TMEM and issues, the others are the
 // epilogue (warp w reads TMEM lanes 32 * (w % 4) ..).  Every wait has a limit; a wait that
@@ -185,8 +187,8 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
                     __nv_bfloat162 h[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        h[j] = __floats2bfloat162_rn(activate_rounded(__uint_as_float(v[2 * j]), p.kind),
-                                                     activate_rounded(__uint_as_float(v[2 * j + 1]), p.kind));
+                        h[j] = __floats2bfloat162_rn(activate(__uint_as_float(v[2 * j]), p.kind),
+                                                     activate(__uint_as_float(v[2 * j + 1]), p.kind));
                     if (n0 + c0 + 32 <= p.rows_w && p.out_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
@@ -209,8 +211,8 @@ expert_rows_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         h[j] = __floats2bfloat162_rn(
-                            activate_rounded(wr * __uint_as_float(v[2 * j]), p.kind) * (wr * __uint_as_float(v[16 + 2 * j])),
-                            activate_rounded(wr * __uint_as_float(v[2 * j + 1]), p.kind) * (wr * __uint_as_float(v[16 + 2 * j + 1])));
+                            activate(wr * __uint_as_float(v[2 * j]), p.kind) * (wr * __uint_as_float(v[16 + 2 * j])),
+                            activate(wr * __uint_as_float(v[2 * j + 1]), p.kind) * (wr * __uint_as_float(v[16 + 2 * j + 1])));
                     if (p.out_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
                         reinterpret_cast<uint4*>(dst)[0] = reinterpret_cast<uint4*>(h)[0];
                         reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<uint4*>(h)[1];
@@ -353,7 +355,7 @@ expert_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         const float wr = p.row_weight ? p.row_weight[p.pair_of_row[r]] : 1.f;
                         const float gate = upper ? other : mine, up = upper ? mine : other;
                         static_cast<__nv_bfloat16*>(p.out)[(size_t)r * p.out_stride + f] =
-                            __float2bfloat16_rn(activate_rounded(wr * gate, p.kind) * (wr * up));
+                            __float2bfloat16_rn(activate(wr * gate, p.kind) * (wr * up));
                     }
                 }
             } else if (n < p.rows_w) {
@@ -363,7 +365,7 @@ expert_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     if (r < row_end) {
                         if (MODE == 2)
                             static_cast<__nv_bfloat16*>(p.out)[(size_t)r * p.out_stride + n] =
-                                __float2bfloat16_rn(activate_rounded(__uint_as_float(v[c]), p.kind));
+                                __float2bfloat16_rn(activate(__uint_as_float(v[c]), p.kind));
                         else
                             static_cast<float*>(p.out)[(size_t)r * p.out_stride + n] = __uint_as_float(v[c]);
                     }
@@ -429,7 +431,7 @@ static int launch_expert_rows(const void* a, const void* w, long long pairs, int
     if (tokens <= 32)
         return launch_expert_few<MODE, 32>(a, w, pairs, experts, K, p, stream);
     // Few columns as long as an expert's rows mostly fit 64 of them: 128 tokens of 8 experts of 1,024 x 1,536, two a
-    // token, 29.5 us, 37.4 in tiles; 300 tokens (128 columns) 41.4, 40.9 in tiles.
+    // token, weights that L2 holds, 29.5 us, 37.4 in tiles; 300 tokens (128 columns) 41.4, 40.9 in tiles.
     if (tokens <= 64 || pairs <= 32LL * experts)
         return launch_expert_few<MODE, 64>(a, w, pairs, experts, K, p, stream);
     // (as many tiles as the pairs make if they spread over the experts)  Narrow ones where they leave no SM a second.

@@ -50,3 +50,27 @@ def test_chosen_experts_tiles(k, D, F, T, E, top, same, weight_on_input):
         size += w * torch.einsum("tf,tdf->td", act.abs(), down.double()[e].abs())
     # the activations become bfloat16 (half a unit of 2^-8) and the sums are 32-bit
     assert ((out.double() - ref).abs() <= (2.0 ** -9 * 1.1 + 1e-5) * size + 1e-6).all()
+
+
+@pytest.mark.parametrize("T", [16, 64, 300])             # 16 and 64 columns, tiles of 128 rows
+def test_the_gate_is_made_in_32_bits(k, T):
+    """Products of one term each, so that the epilogue's arithmetic is all there is: the gate far into its tail too, where
+    1 + exp(-z) is near the largest 32-bit number."""
+    D = F = 64
+    x = torch.eye(D, dtype=torch.bfloat16, device=DEV)[torch.arange(T, device=DEV) % D].contiguous()
+    gate = torch.linspace(-88.0, 20.0, F * D, device=DEV).view(1, F, D).bfloat16()
+    g = torch.Generator(device=DEV).manual_seed(1)
+    up = (torch.randn(1, F, D, generator=g, device=DEV) * 2.0 ** 30).bfloat16()
+    down = torch.eye(F, dtype=torch.bfloat16, device=DEV)[None].contiguous()
+    out = torch.full((T, D), float("nan"), device=DEV)
+    k.chosen_experts(x, torch.zeros(T, 1, dtype=torch.int32, device=DEV), torch.ones(T, 1, device=DEV),
+                     k.interleave_expert_gate_up(gate[0], up[0])[None].contiguous(), down, out,
+                     torch.empty(k.route_words(T, 1), dtype=torch.int32, device=DEV),
+                     torch.empty(T, F, dtype=torch.bfloat16, device=DEV), torch.empty(T, D, device=DEV), "silu",
+                     torch.empty(T, D, dtype=torch.bfloat16, device=DEV), gated=True, interleaved=True, overwrite=True)
+    k.check_error_word()
+    z, u = gate[0].double().t()[torch.arange(T, device=DEV) % D], up[0].double().t()[torch.arange(T, device=DEV) % D]
+    ref = z * torch.sigmoid(z) * u
+    # the rounding to bfloat16 (half a unit of the 8th significant bit: 2^-8 of a value at most) after an exponential of two
+    # units in the last place, a sum, a division and a product (each half a unit of 2^-23)
+    assert ((out.double() - ref).abs() <= (2.0 ** -8 + 8 * 2.0 ** -24) * ref.abs()).all()
