@@ -264,7 +264,7 @@ differential_combine_kernel(const float* __restrict__ att, const TX* __restrict_
 // shared-memory loads of one another.
 constexpr int SSM_CHUNK = 16;
 constexpr int SSM_CW = 2;                               // columns of a warp
-constexpr int SSM_FEW = 4;                              // tokens a sequence, on average, up to which they go one by one
+constexpr int SSM_FEW = 4;                              // tokens of a sequence up to which they go one by one (SCAN_FEW_TOKENS)
 
 // The state row that lane l holds as its i-th: runs of four rows to a lane where a lane has four or more
 // (one 16-byte load of B and of C serves four multiply-adds), else row 32 i + l.
@@ -280,7 +280,7 @@ state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const 
                         long long dt_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                         const float* __restrict__ skip, float* state, float* __restrict__ y,
                         const int* __restrict__ q_start, const int* __restrict__ slots, int heads, int groups, int e,
-                        int N)
+                        int N, int at_least)
 {
     pdl_enter();
     constexpr int THREADS = 32 * COLS / SSM_CW;
@@ -297,7 +297,7 @@ state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const 
     const int col = blockIdx.x * COLS + col_local;      // the warp's first column
     const int row0 = q_start[seq];
     const int q_len = q_start[seq + 1] - row0;
-    if (q_len <= 0)
+    if (q_len < at_least)
         return;
     float* S = state + (((size_t)slots[seq] * heads + h) * e) * N;
     float s[SSM_CW][R];
@@ -440,18 +440,18 @@ state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const 
     }
 }
 
-// The same for steps of about one token a sequence: bound by the state's way from memory and back, so a warp holds
+// The same for sequences of few tokens: bound by the state's way from memory and back, so a warp holds
 // 8 columns (4 of states above 128 rows, 2 above 256) of state rows in 16-byte pieces and nothing goes
 // through shared memory: a lane reads its own rows of a token's B and C, and the columns' sums over the lanes are folded
-// together.  64 sequences of 32 heads of 64 x 128: 77 us with the kernel above (whose block stages a chunk of
-// 16 tokens, of which there is one, behind two barriers).
+// together.  64 sequences of 32 heads of 64 x 128, states that L2 does not hold: 26.9 us, 76.6 with the kernel above (whose
+// block stages a chunk of 16 tokens, of which there is one, behind two barriers).
 template <typename TX, int R>
 __global__ void __launch_bounds__(64)
 state_space_token_kernel(const TX* __restrict__ xbc, long long xbc_stride, const TX* __restrict__ dt_raw,
                          long long dt_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                          const float* __restrict__ skip, float* state, float* __restrict__ y,
                          const int* __restrict__ q_start, const int* __restrict__ slots, int heads, int groups, int e,
-                         int N)
+                         int N, int at_most)
 {
     pdl_enter();
     constexpr int CW = R <= 4 ? 8 : R == 8 ? 4 : 2;     // columns of a warp
@@ -459,7 +459,7 @@ state_space_token_kernel(const TX* __restrict__ xbc, long long xbc_stride, const
     const int g = h / (heads / groups), inner = heads * e;
     const int col = (blockIdx.x * 2 + (threadIdx.x >> 5)) * CW;
     const int row0 = q_start[seq], row1 = q_start[seq + 1];
-    if (row1 <= row0 || col >= e)
+    if (row1 <= row0 || row1 - row0 > at_most || col >= e)
         return;
     float* const S = state + (((size_t)slots[seq] * heads + h) * e + col) * N;
     const bool wide = R >= 4 && N % 4 == 0;             // a lane's runs of four rows are whole and aligned
@@ -887,60 +887,68 @@ CHIBI_API int chibi_differential_combine(const float* att, const void* gate, int
     return launch_status();
 }
 
+struct ScanArgs {
+    const void* xbc;
+    long long xbc_stride;
+    const void* dt_raw;
+    long long dt_stride;
+    const float *dt_bias, *a_log, *skip;
+    float *state, *y;
+    const int *q_start, *slots;
+    int heads, groups, e, N;
+};
+
 template <typename TX, int R, int COLS>
-static void launch_scan(int seqs, cudaStream_t stream, const void* xbc, long long xbc_stride,
-                        const void* dt_raw, long long dt_stride, const float* dt_bias, const float* a_log,
-                        const float* skip, float* state, float* y, const int* q_start, const int* slots, int heads,
-                        int groups, int e, int N)
+static void launch_scan(int seqs, cudaStream_t stream, const ScanArgs& a, int at_least)
 {
-    const dim3 grid((unsigned)((e + COLS - 1) / COLS), (unsigned)heads, (unsigned)seqs);
+    const dim3 grid((unsigned)((a.e + COLS - 1) / COLS), (unsigned)a.heads, (unsigned)seqs);
     const size_t smem = (size_t)2 * (2 * SSM_CHUNK * R * 32 + SSM_CHUNK * COLS + 2 * SSM_CHUNK) * sizeof(float);
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(state_space_scan_kernel<TX, R, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-    launch(state_space_scan_kernel<TX, R, COLS>, grid, dim3(32 * COLS / SSM_CW), smem, stream, (const TX*)xbc,
-           xbc_stride, (const TX*)dt_raw, dt_stride, dt_bias, a_log, skip, state, y, q_start, slots, heads, groups, e, N);
+    launch(state_space_scan_kernel<TX, R, COLS>, grid, dim3(32 * COLS / SSM_CW), smem, stream, (const TX*)a.xbc,
+           a.xbc_stride, (const TX*)a.dt_raw, a.dt_stride, a.dt_bias, a.a_log, a.skip, a.state, a.y, a.q_start, a.slots,
+           a.heads, a.groups, a.e, a.N, at_least);
 }
 
 template <typename TX, int R>
-static void launch_scan_tokens(int seqs, cudaStream_t stream, const void* xbc, long long xbc_stride, const void* dt_raw,
-                               long long dt_stride, const float* dt_bias, const float* a_log, const float* skip,
-                               float* state, float* y, const int* q_start, const int* slots, int heads, int groups, int e,
-                               int N)
+static void launch_scan_tokens(int seqs, cudaStream_t stream, const ScanArgs& a, int at_most)
 {
     constexpr int COLS = 2 * (R <= 4 ? 8 : R == 8 ? 4 : 2);
-    launch(state_space_token_kernel<TX, R>, dim3((unsigned)((e + COLS - 1) / COLS), (unsigned)heads, (unsigned)seqs), dim3(64),
-           0, stream, (const TX*)xbc, xbc_stride, (const TX*)dt_raw, dt_stride, dt_bias, a_log, skip, state, y, q_start,
-           slots, heads, groups, e, N);
+    launch(state_space_token_kernel<TX, R>, dim3((unsigned)((a.e + COLS - 1) / COLS), (unsigned)a.heads, (unsigned)seqs),
+           dim3(64), 0, stream, (const TX*)a.xbc, a.xbc_stride, (const TX*)a.dt_raw, a.dt_stride, a.dt_bias, a.a_log, a.skip,
+           a.state, a.y, a.q_start, a.slots, a.heads, a.groups, a.e, a.N, at_most);
 }
 
+// few: 0: the scan takes all sequences; 1: the kernel for few tokens takes all; 2: that one takes the sequences of up to SSM_FEW
+// tokens and the scan the others.  (The kernel for few tokens wants the state on 16 bytes.)
 CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_stride, const void* dt_raw,
                                      long long dt_stride, const float* dt_bias, const float* a_log, const float* skip,
                                      float* state, float* y, const int* q_start, const int* slots, long long tokens,
-                                     int seqs, int heads, int groups, int e, int N, cudaStream_t stream)
+                                     int seqs, int heads, int groups, int e, int N, int few, cudaStream_t stream)
 {
     if (seqs <= 0)
         return CHIBI_OK;
     if (!xbc || !dt_raw || !dt_bias || !a_log || !skip || !state || !y || heads <= 0 || groups <= 0
-        || heads % groups != 0 || e <= 0 || N <= 0)
+        || heads % groups != 0 || e <= 0 || N <= 0 || few < 0 || few > 2
+        || (few != 0 && (reinterpret_cast<uintptr_t>(state) & 15) != 0))
         return CHIBI_ERR_ARGUMENT;
     if (N > 16 * 32 || heads > 65535 || seqs > 65535)      // (two buffers of a chunk's B and C must fit shared memory)
         return CHIBI_ERR_UNSUPPORTED;
-    // (16-byte pieces of state rows; the state is an array of its own)
-    if (tokens <= SSM_FEW * (long long)seqs && (reinterpret_cast<uintptr_t>(state) & 15) == 0) {
-        const int rows = (N + 31) / 32;
-#define CHIBI_SCAN_TOKENS(RR)                                                                                        \
-    CHIBI_DISPATCH_TYPE(x_type, TX, {                                                                                \
-        launch_scan_tokens<TX, RR>(seqs, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip, state, y, \
-                                   q_start, slots, heads, groups, e, N);                                             \
-    })
+    const ScanArgs a = { xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip, state, y, q_start, slots, heads, groups, e, N };
+    const int rows = (N + 31) / 32;
+    if (few != 0) {
+        const int at_most = few == 1 ? 2147483647 : SSM_FEW;
+#define CHIBI_SCAN_TOKENS(RR) CHIBI_DISPATCH_TYPE(x_type, TX, { launch_scan_tokens<TX, RR>(seqs, stream, a, at_most); })
         if (rows <= 1) CHIBI_SCAN_TOKENS(1);
         else if (rows <= 2) CHIBI_SCAN_TOKENS(2);
         else if (rows <= 4) CHIBI_SCAN_TOKENS(4);
         else if (rows <= 8) CHIBI_SCAN_TOKENS(8);
         else CHIBI_SCAN_TOKENS(16);
 #undef CHIBI_SCAN_TOKENS
-        return launch_status();
+        const int status = launch_status();
+        if (few == 1 || status)
+            return status;
     }
     // blocks of 16 columns, or of 8 where those would leave SMs without a block
     static int sms = 0;
@@ -949,16 +957,15 @@ CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     }
-    const bool narrow = (long long)((e + 15) / 16) * heads * seqs < sms && e > 8;
-    const int rows = (N + 31) / 32;
-#define CHIBI_SCAN(RR)                                                                                       \
-    CHIBI_DISPATCH_TYPE(x_type, TX, {                                                                        \
-        if (narrow)                                                                                          \
-            launch_scan<TX, RR, 8>(seqs, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip,  \
-                                   state, y, q_start, slots, heads, groups, e, N);                          \
-        else                                                                                                 \
-            launch_scan<TX, RR, 16>(seqs, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip, \
-                                    state, y, q_start, slots, heads, groups, e, N);                         \
+    const int at_least = few == 2 ? SSM_FEW + 1 : 1;
+    const long long most = tokens / at_least < seqs ? tokens / at_least : seqs;      // sequences that can have so many
+    const bool narrow = (long long)((e + 15) / 16) * heads * most < sms && e > 8;
+#define CHIBI_SCAN(RR)                                             \
+    CHIBI_DISPATCH_TYPE(x_type, TX, {                              \
+        if (narrow)                                                \
+            launch_scan<TX, RR, 8>(seqs, stream, a, at_least);     \
+        else                                                       \
+            launch_scan<TX, RR, 16>(seqs, stream, a, at_least);    \
     })
     if (rows <= 1) CHIBI_SCAN(1);
     else if (rows <= 2) CHIBI_SCAN(2);
@@ -966,10 +973,7 @@ CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_
     else if (rows <= 8) CHIBI_SCAN(8);
     else {
         // larger states: blocks of 8 columns only (256 threads leave a thread the registers for its rows)
-        CHIBI_DISPATCH_TYPE(x_type, TX, {
-            launch_scan<TX, 16, 8>(seqs, stream, xbc, xbc_stride, dt_raw, dt_stride, dt_bias, a_log, skip, state, y,
-                                   q_start, slots, heads, groups, e, N);
-        });
+        CHIBI_DISPATCH_TYPE(x_type, TX, { launch_scan<TX, 16, 8>(seqs, stream, a, at_least); });
     }
 #undef CHIBI_SCAN
     return launch_status();

@@ -89,7 +89,7 @@ _SIGNATURES = {
         "chibi_latent_heads_append": [P, I, L, I, L, P, P, I, P, F, P, I, I, I, P, P, P, P, P, L, I, I, L, P, P],
         "chibi_head_gate": [P, I, P, L, I, I, P],
         "chibi_differential_combine": [P, P, I, L, F, F, F, P, L, I, I, I, P],
-        "chibi_state_space_scan": [P, I, L, P, L, P, P, P, P, P, P, P, L, I, I, I, I, I, P],
+        "chibi_state_space_scan": [P, I, L, P, L, P, P, P, P, P, P, P, L, I, I, I, I, I, I, P],
         "chibi_gated_group_rms": [P, P, I, L, P, F, P, L, I, I, P],
         "chibi_clamped_swish_gate": [P, I, L, P, L, I, F, F, P],
         "chibi_router_choose": [P, L, P, P, P, L, I, I, I, I, F, I, I, P],

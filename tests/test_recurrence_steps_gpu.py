@@ -97,3 +97,38 @@ def test_steps_without_a_wait_between_them_go_on_from_each_other(k, rule, seqs, 
     for _ in range(3):
         again = run(False)
         assert torch.equal(again[0], state) and torch.equal(again[1], out)
+
+
+# lengths: single tokens only (the kernel for few tokens), single tokens beside a prompt's portion (each kernel its own, the
+# scan's at the edges of four tokens and of its chunks of 16), more than four tokens a sequence on average (the scan)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,launches", [([1] * 20, 1), ([1, 4, 1], 1), ([1] * 63 + [190], 2), ([1, 5, 4, 1], 2), ([3, 16, 1, 1, 1, 2], 2),
+                                           ([1] * 4 + [33] + [1] * 8, 2), ([1, 1, 1, 40], 1), ([5, 5, 5], 1)])
+@pytest.mark.parametrize("heads,e,n", [(2, 64, 128), (3, 10, 5), (2, 24, 300)])
+def test_a_long_sequence_beside_single_tokens(k, heads, e, n, lens, launches, dtype):
+    """A sequence's scan does not go token by token because the others bring one token each, and it gives what it gives alone."""
+    g = torch.Generator(device=DEV).manual_seed(len(lens) + n)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    starts = [0]
+    for m in lens:
+        starts.append(starts[-1] + m)
+    T, S = starts[-1], len(lens)
+    xbc, dt = (rnd(T, heads * e + 2 * n) * 0.5).to(dtype), rnd(T, heads).to(dtype)
+    dt_bias, a_log, skip, first = rnd(heads) - 1, rnd(heads), rnd(heads), rnd(S + 1, heads, e, n)
+    slots = [(3 * i) % S if S % 3 else i for i in range(S)]
+
+    def run(state, y, a, b):
+        k.state_space_scan(xbc[starts[a]:starts[b]], dt[starts[a]:starts[b]], dt_bias, a_log, skip, state, y[starts[a]:starts[b]],
+                           ints([s - starts[a] for s in starts[a:b + 1]]), ints(slots[a:b]), heads, 1, e, n)
+
+    many, one = first.clone(), first.clone()
+    y1, y2 = (torch.full((T, heads * e), float("nan"), device=DEV) for _ in range(2))
+    before = k.launches
+    run(many, y2, 0, S)
+    assert k.launches - before == launches
+    for i in range(S):
+        run(one, y1, i, i + 1)
+    # the same multiply-adds; a sum over the n rows in another order is n roundings of its magnitudes at most
+    bound = lambda a: (n + 16) * 2.0 ** -24 * float(a.abs().max())
+    assert float((y1 - y2).abs().max()) <= bound(y1) and float((one - many).abs().max()) <= bound(one)
+    assert torch.equal(many[S], first[S])
