@@ -876,7 +876,7 @@ class CudaKernels:
                                 chunk, sink)
             return
         if not special and q.dtype == torch.float32 and k_cache.dtype == torch.float32 and v_cache.dtype == torch.float32 \
-                and d in (64, 128):
+                and d in self.FLOAT32_HEAD_DIMS:
             # the 32-bit path's usual head sizes (tiles of query rows for prompts, ranges of keys for single tokens)
             status = self.lib.chibi_attention_f32(
                 _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0), _ptr(q_start),
@@ -914,6 +914,8 @@ class CudaKernels:
             nq, nkv, int(kv_share), page_size, k_cache.shape[0], float(scale), int(window or 0), int(chunk),
             int(max_q_len), float(softcap), _ptr(bias_r1), _ptr(bias_r2), _ptr(sink), _ptr(self.error),
             self._stream()), "attention (tensor cores, prompt)")
+
+    FLOAT32_HEAD_DIMS = (64, 128)       # head sizes that the 32-bit attention kernels take
 
     @staticmethod
     def float32_token_ranks(max_ctx_len: int) -> int:

@@ -249,7 +249,8 @@ class PagedAttention(Mixer):
         if splits is None:
             return None
         s = self.spec
-        return (splits(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) + self.runtime.float32_launch_key(ctx)
+        return (splits(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) \
+            + (self.runtime.float32_launch_key(ctx, s.head_dim) if self.value_dim == s.head_dim else ())
 
     # ---- run
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, overwrite: bool = False, hold: bool = False):

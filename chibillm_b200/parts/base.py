@@ -30,10 +30,12 @@ class Runtime:
     def is_float32(self) -> bool:
         return self.dtype == torch.float32
 
-    def float32_launch_key(self, ctx) -> tuple:
-        """What a captured step of the 32-bit attention kernels depends on besides its data."""
+    def float32_launch_key(self, ctx, head_dim: int) -> tuple:
+        """What a captured step of 32-bit attention over heads of this size depends on besides its data."""
         ranks = getattr(self.kernels, "float32_token_ranks", None)
-        return (ranks(ctx.max_ctx_len),) if self.is_float32 and ranks is not None else ()
+        if not self.is_float32 or ranks is None or head_dim not in self.kernels.FLOAT32_HEAD_DIMS:
+            return ()                # (the plain kernel decides nothing on the host)
+        return (ranks(ctx.max_ctx_len),)
 
 
 # ------------------------------------------------------------------ tensors

@@ -129,7 +129,8 @@ class LatentAttention(Mixer):
         splits = getattr(self.runtime.kernels, "decode_attention_splits", None)
         if splits is None:
             return None
-        return (splits(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),) + self.runtime.float32_launch_key(ctx)
+        return (splits(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),) \
+            + self.runtime.float32_launch_key(ctx, self.key_dim)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, hold: bool = False):
         s, rt = self.spec, self.runtime
