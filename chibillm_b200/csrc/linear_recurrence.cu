@@ -1289,34 +1289,47 @@ static inline int recurrence_sm_count()
     return sms;
 }
 
+// Always asked for: what a block may have by itself counts its kernel's own arrays too (6 KB of the preparing kernel's, and
+// in a timeline build a word of the record), so that a dynamic part below 48 KB may still be refused.
+template <typename KERNEL>
+static int allow_shared(KERNEL kernel, size_t smem)
+{
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        cudaGetLastError();                             // (said here, not by the next launch)
+    return (int)e;
+}
+
 template <int DP, int RT, int CT, int COLS, int RULE, typename TX>
-static void launch_chunks(const RecurrenceParams& p, int seqs, cudaStream_t stream)
+static int launch_chunks(const RecurrenceParams& p, int seqs, cudaStream_t stream)
 {
     const size_t smem = (size_t)(2 * rc_block(DP, RULE) + (RULE == GENERAL ? 2 : 1) * RC * (COLS + 4)) * sizeof(float);
     auto kernel = chunk_recurrence_kernel<DP, RT, CT, COLS, RULE, TX>;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (const int e = allow_shared(kernel, smem))
+        return e;
     launch(kernel, dim3((unsigned)((p.e + COLS - 1) / COLS), (unsigned)p.heads, (unsigned)seqs),
            dim3((DP / RT) * (COLS / CT)), smem, stream, p);
+    return launch_status();
 }
 
 template <int DP, int RULE, typename TX>
-static void launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cudaStream_t stream)
+static int launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cudaStream_t stream)
 {
     const size_t smem = (size_t)(RULE == GENERAL ? 5 * RC + 4 : RULE == DELTA ? 3 * RC + 4 : 2 * RC) * DP * sizeof(float);
     auto prepare = RULE == GENERAL ? general_prepare_kernel<DP, TX> : recurrence_prepare_kernel<DP, RULE == GENERAL ? DELTA : RULE, TX>;
-    if (smem > 44 * 1024)
-        cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (const int e = allow_shared(prepare, smem))
+        return e;
     launch(prepare, dim3((unsigned)((max_q_len + RC - 1) / RC), (unsigned)p.heads, (unsigned)seqs), dim3(256), smem, stream, p);
+    if (const int e = launch_status())
+        return e;
     // as few columns a block as give every SM one block and no more, and the fewer the smaller a thread's piece
     constexpr int RT = DP >= 128 ? 8 : 4;
     const long long per_head = (long long)p.heads * seqs, sms = recurrence_sm_count();
     if (((p.e + 7) / 8) * per_head <= sms)
-        launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, RULE, TX>(p, seqs, stream);
-    else if (((p.e + 15) / 16) * per_head <= sms)
-        launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, RULE, TX>(p, seqs, stream);
-    else
-        launch_chunks<DP, RT, 4, 32, RULE, TX>(p, seqs, stream);
+        return launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, RULE, TX>(p, seqs, stream);
+    if (((p.e + 15) / 16) * per_head <= sms)
+        return launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, RULE, TX>(p, seqs, stream);
+    return launch_chunks<DP, RT, 4, 32, RULE, TX>(p, seqs, stream);
 }
 
 template <int RULE, typename TX>
@@ -1374,15 +1387,14 @@ static int launch_recurrence(const RecurrenceParams& p, int x_type, long long sc
         return CHIBI_ERR_ARGUMENT;
     CHIBI_DISPATCH_TYPE(x_type, TX, {
         if (DP == 32)
-            launch_prompt<32, RULE, TX>(p, seqs, max_q_len, stream);
-        else if (DP == 64)
-            launch_prompt<64, RULE, TX>(p, seqs, max_q_len, stream);
-        else if (DP == 128)
-            launch_prompt<128, RULE, TX>(p, seqs, max_q_len, stream);
-        else
-            launch_prompt<256, RULE, TX>(p, seqs, max_q_len, stream);
+            return launch_prompt<32, RULE, TX>(p, seqs, max_q_len, stream);
+        if (DP == 64)
+            return launch_prompt<64, RULE, TX>(p, seqs, max_q_len, stream);
+        if (DP == 128)
+            return launch_prompt<128, RULE, TX>(p, seqs, max_q_len, stream);
+        return launch_prompt<256, RULE, TX>(p, seqs, max_q_len, stream);
     });
-    return launch_status();
+    return CHIBI_OK;
 }
 
 } // namespace chibi

@@ -38,3 +38,12 @@ def test_the_check_sees_a_lane_that_leaves_by_itself():
 def test_a_wait_that_runs_out_is_a_whole_warps(name):
     with open(os.path.join(CSRC, name)) as f:
         assert lone_waits(f.read()) == []
+
+
+def test_the_recurrences_ask_for_their_shared_memory_whatever_its_size():
+    """A block has 48 KB without asking, its kernel's own arrays among them (general_prepare_kernel's 6 KB beside 42 KB for heads of
+    128, and a word more in a timeline build): the dynamic part alone does not tell."""
+    with open(os.path.join(CSRC, "linear_recurrence.cu")) as f:
+        text = f.read()
+    assert not re.findall(r"if \(smem > [^)]*\)", text)
+    assert text.count("if (const int e = allow_shared(") == 2          # the preparing kernels and the chunk kernels
