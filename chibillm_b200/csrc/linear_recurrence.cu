@@ -337,7 +337,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
         float v = 0.f;
 #pragma unroll
         for (int s = 0; s < RC; ++s)
-            v = fmaf(Bs[t][s], Ms[s][j], v);
+            v = s <= t ? fmaf(Bs[t][s], Ms[s][j], v) : v;      // (later tokens' rows may hold no numbers)
         No[tid] = v;
         Mo[tid] = Ms[t][j];
     }
@@ -605,7 +605,7 @@ general_prepare_kernel(const RecurrenceParams p)
         float v = 0.f;
 #pragma unroll
         for (int s = 0; s < RC; ++s)
-            v = fmaf(-Ms[t][s], Ak[s][j], v);
+            v = s <= t ? fmaf(-Ms[t][s], Ak[s][j], v) : v;     // (later tokens' rows may hold no numbers)
         Ns[t][j] = v;
         Mo[tid] = v;
     }
@@ -615,7 +615,7 @@ general_prepare_kernel(const RecurrenceParams p)
         float v = Bk[t][j];
 #pragma unroll
         for (int s = 0; s < RC; ++s)
-            v = fmaf(Ba[t][s], Ns[s][j], v);
+            v = s <= t ? fmaf(Ba[t][s], Ns[s][j], v) : v;
         No[tid] = v;
     }
     // ---- W and Q, a channel to a thread
@@ -766,10 +766,19 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                 if (p.activate)
                     vt[i][j] = lr_silu<TX>(vt[i][j]);
             }
+        // A value that is no number would reach the tokens before it through N's zeros: a warp that has one is careful.
+        bool finite = true;
+#pragma unroll
+        for (int i = 0; i < VR; ++i)
+#pragma unroll
+            for (int j = 0; j < CT; ++j)
+                finite = finite && fabsf(vt[i][j]) < INFINITY;
+        const bool numbers = __all_sync(0xffffffffu, finite);
         if (c + 1 < chunks)
             fetch_v(base + RC);
-        // A S_0 + N V, folded: thread lr ends with values lr OWN .. of the [token][column] tile
-        auto product = [&](const float* A, const float* N, float (&acc)[SUMS]) {
+        // A S_0 + N V, folded: thread lr ends with values lr OWN .. of the [token][column] tile.  N is zero above the diagonal;
+        // `careful`: those products are left out.
+        auto sums = [&](const float* A, const float* N, float (&acc)[SUMS], const bool careful) {
 #pragma unroll
             for (int t = 0; t < RC; ++t) {
                 uint64_t pair[CT];
@@ -793,12 +802,19 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                     const float m = L <= RC || lr < RC ? N[t * RC + lr + L * i] : 0.f;
 #pragma unroll
                     for (int j = 0; j < CT; ++j)
-                        s[j] = fmaf(m, vt[i][j], s[j]);
+                        if (!careful || lr + L * i <= t)
+                            s[j] = fmaf(m, vt[i][j], s[j]);
                 }
 #pragma unroll
                 for (int j = 0; j < CT; ++j)
                     acc[CT * t + j] = s[j];
             }
+        };
+        auto product = [&](const float* A, const float* N, float (&acc)[SUMS]) {
+            if (__builtin_expect(numbers, 1))
+                sums(A, N, acc, false);
+            else
+                sums(A, N, acc, true);
 #pragma unroll
             for (int o = L / 2, half = SUMS / 2; o >= 1; o >>= 1, half >>= 1) {
                 const bool upper = (lr & o) != 0;

@@ -1,0 +1,76 @@
+"""The recurrences over prompts, chunk by chunk: what a chunk may not do to the tokens before, and which calls it takes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+RULES = ["delta", "decayed", "general"]
+
+
+@pytest.fixture(scope="module")
+def k():
+    from chibillm_b200.kernels.ops import CudaKernels
+    return CudaKernels(torch.device(DEV))
+
+
+def ints(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+class Step:
+    """A step's inputs, and its outputs and states under one of the three rules."""
+
+    def __init__(self, k, rule, lens, heads, d, dtype=torch.float32, seed=0):
+        self.k, self.rule, self.lens, self.heads, self.d = k, rule, lens, heads, d
+        g = torch.Generator(device=DEV).manual_seed(d + seed)
+        rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)
+        T, W = sum(lens), heads * d
+        # r | k | v | gate | removal | low of the generalised rule, of which the others take the first three as q | k | v
+        self.x, self.logits, self.beta = rnd(T, 5 * W + 8).to(dtype), rnd(T, W), rnd(T, heads).to(dtype)
+        self.a_log, self.bias, self.removal = rnd(heads), rnd(W), rnd(W)
+        self.decay = torch.rand(heads, generator=g, device=DEV)
+        self.first = rnd(len(lens), heads, d, d)
+        self.starts = [0]
+        for n in lens:
+            self.starts.append(self.starts[-1] + n)
+
+    def run(self, longest=None):
+        k, H, d, W = self.k, self.heads, self.d, self.heads * self.d
+        state, o = self.first.clone(), torch.full((self.x.shape[0], W), float("nan"), device=DEV)
+        q_start, slots, longest = ints(self.starts), ints(list(range(len(self.lens)))), longest or max(self.lens)
+        if self.rule == "delta":
+            k.channel_delta(self.x[:, :3 * W], self.logits, self.beta, self.a_log, self.bias, state, o, q_start, slots, H, H, d,
+                            d, 1e-6, d ** -0.5, longest)
+        elif self.rule == "decayed":
+            k.decayed_attention(self.x[:, :3 * W], self.decay, state, o, q_start, slots, H, d, d, longest)
+        else:
+            k.delta_rule(self.x, self.logits, self.bias, self.removal, state, o, q_start, slots, H, d, 8, 0.6, 1e-6, longest)
+        return o, state
+
+
+# the chunk kernel's cuts: 8, 16 and 32 columns a block, 8 to 32 threads along the rows
+@pytest.mark.parametrize("d,heads", [(20, 2), (20, 60), (64, 2), (64, 20), (64, 40), (128, 2), (128, 12), (128, 20), (200, 2), (200, 6),
+                                     (200, 12)])
+@pytest.mark.parametrize("rule", RULES)
+def test_what_is_no_number_reaches_later_tokens_only(k, rule, d, heads):
+    """One value, key, query, decay's logit or rate that is no number: the tokens before it, in its chunk of 16 and its tile of
+    four too, and the other heads keep their bits."""
+    step = Step(k, rule, [40], heads, d)
+    clean, _ = step.run()
+    assert torch.isfinite(clean).all()
+    W, h = heads * d, heads - 1
+    for at in (16, 21, 31):
+        for part, what in enumerate(["query", "key", "value", None, "rate", "logit"]):
+            if what is None or (rule != "general" and what == "rate") or (rule == "decayed" and what == "logit"):
+                continue
+            for bad in (float("nan"), float("inf")):
+                where = step.logits[at] if what == "logit" else step.x[at]
+                column = h * d + 3 + (0 if what == "logit" else part * W)
+                kept = where[column].clone()
+                where[column] = bad
+                o, _ = step.run()
+                where[column] = kept
+                assert torch.equal(o[:at], clean[:at]), f"{bad} as token {at}'s {what} reached an earlier token"
+                assert torch.equal(o[:, :h * d], clean[:, :h * d]), f"{bad} as token {at}'s {what} reached another head"
+                if what != "logit" and bad != bad:
+                    assert torch.isnan(o[at]).any()
