@@ -291,8 +291,10 @@ gemm_f32_tile_kernel(const F32Params p)
 // the rows of x beside them, which all lanes read at the same place: MT + NR reads of 16 bytes (four cycles
 // each) to 16 NR bytes of weights a lane, so more rows of x want more rows of weights to a lane to stay behind
 // memory.  The four warps of a CTA, and the CTAs of a cluster where the tiles of 32 NR rows are few, take
-// the parts in turn; a CTA that is alone with its tiles walks over several.  The first weights are asked
-// for before the wait for the kernel ahead.
+// the parts in turn; a CTA that is alone with its tiles walks over several.  The first weights are asked for in L2
+// before the wait for the kernel ahead, and read after it, because that kernel may be the one that writes them (fetched into
+// shared memory before the wait, one row of 4,096 x 1,024 / 1,024 x 3,072 / 151,936 x 1,024 takes 5.5, 5.8, 94.8 us; so 5.8,
+// 7.0, 103.6).
 template <int MT, int NR, int STAGES>
 __global__ void __launch_bounds__(128)
 gemm_f32_few_kernel(const F32Params p)
@@ -353,7 +355,13 @@ gemm_f32_few_kernel(const F32Params p)
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s)
             if (at.tile < p.tiles) {
-                fetch_w(at, s);
+                const int k = ((slot + at.part * slots) * part_blocks + at.block) * F32_KB;
+#pragma unroll
+                for (int j = 0; j < NR; ++j) {
+                    const int n = at.tile * ROWS + 32 * j + lane;
+                    if (n < p.N && k < p.K)
+                        prefetch_l2(p.w + (size_t)n * p.w_stride + k);
+                }
                 advance(at);
             }
     }
@@ -362,6 +370,7 @@ gemm_f32_few_kernel(const F32Params p)
 #pragma unroll
         for (int s = 0; s < STAGES - 1; ++s) {
             if (ahead.tile < p.tiles) {
+                fetch_w(ahead, s);
                 fetch_x(ahead, s);
                 advance(ahead);
             }
@@ -544,10 +553,10 @@ static int gemm_f32(const float* x, const float* w, float* out, const float* res
     p.part = (sixteenth + F32_KB - 1) / F32_KB * F32_KB;
     p.part = p.part < 128 ? 128 : p.part;
     p.parts = (K + p.part - 1) / p.part;
-    // Few rows to 48 (blocks of 16 above 8), to 128 where N is small: 4,096 x 1,024 / 1,024 x 3,072 take 6.6, 7.7 us with
+    // Few rows to 48 (blocks of 16 above 8), to 128 where N is small: 4,096 x 1,024 / 1,024 x 3,072 take 6.7, 8.1 us with
     // 4 rows, 30, 26 us with 48 (50 in tiles of 64 rows), 30, 26 with 64 (37, 43), 58, 44 with 128 (39, 53); the
     // kernel for all before this 150, 180 us from one row to 64.  From 5 rows on, where the weights'
-    // tiles fill the SMs (N >= 64 x 148), a lane takes two of their rows (151,936 x 1,024: 8 rows 155 -> 125 us, 16 rows
+    // tiles fill the SMs (N >= 64 x 148), a lane takes two of their rows (151,936 x 1,024: 8 rows 155 -> 130 us, 16 rows
     // 246 -> 173; with fewer tiles two rows a lane leave SMs idle, 4,096 x 1,024: 7.9 -> 10.9).
     if (M <= 1)
         return f32_few<1, 1, 6>(p, stream);

@@ -161,3 +161,25 @@ def test_single_tokens_with_fewer_ranges_than_keys(k, ranks, monkeypatch):
                 min_q_len=1)
     exact = exact_attention(q, keys, values, table, [1], [c], 4, 2, d, 16, d ** -0.5, None, None, None, None, None)
     assert float((out.double() - exact).abs().max()) <= 2 * 6 * 16 * (d / 4 + 16) * UNIT
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4, 8, 16, 48, 70, 300])
+def test_linear_float32_reads_weights_that_the_kernel_ahead_wrote(k, rows):
+    """Every kernel starts before the one ahead has ended: no weight is read before that."""
+    N, K = 4096, 1024
+    first, x = rnd(N, K, seed=7), rnd(rows, K, seed=8)
+    for wait in (True, False, False, False):
+        ws, outs = [first.clone() for _ in range(4)], [torch.full((rows, N), float("nan"), device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        for w, out in zip(ws, outs):
+            k.scale(w, 2.0)
+            if wait:
+                torch.cuda.synchronize()
+            k.linear(x, w, out)
+        torch.cuda.synchronize()
+        if wait:
+            right = outs
+        assert all(torch.equal(a, b) for a, b in zip(outs, right))
+    plain = torch.full((rows, N), float("nan"), device="cuda")
+    k.linear(x, first, plain)                            # (a power of two scales every sum exactly)
+    assert torch.equal(right[0], 2 * plain)
