@@ -333,6 +333,20 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
     launch_cluster(kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
 }
 
+// SMs of the current device, asked for once (148 on a B200, and if the driver does not say).
+inline int device_sm_count()
+{
+    static int count = 0;
+    if (count == 0) {
+        int device = 0, n = 0;
+        if (cudaGetDevice(&device) != cudaSuccess
+            || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0)
+            return 148;
+        count = n;
+    }
+    return count;
+}
+
 inline int launch_status()
 {
     const cudaError_t e = cudaGetLastError();

@@ -40,7 +40,7 @@ namespace chibi {
 
 using namespace sm100;
 
-constexpr int XT_M = 128, XT_K = 64, XT_UMMA_K = 16, XT_THREADS = 192, XT_MANY_THREADS = 320, XT_SMS = 148;
+constexpr int XT_M = 128, XT_K = 64, XT_UMMA_K = 16, XT_THREADS = 192, XT_MANY_THREADS = 320;
 template <int XT_N> struct ManyTile {
     static constexpr int STAGES = XT_N == 256 ? 4 : 6, A_BYTES = XT_M * XT_K * 2, STAGE_BYTES = A_BYTES + XT_N * XT_K * 2;
     static constexpr size_t SMEM = STAGES * STAGE_BYTES + (2 * STAGES + 4) * 8 + 16 + 1024;
@@ -416,8 +416,8 @@ static int launch_expert_many(const void* a, const void* w, long long pairs, int
             return (int)e;
         configured = true;
     }
-    const long long tiles = (long long)((p.rows_w + XT_N - 1) / XT_N) * p.max_tiles;
-    launch(expert_rows_tc_kernel<MODE, XT_N>, dim3((unsigned)(tiles < XT_SMS ? tiles : XT_SMS)), dim3(XT_MANY_THREADS),
+    const long long tiles = (long long)((p.rows_w + XT_N - 1) / XT_N) * p.max_tiles, sms = device_sm_count();
+    launch(expert_rows_tc_kernel<MODE, XT_N>, dim3((unsigned)(tiles < sms ? tiles : sms)), dim3(XT_MANY_THREADS),
            ManyTile<XT_N>::SMEM, stream, map_a, map_b, p);
     return launch_status();
 }
@@ -436,7 +436,7 @@ static int launch_expert_rows(const void* a, const void* w, long long pairs, int
         return launch_expert_few<MODE, 64>(a, w, pairs, experts, K, p, stream);
     // (as many tiles as the pairs make if they spread over the experts)  Narrow ones where they leave no SM a second.
     const long long spread = pairs / XT_M + (pairs < experts ? pairs : experts);
-    if (spread * ((p.rows_w + 127) / 128) <= XT_SMS)
+    if (spread * ((p.rows_w + 127) / 128) <= device_sm_count())
         return launch_expert_many<MODE, 128>(a, w, pairs, experts, K, p, stream);
     return launch_expert_many<MODE, 256>(a, w, pairs, experts, K, p, stream);
 }

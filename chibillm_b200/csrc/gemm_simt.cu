@@ -95,7 +95,6 @@ gemm_simt_kernel(const TX* __restrict__ x, const TW* __restrict__ w, TO* __restr
 // sum are the two halves of one 64-bit register: fma.rn.f32x2 takes two neighbouring places of both operands
 // as they lie in shared memory (each half rounded like fmaf), so neither operand is transposed or
 // doubled on its way.  Rows lie 36 floats apart there: the 16 bytes of eight rows fall on all 32 banks.
-constexpr int F32_SMS = 148;
 constexpr int F32_KB = 32, F32_ROW = F32_KB + 4;        // places of a stage; floats from row to row
 constexpr int F32_GROUP = 4;                            // parts of a group
 constexpr int F32_GROUPS = 4;                           // most groups of a sum
@@ -514,7 +513,7 @@ static int f32_few(F32Params p, cudaStream_t stream)
     // Two CTAs to an SM.  The tiles fill them, or the parts of a tile are shared by 2 or 4 CTAs while that needs no
     // second round and leaves every warp a part.
     p.tiles = (p.N + 32 * NR - 1) / (32 * NR);
-    const int blocks = (p.M + MT - 1) / MT, slots = 2 * F32_SMS / blocks;
+    const int blocks = (p.M + MT - 1) / MT, slots = 2 * device_sm_count() / blocks;
     p.ranks = 1;
     while (p.ranks < 4 && p.tiles * p.ranks * 2 <= slots && 8 * p.ranks <= p.parts)
         p.ranks *= 2;
@@ -530,10 +529,10 @@ static int f32_tiles(F32Params p, cudaStream_t stream)
     // 1,024 x 2,048 38 -> 50 us), and one alone takes 0.8 of the time of two (512 rows of 1,024 x 2,048, 128 tiles: 134 us
     // whole, 76 shared).  The busiest SM's time in groups of parts, with an eighth of one for a CTA's start and end.
     const long long tiles = (long long)((p.N + 63) / 64) * ((p.M + 63) / 64);
-    const int groups = (p.parts + F32_GROUP - 1) / F32_GROUP;
+    const int groups = (p.parts + F32_GROUP - 1) / F32_GROUP, sms = device_sm_count();
     double least = 0.0;
     for (int ranks = 1; ranks <= groups; ranks *= 2) {
-        const long long ctas = (tiles * ranks + F32_SMS - 1) / F32_SMS;
+        const long long ctas = (tiles * ranks + sms - 1) / sms;
         const double cost = ((double)(ctas / 2) + (ctas % 2 ? 0.8 : 0.0)) * ((groups + ranks - 1) / ranks + 0.125);
         if (ranks == 1 || cost < least) {
             p.ranks = ranks;
@@ -564,7 +563,7 @@ static int gemm_f32(const float* x, const float* w, float* out, const float* res
         return f32_few<2, 1, 4>(p, stream);
     if (M <= 4)
         return f32_few<4, 1, 4>(p, stream);
-    const bool wide = N >= 64 * F32_SMS;
+    const bool wide = N >= 64 * device_sm_count();
     if (M <= 8)
         return wide ? f32_few<8, 2, 2>(p, stream) : f32_few<8, 1, 4>(p, stream);
     if (M <= 48 || (M <= 128 && (long long)((N + 31) / 32) * ((M + 15) / 16) <= 512))

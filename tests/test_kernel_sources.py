@@ -47,3 +47,9 @@ def test_the_recurrences_ask_for_their_shared_memory_whatever_its_size():
         text = f.read()
     assert not re.findall(r"if \(smem > [^)]*\)", text)
     assert text.count("if (const int e = allow_shared(") == 2          # the preparing kernels and the chunk kernels
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh"))))
+def test_rules_ask_the_device_for_its_sms(name):
+    with open(os.path.join(CSRC, name)) as f:
+        assert not re.findall(r"constexpr[^;]*\b148\b", re.sub(r"//[^\n]*", "", f.read()))
