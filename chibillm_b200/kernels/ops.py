@@ -1172,6 +1172,8 @@ class CudaKernels:
         if proj.shape[1] != 5 * W + rank or state.dtype != torch.float32 or not state.is_contiguous() \
                 or tuple(state.shape[1:]) != (heads, d, d):
             raise KernelError("delta_rule: proj [T, 5 * heads * d + rank] and state float32 [slots, heads, d, d]")
+        if rank <= 0:
+            raise KernelError("delta_rule: the rank of the decay's projection must be positive")
         seqs = state_slots.numel()
         scratch = self._recurrence_scratch(T, seqs, heads, d, 2, max_q_len)
         self.launches += 2 if scratch is not None and d <= 256 else 1

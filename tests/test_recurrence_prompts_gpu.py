@@ -74,3 +74,12 @@ def test_what_is_no_number_reaches_later_tokens_only(k, rule, d, heads):
                 assert torch.equal(o[:, :h * d], clean[:, :h * d]), f"{bad} as token {at}'s {what} reached another head"
                 if what != "logit" and bad != bad:
                     assert torch.isnan(o[at]).any()
+
+
+def test_a_decay_without_a_rank_is_refused(k):
+    from chibillm_b200.kernels.ops import KernelError
+    step = Step(k, "general", [1], 2, 32)
+    W = 64
+    with pytest.raises(KernelError):
+        k.delta_rule(step.x[:, :5 * W], step.logits, step.bias, step.removal, step.first, torch.empty(1, W, device=DEV), ints([0, 1]),
+                     ints([0]), 2, 32, 0, 0.6, 1e-6, 1)
