@@ -766,19 +766,46 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                 if (p.activate)
                     vt[i][j] = lr_silu<TX>(vt[i][j]);
             }
-        // A value that is no number would reach the tokens before it through N's zeros: a warp that has one is careful.
-        bool finite = true;
+        if (RULE != DELTA) {                            // (the values as they are: they go into the state)
+            float* const to = RULE == GENERAL ? Vs : Us;
 #pragma unroll
-        for (int i = 0; i < VR; ++i)
+            for (int i = 0; i < VR; ++i)
 #pragma unroll
-            for (int j = 0; j < CT; ++j)
-                finite = finite && fabsf(vt[i][j]) < INFINITY;
-        const bool numbers = __all_sync(0xffffffffu, finite);
+                for (int j = 0; j < CT; ++j)
+                    if (lr + L * i < RC)
+                        to[(lr + L * i) * CP + c0 + j] = vt[i][j];
+        }
+        // A value that is no number would reach the tokens before it through N's zeros.  The products take it as zero, and what
+        // they give its column from its token on is no number: byte j of `from` is column j's first such token.
+        uint32_t from = 0x10101010u;
+        {
+            bool finite = true;
+#pragma unroll
+            for (int i = 0; i < VR; ++i)
+#pragma unroll
+                for (int j = 0; j < CT; ++j)
+                    finite = finite && fabsf(vt[i][j]) < INFINITY;
+            if (!__all_sync(0xffffffffu, finite)) {
+#pragma unroll
+                for (int j = 0; j < CT; ++j) {
+                    uint32_t first = RC;
+#pragma unroll
+                    for (int i = VR - 1; i >= 0; --i)
+                        if (!(fabsf(vt[i][j]) < INFINITY)) {
+                            first = lr + L * i;
+                            vt[i][j] = 0.f;
+                        }
+#pragma unroll
+                    for (int o = L / 2; o >= 1; o >>= 1)
+                        first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+                    from = (from & ~(255u << 8 * j)) | first << 8 * j;
+                }
+            }
+        }
         if (c + 1 < chunks)
             fetch_v(base + RC);
-        // A S_0 + N V, folded: thread lr ends with values lr OWN .. of the [token][column] tile.  N is zero above the diagonal;
-        // `careful`: those products are left out.
-        auto sums = [&](const float* A, const float* N, float (&acc)[SUMS], const bool careful) {
+        // A S_0 + N V, folded: thread lr ends with values lr OWN .. of the [token][column] tile
+        auto product = [&](const float* A, const float* N, float (&acc)[SUMS]) {
 #pragma unroll
             for (int t = 0; t < RC; ++t) {
                 uint64_t pair[CT];
@@ -802,19 +829,12 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                     const float m = L <= RC || lr < RC ? N[t * RC + lr + L * i] : 0.f;
 #pragma unroll
                     for (int j = 0; j < CT; ++j)
-                        if (!careful || lr + L * i <= t)
-                            s[j] = fmaf(m, vt[i][j], s[j]);
+                        s[j] = fmaf(m, vt[i][j], s[j]);
                 }
 #pragma unroll
                 for (int j = 0; j < CT; ++j)
                     acc[CT * t + j] = s[j];
             }
-        };
-        auto product = [&](const float* A, const float* N, float (&acc)[SUMS]) {
-            if (__builtin_expect(numbers, 1))
-                sums(A, N, acc, false);
-            else
-                sums(A, N, acc, true);
 #pragma unroll
             for (int o = L / 2, half = SUMS / 2; o >= 1; o >>= 1, half >>= 1) {
                 const bool upper = (lr & o) != 0;
@@ -825,6 +845,12 @@ chunk_recurrence_kernel(const RecurrenceParams p)
                     acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
                 }
             }
+            if (from != 0x10101010u) {
+#pragma unroll
+                for (int i = 0; i < OWN; ++i)
+                    if ((lr * OWN + i) / CT >= (int)(from >> 8 * ((lr * OWN + i) % CT) & 255u))
+                        acc[i] = nanf("");
+            }
         };
         if (RULE != LINEAR) {
             float acc[SUMS];
@@ -832,21 +858,6 @@ chunk_recurrence_kernel(const RecurrenceParams p)
 #pragma unroll
             for (int i = 0; i < OWN; ++i)
                 Us[((lr * OWN + i) / CT) * CP + c0 + (lr * OWN + i) % CT] = acc[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < VR; ++i)
-#pragma unroll
-                for (int j = 0; j < CT; ++j)
-                    if (lr + L * i < RC)
-                        Us[(lr + L * i) * CP + c0 + j] = vt[i][j];
-        }
-        if (RULE == GENERAL) {
-#pragma unroll
-            for (int i = 0; i < VR; ++i)
-#pragma unroll
-                for (int j = 0; j < CT; ++j)
-                    if (lr + L * i < RC)
-                        Vs[(lr + L * i) * CP + c0 + j] = vt[i][j];
         }
         __syncthreads();
         {
