@@ -87,11 +87,58 @@ struct RecurrenceParams {
     float* scratch;
     const int* q_start;
     const int* slots;
-    int heads, qk_heads, d, e;
+    int seqs, heads, qk_heads, d, e;
 };
 
+// The chunk whose block of the scratch array is number `slot` (a sequence's chunks start at slot q_start / 16 + sequence): its
+// first row and its number of tokens, which is not above 0 where no chunk lies.  Called by whole warps; a lane looks at four
+// sequences, so that up to 128 take one round of loads.
+__device__ __forceinline__ int2 rc_chunk_of(const RecurrenceParams& p, int slot)
+{
+    if (p.seqs == 1) {
+        const int row = p.q_start[0] + (slot - p.q_start[0] / RC) * RC;
+        return make_int2(row, slot < p.q_start[0] / RC ? 0 : min(RC, p.q_start[1] - row));
+    }
+    constexpr int EACH = 4, ALL = 32 * EACH;
+    const int lane = threadIdx.x & 31;
+    int low = 0, among = p.seqs;                        // the sequence is one of low .. low + among - 1
+    int starts[EACH], c, step;
+    do {
+        step = (among + ALL - 1) / ALL;
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int s = low + (lane + 32 * i) * step;
+            starts[i] = s <= p.seqs ? p.q_start[s] : 2147483647;
+        }
+        c = 0;                                          // how many of them start no later (they are the first ones)
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) {
+            const int at = (lane + 32 * i) * step;
+            c += __popc(__ballot_sync(0xffffffffu, at < among && starts[i] / RC + low + at <= slot));
+        }
+        if (c == 0)
+            return make_int2(0, 0);
+        low += (c - 1) * step;
+        among = min(step, among - (c - 1) * step);
+    } while (step > 1);
+    int first = 0, end = 0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        const int f = __shfl_sync(0xffffffffu, starts[i], (c - 1) & 31), e = __shfl_sync(0xffffffffu, starts[i], c & 31);
+        first = (c - 1) / 32 == i ? f : first;
+        end = c / 32 == i ? e : end;
+    }
+    if (c == ALL)
+        end = p.q_start[low + 1];
+    const int base = (slot - (first / RC + low)) * RC;
+    return make_int2(first + base, min(RC, end - first - base));
+}
+
 // ---------------------------------------------------------------- per chunk and head: what the chunk kernel needs
-// grid (chunks, heads, sequences), eight warps.  The inner products of a chunk's tokens come in tiles of four
+// grid (chunks, heads), eight warps.  The chunks of all sequences in one list, as many as the step's rows can make: by the
+// longest sequence, a step of 63 single tokens and a portion of 1,024 is 131,072 blocks (32 heads), of which 4,064 have work
+// (the generalised rule 328 us, 262 by the list), and a sequence longer than the host said would have no chunks.
+// The inner products of a chunk's tokens come in tiles of four
 // sources s and four targets t, lanes along the channels.  Off the diagonal the sources are decayed to the
 // targets' first token and the targets from there, so that a tile is a plain product; on it the sources are
 // decayed token by token.  A tile's 32 sums over the lanes are folded together.  Bound by the latency of its short
@@ -118,17 +165,16 @@ recurrence_prepare_kernel(const RecurrenceParams p)
     __shared__ __align__(16) float Bs[RC][RC];
     __shared__ __align__(16) float Ms[RC][RC];
     __shared__ float bs[RC], power[RC + 1];
-    const int h = blockIdx.y, seq = blockIdx.z;
-    const int row0 = p.q_start[seq];
-    const int base = blockIdx.x * RC;
-    const int n = min(RC, p.q_start[seq + 1] - row0 - base);
+    const int h = blockIdx.y;
+    const int2 chunk = rc_chunk_of(p, blockIdx.x);
+    const int row0 = chunk.x, n = chunk.y;              // the chunk's first row, its tokens
     if (n <= 0)
         return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int d = p.d, kh = h / (p.heads / p.qk_heads);
-    const TX* q = static_cast<const TX*>(p.q) + (size_t)(row0 + base) * p.stride + kh * d;
-    const TX* k = static_cast<const TX*>(p.k) + (size_t)(row0 + base) * p.stride + kh * d;
-    float* KE = p.scratch + ((size_t)((row0 / RC) + seq + blockIdx.x) * p.heads + h) * rc_block(DP, RULE);
+    const TX* q = static_cast<const TX*>(p.q) + (size_t)row0 * p.stride + kh * d;
+    const TX* k = static_cast<const TX*>(p.k) + (size_t)row0 * p.stride + kh * d;
+    float* KE = p.scratch + ((size_t)blockIdx.x * p.heads + h) * rc_block(DP, RULE);
     float* GE = KE + RC * DP;
     float* Qo = GE + DP;
     float* No = Qo + RC * DP;                           // B M, or B
@@ -150,7 +196,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
                 kr[u] = k[(size_t)t * p.stride + c];
                 qr[u] = q[(size_t)t * p.stride + c];
                 if (RULE == DELTA)
-                    zr[u] = p.logits[(size_t)(row0 + base + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
+                    zr[u] = p.logits[(size_t)(row0 + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
             }
         }
 #pragma unroll
@@ -167,7 +213,7 @@ recurrence_prepare_kernel(const RecurrenceParams p)
     }
     if (tid < RC) {
         if (RULE == DELTA) {
-            bs[tid] = tid < n ? 1.f / (1.f + expf(-to_f32(static_cast<const TX*>(p.beta)[(size_t)(row0 + base + tid)
+            bs[tid] = tid < n ? 1.f / (1.f + expf(-to_f32(static_cast<const TX*>(p.beta)[(size_t)(row0 + tid)
                                                                                         * p.beta_stride + h]))) : 0.f;
         } else {
             float v = 1.f;
@@ -405,19 +451,18 @@ general_prepare_kernel(const RecurrenceParams p)
     float* gs = rs + RC * DP;                           // decays
     float* gg = gs + RC * DP;                           // [4][DP]: the decays' products over four tokens each
     __shared__ __align__(16) float Aa[RC][RC], Ak[RC][RC], Ba[RC][RC], Bk[RC][RC], Ms[RC][RC], Ns[RC][RC];
-    const int h = blockIdx.y, seq = blockIdx.z;
-    const int row0 = p.q_start[seq];
-    const int base = blockIdx.x * RC;
-    const int n = min(RC, p.q_start[seq + 1] - row0 - base);
+    const int h = blockIdx.y;
+    const int2 chunk = rc_chunk_of(p, blockIdx.x);
+    const int row0 = chunk.x, n = chunk.y;              // the chunk's first row, its tokens
     if (n <= 0)
         return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int d = p.d;
-    const size_t at0 = (size_t)(row0 + base) * p.stride + h * d;
+    const size_t at0 = (size_t)row0 * p.stride + h * d;
     const TX* r = static_cast<const TX*>(p.q) + at0;
     const TX* k = static_cast<const TX*>(p.k) + at0;
     const TX* a = static_cast<const TX*>(p.removal) + at0;
-    float* KE = p.scratch + ((size_t)((row0 / RC) + seq + blockIdx.x) * p.heads + h) * rc_block(DP, GENERAL);
+    float* KE = p.scratch + ((size_t)blockIdx.x * p.heads + h) * rc_block(DP, GENERAL);
     float* GE = KE + RC * DP;
     float* Qo = GE + DP;
     float* No = Qo + RC * DP;
@@ -438,7 +483,7 @@ general_prepare_kernel(const RecurrenceParams p)
                 kr[u] = k[(size_t)t * p.stride + c];
                 rr[u] = r[(size_t)t * p.stride + c];
                 ar[u] = a[(size_t)t * p.stride + c];
-                zr[u] = p.logits[(size_t)(row0 + base + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
+                zr[u] = p.logits[(size_t)(row0 + t) * p.logit_stride + h * d + c] + p.dt_bias[h * d + c];
             }
         }
 #pragma unroll
@@ -1340,23 +1385,23 @@ static int launch_chunks(const RecurrenceParams& p, int seqs, cudaStream_t strea
 }
 
 template <int DP, int RULE, typename TX>
-static int launch_prompt(const RecurrenceParams& p, int seqs, int max_q_len, cudaStream_t stream)
+static int launch_prompt(const RecurrenceParams& p, long long tokens, cudaStream_t stream)
 {
     const size_t smem = (size_t)(RULE == GENERAL ? 5 * RC + 4 : RULE == DELTA ? 3 * RC + 4 : 2 * RC) * DP * sizeof(float);
     auto prepare = RULE == GENERAL ? general_prepare_kernel<DP, TX> : recurrence_prepare_kernel<DP, RULE == GENERAL ? DELTA : RULE, TX>;
     if (const int e = allow_shared(prepare, smem))
         return e;
-    launch(prepare, dim3((unsigned)((max_q_len + RC - 1) / RC), (unsigned)p.heads, (unsigned)seqs), dim3(256), smem, stream, p);
+    launch(prepare, dim3((unsigned)(tokens / RC + p.seqs), (unsigned)p.heads), dim3(256), smem, stream, p);
     if (const int e = launch_status())
         return e;
     // as few columns a block as give every SM one block and no more, and the fewer the smaller a thread's piece
     constexpr int RT = DP >= 128 ? 8 : 4;
-    const long long per_head = (long long)p.heads * seqs, sms = recurrence_sm_count();
+    const long long per_head = (long long)p.heads * p.seqs, sms = recurrence_sm_count();
     if (((p.e + 7) / 8) * per_head <= sms)
-        return launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, RULE, TX>(p, seqs, stream);
+        return launch_chunks<DP, RT, DP >= 256 ? 2 : 1, 8, RULE, TX>(p, p.seqs, stream);
     if (((p.e + 15) / 16) * per_head <= sms)
-        return launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, RULE, TX>(p, seqs, stream);
-    return launch_chunks<DP, RT, 4, 32, RULE, TX>(p, seqs, stream);
+        return launch_chunks<DP, DP >= 256 ? 8 : 4, DP >= 128 ? 4 : 2, 16, RULE, TX>(p, p.seqs, stream);
+    return launch_chunks<DP, RT, 4, 32, RULE, TX>(p, p.seqs, stream);
 }
 
 template <int RULE, typename TX>
@@ -1414,12 +1459,12 @@ static int launch_recurrence(const RecurrenceParams& p, int x_type, long long sc
         return CHIBI_ERR_ARGUMENT;
     CHIBI_DISPATCH_TYPE(x_type, TX, {
         if (DP == 32)
-            return launch_prompt<32, RULE, TX>(p, seqs, max_q_len, stream);
+            return launch_prompt<32, RULE, TX>(p, tokens, stream);
         if (DP == 64)
-            return launch_prompt<64, RULE, TX>(p, seqs, max_q_len, stream);
+            return launch_prompt<64, RULE, TX>(p, tokens, stream);
         if (DP == 128)
-            return launch_prompt<128, RULE, TX>(p, seqs, max_q_len, stream);
-        return launch_prompt<256, RULE, TX>(p, seqs, max_q_len, stream);
+            return launch_prompt<128, RULE, TX>(p, tokens, stream);
+        return launch_prompt<256, RULE, TX>(p, tokens, stream);
     });
     return CHIBI_OK;
 }
@@ -1474,6 +1519,7 @@ CHIBI_API int chibi_channel_delta(const void* qkv, int x_type, long long stride,
     p.scratch = scratch;
     p.q_start = q_start;
     p.slots = slots;
+    p.seqs = seqs;
     p.heads = heads;
     p.qk_heads = qk_heads;
     p.d = d;
@@ -1503,6 +1549,7 @@ CHIBI_API int chibi_decayed_attention(const void* qkv, int x_type, long long str
     p.scratch = scratch;
     p.q_start = q_start;
     p.slots = slots;
+    p.seqs = seqs;
     p.heads = heads;
     p.qk_heads = heads;
     p.d = d;
@@ -1540,6 +1587,7 @@ CHIBI_API int chibi_delta_rule(const void* proj, int x_type, long long stride, c
     p.scratch = scratch;
     p.q_start = q_start;
     p.slots = slots;
+    p.seqs = seqs;
     p.heads = heads;
     p.qk_heads = heads;
     p.d = d;

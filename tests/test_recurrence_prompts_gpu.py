@@ -76,6 +76,36 @@ def test_what_is_no_number_reaches_later_tokens_only(k, rule, d, heads):
                     assert torch.isnan(o[at]).any()
 
 
+@pytest.mark.parametrize("lens", [[40], [1, 33, 1, 1, 16, 17], [1] * 40 + [70] + [3] * 30])
+@pytest.mark.parametrize("rule", RULES)
+def test_the_longest_sequence_is_a_hint(k, rule, lens):
+    """A number of tokens below that of the longest sequence picks no other chunks than the right one."""
+    step = Step(k, rule, lens, 2, 64)
+    right, wrong = step.run(), step.run(longest=5)
+    assert torch.equal(right[0], wrong[0]) and torch.equal(right[1], wrong[1])
+
+
+# sequences without a token, of single tokens, of whole chunks and a token more; 128 of them (what one look finds), one more or
+# less, and many more
+@pytest.mark.parametrize("lens", [[0, 16, 0, 0, 17, 1, 0], [1] * 31 + [50], [20] + [1] * 64 + [33], [1] * 126 + [50], [1] * 127 + [50],
+                                  [1] * 128 + [50], [2] * 700 + [18] + [1] * 400])
+@pytest.mark.parametrize("rule", RULES)
+def test_every_sequence_of_a_mixed_step_gets_its_chunks(k, rule, lens):
+    step = Step(k, rule, lens, 1, 32)
+    o, state = step.run()
+    for s in {0, 1, len(lens) // 2, len(lens) - 2, len(lens) - 1, max(range(len(lens)), key=lambda i: lens[i])}:
+        a, b = step.starts[s], step.starts[s + 1]
+        if a == b:
+            assert torch.equal(state[s], step.first[s])
+            continue
+        alone = Step(k, rule, [b - a], 1, 32)
+        alone.x, alone.logits, alone.beta, alone.first = step.x[a:b], step.logits[a:b], step.beta[a:b], step.first[s:s + 1]
+        alone.a_log, alone.bias, alone.removal, alone.decay = step.a_log, step.bias, step.removal, step.decay
+        # (the longest said to be five or more: chunks, as in the mixed step)
+        one_o, one_state = alone.run(longest=max(5, b - a))
+        assert torch.equal(o[a:b], one_o) and torch.equal(state[s:s + 1], one_state)
+
+
 def test_a_decay_without_a_rank_is_refused(k):
     from chibillm_b200.kernels.ops import KernelError
     step = Step(k, "general", [1], 2, 32)
