@@ -273,14 +273,16 @@ template <int R> __device__ __forceinline__ int ssm_row(int i, int l)
     return R >= 4 ? (i >> 2) * 128 + l * 4 + (i & 3) : i * 32 + l;
 }
 
-// COLS: value columns of a block: 16, or 8 where 16 would leave SMs without a block.
-template <typename TX, int R, int COLS>
+// COLS: value columns of a block: 16, or 8 where 16 would leave SMs without a block.  AT_LEAST: tokens of the sequences that it
+// takes: 1, or SSM_FEW + 1 where the kernel for few tokens takes the others.  (Compiled in: with the number among the arguments a
+// step of eight single tokens and a portion of 200 took 47 us and not 37, its blocks falling to the SMs otherwise.)
+template <typename TX, int R, int COLS, int AT_LEAST>
 __global__ void __launch_bounds__(32 * COLS / SSM_CW)
 state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const TX* __restrict__ dt_raw,
                         long long dt_stride, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                         const float* __restrict__ skip, float* state, float* __restrict__ y,
                         const int* __restrict__ q_start, const int* __restrict__ slots, int heads, int groups, int e,
-                        int N, int at_least)
+                        int N)
 {
     pdl_enter();
     constexpr int THREADS = 32 * COLS / SSM_CW;
@@ -297,7 +299,7 @@ state_space_scan_kernel(const TX* __restrict__ xbc, long long xbc_stride, const 
     const int col = blockIdx.x * COLS + col_local;      // the warp's first column
     const int row0 = q_start[seq];
     const int q_len = q_start[seq + 1] - row0;
-    if (q_len < at_least)
+    if (q_len < AT_LEAST)
         return;
     float* S = state + (((size_t)slots[seq] * heads + h) * e) * N;
     float s[SSM_CW][R];
@@ -898,17 +900,17 @@ struct ScanArgs {
     int heads, groups, e, N;
 };
 
-template <typename TX, int R, int COLS>
-static void launch_scan(int seqs, cudaStream_t stream, const ScanArgs& a, int at_least)
+template <typename TX, int R, int COLS, int AT_LEAST>
+static void launch_scan(int seqs, cudaStream_t stream, const ScanArgs& a)
 {
     const dim3 grid((unsigned)((a.e + COLS - 1) / COLS), (unsigned)a.heads, (unsigned)seqs);
     const size_t smem = (size_t)2 * (2 * SSM_CHUNK * R * 32 + SSM_CHUNK * COLS + 2 * SSM_CHUNK) * sizeof(float);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute(state_space_scan_kernel<TX, R, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(state_space_scan_kernel<TX, R, COLS, AT_LEAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem);
-    launch(state_space_scan_kernel<TX, R, COLS>, grid, dim3(32 * COLS / SSM_CW), smem, stream, (const TX*)a.xbc,
+    launch(state_space_scan_kernel<TX, R, COLS, AT_LEAST>, grid, dim3(32 * COLS / SSM_CW), smem, stream, (const TX*)a.xbc,
            a.xbc_stride, (const TX*)a.dt_raw, a.dt_stride, a.dt_bias, a.a_log, a.skip, a.state, a.y, a.q_start, a.slots,
-           a.heads, a.groups, a.e, a.N, at_least);
+           a.heads, a.groups, a.e, a.N);
 }
 
 template <typename TX, int R>
@@ -960,20 +962,25 @@ CHIBI_API int chibi_state_space_scan(const void* xbc, int x_type, long long xbc_
     const int at_least = few == 2 ? SSM_FEW + 1 : 1;
     const long long most = tokens / at_least < seqs ? tokens / at_least : seqs;      // sequences that can have so many
     const bool narrow = (long long)((e + 15) / 16) * heads * most < sms && e > 8;
-#define CHIBI_SCAN(RR)                                             \
-    CHIBI_DISPATCH_TYPE(x_type, TX, {                              \
-        if (narrow)                                                \
-            launch_scan<TX, RR, 8>(seqs, stream, a, at_least);     \
-        else                                                       \
-            launch_scan<TX, RR, 16>(seqs, stream, a, at_least);    \
+#define CHIBI_SCAN(RR, COLS)                                               \
+    CHIBI_DISPATCH_TYPE(x_type, TX, {                                      \
+        if (few == 2)                                                      \
+            launch_scan<TX, RR, COLS, SSM_FEW + 1>(seqs, stream, a);       \
+        else                                                               \
+            launch_scan<TX, RR, COLS, 1>(seqs, stream, a);                 \
     })
-    if (rows <= 1) CHIBI_SCAN(1);
-    else if (rows <= 2) CHIBI_SCAN(2);
-    else if (rows <= 4) CHIBI_SCAN(4);
-    else if (rows <= 8) CHIBI_SCAN(8);
-    else {
-        // larger states: blocks of 8 columns only (256 threads leave a thread the registers for its rows)
-        CHIBI_DISPATCH_TYPE(x_type, TX, { launch_scan<TX, 16, 8>(seqs, stream, a, at_least); });
+    // (states above 256 rows: blocks of 8 columns only, 256 threads leave a thread the registers for its rows)
+    if (rows > 8) CHIBI_SCAN(16, 8);
+    else if (narrow) {
+        if (rows <= 1) CHIBI_SCAN(1, 8);
+        else if (rows <= 2) CHIBI_SCAN(2, 8);
+        else if (rows <= 4) CHIBI_SCAN(4, 8);
+        else CHIBI_SCAN(8, 8);
+    } else {
+        if (rows <= 1) CHIBI_SCAN(1, 16);
+        else if (rows <= 2) CHIBI_SCAN(2, 16);
+        else if (rows <= 4) CHIBI_SCAN(4, 16);
+        else CHIBI_SCAN(8, 16);
     }
 #undef CHIBI_SCAN
     return launch_status();
