@@ -17,3 +17,9 @@ def test_32_bit_attention_is_captured_anew_only_where_its_kernels_depend_on_the_
     keys = [runtime.float32_launch_key(SimpleNamespace(max_ctx_len=n), head_dim) for n in (1, 64, 65, 128, 129, 256, 257, 5000)]
     assert len(set(keys)) == (4 if differs else 1)
     assert all(len(k) == (1 if differs else 0) for k in keys)
+
+
+def test_a_question_about_scratch_is_no_launch():
+    """The table of launches (--profile) has no line for an entry point that only answers."""
+    from chibillm_b200.kernels import profile
+    assert "chibi_recurrence_scratch" in profile._NOT_LAUNCHES
