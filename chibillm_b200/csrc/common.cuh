@@ -291,7 +291,8 @@ inline void launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size
 // after it, however early programmatic dependent launch lets it start, therefore
 // runs after all that was written before the embedding: the step's index arrays
 // (positions, sequence of each token, lengths, block tables) and the cache
-// entries of earlier steps.  Kernels may read those before their pdl_wait().
+// entries of earlier steps.  Kernels may read those before their pdl_wait(), and the tcgen05 products their
+// weights, which nothing in flight writes (CudaKernels.linear says so).
 template <typename... KArgs, typename... Args>
 inline void launch_ordered(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                            Args&&... args)

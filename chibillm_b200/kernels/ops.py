@@ -701,6 +701,8 @@ class CudaKernels:
     def linear(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor,
                residual: Optional[torch.Tensor] = None, defer: bool = False) -> Optional[PendingSum]:
         """out[M, N] = x[M, K] @ w[N, K]^T (+ residual, 32-bit, may alias out).
+        bfloat16 products read w before the kernel ahead of them has ended: it is constant, or no kernel of this package
+        in flight on the stream writes it (32-bit products wait first).
         With ``defer`` (together with a residual that aliases out, or without one) a split
         product is left pending -- the caller adds it, or takes it for ``out`` -- and is returned."""
         if isinstance(x, ScaledRows):
