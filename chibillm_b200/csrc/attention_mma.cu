@@ -63,9 +63,12 @@ struct AttnParams {
     float scale_log2;              // scale * log2(e)
     int window;
     int chunk;                     // 0: none; else a row sees only keys of its own block of this many positions
+    int seqs;                      // decode: all sequences of the step
     int splits;                    // decode: key ranges per sequence
-    float* scratch_o;              // decode: [S, nq, splits, D]
-    float* scratch_ml;             // decode: [S, nq, splits, 2]
+    int units;                     // decode: > 0: key ranges of all sequences together, cut by decode_unit
+    int by_length;                 // decode: the sequences with the most keys start first
+    float* scratch_o;              // decode: [S, nq, splits, D], or [units, nq, D]
+    float* scratch_ml;             // decode: the same with 2 numbers
     // decode, optional: q (and the newest key and value) are not in `q` and the caches yet but
     // still the partial sums of the q | k | v product: the kernel adds them up, applies the per-head
     // norm and the rotation itself and appends the new key and value (head size 128 only)
@@ -462,6 +465,121 @@ __device__ __forceinline__ void build_q_from_partial(const AttnParams& p, int t,
         __threadfence();                                      // the copies of the last tile read them back
 }
 
+// ---- which keys a decode CTA takes, from the sequences' lengths (whole warps; the lengths were written before the step's
+// first kernel, so this comes before the wait for the kernel ahead)
+constexpr int DEC_UNIT_SEQS = 128;           // sequences that decode_unit can deal with
+constexpr int DEC_ORDER_SEQS = DEC_WARPS * 32;   // that sequence_of_rank can
+constexpr int DEC_LEAST_TILES = 8;           // 128 keys: two tiles for each warp
+
+// Tiles of 16 visible keys of a sequence's one token; 0 for a sequence that brings another number of tokens.
+__device__ __forceinline__ int decode_tiles(const AttnParams& p, int s)
+{
+    if (s >= p.seqs || p.q_start[s + 1] - p.q_start[s] != 1)
+        return 0;
+    const int pos = p.ctx_len[s] - 1;
+    return (pos + 1 - first_visible_key(pos, p.window, p.chunk) + DEC_TILE - 1) / DEC_TILE;
+}
+
+struct DecodeUnit {
+    int seq;               // -1: none
+    int range, ranges;     // which key range of the sequence, and how many it has
+    int first_unit;        // the sequence's first unit
+    int tiles;             // tiles of a range
+};
+
+// Cuts the sequences' keys into at most p.units ranges of c tiles (the last of a sequence shorter), c as small as that
+// allows.  Ranges of one length, not so many to every sequence: with as many CTAs as are resident at once the time is that
+// of the longest range.  The lanes try 32 values of c at a time.  `unit` >= 0 asks for that range,
+// else for the ranges of sequence `seq`.
+__device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, int unit, int seq)
+{
+    constexpr int EACH = DEC_UNIT_SEQS / 32;
+    const int lane = threadIdx.x & 31;
+    int t[EACH], most = 0, total = 0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        t[i] = 32 * i < p.seqs ? decode_tiles(p, lane + 32 * i) : 0;
+        most = max(most, t[i]);
+        total += t[i];
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    total = __reduce_add_sync(0xffffffffu, total);
+    // (at most 32 ranges of a sequence: every one is a partial result for the merge to fetch)
+    int low = max(max(DEC_LEAST_TILES, (most + 31) / 32), (total + p.units - 1) / p.units);
+    int high = max(low, most);                           // (one range each is no more than p.units)
+    // ceil(t / c) as a product with 2^32 / c, rounded up: exact below 2^15 tiles, and one too many (an empty range) at most
+    auto ranges_of = [](int tiles, int c, uint32_t inverse) { return (int)__umulhi((uint32_t)(tiles + c - 1), inverse); };
+    auto inverse_of = [](int c) { return 0xffffffffu / (uint32_t)c + 1u; };
+    while (low < high) {
+        const int step = (high - low + 30) / 31;
+        const int c = min(high, low + lane * step);
+        const uint32_t inverse = inverse_of(c);
+        int sum = 0;
+#pragma unroll
+        for (int i = 0; i < EACH; ++i)
+            if (32 * i < p.seqs) {
+                const int n = min(32, p.seqs - 32 * i);
+                for (int k = 0; k < n; ++k)
+                    sum += ranges_of(__shfl_sync(0xffffffffu, t[i], k), c, inverse);
+            }
+        // the values are in order, so the first that fits is the lowest lane's; (high fits always)
+        const int first = __ffs(__ballot_sync(0xffffffffu, sum <= p.units || c == high)) - 1;
+        high = min(high, low + first * step);
+        low = step == 1 ? high : min(high, low + max(first - 1, 0) * step + 1);
+        if (first == 0)
+            low = high;
+    }
+    const uint32_t inverse = inverse_of(high);
+    DecodeUnit u { -1, 0, 0, 0, high };
+    int before = 0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        if (32 * i >= p.seqs)
+            break;
+        const int n = t[i] > 0 ? ranges_of(t[i], high, inverse) : 0;
+        int end = n;                                     // of lane's ranges, in the order of the sequences
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int other = __shfl_up_sync(0xffffffffu, end, o);
+            end += lane >= o ? other : 0;
+        }
+        const int first = before + end - n;
+        const uint32_t mine = __ballot_sync(0xffffffffu, unit >= 0 ? (unit >= first && unit < first + n) : lane + 32 * i == seq);
+        if (mine) {
+            const int l = __ffs(mine) - 1;
+            u.seq = 32 * i + l;
+            u.first_unit = __shfl_sync(0xffffffffu, first, l);
+            u.ranges = __shfl_sync(0xffffffffu, n, l);
+            u.range = unit - u.first_unit;
+        }
+        before += __shfl_sync(0xffffffffu, end, 31);
+    }
+    return u;
+}
+
+// The sequence that has the rank-th most keys, for the whole block (one sequence to a thread): with more CTAs than are
+// resident at once, what starts last should be short (64 sequences of 1,046 to 4,096 keys, 8 kv heads, two CTAs to an SM: the
+// SM with the most keys has 1.5 times the average in the batch's order).
+__device__ __forceinline__ int sequence_of_rank(const AttnParams& p, int rank)
+{
+    __shared__ __align__(16) int length[DEC_ORDER_SEQS];
+    __shared__ int found;
+    const int s = threadIdx.x;
+    // (distinct, earlier sequences first among equals; -1 is no sequence)
+    const int key = s < p.seqs ? min(decode_tiles(p, s), (1 << 22) - 1) * DEC_ORDER_SEQS + DEC_ORDER_SEQS - 1 - s : -1;
+    length[s] = key;
+    __syncthreads();
+    int longer = 0;
+    for (int i = 0; i < p.seqs; i += 4) {
+        const int4 other = *reinterpret_cast<const int4*>(length + i);
+        longer += (other.x > key) + (other.y > key) + (other.z > key) + (other.w > key);
+    }
+    if (key >= 0 && longer == rank)
+        found = s;
+    __syncthreads();
+    return found;
+}
+
 __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnParams p)
 {
     pdl_trigger();
@@ -472,7 +590,15 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     // The index arrays, the block table and every key before the newest one were written
     // before this step's first kernel: the first tiles are on their way while the kernel
     // that writes q and the newest key still runs.
-    const int seq = blockIdx.z, split = blockIdx.x;
+    int seq = blockIdx.z, split = blockIdx.x, ranges = p.splits, unit_tiles = 0;
+    if (p.units > 0) {
+        const DecodeUnit u = decode_unit(p, blockIdx.x, -1);
+        if (u.seq < 0)
+            return;
+        seq = u.seq, split = u.range, ranges = u.ranges, unit_tiles = u.tiles;
+    } else if (p.by_length) {
+        seq = sequence_of_rank(p, blockIdx.z);
+    }
     const int row_blocks = (p.group + 15) / 16;
     const int kv_head = blockIdx.y / row_blocks, row_block = blockIdx.y - kv_head * row_blocks;
     const int t = p.q_start[seq];
@@ -483,7 +609,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     const int first = first_visible_key(pos, p.window, p.chunk);
     const int key_end = pos + 1;
     const int tiles_total = (key_end - first + DEC_TILE - 1) / DEC_TILE;
-    const int tiles_per_split = (tiles_total + p.splits - 1) / p.splits;
+    const int tiles_per_split = unit_tiles > 0 ? unit_tiles : (tiles_total + p.splits - 1) / p.splits;
     const int tile_begin = split * tiles_per_split;
     int tile_end = tile_begin + tiles_per_split;
     if (tile_end > tiles_total)
@@ -644,11 +770,11 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
             lsum += ml[w * 16 + row] * f;
         }
         const int head = head0 + row;
-        if (p.splits == 1) {
+        if (ranges == 1) {
             lsum += sink_weight(p.sink, head, mmax);
             p.out[((size_t)t * p.nq + head) * D + c] = __float2bfloat16_rn(lsum > 0.f ? acc / lsum : 0.f);
         } else {
-            const size_t slot = ((size_t)seq * p.nq + head) * p.splits + split;
+            const size_t slot = p.units > 0 ? (size_t)blockIdx.x * p.nq + head : ((size_t)seq * p.nq + head) * p.splits + split;
             p.scratch_o[slot * D + c] = acc;
             if (c == 0) {
                 p.scratch_ml[slot * 2] = mmax;
@@ -658,26 +784,35 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     }
 }
 
-// Merges the key ranges of one (sequence, head): one block of D threads.
+// Merges the key ranges of one (sequence, head): one block of D threads (whole warps).
 __global__ void attn_decode_merge_kernel(const AttnParams p)
 {
     pdl_trigger();
-    const int seq = blockIdx.y, head = blockIdx.x, c = threadIdx.x;
+    const int seq = blockIdx.y, head = blockIdx.x, c = min((int)threadIdx.x, D - 1);
     const int t = p.q_start[seq];                     // written before the step's first kernel
     if (p.q_start[seq + 1] - t != 1)
         return;
+    int ranges = p.splits, step = 1;
+    size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
+    if (p.units > 0) {
+        const DecodeUnit u = decode_unit(p, -1, seq);
+        if (u.ranges <= 1)
+            return;                                   // (the attention kernel has written the row)
+        ranges = u.ranges;
+        step = p.nq;
+        slot0 = (size_t)u.first_unit * p.nq + head;
+    }
     pdl_wait();
-    const size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
     // eight key ranges at a time, all their loads in flight together
     float m_run = -INFINITY, acc = 0.f, lsum = 0.f;
-    for (int s0 = 0; s0 < p.splits; s0 += 8) {
+    for (int s0 = 0; s0 < ranges; s0 += 8) {
         float mv[8], lv[8], ov[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-            const bool in = s0 + u < p.splits;
-            mv[u] = in ? p.scratch_ml[(slot0 + s0 + u) * 2] : -INFINITY;
-            lv[u] = in ? p.scratch_ml[(slot0 + s0 + u) * 2 + 1] : 0.f;
-            ov[u] = in ? p.scratch_o[(slot0 + s0 + u) * D + c] : 0.f;
+            const bool in = s0 + u < ranges;
+            mv[u] = in ? p.scratch_ml[(slot0 + (size_t)(s0 + u) * step) * 2] : -INFINITY;
+            lv[u] = in ? p.scratch_ml[(slot0 + (size_t)(s0 + u) * step) * 2 + 1] : 0.f;
+            ov[u] = in ? p.scratch_o[(slot0 + (size_t)(s0 + u) * step) * D + c] : 0.f;
         }
         float m_new = m_run;
 #pragma unroll
@@ -696,7 +831,8 @@ __global__ void attn_decode_merge_kernel(const AttnParams p)
         m_run = m_new;
     }
     lsum += sink_weight(p.sink, head, m_run);
-    p.out[((size_t)t * p.nq + head) * D + c] = __float2bfloat16_rn(lsum > 0.f ? acc / lsum : 0.f);
+    if (threadIdx.x < D)
+        p.out[((size_t)t * p.nq + head) * D + c] = __float2bfloat16_rn(lsum > 0.f ? acc / lsum : 0.f);
 }
 
 // ------------------------------------------------------------------ prefill
@@ -851,9 +987,34 @@ CHIBI_API int chibi_attention_mma_head_dim() { return D; }
 CHIBI_API int chibi_attention_mma_value_dim() { return DV; }
 
 // Scratch floats that a decode launch with these sizes needs.
-CHIBI_API long long chibi_attention_mma_scratch_floats(int seqs, int nq, int splits)
+// The decode kernels on p's sequences: `splits` key ranges each, or, where `units` is above 0, that many ranges of all
+// sequences together, cut on the device by the sequences' lengths.
+static int launch_decode(AttnParams& p, int seqs, int splits, int units, int by_length, float* scratch,
+                         long long scratch_floats, cudaStream_t stream)
 {
-    return splits > 1 ? (long long)seqs * nq * splits * (D + 2) : 0;
+    if (splits < 1 || units < 0 || (units > 0 && (units < seqs || seqs > DEC_UNIT_SEQS)) || (by_length && seqs > DEC_ORDER_SEQS))
+        return CHIBI_ERR_ARGUMENT;
+    p.seqs = seqs;
+    p.splits = splits;
+    p.units = units;
+    p.by_length = by_length;
+    const bool merge = splits > 1 || units > 0;
+    if (merge) {
+        const long long parts = (units > 0 ? (long long)units : (long long)seqs * splits) * p.nq;
+        if (!scratch || scratch_floats < parts * (D + 2))
+            return CHIBI_ERR_ARGUMENT;
+        p.scratch_o = scratch;
+        p.scratch_ml = scratch + (size_t)parts * D;
+    }
+    const int row_blocks = (p.group + 15) / 16;
+    const dim3 grid(units > 0 ? units : splits, p.nkv * row_blocks, units > 0 ? 1 : seqs);
+    launch(attn_decode_kernel, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, p);
+    int st = launch_status();
+    if (st == CHIBI_OK && merge) {
+        launch(attn_decode_merge_kernel, dim3(dim3(p.nq, seqs)), dim3((D + 31) / 32 * 32), 0, stream, p);
+        st = launch_status();
+    }
+    return st;
 }
 
 // mode bit 0: run the decode kernel (one-token sequences); bit 1: run the
@@ -862,7 +1023,7 @@ CHIBI_API int chibi_attention_mma(const void* q, const void* k_cache, const void
                                   const int* block_table, int table_stride, const int* seq_rows,
                                   const int* q_start, const int* ctx_len, int seqs, int nq, int nkv, int page_size,
                                   int num_pages, float scale, int window, int chunk, int mode, int max_q_len,
-                                  int splits, float* scratch, long long scratch_floats, float softcap,
+                                  int splits, int units, int by_length, float* scratch, long long scratch_floats, float softcap,
                                   const float* bias_r1, const float* bias_r2, const float* sink, int* error,
                                   cudaStream_t stream);
 
@@ -926,7 +1087,7 @@ CHIBI_API int chibi_attention_mma(const void* q, const void* k_cache, const void
                                   const int* block_table, int table_stride, const int* seq_rows,
                                   const int* q_start, const int* ctx_len, int seqs, int nq, int nkv, int page_size,
                                   int num_pages, float scale, int window, int chunk, int mode, int max_q_len,
-                                  int splits, float* scratch, long long scratch_floats, float softcap,
+                                  int splits, int units, int by_length, float* scratch, long long scratch_floats, float softcap,
                                   const float* bias_r1, const float* bias_r2, const float* sink, int* error,
                                   cudaStream_t stream)
 {
@@ -975,25 +1136,9 @@ CHIBI_API int chibi_attention_mma(const void* q, const void* k_cache, const void
         configured = true;
     }
     if (mode & 1) {
-        if (splits > 1) {
-            const long long need = chibi_attention_mma_scratch_floats(seqs, nq, splits);
-            if (!scratch || scratch_floats < need)
-                return CHIBI_ERR_ARGUMENT;
-            p.scratch_o = scratch;
-            p.scratch_ml = scratch + (size_t)seqs * nq * splits * D;
-        }
-        const int row_blocks = (p.group + 15) / 16;
-        const dim3 grid(splits, nkv * row_blocks, seqs);
-        launch(attn_decode_kernel, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, p);
-        int st = launch_status();
+        const int st = launch_decode(p, seqs, splits, units, by_length, scratch, scratch_floats, stream);
         if (st != CHIBI_OK)
             return st;
-        if (splits > 1) {
-            launch(attn_decode_merge_kernel, dim3(dim3(nq, seqs)), dim3(D), 0, stream, p);
-            st = launch_status();
-            if (st != CHIBI_OK)
-                return st;
-        }
     }
     if (mode & 2) {
         const long long rows = (long long)max_q_len * p.group;
@@ -1015,7 +1160,7 @@ CHIBI_API int chibi_attention_decode_fused(const float* partial, int partial_spl
                                            long long tokens, void* k_cache, void* v_cache, void* out,
                                            const int* block_table, int table_stride, const int* seq_rows,
                                            const int* q_start, const int* ctx_len, int seqs, int nq, int nkv,
-                                           int page_size, int num_pages, float scale, int window, int chunk, int splits,
+                                           int page_size, int num_pages, float scale, int window, int chunk, int splits, int units,
                                            float* scratch, long long scratch_floats, const void* q_norm_w,
                                            const void* k_norm_w, const float* inv_freq, float eps, float offset,
                                            int append, int* error, cudaStream_t stream)
@@ -1067,20 +1212,5 @@ CHIBI_API int chibi_attention_decode_fused(const float* partial, int partial_spl
             return (int)e;
         configured = true;
     }
-    if (splits > 1) {
-        const long long need = chibi_attention_mma_scratch_floats(seqs, nq, splits);
-        if (!scratch || scratch_floats < need)
-            return CHIBI_ERR_ARGUMENT;
-        p.scratch_o = scratch;
-        p.scratch_ml = scratch + (size_t)seqs * nq * splits * D;
-    }
-    launch(attn_decode_kernel, dim3(splits, nkv, seqs), dim3(DEC_WARPS * 32), DEC_SMEM, stream, p);
-    int st = launch_status();
-    if (st != CHIBI_OK)
-        return st;
-    if (splits > 1) {
-        launch(attn_decode_merge_kernel, dim3(dim3(nq, seqs)), dim3(D), 0, stream, p);
-        st = launch_status();
-    }
-    return st;
+    return launch_decode(p, seqs, splits, units, 0, scratch, scratch_floats, stream);
 }

@@ -8,7 +8,7 @@ nothing once its workspace exists) and launch on torch's current stream.
 from __future__ import annotations
 
 import ctypes
-from typing import Dict, Optional
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -955,6 +955,28 @@ class CudaKernels:
                 best, least = s, cost
         return best
 
+    def decode_attention_units(self, seqs: int, nq: int, nkv: int, splits: int, max_ctx_len: int) -> Tuple[int, int]:
+        """How the decode attention kernel deals with sequences of different lengths (which the host does not know
+        here): (key ranges of all sequences together, or 0; whether the longest sequences start first).  Where
+        ``splits`` ranges each fit the resident CTAs, the same number of CTAs goes to ranges of one length instead, cut
+        on the device (16 sequences of 1,500 to 6,000 keys, 8 kv heads: 64.4 -> 48.2 us; of equal lengths 70.1 and 71.4:
+        the ranges are the same then, and finding them costs a microsecond, so not below 512 keys a range).
+        Where even one each does not fit, a range costs more than it evens out, and the order does: 64 sequences of
+        1,046 to 4,096 keys 145.5 -> 109.4 us, of equal lengths 179.9 and 180.8.  More sequences than the kernels' searches
+        take, and contexts too short to be worth them, stay in equal shares and in the batch's order."""
+        per_seq = nkv * ((nq // nkv + 15) // 16)
+        slots = 2 * self.sm_count
+        if seqs * per_seq > slots:
+            return 0, int(splits == 1 and 1 < seqs <= 128 and max_ctx_len >= 1024)
+        if splits == 1 or not 1 < seqs <= 128 or max_ctx_len < 512 * splits:
+            return 0, 0
+        return min(slots // per_seq, 32 * seqs), 0
+
+    def decode_attention_key(self, seqs: int, nq: int, nkv: int, max_ctx_len: int) -> Tuple[int, int, int]:
+        """What a captured decode step depends on besides its data."""
+        splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
+        return (splits, *self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len))
+
     def prompt_attention_key_ranges(self, seqs: int, nq: int, nkv: int, max_q_len: int, max_ctx_len: int) -> int:
         """Key ranges per row tile of the tcgen05 prompt attention: 1 unless the step
         has so few query rows that the CTAs (a tile of 128 rows for each kv head and
@@ -1025,15 +1047,16 @@ class CudaKernels:
                     return
             elif status != -2:
                 _check(status, "attention (tcgen05, tied values)")
-        splits, scratch = 1, None
+        splits, units, by_length, scratch = 1, 0, 0, None
         if mode & 1:
             splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
-            if splits > 1:
-                scratch = self._scratch(seqs * nq * splits * (d + 2))
+            units, by_length = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)
+            if splits > 1 or units:
+                scratch = self._scratch((units or seqs * splits) * nq * (d + 2))
         status = lib.chibi_attention_mma(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0),
             _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv, page_size, k_cache.shape[0], float(scale),
-            int(window or 0), int(chunk), mode, int(max_q_len), splits, _ptr(scratch),
+            int(window or 0), int(chunk), mode, int(max_q_len), splits, units, by_length, _ptr(scratch),
             scratch.numel() if scratch is not None else 0, float(softcap), _ptr(bias_r1), _ptr(bias_r2),
             _ptr(sink), _ptr(self.error), self._stream())
         self.launches += (1 if mode & 1 else 0) + (1 if mode & 1 and splits > 1 else 0) + (1 if mode & 2 else 0)
@@ -1077,11 +1100,12 @@ class CudaKernels:
             lib = self._load("chibi_attention_mma", (f"CHIBI_HEAD_DIM={d}",))
             lib = self._attention_libs[d] = self._profiled(lib)
         splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
-        scratch = self._scratch(seqs * nq * splits * (d + 2)) if splits > 1 else None
+        units = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)[0]
+        scratch = self._scratch((units or seqs * splits) * nq * (d + 2)) if splits > 1 else None
         status = lib.chibi_attention_decode_fused(
             _ptr(pending.partial), pending.splits, width, seqs, _ptr(k_cache), _ptr(v_cache), _ptr(out),
             _ptr(block_table), block_table.stride(0), _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv,
-            page_size, k_cache.shape[0], float(scale), int(window or 0), 0, splits, _ptr(scratch),
+            page_size, k_cache.shape[0], float(scale), int(window or 0), 0, splits, units, _ptr(scratch),
             scratch.numel() if scratch is not None else 0, _ptr(q_norm_w), _ptr(k_norm_w), _ptr(inv_freq),
             float(eps), float(norm_offset), 1 if append else 0, _ptr(self.error), self._stream())
         if status == -2:

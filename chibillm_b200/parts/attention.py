@@ -245,11 +245,11 @@ class PagedAttention(Mixer):
         k = self.runtime.kernels
         if self.prepared and (self.maps > 1 or self.value_dim != self.spec.head_dim):
             return ()                        # the plain attention kernel: nothing is decided on the host
-        splits = getattr(k, "decode_attention_splits", None)
-        if splits is None:
+        decode = getattr(k, "decode_attention_key", None)
+        if decode is None:
             return None
         s = self.spec
-        return (splits(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) \
+        return (decode(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) \
             + (self.runtime.float32_launch_key(ctx, s.head_dim) if self.value_dim == s.head_dim else ())
 
     # ---- run

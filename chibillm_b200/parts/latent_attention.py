@@ -126,10 +126,10 @@ class LatentAttention(Mixer):
         return True               # x goes to the first product and nowhere else
 
     def launch_key(self, ctx):
-        splits = getattr(self.runtime.kernels, "decode_attention_splits", None)
-        if splits is None:
+        decode = getattr(self.runtime.kernels, "decode_attention_key", None)
+        if decode is None:
             return None
-        return (splits(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),) \
+        return (decode(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),) \
             + self.runtime.float32_launch_key(ctx, self.key_dim)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, hold: bool = False):
