@@ -40,6 +40,7 @@ struct AttnTcParams {
     int kv_splits;                 // 1: none
     float* part_o;                 // [tokens][nq][kv_splits][D]
     float* part_ml;                // [tokens][nq][kv_splits][2]
+    int q_by_tma;                  // the query rows come by TMA (a tile of 128 rows is whole tokens)
     const float* sink;             // [nq] or null: exp(sink[head]) joins the softmax's denominator, once
 };
 

@@ -450,7 +450,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
 // O[row, :] *= f for this thread's row of an output accumulator in TMEM (a rare
 // event: kept out of line so that its registers do not count against the loop).
-__device__ __noinline__ void rescale_output_row(uint32_t o_addr, float f)
+__device__ __forceinline__ void rescale_output_row(uint32_t o_addr, float f)
 {
 #pragma unroll 1
     for (int c0 = 0; c0 < D; c0 += 32) {
@@ -472,20 +472,64 @@ __device__ __noinline__ void rescale_output_row(uint32_t o_addr, float f)
 // packed bfloat16 and is the A operand of the P V product).  While one group
 // works on its S tile the tensor core multiplies for the other.
 //
-//   warp 0      TMA loader (as above)
-//   warp 1      MMA issuer:  S_q = Q_q K^T,  O_q += P_q V  for q = 0, 1 in turn
-//   warps 2..5  softmax of tile 0;  warps 6..9  softmax of tile 1
+//   warp 0       TMA loader: the query rows (where a tile of 128 is whole tokens), then keys and values as above
+//   warp 1       MMA issuer:  S_q = Q_q K^T,  O_q += P_q V  for q = 0, 1 in turn
+//   warps 2, 3   none (registers are given back by warp groups of four)
+//   warps 4..7   softmax of tile 0;  warps 8..11  softmax of tile 1
+//
+// What bounds it is each tile's chain softmax -> P V -> next Q K^T, and a CTA's start and end.  A softmax thread holds its
+// whole row of S (224 registers: the first four warps give theirs back), so that the row leaves TMEM once for both the
+// maximum and the exponentials; scale, differences and sums are made two at a time (fma.rn.f32x2).  The queries
+// come by TMA, asked for together with the first keys and values before anything else is set up, and the output goes out
+// by way of shared memory in whole lines.  2,048 / 8,192 tokens of 32 heads of 128 on 8 key heads: 70.6 / 649 us with two
+// readings of S in pieces, queries through registers and rows written lane by lane; 45.0 / 455 so (0.47 / 0.75
+// of the measured product rate).  Three prompts of up to 1,500 tokens of 16 heads of 64: 61.5 -> 45.5.
 //
 // TMEM: S_0 at column 0, S_1 at 128, O_0 at 256, O_1 at 384.
-constexpr int ATC2_THREADS = 320;
+constexpr int ATC2_THREADS = 384;
 constexpr int SMEM2_TILES = 2 * Q_BYTES + 4 * KV_TILE_BYTES;
-constexpr int NUM_BARS2 = 14;
+constexpr int NUM_BARS2 = 16;
 constexpr size_t ATC2_SMEM = SMEM2_TILES + NUM_BARS2 * 8 + 16 + 1024;
+// Registers of a thread: what the block is launched with, and what the loader's and the softmax groups' threads have then.
+constexpr int ATC2_REGS = 168, ATC2_REGS_FEW = 56, ATC2_REGS_MANY = 224;
+static_assert(ATC2_REGS_FEW + 2 * ATC2_REGS_MANY <= 3 * ATC2_REGS, "more registers than the block has");
+
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Two 32-bit numbers in one register pair.
+__device__ __forceinline__ uint64_t pair_of(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 halves_of(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t pair_add(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 
 template <int OPT>
 __global__ void __launch_bounds__(ATC2_THREADS, 1)
-attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                        const AttnTcParams p)
+attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                        const __grid_constant__ CUtensorMap map_v, const AttnTcParams p)
 {
     pdl_enter();
     extern __shared__ uint8_t smem_raw[];
@@ -501,6 +545,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     uint64_t* s_full = bars + 8;      // [2] per query tile, MMA commit
     uint64_t* p_full = bars + 10;     // [2] per query tile, 128 threads
     uint64_t* o_done = bars + 12;     // [2] per query tile, MMA commit
+    uint64_t* q_full = bars + 14;     // [2] per query tile, TMA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS2);
 
     const int seq = blockIdx.z;
@@ -536,32 +581,80 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     }
     const int n_tiles = max(nt[0], nt[1]);
 
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&k_full[i], 1);
-            mbar_init(&v_full[i], 1);
-            mbar_init(&k_empty[i], 1);
-            mbar_init(&v_empty[i], 1);
-            mbar_init(&s_full[i], 1);
-            mbar_init(&p_full[i], 128);
-            mbar_init(&o_done[i], 1);
+    // Lane i of the loader brings page i of every 128-key tile (at most 16 pages: page_size >= 8).  It looks its page
+    // up one tile ahead, so the dependent read of the block table is over by the time the stage is free.
+    const int pages_per_tile = KEYS / p.page_size;
+    auto first_row_of = [&](int j) -> long long {
+        const int key = key_begin + j * KEYS + lane * p.page_size;
+        if (lane >= pages_per_tile || key >= key_end)
+            return p.cache_rows;          // past the context: read outside the array, zeros
+        const int page = table[key / p.page_size];
+        if (page < 0 || page >= p.num_pages) {
+            if (p.error)
+                atomicExch(p.error, 3);
+            return p.cache_rows;
         }
-        fence_barrier_init();
-    }
-    if (warp == 1) {
+        return ((long long)page * p.nkv + kv_head) * p.page_size;
+    };
+    auto load = [&](int which, int j, long long row) {             // keys, or values; the whole warp
+        const int st = j & 1;
+        uint64_t* full = which ? &v_full[st] : &k_full[st];
+        uint8_t* dst = (which ? v_s : k_s) + st * KV_TILE_BYTES;
+        if (lane == 0) {
+            if (j >= 2)
+                mbar_wait(which ? &v_empty[st] : &k_empty[st], ((j >> 1) - 1) & 1, p.error, 41);
+            mbar_arrive_expect_tx(full, KV_TILE_BYTES);
+        }
+        __syncwarp();
+        if (lane < pages_per_tile) {
+            for (int h = 0; h < HALVES; ++h)
+                tma_load_2d(dst + h * (KEYS * 128) + lane * p.page_size * 128, which ? &map_v : &map_k,
+                            full, h * 64, (int)row);
+        }
+    };
+    long long row = 0;
+    if (warp == 0) {
+        // the loader starts by itself: queries, first keys and first values are on their way while the others set up
+        if (lane == 0) {
+            for (int i = 0; i < 2; ++i) {
+                mbar_init(&k_full[i], 1);
+                mbar_init(&v_full[i], 1);
+                mbar_init(&k_empty[i], 1);
+                mbar_init(&v_empty[i], 1);
+                mbar_init(&s_full[i], 1);
+                mbar_init(&p_full[i], 128);
+                mbar_init(&o_done[i], 1);
+                mbar_init(&q_full[i], 1);
+            }
+            fence_barrier_init();
+            if (p.q_by_tma) {
+                for (int q = 0; q < 2; ++q)
+                    if (nt[q] > 0) {
+                        mbar_arrive_expect_tx(&q_full[q], Q_BYTES);
+                        for (int h = 0; h < HALVES; ++h)
+                            tma_load_3d(q_s + q * Q_BYTES + h * (ROWS * 128), &map_q, &q_full[q], h * 64,
+                                        kv_head * p.group, t0 + (row0 + q * ROWS) / p.group);
+                    }
+            }
+        }
+        row = first_row_of(0);
+        __syncwarp();
+        load(0, 0, row);
+        load(1, 0, row);
+    } else if (warp == 1) {
         tmem_alloc(tmem_slot, 512);
         tmem_relinquish();
     }
-    // query rows -> shared memory in the swizzled K-major layout (all threads help)
-    {
-        // all of a thread's loads go out before the first store
+    if (!p.q_by_tma) {
+        // query rows -> shared memory in the swizzled K-major layout (all threads help), all of a thread's loads before the
+        // first store
         constexpr int PIECES = (2 * ROWS * (D / 8) + ATC2_THREADS - 1) / ATC2_THREADS;
         uint4 v[PIECES];
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
             const int c = threadIdx.x + i * ATC2_THREADS;
-            const int row = c / (D / 8), chunk = c - row * (D / 8);     // row 0 .. 255
-            const int r = row0 + row;
+            const int qrow = c / (D / 8), chunk = c - qrow * (D / 8);     // row 0 .. 255
+            const int r = row0 + qrow;
             v[i] = make_uint4(0, 0, 0, 0);
             if (c < 2 * ROWS * (D / 8) && r < rows_total) {
                 const int tok = r / p.group, h = r - tok * p.group;
@@ -571,77 +664,46 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
             const int c = threadIdx.x + i * ATC2_THREADS;
-            const int row = c / (D / 8), chunk = c - row * (D / 8);
+            const int qrow = c / (D / 8), chunk = c - qrow * (D / 8);
             if (c < 2 * ROWS * (D / 8))
-                *reinterpret_cast<uint4*>(q_s + (row >> 7) * Q_BYTES + (chunk >> 3) * (ROWS * 128)
-                                          + swizzled_chunk(row & 127, chunk & 7)) = v[i];
+                *reinterpret_cast<uint4*>(q_s + (qrow >> 7) * Q_BYTES + (chunk >> 3) * (ROWS * 128)
+                                          + swizzled_chunk(qrow & 127, chunk & 7)) = v[i];
         }
+        fence_proxy_async();           // the tensor core reads what these threads wrote
     }
-    fence_proxy_async();               // the tensor core reads what these threads wrote
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
-    timeline_mark(0);                  // the query rows are in shared memory
+    timeline_mark(0);                  // barriers and TMEM are there (and the query rows, if not by TMA)
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0) {
-        if (lane == 0) {
-            tma_prefetch_descriptor(&map_k);
-            tma_prefetch_descriptor(&map_v);
-        }
-        const int pages_per_tile = KEYS / p.page_size;
-        auto first_row_of = [&](int j) -> long long {
-            const int key = key_begin + j * KEYS + lane * p.page_size;
-            if (lane >= pages_per_tile || key >= key_end)
-                return p.cache_rows;      // past the context: read outside the array, zeros
-            const int page = table[key / p.page_size];
-            if (page < 0 || page >= p.num_pages) {
-                if (p.error)
-                    atomicExch(p.error, 3);
-                return p.cache_rows;
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ATC2_REGS_FEW));
+        if (warp == 0) {
+            for (int j = 1; j < n_tiles; ++j) {
+                row = first_row_of(j);
+                load(0, j, row);
+                load(1, j, row);
             }
-            return ((long long)page * p.nkv + kv_head) * p.page_size;
-        };
-        long long row = n_tiles > 0 ? first_row_of(0) : 0;
-        for (int j = 0; j < n_tiles; ++j) {
-            const long long row_next = j + 1 < n_tiles ? first_row_of(j + 1) : 0;
-            const int st = j & 1;
-            const uint32_t round = j >> 1;
-            for (int which = 0; which < 2; ++which) {       // keys, then values
-                uint64_t* full = which ? &v_full[st] : &k_full[st];
-                uint64_t* empty = which ? &v_empty[st] : &k_empty[st];
-                uint8_t* dst = (which ? v_s : k_s) + st * KV_TILE_BYTES;
-                if (lane == 0) {
-                    if (round > 0)
-                        mbar_wait(empty, (round - 1) & 1, p.error, 41);
-                    mbar_arrive_expect_tx(full, KV_TILE_BYTES);
-                }
-                __syncwarp();
-                if (lane < pages_per_tile) {
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(dst + h * (KEYS * 128) + lane * p.page_size * 128, which ? &map_v : &map_k,
-                                    full, h * 64, (int)row);
-                }
-            }
-            row = row_next;
-        }
-    } else if (warp == 1) {
-        if (elect_one()) {
+        } else if (warp == 1 && elect_one()) {
             constexpr uint32_t idesc_qk = make_idesc_bf16_f32(ROWS, KEYS);
             constexpr uint32_t idesc_pv = make_idesc_bf16_f32(ROWS, D) | (1u << 16);    // B is MN-major
             // tile 1 is the last user of a key/value tile that it needs at all
             auto last_user = [&](int q, int j) { return q == (j < nt[1] ? 1 : 0); };
+            // (descriptors of a tile's first 16 columns or keys; the others are constants away in units of 16 bytes)
+            const uint64_t q_desc = make_kmajor_sw128_desc(smem_addr(q_s)), k_desc = make_kmajor_sw128_desc(smem_addr(k_s));
+            const uint64_t v_desc = make_mnmajor_sw128_desc(smem_addr(v_s), KEYS * 128);
             auto issue_qk = [&](int q, int j) {
                 const int st = j & 1;
+                if (j == 0 && p.q_by_tma)
+                    mbar_wait(&q_full[q], 0, p.error, 49);
                 mbar_wait(&k_full[st], (j >> 1) & 1, p.error, 42);
                 tcgen05_fence_after();
-                const uint32_t q_addr = smem_addr(q_s + q * Q_BYTES);
-                const uint32_t k_addr = smem_addr(k_s + st * KV_TILE_BYTES);
+                const uint64_t a = q_desc + q * (Q_BYTES >> 4), b = k_desc + st * (KV_TILE_BYTES >> 4);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    const uint32_t off = (ks >> 2) * (ROWS * 128) + (ks & 3) * 32;
-                    tcgen05_mma_bf16(tmem_base + q * 128, make_kmajor_sw128_desc(q_addr + off),
-                                     make_kmajor_sw128_desc(k_addr + off), idesc_qk, ks > 0 ? 1u : 0u);
+                    const uint32_t off = ((ks >> 2) * (ROWS * 128) + (ks & 3) * 32) >> 4;
+                    tcgen05_mma_bf16(tmem_base + q * 128, a + off, b + off, idesc_qk, ks > 0 ? 1u : 0u);
                 }
                 tcgen05_commit(&s_full[q]);
                 if (last_user(q, j))
@@ -649,37 +711,37 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
             };
             auto issue_pv = [&](int q, int j) {
                 const int st = j & 1;
-                mbar_wait(&p_full[q], j & 1, p.error, 43);            // P_q(j) is in TMEM
                 mbar_wait(&v_full[st], (j >> 1) & 1, p.error, 44);
+                mbar_wait(&p_full[q], j & 1, p.error, 43);            // P_q(j) is in TMEM
                 tcgen05_fence_after();
-                const uint32_t v_addr = smem_addr(v_s + st * KV_TILE_BYTES);
+                const uint64_t b = v_desc + st * (KV_TILE_BYTES >> 4);
+                const uint32_t more = j > 0 ? 1u : 0u;
 #pragma unroll
                 for (int ks = 0; ks < KEYS / 16; ++ks)
-                    tcgen05_mma_bf16_a_tmem(tmem_base + 256 + q * 128, tmem_base + q * 128 + ks * 8,
-                                            make_mnmajor_sw128_desc(v_addr + ks * 16 * 128, KEYS * 128), idesc_pv,
-                                            (j > 0 || ks > 0) ? 1u : 0u);
+                    tcgen05_mma_bf16_a_tmem(tmem_base + 256 + q * 128, tmem_base + q * 128 + ks * 8, b + ks * (16 * 128 >> 4),
+                                            idesc_pv, ks > 0 ? 1u : more);
                 tcgen05_commit(&o_done[q]);
                 if (last_user(q, j))
                     tcgen05_commit(&v_empty[st]);
             };
-            for (int q = 0; q < 2; ++q)
-                if (nt[q] > 0)
-                    issue_qk(q, 0);
-            for (int j = 0; j < n_tiles; ++j) {
-                for (int q = 0; q < 2; ++q) {
-                    if (j < nt[q]) {
-                        issue_pv(q, j);
-                        if (j + 1 < nt[q])
-                            issue_qk(q, j + 1);       // S_q may be overwritten: the products of one thread run in order
-                    }
-                }
+            // one turn for each tile in order, the products of tile j - 1's probabilities before tile j's scores (S_q may be
+            // overwritten: the products of one thread run in order)
+#pragma unroll 1
+            for (int turn = 0; turn < 2 * (n_tiles + 1); ++turn) {
+                const int q = turn & 1, j = turn >> 1;
+                if (j > 0 && j - 1 < nt[q])
+                    issue_pv(q, j - 1);
+                if (j < nt[q])
+                    issue_qk(q, j);
             }
         }
+        __syncwarp();
     } else {
-        const int q = warp >= 6 ? 1 : 0;                     // this warp group's query tile
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ATC2_REGS_MANY));
+        const int q = warp >= 8 ? 1 : 0;                     // this warp group's query tile
         const int quarter = warp & 3;
-        const int row = quarter * 32 + lane;                 // this thread's row of the tile = its TMEM lane
-        const int r = row0 + q * ROWS + row;
+        const int row_in_tile = quarter * 32 + lane;         // this thread's row of the tile = its TMEM lane
+        const int r = row0 + q * ROWS + row_in_tile;
         const bool live = r < rows_total;
         const int tok = live ? r / p.group : 0;
         const int pos = live ? pos0 + tok : -1;
@@ -689,8 +751,8 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         const uint32_t o_addr = lane_addr + 256 + q * 128;
         const int my_tiles = nt[q];
         float m = -INFINITY, l = 0.f;
-        // options of the score: both passes over the row bring their piece to its final form (in
-        // units of log2) right after it is read, and the scale below is 1
+        // with options of the score a row is brought to its final form (in units of log2) right after it is read, and the
+        // scale below is 1
         constexpr bool options = OPT == OPT_ANY || OPT == OPT_CAP;
         const float sl2 = OPT != OPT_NONE ? 1.f : p.scale_log2;
         const int bias_head = kv_head * p.group + (live ? r - tok * p.group : 0);
@@ -700,83 +762,62 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         for (int j = 0; j < my_tiles; ++j) {
             const int st = j & 1;
             const int key0 = key_begin + j * KEYS;
-            mbar_wait(&s_full[q], j & 1, p.error, 45);
+            mbar_wait_warp(&s_full[q], j & 1, p.error, 45);
             tcgen05_fence_after();
-
-            // Two passes over the S row in TMEM, 32 columns at a time (the next piece is on its way
-            // while this one is worked on): the maximum, then P = exp2(S * scale - m) as packed
-            // bfloat16 pairs, which overwrite the columns of S already read.
-            const bool masked = __any_sync(0xffffffffu, key0 + KEYS - 1 > pos || key0 < first);
-            // With options the first pass brings a piece to its final form and writes it back to its
-            // columns; the second pass reads finished (and masked) scores and changes nothing.
-            // With a linear bias alone both passes make the scores anew; the second takes the exponents' base off
-            // on the way.
-            const float slope = OPT == OPT_LINEAR ? r1 * 1.4426950408889634f : 0.f;
-            const float at0 = OPT == OPT_LINEAR ? slope * (float)(key0 - pos) : 0.f;
-            auto mask_piece = [&](uint32_t (&v)[32], int c0, bool second = false, float off = 0.f) {
-                if (options && second)
-                    return;
-                if (OPT == OPT_LINEAR) {
+            uint32_t sv[KEYS];
 #pragma unroll
-                    for (int i = 0; i < 32; ++i)
-                        v[i] = __float_as_uint(fmaf(__uint_as_float(v[i]), p.scale_log2, fmaf((float)(c0 + i), slope, at0 - off)));
-                }
-                if (OPT == OPT_CAP) {
-                    cap_scores(v, p.scale, p.softcap, two_over_cap_log2);
-                } else if (options) {
+            for (int c0 = 0; c0 < KEYS; c0 += 32)
+                tmem_load_32x32(s_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(&sv[c0]));
+            tmem_load_wait();
+            if (OPT == OPT_LINEAR) {
+                // score - slope * (pos - key), in units of log2; keys after pos are masked below
+                const float slope = r1 * 1.4426950408889634f, at0 = slope * (float)(key0 - pos);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        float x = __uint_as_float(v[i]) * p.scale;
-                        if (p.softcap > 0.f)
-                            x = p.softcap * (1.f - __fdividef(2.f, fast_exp2(x * two_over_cap_log2) + 1.f));
-                        const int dist = pos - (key0 + c0 + i);
-                        x -= linear_bias ? r1 * (float)(dist > 0 ? dist : 0) : r1 * __logf(1.f + r2 * (float)(dist > 0 ? dist : 0));
-                        v[i] = __float_as_uint(x * 1.4426950408889634f);
-                    }
-                }
-                if (masked) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int key = key0 + c0 + i;
-                        if (!(key <= pos && key >= first))
-                            v[i] = 0xff800000u;              // -inf
-                    }
-                }
-            };
-            uint32_t pa[32], pb[32];
-            float mx4[4] = { -INFINITY, -INFINITY, -INFINITY, -INFINITY };
-            tmem_load_32x32(s_addr, pa);
-#pragma unroll
-            for (int c0 = 0; c0 < KEYS; c0 += 64) {
-                tmem_load_wait();
-                tmem_load_32x32(s_addr + c0 + 32, pb);
-                mask_piece(pa, c0);
-                if (options)
-                    tmem_store_32x32(s_addr + c0, pa);
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(pa[i]));
-                tmem_load_wait();
-                if (c0 + 64 < KEYS)
-                    tmem_load_32x32(s_addr + c0 + 64, pa);
-                mask_piece(pb, c0 + 32);
-                if (options)
-                    tmem_store_32x32(s_addr + c0 + 32, pb);
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(pb[i]));
+                for (int i = 0; i < KEYS; ++i)
+                    sv[i] = __float_as_uint(fmaf(__uint_as_float(sv[i]), p.scale_log2, fmaf((float)i, slope, at0)));
             }
-            if (options)
-                tmem_store_wait();                           // the finished scores are in their columns
-            tmem_load_32x32(s_addr, pa);                     // the second pass starts while the maximum settles
+            if (OPT == OPT_CAP) {
+                cap_scores(sv, p.scale, p.softcap, two_over_cap_log2);
+            } else if (options) {
+#pragma unroll
+                for (int i = 0; i < KEYS; ++i) {
+                    float x = __uint_as_float(sv[i]) * p.scale;
+                    if (p.softcap > 0.f)
+                        x = p.softcap * (1.f - __fdividef(2.f, fast_exp2(x * two_over_cap_log2) + 1.f));
+                    const int dist = pos - (key0 + i);
+                    x -= linear_bias ? r1 * (float)(dist > 0 ? dist : 0) : r1 * __logf(1.f + r2 * (float)(dist > 0 ? dist : 0));
+                    sv[i] = __float_as_uint(x * 1.4426950408889634f);
+                }
+            }
+            // masks only where a row's visible range ends inside the tile; the warp takes one path
+            if (__any_sync(0xffffffffu, key0 + KEYS - 1 > pos || key0 < first)) {
+#pragma unroll
+                for (int i = 0; i < KEYS; ++i) {
+                    const int key = key0 + i;
+                    if (!(key <= pos && key >= first))
+                        sv[i] = 0xff800000u;                 // -inf
+                }
+            }
+            float mx4[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                mx4[u] = max3(__uint_as_float(sv[u]), __uint_as_float(sv[u + 4]), __uint_as_float(sv[u + 8]));
+#pragma unroll
+            for (int i = 12; i < KEYS - 4; i += 8) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    mx4[u] = max3(mx4[u], __uint_as_float(sv[i + u]), __uint_as_float(sv[i + 4 + u]));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                mx4[u] = fmaxf(mx4[u], __uint_as_float(sv[KEYS - 4 + u]));
             float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            mx *= sl2;                                     // the scale is positive
+            mx *= sl2;                                       // the scale is positive
             const bool grow = mx > m + 8.f;                  // also true for the first visible key (m = -inf)
             if (__any_sync(0xffffffffu, grow && m != -INFINITY && j > 0)) {
                 // rescale what has accumulated: the product of tile j-1 must have landed first
-                mbar_wait(&o_done[q], (j - 1) & 1, p.error, 46);
+                mbar_wait_warp(&o_done[q], (j - 1) & 1, p.error, 46);
                 tcgen05_fence_after();
-                tmem_load_wait();
                 rescale_output_row(o_addr, (grow && m != -INFINITY) ? fast_exp2(m - mx) : 1.f);
             }
             if (grow) {
@@ -784,38 +825,30 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 m = mx;
             }
             const float base = m == -INFINITY ? 0.f : m;
-            float sum4[4] = { 0.f, 0.f, 0.f, 0.f };
-            auto exp_piece = [&](uint32_t (&v)[32], int c0) {
-                mask_piece(v, c0, true, base);
+            const uint64_t scale2 = pair_of(sl2, sl2), base2 = pair_of(-base, -base);
+            uint64_t sum2[4] = { 0, 0, 0, 0 };
+#pragma unroll
+            for (int c0 = 0; c0 < KEYS; c0 += 32) {
                 uint32_t packed[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float a = __uint_as_float(v[2 * i]), b = __uint_as_float(v[2 * i + 1]);
-                    const float p0 = fast_exp2(OPT == OPT_LINEAR ? a : fmaf(a, sl2, -base));
-                    const float p1 = fast_exp2(OPT == OPT_LINEAR ? b : fmaf(b, sl2, -base));
-                    sum4[i & 3] += p0 + p1;
+                    const uint64_t s2 = pair_of(__uint_as_float(sv[c0 + 2 * i]), __uint_as_float(sv[c0 + 2 * i + 1]));
+                    const float2 e = halves_of(OPT == OPT_NONE ? pair_fma(s2, scale2, base2) : pair_add(s2, base2));
+                    const float p0 = fast_exp2(e.x), p1 = fast_exp2(e.y);
+                    sum2[i & 3] = pair_add(sum2[i & 3], pair_of(p0, p1));
                     const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
                     packed[i] = *reinterpret_cast<const uint32_t*>(&h);
                 }
-                tmem_store_32x16(s_addr + (c0 >> 1), packed);   // behind the columns still to be read
-            };
-#pragma unroll
-            for (int c0 = 0; c0 < KEYS; c0 += 64) {
-                tmem_load_wait();
-                tmem_load_32x32(s_addr + c0 + 32, pb);
-                exp_piece(pa, c0);
-                tmem_load_wait();
-                if (c0 + 64 < KEYS)
-                    tmem_load_32x32(s_addr + c0 + 64, pa);
-                exp_piece(pb, c0 + 32);
+                tmem_store_32x16(s_addr + (c0 >> 1), packed);
             }
-            l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            const float2 s01 = halves_of(pair_add(sum2[0], sum2[1])), s23 = halves_of(pair_add(sum2[2], sum2[3]));
+            l += (s01.x + s01.y) + (s23.x + s23.y);
             // values past the context may be anything (a page is loaded whole): make them zero, so
             // that 0 * value stays 0.  Only the CTA's last tile can hold such keys.
             if (key0 + KEYS > key_end) {
                 mbar_wait(&v_full[st], (j >> 1) & 1, p.error, 47);
                 uint8_t* v_tile = v_s + st * KV_TILE_BYTES;
-                for (int c = row; c < (key0 + KEYS - key_end) * (D / 8); c += 128) {
+                for (int c = row_in_tile; c < (key0 + KEYS - key_end) * (D / 8); c += 128) {
                     const int krow = key_end - key0 + c / (D / 8), chunk = c % (D / 8);
                     *reinterpret_cast<uint4*>(v_tile + (chunk >> 3) * (KEYS * 128) + swizzled_chunk(krow, chunk & 7)) =
                         make_uint4(0, 0, 0, 0);
@@ -829,29 +862,39 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 timeline_mark(1);      // the first tile's probabilities are written
         }
         timeline_mark(2);              // the last tile's probabilities are written
-        // the last product has landed: normalise and write the rows out
+        // The last product has landed: normalise, and write the rows out by way of the tile's query rows (which are done
+        // with): neighbouring lanes then store neighbouring pieces of a row.
         if (my_tiles > 0) {
-            mbar_wait(&o_done[q], (my_tiles - 1) & 1, p.error, 48);
+            mbar_wait_warp(&o_done[q], (my_tiles - 1) & 1, p.error, 48);
             tcgen05_fence_after();
             const int head = kv_head * p.group + (live ? r - tok * p.group : 0);      // (rows past the end have none)
             l += sink_weight(p.sink, head, m);
             const float inv = l > 0.f ? 1.f / l : 0.f;
-            __nv_bfloat16* dst_row = p.out + ((size_t)(t0 + tok) * p.nq + head) * D;
+            uint8_t* const tile = q_s + q * Q_BYTES + quarter * 32 * (D * 2);         // 32 rows of this warp
+            constexpr int CHUNKS = D / 8;
+            uint32_t ov[D];
 #pragma unroll
-            for (int c0 = 0; c0 < D; c0 += 32) {
-                uint32_t ov[32];
-                tmem_load_32x32(o_addr + c0, ov);
-                tmem_load_wait();
-                if (live) {
+            for (int c0 = 0; c0 < D; c0 += 32)
+                tmem_load_32x32(o_addr + c0, *reinterpret_cast<uint32_t(*)[32]>(&ov[c0]));
+            tmem_load_wait();
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        __nv_bfloat162 h[4];
+            for (int c = 0; c < CHUNKS; ++c) {
+                __nv_bfloat162 h[4];
 #pragma unroll
-                        for (int u = 0; u < 4; ++u)
-                            h[u] = __floats2bfloat162_rn(__uint_as_float(ov[8 * c + 2 * u]) * inv,
-                                                         __uint_as_float(ov[8 * c + 2 * u + 1]) * inv);
-                        reinterpret_cast<uint4*>(dst_row + c0)[c] = *reinterpret_cast<uint4*>(h);
-                    }
+                for (int u = 0; u < 4; ++u)
+                    h[u] = __floats2bfloat162_rn(__uint_as_float(ov[8 * c + 2 * u]) * inv,
+                                                 __uint_as_float(ov[8 * c + 2 * u + 1]) * inv);
+                *reinterpret_cast<uint4*>(tile + lane * (D * 2) + ((c ^ (lane & 7)) << 4)) = *reinterpret_cast<uint4*>(h);
+            }
+            __syncwarp();
+            const int warp_row0 = row0 + q * ROWS + quarter * 32;
+#pragma unroll 4
+            for (int i = lane; i < 32 * CHUNKS; i += 32) {
+                const int rr = i / CHUNKS, c = i % CHUNKS, at = warp_row0 + rr;
+                if (at < rows_total) {
+                    const int t = at / p.group, h = at - t * p.group;
+                    *reinterpret_cast<uint4*>(p.out + ((size_t)(t0 + t) * p.nq + kv_head * p.group + h) * D + 8 * c) =
+                        *reinterpret_cast<const uint4*>(tile + rr * (D * 2) + ((c ^ (rr & 7)) << 4));
                 }
             }
         }
@@ -960,9 +1003,10 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
         || !tensor_map_2d(v_cache, p.cache_rows, D, D, page_size, &mv))
         return CHIBI_ERR_UNSUPPORTED;
     using Kernel = void (*)(const CUtensorMap, const CUtensorMap, const AttnTcParams);
+    using Kernel2 = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnTcParams);
     static const Kernel one_tile[4] = { attn_prefill_tc_kernel<OPT_NONE>, attn_prefill_tc_kernel<OPT_ANY>,
                                         attn_prefill_tc_kernel<OPT_LINEAR>, attn_prefill_tc_kernel<OPT_CAP> };
-    static const Kernel two_tiles[4] = { attn_prefill_tc2_kernel<OPT_NONE>, attn_prefill_tc2_kernel<OPT_ANY>,
+    static const Kernel2 two_tiles[4] = { attn_prefill_tc2_kernel<OPT_NONE>, attn_prefill_tc2_kernel<OPT_ANY>,
                                          attn_prefill_tc2_kernel<OPT_LINEAR>, attn_prefill_tc2_kernel<OPT_CAP> };
     static bool configured = false;
     if (!configured) {
@@ -970,6 +1014,12 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
             cudaError_t e = cudaFuncSetAttribute(one_tile[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC_SMEM);
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(two_tiles[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC2_SMEM);
+            // (a softmax group that asked for more registers than the block was launched with would wait for good)
+            cudaFuncAttributes attr {};
+            if (e == cudaSuccess)
+                e = cudaFuncGetAttributes(&attr, two_tiles[i]);
+            if (e == cudaSuccess && attr.numRegs < ATC2_REGS)
+                return CHIBI_ERR_ARGUMENT;
             if (e != cudaSuccess)
                 return (int)e;
         }
@@ -988,7 +1038,9 @@ CHIBI_API int chibi_attention_prefill_tc(const void* q, const void* k_cache, con
              && one_tile_is_faster(rows, p.group, max_q_len, max_ctx_len, tokens, nkv, window, chunk, sms));
     if (variant == 2 || (variant == 0 && two)) {
         const dim3 grid2((unsigned)((rows + 2 * ROWS - 1) / (2 * ROWS)), nkv, seqs);
-        launch(two_tiles[options], grid2, dim3(ATC2_THREADS), ATC2_SMEM, stream, mk, mv, p);
+        CUtensorMap mq = mk;                          // (not used where a tile's rows are not whole tokens)
+        p.q_by_tma = tokens > 0 && ROWS % p.group == 0 && tensor_map_of_heads(q, tokens, nq, D, p.group, ROWS / p.group, &mq);
+        launch(two_tiles[options], grid2, dim3(ATC2_THREADS), ATC2_SMEM, stream, mq, mk, mv, p);
         return launch_status();
     }
     if (kv_splits > 1) {

@@ -92,6 +92,22 @@ inline bool tensor_map_of_rows(const void* ptr, long long rows, long long cols, 
     return true;
 }
 
+// A map over [tokens][heads][d] bfloat16, without gaps: a box is 64 columns of box_heads heads of box_tokens tokens, token by
+// token.  (Made anew by each call: activations do not stay where they are as caches and weights do.)
+inline bool tensor_map_of_heads(const void* ptr, long long tokens, int heads, int d, int box_heads, int box_tokens, CUtensorMap* out)
+{
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn)
+        return false;
+    const cuuint64_t dims[3] = { (cuuint64_t)d, (cuuint64_t)heads, (cuuint64_t)tokens };
+    const cuuint64_t strides[2] = { (cuuint64_t)d * 2, (cuuint64_t)heads * d * 2 };
+    const cuuint32_t box[3] = { (cuuint32_t)TENSOR_MAP_BOX_COLS, (cuuint32_t)box_heads, (cuuint32_t)box_tokens };
+    const cuuint32_t elem[3] = { 1, 1, 1 };
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, elem,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 inline bool tensor_map_2d(const void* ptr, long long rows, long long cols, long long stride, int box_rows,
                           CUtensorMap* out)
 {
