@@ -1,13 +1,16 @@
 // Causal grouped-query attention of the 32-bit path over the paged cache, head sizes 64 and 128: all operands and
-// results 32-bit, scores and sums by 32-bit multiply-adds (attention_generic.cu says what is computed and which options
+// results 32-bit (attention_generic.cu says what is computed and which options
 // the scores have; it takes the other sizes and types).  Two kernels, one for the sequences that bring one token to a step
 // and one for those that bring more.  In both, the order of a row's operations depends on its own position (and on
 // whether it came alone), never on the batch around it.
 #define CHIBI_UNIT attention_f32
 #define CHIBI_UNIT_ID 17
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace chibi {
+
+using namespace sm100;
 
 struct AttentionF32 {
     const float* q;
@@ -101,265 +104,529 @@ __device__ __forceinline__ float af_score(const AttentionF32& p, float dot, floa
 __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -INFINITY ? 0.f : expf(m - m_new); }
 
 // ---------------------------------------------------------------- sequences that bring several tokens
-// grid (4 CTAs for each row tile, kv heads, sequences), 128 threads.  A tile is 64 rows, the group's heads of
-// neighbouring tokens; the keys are taken 32 at a time, from a multiple of 32 on, and blocks of 64 keys (counted from the
-// sequence's start) go to the four CTAs of a cluster in turn, which add up what they found at the end: a causal
-// tile's keys spread evenly, and few rows make four times the CTAs (three prompts of up to 400 tokens of 16 heads:
-// 137 us with one CTA a tile).  A thread owns rows ty + 16 i; of the scores
-// the keys tx + 8 j, of the output the columns 4 tx + 32 j .. + 3, so a row's eight threads sit side by side in a warp:
-// its maximum and sum are three shuffles, and its probabilities reach them through shared memory without a block
-// barrier.  The next keys are fetched while the values are used and the other way round.  Scores take two
-// neighbouring features at a time (fma.rn.f32x2), the output two neighbouring columns.  Bound by the reads of
-// shared memory beside the multiply-adds (8 reads of 16 bytes, 32 cycles, to 16 cycles of multiply-adds for the
-// scores; 80 to 64 for the output); 76 KB a CTA, three to an SM.
-constexpr int AF_ROWS = 64, AF_KEYS = 32, AF_P = AF_KEYS + 4, AF_RANKS = 4, AF_BLOCK = 64;
+// On the 5th-generation tensor cores.  A 32-bit number is the sum of three bfloat16 numbers (its leading 8 bits, the next
+// 8 of what is left, the last 8, each rounded to nearest), so a product of two is the sum of nine exact products of 8 by
+// 8 bits; the three smallest (below 2^-26 of the whole) are left out, the other six are tcgen05.mma with 32-bit
+// accumulators.  What limits the precision is the accumulator, which the tensor core cuts off instead of rounding: so
+// every sum over 64 features or keys has an accumulator of its own, that takes the five small products first and the
+// large one last, and those sums are added in plain 32-bit arithmetic.  Relative error against 64 bits, 3 prompts of up to
+// 400 tokens: 1.6e-7, by multiply-adds (fma.rn.f32x2) before 2.1e-7.
+//
+// A CTA owns 128 query rows of one kv head, (token, head of the group) pairs, and walks over the keys in blocks of 64, counted
+// from the sequence's start: what a row gives does not depend on the rows beside it (a key that it does not see has
+// probability 0 and leaves its sums as they are).  Warp 0 issues the MMAs.  Warps 4 to 19 do the rest: four threads own a
+// row, a quarter of a block's keys and of the output's columns each; all of them bring queries, keys and values (in registers, a
+// block ahead), split them and write the parts into the swizzled tiles that the MMAs read; probabilities go through TMEM as the
+// A operand.  S = Q K^T of the next block runs while a block's softmax is made, O = P V while the next keys are split.
+// Bound by the products beside the threads' work: 48 MMAs of 128 x 64 x 16 (shared memory: 48 cycles each) and 24 of
+// 128 x D x 16 (64) a block, 3,900 cycles for heads of 128.  An issuing thread waits while they run (issued by one of the
+// working warps a block took 11,400).  Heads of 128, us by multiply-adds (64 rows a CTA, four CTAs to a row tile's keys) and
+// so: 3 prompts of up to 400 tokens of 16 heads 109 and 38, 4 of up to 600 after 800 of 32 heads 1,235 and 322, 64 tokens after 800
+// of 16 heads 86 and 64, 100 after 4,000 417 and 298, 4 after 800 78 and 59.
+//
+// Numbers that are none: a key or query with one marks its scores, which are then summed by multiply-adds; a value adds
+// itself to the columns of the rows that see it.
+constexpr int AT_ROWS = 128, AT_KEYS = 64, AT_WORKERS = 512, AT_THREADS = 128 + AT_WORKERS;
+constexpr int AT_REGS = 96, AT_REGS_FEW = 32, AT_REGS_MANY = 112;    // of a thread at launch, of the first four warps', of the others'
+static_assert(AT_REGS_FEW + 4 * AT_REGS_MANY <= 5 * AT_REGS, "more registers than the block has");
+constexpr int AT_SHARE = AT_WORKERS / AT_ROWS, AT_OWN = AT_KEYS / AT_SHARE;     // threads of a row; keys of a thread
 
-template <int D> constexpr size_t af_shared()
+template <int D> struct AtShape {
+    static constexpr int SLICES = D / 64;                        // 64 features are a swizzled line
+    static constexpr int Q_PLANE = AT_ROWS * D * 2, KV_PLANE = AT_KEYS * D * 2;
+    static constexpr int TILES = 3 * Q_PLANE + 6 * KV_PLANE;
+    static constexpr size_t SHARED = 1024 + TILES + 64 + 4 * (AT_SHARE * AT_ROWS + 20 + AT_ROWS);
+    static constexpr uint32_t S_COLS = 64 * SLICES;              // TMEM: two buffers of S, three parts of P, O
+    static constexpr uint32_t P_AT = 2 * S_COLS, O_AT = P_AT + 96, TMEM = O_AT + D <= 256 ? 256 : 512;
+};
+
+__device__ __forceinline__ uint32_t at_pair(float a, float b)
 {
-    return sizeof(float) * (AF_ROWS * (D + 4) + AF_KEYS * (D + 4) + AF_KEYS * D + AF_ROWS * AF_P);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
+// What is left of two numbers without their bfloat16 parts (exact).
+__device__ __forceinline__ uint64_t at_rest(uint64_t v, uint32_t pair)
+{
+    const uint64_t parts = af_pair(__uint_as_float(pair << 16), __uint_as_float(pair & 0xffff0000u));
+    return af_fma2(parts, 0xbf800000bf800000ull, v);             // (-1, -1)
+}
+__device__ __forceinline__ uint32_t at_pair(uint64_t v)
+{
+    const float2 h = af_halves(v);
+    return at_pair(h.x, h.y);
+}
+__device__ __forceinline__ void at_put(uint32_t at, uint32_t a, uint32_t b)
+{
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
+}
+// A number whose leading part would be infinite: none (0 and true), or so large that its part is cut off instead of rounded.
+__device__ __noinline__ bool at_odd_parts(float v, uint32_t parts[3])
+{
+    parts[0] = parts[1] = parts[2] = 0;
+    if (!(fabsf(v) < INFINITY))
+        return true;
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t cut = __float_as_uint(v) & 0xffff0000u;
+        parts[i] = cut >> 16;
+        v -= __uint_as_float(cut);
+    }
+    return false;
+}
+// Writes the three parts of four numbers, `plane` bytes apart; adds to `none` what is no number if one of them is none, or so
+// large that its leading part is infinite.
+__device__ __forceinline__ void at_split(float4 v, uint32_t at, uint32_t plane, uint64_t& none)
+{
+    uint64_t x = af_pair(v.x, v.y), y = af_pair(v.z, v.w);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t a = at_pair(x), b = at_pair(y);
+        at_put(at + i * plane, a, b);
+        if (i < 2) {
+            x = at_rest(x, a);
+            y = at_rest(y, b);
+        }
+    }
+    none = af_fma2(x, 0x3f8000003f800000ull, af_fma2(y, 0x3f8000003f800000ull, none));      // (infinite parts leave no numbers)
+}
+// The same for numbers among which some are none or very large; true if one is none (its parts are 0 then).
+__device__ __noinline__ bool at_split_odd(float4 v, uint32_t at, uint32_t plane)
+{
+    uint32_t parts[4][3];
+    bool none = at_odd_parts(v.x, parts[0]);
+    none |= at_odd_parts(v.y, parts[1]);
+    none |= at_odd_parts(v.z, parts[2]);
+    none |= at_odd_parts(v.w, parts[3]);
+    for (int i = 0; i < 3; ++i)
+        at_put(at + i * plane, parts[0][i] | parts[1][i] << 16, parts[2][i] | parts[3][i] << 16);
+    return none;
+}
+__device__ __forceinline__ bool at_none(uint64_t v)
+{
+    const float2 h = af_halves(v);
+    return !(fabsf(h.x + h.y) < INFINITY);
+}
+__device__ __noinline__ float at_dot(const float* a, const float* b, int d)
+{
+    float s = 0.f;
+    for (int i = 0; i < d; ++i)
+        s = fmaf(a[i], b[i], s);
+    return s;
+}
+// The warps that share 32 rows.
+__device__ __forceinline__ void at_row_sync(int barrier)
+{
+    asm volatile("barrier.cta.sync.aligned %0, %1;" ::"r"(barrier), "n"(32 * AT_SHARE) : "memory");
+}
+// MN-major operand (V: [key][d]) in swizzled slices of 64 columns, `slice` bytes apart.
+__device__ __forceinline__ uint64_t at_values_desc(uint32_t smem_byte_addr, uint32_t slice)
+{
+    return static_cast<uint64_t>((smem_byte_addr & 0x3ffff) >> 4) | static_cast<uint64_t>((slice >> 4) & 0x3fff) << 16
+        | static_cast<uint64_t>(1024 >> 4) << 32 | static_cast<uint64_t>(1) << 46 | static_cast<uint64_t>(2) << 61;
 }
 
-template <int D>
-__global__ void __launch_bounds__(128, 3)
+template <int COUNT> __device__ __forceinline__ void at_tmem_load(uint32_t at, uint32_t (&r)[COUNT])
+{
+    static_assert(COUNT == 16 || COUNT == 32);
+    if constexpr (COUNT == 32)
+        tmem_load_32x32(at, r);
+    else
+        tmem_load_32x16(at, r);
+}
+
+template <int D, bool OPTIONS>
+__global__ void __launch_bounds__(AT_THREADS, 1)
 attention_f32_prompt_kernel(const AttentionF32 p)
 {
     pdl_enter();
-    constexpr int DS = D + 4, QUADS = D / 4, CJ = D / 32;
-    extern __shared__ __align__(16) float af_sm[];
-    float* const Q = af_sm;                             // [AF_ROWS][DS]
-    float* const K = Q + AF_ROWS * DS;                  // [AF_KEYS][DS]
-    float* const V = K + AF_KEYS * DS;                  // [AF_KEYS][D]
-    float* const P = V + AF_KEYS * D;                   // [AF_ROWS][AF_P]
-    const int tid = threadIdx.x, lane = tid & 31, tx = tid & 7, ty = tid >> 3;
+    using Shape = AtShape<D>;
+    constexpr int QUADS = D / 4, PASS = AT_WORKERS / QUADS;      // rows that all threads bring at a time
+    constexpr int KV_EACH = AT_KEYS / PASS, Q_EACH = AT_ROWS / PASS;
+    extern __shared__ uint8_t at_raw[];
+    uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(at_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t q_s = smem_addr(smem), k_s = q_s + 3 * Shape::Q_PLANE, v_s = k_s + 3 * Shape::KV_PLANE;
+    uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + Shape::TILES);
+    uint64_t* const keys_there = bars;           // working threads: the keys are written
+    uint64_t* const p_there = bars + 1;          // working threads: probabilities and values are written
+    uint64_t* const s_done = bars + 2;           // MMA commit
+    uint64_t* const o_done = bars + 3;           // MMA commit
+    uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
+    float* const exchange = reinterpret_cast<float*>(bars + 8);          // [4][128]
+    // marks of what holds a number that is none: keys [4][2] and values [4][2] of a block's 64 (block j in place j % 4), any at
+    // all, queries [128]
+    uint32_t* const odd_keys = reinterpret_cast<uint32_t*>(exchange + AT_SHARE * AT_ROWS);
+    uint32_t* const odd_values = odd_keys + 8;
+    uint32_t* const odd_any = odd_values + 8;
+    int* const odd_row = reinterpret_cast<int*>(odd_any + 4);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int seq = blockIdx.z, kv_head = blockIdx.y, G = p.nq / p.nkv;
     const int row0 = p.q_start[seq], q_len = p.q_start[seq + 1] - row0;
     if (q_len <= 1)
-        return;                                         // (a single token is the other kernel's)
-    const int all_rows = q_len * G, tiles = (all_rows + AF_ROWS - 1) / AF_ROWS;
-    const int pos0 = p.ctx_len[seq] - q_len;            // the first token's position
+        return;                                                  // (a single token is the other kernel's)
+    const int all_rows = q_len * G, tile = (all_rows + AT_ROWS - 1) / AT_ROWS - 1 - (int)blockIdx.x;     // most keys first
+    if (tile < 0)
+        return;
+    const int pos0 = p.ctx_len[seq] - q_len;                     // the first token's position
     const int* const table = p.block_table + (size_t)(p.seq_rows ? p.seq_rows[seq] : seq) * p.table_stride;
+    const int first_row = tile * AT_ROWS, last_pos = pos0 + (min(first_row + AT_ROWS, all_rows) - 1) / G;
+    const int oldest = first_visible_key(pos0 + first_row / G, p.window, p.chunk);      // (older pages may be gone)
+    const int begin = oldest / AT_KEYS * AT_KEYS, blocks = (last_pos - begin) / AT_KEYS + 1;
 
-    const int rank = blockIdx.x % AF_RANKS;
-    float* const ml = P;                                // at the end: [AF_ROWS] maxima, [AF_ROWS] sums
-    float* const part = K;                              // and, over keys and values, [AF_ROWS][D] sums
+    if (tid == 0) {
+        mbar_init(keys_there, AT_WORKERS);
+        mbar_init(p_there, AT_WORKERS);
+        mbar_init(s_done, 1);
+        mbar_init(o_done, 1);
+        fence_barrier_init();
+    }
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, Shape::TMEM);
+        tmem_relinquish();
+    }
+    if (tid < AT_ROWS)
+        odd_row[tid] = 0;
+    if (tid < 20)
+        odd_keys[tid] = 0;
 
-    // the tiles with the most keys first
-    for (int tile = tiles - 1 - (int)blockIdx.x / AF_RANKS; tile >= 0; tile -= gridDim.x / AF_RANKS) {
-        const int first_row = tile * AF_ROWS, last_row = min(first_row + AF_ROWS, all_rows) - 1;
-        const int last_pos = pos0 + last_row / G;
-        const int oldest = first_visible_key(pos0 + first_row / G, p.window, p.chunk);      // (older pages may be gone)
-        const int visible = oldest & ~(AF_KEYS - 1);
-        // this CTA's blocks: those whose number is rank modulo AF_RANKS
-        const int block = visible / AF_BLOCK, mine = block + (rank + AF_RANKS - block % AF_RANKS) % AF_RANKS;
-        const int begin = mine == block ? visible : mine * AF_BLOCK;
-        auto after = [&](int base) {
-            const int next = base + AF_KEYS;
-            return next % AF_BLOCK ? next : next + (AF_RANKS - 1) * AF_BLOCK;
-        };
-        __syncthreads();                                // (the tile before is through)
-        for (int c = tid; c < AF_ROWS * QUADS; c += 128) {
-            const int r = c / QUADS, at = 4 * (c % QUADS), row = first_row + r;
-            const bool there = row < all_rows;
-            af_copy16(Q + r * DS + at,
-                      there ? p.q + ((size_t)(row0 + row / G) * p.nq + kv_head * G + row % G) * D + at : p.q, there ? 16 : 0);
-        }
-        // rows of keys or values: lane l looks the page of key l up, a row is copied by QUADS threads
-        unsigned usable = 0;                            // keys of the tile whose page is one of the pool's
-        auto fetch = [&](const float* cache, float* dst, int stride, int base) {
-            const int u = base + lane;
-            long long at = -1;
-            if (u >= oldest && u <= last_pos) {
-                const int page = table[u / p.page_size];
-                if (page < 0 || page >= p.num_pages) {
-                    if (p.error)
-                        atomicExch(p.error, 3);
-                } else {
-                    at = (((long long)page * p.nkv + kv_head) * p.page_size + u % p.page_size) * D;
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AT_REGS_FEW));
+        if (warp == 0 && elect_one()) {
+            constexpr uint32_t idesc_s = make_idesc_bf16_f32(AT_ROWS, AT_KEYS), idesc_o = make_idesc_bf16_f32(AT_ROWS, D) | (1u << 16);
+            const uint64_t q_desc = make_kmajor_sw128_desc(q_s), k_desc = make_kmajor_sw128_desc(k_s);
+            const uint64_t v_desc = at_values_desc(v_s, AT_KEYS * 128);
+            auto scores = [&](int j) {
+                uint64_t a = q_desc, b = k_desc;
+                asm volatile("" : "+l"(a), "+l"(b));                 // (or 48 sums of constants wait in registers from block to block)
+                mbar_wait(keys_there, j & 1, p.error, 71);
+                tcgen05_fence_after();
+#pragma unroll
+                for (int slice = 0; slice < Shape::SLICES; ++slice) {
+                    const uint32_t d = tmem + (j & 1) * Shape::S_COLS + slice * 64;
+                    auto product = [&](int pq, int pk, int ks, uint32_t more) {
+                        tcgen05_mma_bf16(d, a + ((pq * Shape::Q_PLANE + slice * AT_ROWS * 128 + ks * 32) >> 4),
+                                         b + ((pk * Shape::KV_PLANE + slice * AT_KEYS * 128 + ks * 32) >> 4), idesc_s, more);
+                    };
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        product(2, 0, ks, ks > 0 ? 1u : 0u);
+                        product(1, 1, ks, 1u);
+                        product(1, 0, ks, 1u);
+                        product(0, 2, ks, 1u);
+                        product(0, 1, ks, 1u);
+                    }
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        product(0, 0, ks, 1u);
                 }
+                tcgen05_commit(s_done);
+            };
+            auto outputs = [&](int j) {
+                uint64_t b = v_desc;
+                asm volatile("" : "+l"(b));
+                mbar_wait(p_there, j & 1, p.error, 72);
+                tcgen05_fence_after();
+                auto product = [&](int pp, int pv, int ks, uint32_t more) {
+                    tcgen05_mma_bf16_a_tmem(tmem + Shape::O_AT, tmem + Shape::P_AT + pp * 32 + ks * 8,
+                                            b + ((pv * Shape::KV_PLANE + ks * 16 * 128) >> 4), idesc_o, more);
+                };
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                    product(2, 0, ks, ks > 0 ? 1u : 0u);
+                    product(1, 1, ks, 1u);
+                    product(1, 0, ks, 1u);
+                    product(0, 2, ks, 1u);
+                    product(0, 1, ks, 1u);
+                }
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                    product(0, 0, ks, 1u);
+                tcgen05_commit(o_done);
+            };
+            scores(0);
+            for (int j = 0; j < blocks; ++j) {
+                if (j + 1 < blocks)
+                    scores(j + 1);
+                outputs(j);
             }
-#pragma unroll
-            for (int i = 0; i < AF_KEYS * QUADS / 128; ++i) {
-                const int c = tid + 128 * i, r = c / QUADS, x = 4 * (c % QUADS);
-                const long long from = __shfl_sync(0xffffffffu, at, r);
-                af_copy16(dst + r * stride + x, from >= 0 ? cache + from + x : cache, from >= 0 ? 16 : 0);
-            }
-            af_commit();
-            return __ballot_sync(0xffffffffu, at >= 0);
-        };
-
-        int pos[4];
-        float r1[4], r2[4], m[4], l[4];
-        uint64_t O[4][CJ][2];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = min(first_row + ty + 16 * i, all_rows - 1), h = kv_head * G + row % G;
-            pos[i] = pos0 + row / G;
-            r1[i] = p.bias_r1 ? p.bias_r1[h] : 0.f;
-            r2[i] = p.bias_r2 ? p.bias_r2[h] : 0.f;
-            m[i] = -INFINITY;
-            l[i] = 0.f;
-#pragma unroll
-            for (int j = 0; j < CJ; ++j)
-                O[i][j][0] = O[i][j][1] = 0;
         }
-        usable = fetch(p.k_cache, K, DS, begin);        // (one group with the queries)
-        for (int base = begin; base <= last_pos; base = after(base)) {
-            const unsigned keys = usable;
-            af_wait<0>();
-            __syncthreads();                            // the keys are there; everyone is through with the values before
-            fetch(p.v_cache, V, D, base);
-            uint64_t S[4][4];
+        __syncwarp();
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AT_REGS_MANY));
+        // four columns of rows line + PASS i of a tile: where they lie in a part of the queries, and of the keys or values
+        static_assert(PASS % 8 == 0);
+        const int worker = tid - (AT_THREADS - AT_WORKERS), quad = worker % QUADS, line = worker / QUADS;
+        const uint32_t inside = (uint32_t)((line >> 3) * 1024 + (line & 7) * 128 + ((((4 * quad & 63) >> 3) ^ (line & 7)) << 4) + (quad & 1) * 8);
+        const uint32_t q_at = (quad >> 4) * (AT_ROWS * 128) + inside, kv_at = (quad >> 4) * (AT_KEYS * 128) + inside;
+        // Which rows of the cache a warp brings of a block's keys and values (-1: none): lane i looks up the i-th.
+        constexpr int WARP_ROWS = 32 / QUADS > 1 ? 32 / QUADS : 1, FOUND = KV_EACH * WARP_ROWS;
+        static_assert(AT_WORKERS % QUADS == 0 && QUADS <= 32 && FOUND <= 32);
+        auto lookup = [&](int base) {                                // the page, as it stands in the table
+            const int u = base + worker / QUADS / WARP_ROWS * WARP_ROWS + lane % WARP_ROWS + PASS * (lane / WARP_ROWS);
+            return lane < FOUND && u >= oldest && u <= last_pos ? table[u / p.page_size] : -2;
+        };
+        auto row_in = [&](int base, int page) {                      // and the key's row there
+            const int u = base + worker / QUADS / WARP_ROWS * WARP_ROWS + lane % WARP_ROWS + PASS * (lane / WARP_ROWS);
+            if (page < 0 || page >= p.num_pages) {
+                if (page != -2 && p.error)
+                    atomicExch(p.error, 3);
+                return -1;
+            }
+            return (page * p.nkv + kv_head) * p.page_size + u % p.page_size;
+        };
+        auto fetch = [&](const float* cache, int found, float4 (&v)[KV_EACH]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < KV_EACH; ++i) {
+                const int at = __shfl_sync(0xffffffffu, found, WARP_ROWS * i + lane / QUADS);
+                v[i] = at >= 0 ? *reinterpret_cast<const float4*>(cache + (size_t)at * D + 4 * quad) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        };
+        auto spread = [&](const float4 (&v)[KV_EACH], uint32_t to, uint32_t* flags) {
+            uint64_t none = 0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    S[i][j] = 0;
-#pragma unroll 4
-            for (int c = 0; c < D; c += 4) {
-                ulonglong2 a[4];
+            for (int i = 0; i < KV_EACH; ++i)
+                at_split(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE, none);
+            if (at_none(none)) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    a[i] = *reinterpret_cast<const ulonglong2*>(Q + (ty + 16 * i) * DS + c);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(K + (tx + 8 * j) * DS + c);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        S[i][j] = af_fma2(a[i].x, b.x, S[i][j]);
-                        S[i][j] = af_fma2(a[i].y, b.y, S[i][j]);
+                for (int i = 0; i < KV_EACH; ++i) {
+                    const int r = line + PASS * i;
+                    if (at_split_odd(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE)) {
+                        atomicOr(&flags[r >> 5], 1u << (r & 31));
+                        *odd_any = 1;
                     }
                 }
             }
-            // every row sees every key of this tile?
-            const bool whole = base + AF_KEYS - 1 <= pos0 + first_row / G && keys == 0xffffffffu
-                && base >= first_visible_key(last_pos, p.window, p.chunk);
-            int low[4], high[4];                        // the keys of the tile that a row sees
+        };
+        float4 kn[KV_EACH], vn[KV_EACH];
+        int page[3], found[2];                                       // pages of blocks j + 1 .. j + 3 (looked up long before they are
+                                                                     // looked at); rows of blocks j + 1 and j + 2
+        {
+            const int first_page = lookup(begin);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                low[i] = whole ? 0 : max(first_visible_key(pos[i], p.window, p.chunk) - base, 0);
-                high[i] = whole ? AF_KEYS - 1 : min(pos[i] - base, AF_KEYS - 1);
-                float s[4], most = -INFINITY;
+            for (int i = 0; i < 3; ++i)
+                page[i] = lookup(begin + (i + 1) * AT_KEYS);
+            found[0] = row_in(begin, first_page);
+        }
+        fetch(p.k_cache, found[0], kn);
+        fetch(p.v_cache, found[0], vn);
+        found[0] = row_in(begin + AT_KEYS, page[0]);
+        found[1] = row_in(begin + 2 * AT_KEYS, page[1]);
+        int ahead = page[2];
+        // the queries, in two goes
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int kk = tx + 8 * j;
-                    const float2 halves = af_halves(S[i][j]);
-                    s[j] = af_score(p, halves.x + halves.y, r1[i], r2[i], pos[i] - base - kk);
-                    if (kk < low[i] || kk > high[i] || !(keys >> kk & 1))
-                        s[j] = -INFINITY;
-                    most = fmaxf(most, s[j]);
-                }
+        for (int half = 0; half < 2; ++half) {
+            float4 v[Q_EACH / 2];
 #pragma unroll
-                for (int o = 4; o > 0; o >>= 1)
-                    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-                const float m_new = fmaxf(m[i], most);
-                const float keep = af_keep(m[i], m_new);
-                float sum = 0.f;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float e = s[j] == -INFINITY ? 0.f : expf(s[j] - m_new);
-                    P[(ty + 16 * i) * AF_P + tx + 8 * j] = e;
-                    sum += e;
-                }
-#pragma unroll
-                for (int o = 4; o > 0; o >>= 1)
-                    sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                l[i] = l[i] * keep + sum;
-                m[i] = m_new;
-                const uint64_t k2 = af_pair(keep, keep);
-#pragma unroll
-                for (int j = 0; j < CJ; ++j) {
-                    O[i][j][0] = af_mul2(O[i][j][0], k2);
-                    O[i][j][1] = af_mul2(O[i][j][1], k2);
-                }
+            for (int i = 0; i < Q_EACH / 2; ++i) {
+                const int row = first_row + line + PASS * (i + half * (Q_EACH / 2));
+                v[i] = row < all_rows ? *reinterpret_cast<const float4*>(p.q + ((size_t)(row0 + row / G) * p.nq + kv_head * G + row % G) * D + 4 * quad)
+                                      : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            af_wait<0>();
-            __syncthreads();                            // the values are there (and the row's probabilities)
-            if (after(base) <= last_pos)
-                usable = fetch(p.k_cache, K, DS, after(base));
-            auto values = [&](bool all) {
-#pragma unroll 2
-                for (int kk = 0; kk < AF_KEYS; kk += 4) {
-                    float4 e[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        e[i] = *reinterpret_cast<const float4*>(P + (ty + 16 * i) * AF_P + kk);
+            for (int i = 0; i < Q_EACH / 2; ++i) {
+                const int r = line + PASS * (i + half * (Q_EACH / 2));
+                uint64_t none = 0;
+                const uint32_t to = q_s + q_at + (i + half * (Q_EACH / 2)) * (PASS / 8) * 1024;
+                at_split(v[i], to, Shape::Q_PLANE, none);
+                if (at_none(none) && at_split_odd(v[i], to, Shape::Q_PLANE))
+                    odd_row[r] = *odd_any = 1;
+            }
+        }
+        spread(kn, k_s, odd_keys);
+        fence_proxy_async();
+        mbar_arrive(keys_there);
+        if (blocks > 1)
+            fetch(p.k_cache, found[0], kn);
+
+        // ---- a thread's row, its part of the keys and of the columns
+        const int quarter = warp & 3, part = (warp - 4) >> 2, r = quarter * 32 + lane, barrier = 1 + quarter;
+        const int row = min(first_row + r, all_rows - 1), h = kv_head * G + row % G, pos = pos0 + row / G;
+        const uint32_t lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+        const float r1 = p.bias_r1 ? p.bias_r1[h] : 0.f, r2 = p.bias_r2 ? p.bias_r2[h] : 0.f;
+        const int first = first_visible_key(pos, p.window, p.chunk);
+        constexpr int COLS = D / AT_SHARE;
+        uint64_t O[COLS / 2];
+        float m = -INFINITY, l = 0.f;
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        ulonglong2 v[CJ];
+        for (int c = 0; c < COLS / 2; ++c)
+            O[c] = 0;
+        auto key_at = [&](int key) -> long long {                    // where a key's numbers begin, -1 if its page is none of the pool's
+            const int page = table[key / p.page_size];
+            return page < 0 || page >= p.num_pages ? -1 : (long long)((page * p.nkv + kv_head) * p.page_size + key % p.page_size) * D;
+        };
+        auto add_output = [&](int j) {                // what block j's product has found
+            mbar_wait_warp(o_done, j & 1, p.error, 74);
+            tcgen05_fence_after();
+            uint32_t v[COLS];
+            at_tmem_load(lanes + Shape::O_AT + part * COLS, v);
+            tmem_load_wait();
 #pragma unroll
-                        for (int j = 0; j < CJ; ++j)
-                            v[j] = *reinterpret_cast<const ulonglong2*>(V + (kk + u) * D + 4 * tx + 32 * j);
+            for (int c = 0; c < COLS / 2; ++c)
+                O[c] = af_fma2(O[c], 0x3f8000003f800000ull, af_pair(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])));
+            if (*odd_any)
+                for (int i = 0; i < AT_KEYS; ++i) {
+                    const int key = begin + j * AT_KEYS + i;
+                    if ((odd_values[2 * (j & 3) + (i >> 5)] >> (i & 31) & 1) && key <= pos && key >= first) {
+                        const float* const v = p.v_cache + key_at(key) + part * COLS;        // (what is marked has been read)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float w = u == 0 ? e[i].x : u == 1 ? e[i].y : u == 2 ? e[i].z : e[i].w;
-                            const uint64_t w2 = af_pair(w, w);
-                            // (a key that the row does not see adds nothing, whatever its value holds)
-                            if (all || (kk + u >= low[i] && kk + u <= high[i])) {
-#pragma unroll
-                                for (int j = 0; j < CJ; ++j) {
-                                    O[i][j][0] = af_fma2(w2, v[j].x, O[i][j][0]);
-                                    O[i][j][1] = af_fma2(w2, v[j].y, O[i][j][1]);
-                                }
-                            }
+                        for (int c = 0; c < COLS / 2; ++c) {
+                            const float x = v[2 * c], y = v[2 * c + 1];
+                            const float2 o = af_halves(O[c]);
+                            O[c] = af_pair(o.x + (fabsf(x) < INFINITY ? 0.f : x), o.y + (fabsf(y) < INFINITY ? 0.f : y));
                         }
                     }
                 }
-            };
-            if (whole)
-                values(true);
-            else
-                values(false);
-        }
-        af_wait<0>();
-        __syncthreads();                                // keys and values are through: their place takes the sums
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = ty + 16 * i;
-#pragma unroll
-            for (int j = 0; j < CJ; ++j)
-                *reinterpret_cast<ulonglong2*>(part + r * D + 4 * tx + 32 * j) = make_ulonglong2(O[i][j][0], O[i][j][1]);
-            if (tx == 0) {
-                ml[r] = m[i];
-                ml[AF_ROWS + r] = l[i];
+        };
+        for (int j = 0; j < blocks; ++j) {
+            const int base = begin + j * AT_KEYS;
+            mbar_wait_warp(s_done, j & 1, p.error, 73);
+            tcgen05_fence_after();
+            // (places of blocks that all threads are through with: everyone has written keys j)
+            if (worker < 2) {
+                odd_keys[2 * ((j + 2) & 3) + worker] = 0;
+                odd_values[2 * ((j + 1) & 3) + worker] = 0;
             }
-        }
-        af_cluster_sync();
-        // each CTA finishes a quarter of the rows
-        constexpr int OWN = AF_ROWS / AF_RANKS;
-        for (int c = tid; c < OWN * QUADS; c += 128) {
-            const int r = rank * OWN + c / QUADS, at = 4 * (c % QUADS), row = first_row + r;
-            if (row >= all_rows)
-                continue;
-            float pm[AF_RANKS], pl[AF_RANKS];
-            float4 po[AF_RANKS];
-#pragma unroll
-            for (int x = 0; x < AF_RANKS; ++x) {
-                pm[x] = af_peer(ml + r, x);
-                pl[x] = af_peer(ml + AF_ROWS + r, x);
-                po[x] = af_peer4(part + r * D + at, x);
+            // the next block's scores are made while this one's are worked on
+            if (j + 1 < blocks) {
+                spread(kn, k_s, odd_keys + 2 * ((j + 1) & 3));
+                fence_proxy_async();
+                tcgen05_fence_before();
+                mbar_arrive(keys_there);
+                if (j + 2 < blocks)
+                    fetch(p.k_cache, found[1], kn);
             }
-            const int h = kv_head * G + row % G;
-            const float sink = p.sink ? p.sink[h] : -INFINITY;
-            float top = sink;
+            float s[AT_OWN];
+            {
+                uint32_t v[Shape::SLICES][AT_OWN];
 #pragma unroll
-            for (int x = 0; x < AF_RANKS; ++x)
-                top = fmaxf(top, pm[x]);
-            float sum = p.sink ? af_keep(sink, top) : 0.f;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int slice = 0; slice < Shape::SLICES; ++slice)
+                    at_tmem_load(lanes + (j & 1) * Shape::S_COLS + slice * 64 + part * AT_OWN, v[slice]);
+                tmem_load_wait();
 #pragma unroll
-            for (int x = 0; x < AF_RANKS; ++x) {
-                const float keep = af_keep(pm[x], top);
-                sum = fmaf(pl[x], keep, sum);           // (a CTA without a key for the row has zeros)
-                v.x = fmaf(po[x].x, keep, v.x);
-                v.y = fmaf(po[x].y, keep, v.y);
-                v.z = fmaf(po[x].z, keep, v.z);
-                v.w = fmaf(po[x].w, keep, v.w);
+                for (int i = 0; i < AT_OWN; ++i) {
+                    s[i] = __uint_as_float(v[0][i]);
+                    if (Shape::SLICES > 1)
+                        s[i] += __uint_as_float(v[Shape::SLICES - 1][i]);
+                }
             }
-            const float inv = sum > 0.f ? 1.f / sum : 0.f;
-            *reinterpret_cast<float4*>(p.out + ((size_t)(row0 + row / G) * p.nq + h) * D + at) =
-                make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+            const int key0 = base + part * AT_OWN;
+            if (*odd_any) {
+                const uint32_t marked = odd_row[r] ? 0xffffffffu : odd_keys[2 * (j & 3) + part / 2] >> (part & 1) * AT_OWN;
+                for (int i = 0; i < AT_OWN; ++i)
+                    if (marked >> i & 1 && key0 + i <= pos && key0 + i >= first && key_at(key0 + i) >= 0) {
+                        const float dot = at_dot(p.q + ((size_t)(row0 + row / G) * p.nq + h) * D, p.k_cache + key_at(key0 + i), D);
+#pragma unroll
+                        for (int u = 0; u < AT_OWN; ++u)
+                            s[u] = u == i ? dot : s[u];
+                    }
+            }
+            // every row sees every key of these?
+            const bool whole = __all_sync(0xffffffffu, key0 + AT_OWN - 1 <= pos && key0 >= first);
+            float most = -INFINITY;
+#pragma unroll
+            for (int i = 0; i < AT_OWN; ++i)
+                s[i] = OPTIONS ? af_score(p, s[i], r1, r2, pos - key0 - i) : s[i] * p.scale;
+            if (!whole) {
+#pragma unroll
+                for (int i = 0; i < AT_OWN; ++i)
+                    if (key0 + i > pos || key0 + i < first)
+                        s[i] = -INFINITY;
+            }
+#pragma unroll
+            for (int i = 0; i < AT_OWN; ++i)
+                most = fmaxf(most, s[i]);
+            exchange[part * AT_ROWS + r] = most;
+            at_row_sync(barrier);
+            float m_new = m;
+#pragma unroll
+            for (int x = 0; x < AT_SHARE; ++x)
+                m_new = fmaxf(m_new, exchange[x * AT_ROWS + r]);
+            at_row_sync(barrier);                                    // (read before the next block's are written)
+            const float keep = af_keep(m, m_new), least = m_new == -INFINITY ? 0.f : m_new;
+            m = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < AT_OWN; ++i) {
+                s[i] = expf(s[i] - least);                           // (of a hidden key: 0)
+                sum += s[i];
+            }
+            l = l * keep + sum;
+            if (j > 0)
+                add_output(j - 1);
+            const uint64_t keep2 = af_pair(keep, keep);
+#pragma unroll
+            for (int c = 0; c < COLS / 2; ++c)
+                O[c] = af_mul2(O[c], keep2);
+            uint64_t s2[AT_OWN / 2];
+#pragma unroll
+            for (int i = 0; i < AT_OWN / 2; ++i)
+                s2[i] = af_pair(s[2 * i], s[2 * i + 1]);
+#pragma unroll
+            for (int plane = 0; plane < 3; ++plane) {
+                uint32_t pairs[AT_OWN / 2];
+#pragma unroll
+                for (int i = 0; i < AT_OWN / 2; ++i) {
+                    pairs[i] = at_pair(s2[i]);
+                    s2[i] = at_rest(s2[i], pairs[i]);
+                }
+                tmem_store_32x8(lanes + Shape::P_AT + plane * 32 + part * (AT_OWN / 2), pairs);
+            }
+            spread(vn, v_s, odd_values + 2 * (j & 3));
+            tmem_store_wait();
+            fence_proxy_async();
+            tcgen05_fence_before();
+            mbar_arrive(p_there);
+            if (j + 1 < blocks)
+                fetch(p.v_cache, found[0], vn);
+            found[0] = found[1];
+            found[1] = row_in(base + 3 * AT_KEYS, ahead);
+            ahead = lookup(base + 4 * AT_KEYS);
         }
-        af_cluster_sync();                              // nobody goes on while its sums are read
+        add_output(blocks - 1);
+        // ---- the row's sum of all its threads, and the rows by way of the queries' place: neighbouring lanes store neighbouring pieces
+        exchange[part * AT_ROWS + r] = l;
+        at_row_sync(barrier);
+        l = 0.f;
+#pragma unroll
+        for (int x = 0; x < AT_SHARE; ++x)
+            l += exchange[x * AT_ROWS + r];
+        if (p.sink) {
+            const float sink = p.sink[h], top = fmaxf(sink, m), keep = af_keep(m, top);
+            l = l * keep + af_keep(sink, top);
+            const uint64_t keep2 = af_pair(keep, keep);
+#pragma unroll
+            for (int c = 0; c < COLS / 2; ++c)
+                O[c] = af_mul2(O[c], keep2);
+        }
+        const float inv = l > 0.f ? 1.f / l : 0.f;
+        constexpr int CHUNKS = D / 4, SHARE = CHUNKS / AT_SHARE;     // pieces of 16 bytes of a row, and a thread's
+        uint8_t* const rows = smem + quarter * 32 * (D * 4);
+#pragma unroll
+        for (int c = 0; c < SHARE; ++c) {
+            const float2 a = af_halves(O[2 * c]), b = af_halves(O[2 * c + 1]);
+            *reinterpret_cast<float4*>(rows + lane * (D * 4) + (((part * SHARE + c) ^ (lane & 7)) << 4)) =
+                make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+        }
+        at_row_sync(barrier);
+#pragma unroll 4
+        for (int i = part * 32 * SHARE + lane; i < (part + 1) * 32 * SHARE; i += 32) {
+            const int rr = i / CHUNKS, c = i % CHUNKS, to = first_row + quarter * 32 + rr;
+            if (to < all_rows)
+                *reinterpret_cast<float4*>(p.out + ((size_t)(row0 + to / G) * p.nq + kv_head * G + to % G) * D + 4 * c) =
+                    *reinterpret_cast<const float4*>(rows + rr * (D * 4) + ((c ^ (rr & 7)) << 4));
+        }
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tcgen05_fence_after();
+        tmem_dealloc(tmem, Shape::TMEM);
     }
 }
 
@@ -563,19 +830,24 @@ static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min
 {
     const int G = p.nq / p.nkv;
     if (max_q_len > 1) {
-        static bool configured = false;
-        if (!configured) {
-            const cudaError_t e = cudaFuncSetAttribute(attention_f32_prompt_kernel<D>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)af_shared<D>());
-            if (e != cudaSuccess)
-                return (int)e;
-            configured = true;
+        const bool options = p.softcap > 0.f || p.bias_r1;
+        const auto kernel = options ? attention_f32_prompt_kernel<D, true> : attention_f32_prompt_kernel<D, false>;
+        static bool configured[2] = { false, false };
+        if (!configured[options]) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AtShape<D>::SHARED);
+            // (threads that asked for more registers than the block was launched with would wait for good)
+            cudaFuncAttributes attr {};
+            const cudaError_t a = e == cudaSuccess ? cudaFuncGetAttributes(&attr, kernel) : e;
+            if (a != cudaSuccess)
+                return (int)a;
+            if (attr.numRegs < AT_REGS)
+                return CHIBI_ERR_ARGUMENT;
+            configured[options] = true;
         }
-        const long long tiles = ((long long)max_q_len * G + AF_ROWS - 1) / AF_ROWS;
-        if (tiles * AF_RANKS > 2147483647LL)
+        const long long tiles = ((long long)max_q_len * G + AT_ROWS - 1) / AT_ROWS;
+        if (tiles > 2147483647LL || (long long)p.num_pages * p.nkv * p.page_size > 2147483647LL)
             return CHIBI_ERR_UNSUPPORTED;
-        launch_cluster_x(attention_f32_prompt_kernel<D>, dim3((unsigned)tiles * AF_RANKS, p.nkv, seqs), dim3(128), af_shared<D>(),
-                         stream, AF_RANKS, p);
+        launch(kernel, dim3((unsigned)tiles, p.nkv, seqs), dim3(AT_THREADS), AtShape<D>::SHARED, stream, p);
         if (const int status = launch_status())
             return status;
     }
