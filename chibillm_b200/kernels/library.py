@@ -26,6 +26,7 @@ _SIGNATURES = {
         "chibi_cast": [P, I, P, I, L, P],
         "chibi_add_into": [P, P, I, L, P],
         "chibi_gemm_simt": [P, I, P, I, P, I, P, I, I, I, L, L, L, L, P],
+        "chibi_gemm_f32": [P, P, P, P, I, I, I, L, L, L, L, I, I, P, P],
         "chibi_gemm_bf16_splits": [I, I, I],
         "chibi_gemm_bf16_splits_capped": [I, I, I, I],
         "chibi_gemm_bf16": [P, P, P, I, P, I, I, I, L, L, L, L, P, L, P, P],

@@ -748,6 +748,14 @@ class CudaKernels:
                 if status != -2:
                     _check(status, "linear (tensor cores)")
         self.launches += 1
+        if x.dtype == w.dtype == out.dtype == torch.float32:
+            status = self.lib.chibi_gemm_f32(
+                _ptr(x), _ptr(w), _ptr(out), _ptr(residual), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+                residual.stride(0) if residual is not None else 0, 0, 0, _ptr(self.error), self._stream())
+            if status == 0:
+                return
+            if status != -2:
+                _check(status, "linear (32-bit, tensor cores)")
         _check(self.lib.chibi_gemm_simt(
             _ptr(x), _code(x), _ptr(w), _code(w), _ptr(out), _code(out), _ptr(residual), M, N, K,
             x.stride(0), w.stride(0), out.stride(0),

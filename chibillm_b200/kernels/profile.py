@@ -31,7 +31,8 @@ _NOT_LAUNCHES = ("chibi_gemm_bf16_splits", "chibi_gemm_bf16_splits_capped", "chi
 
 # where M, N, K stand among the arguments of the matrix products
 _PRODUCT_SIZES = {"chibi_gemm_bf16": (5, 6, 7), "chibi_gemm_bf16_rows": (5, 6, 7), "chibi_gemm_bf16_fused": (5, 6, 7),
-                  "chibi_gemm_bf16_partial": (2, 3, 4), "chibi_gemm_simt": (7, 8, 9)}
+                  "chibi_gemm_bf16_partial": (2, 3, 4), "chibi_gemm_simt": (7, 8, 9),
+                  "chibi_gemm_f32": (4, 5, 6)}
 
 
 def launch_name(function: str, args: tuple) -> str:
