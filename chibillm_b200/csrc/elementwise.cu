@@ -608,6 +608,26 @@ __global__ void swiglu_kernel(const TX* __restrict__ gate_up, TO* __restrict__ o
     }
 }
 
+// Any types, inter a multiple of 4: four values per thread, a row to blockIdx.y.  (A value a thread, with a 64-bit division for its
+// place, was bound by that division: 484 rows of 3,072 in 32 bits 8.5 us, so 2.8, 1,200 of 12,288 50.0 and 26.3, 4 of 3,072 1.38 and
+// 1.32.)
+template <typename TX, typename TO>
+__global__ void swiglu_vec4_kernel(const TX* __restrict__ gate_up, TO* __restrict__ out, int inter)
+{
+    pdl_enter();
+    const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= inter)
+        return;
+    const size_t row = blockIdx.y;
+    float g[4], u[4];
+    Vec4<TX>::load(gate_up + row * 2 * inter + c, g);
+    Vec4<TX>::load(gate_up + row * 2 * inter + inter + c, u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        g[i] = (g[i] / (1.f + expf(-g[i]))) * u[i];
+    Vec4<TO>::store(out + row * inter + c, g);
+}
+
 // bfloat16 in and out, inter a multiple of 8: eight values per thread.
 __global__ void swiglu_bf16x8_kernel(const __nv_bfloat16* __restrict__ gate_up,
                                      __nv_bfloat16* __restrict__ out, int inter)
@@ -860,8 +880,15 @@ CHIBI_API int chibi_swiglu(const void* gate_up, int x_type, void* out, int out_t
         launch(swiglu_bf16x8_kernel, dim3(grid), dim3(256), 0, stream, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, inter);
         return launch_status();
     }
+    const bool vec = inter % 4 == 0 && rows <= 65535
+        && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    const int threads = rows < 128 ? 64 : 256;         // (few rows: a block to as many SMs as there are)
     CHIBI_DISPATCH_TYPE(x_type, TX, CHIBI_DISPATCH_TYPE(out_type, TO, {
-        launch(swiglu_kernel<TX, TO>, dim3(grid_for(rows * inter, 256)), dim3(256), 0, stream, 
+        if (vec)
+            launch(swiglu_vec4_kernel<TX, TO>, dim3((unsigned)((inter / 4 + threads - 1) / threads), (unsigned)rows), dim3(threads), 0,
+                   stream, (const TX*)gate_up, (TO*)out, inter);
+        else
+            launch(swiglu_kernel<TX, TO>, dim3(grid_for(rows * inter, 256)), dim3(256), 0, stream,
             (const TX*)gate_up, (TO*)out, rows, inter);
     }));
     return launch_status();
