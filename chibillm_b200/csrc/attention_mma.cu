@@ -593,8 +593,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     int seq = blockIdx.z, split = blockIdx.x, ranges = p.splits, unit_tiles = 0;
     if (p.units > 0) {
         const DecodeUnit u = decode_unit(p, blockIdx.x, -1);
-        if (u.seq < 0)
+        if (u.seq < 0) {
+            pdl_wait();                               // (every way out waits: the next kernel waits for this one alone)
             return;
+        }
         seq = u.seq, split = u.range, ranges = u.ranges, unit_tiles = u.tiles;
     } else if (p.by_length) {
         seq = sequence_of_rank(p, blockIdx.z);
@@ -602,8 +604,10 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     const int row_blocks = (p.group + 15) / 16;
     const int kv_head = blockIdx.y / row_blocks, row_block = blockIdx.y - kv_head * row_blocks;
     const int t = p.q_start[seq];
-    if (p.q_start[seq + 1] - t != 1)
+    if (p.q_start[seq + 1] - t != 1) {
+        pdl_wait();
         return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pos = p.ctx_len[seq] - 1;
     const int first = first_visible_key(pos, p.window, p.chunk);
@@ -784,20 +788,26 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     }
 }
 
-// Merges the key ranges of one (sequence, head): one block of D threads (whole warps).
+// Merges the key ranges of one (sequence, head): one block of D threads (whole warps).  Every way out of it waits for the
+// attention kernel: the kernel behind waits for this one alone, and where no sequence has ranges to merge it would otherwise
+// read rows that are not written yet.
 __global__ void attn_decode_merge_kernel(const AttnParams p)
 {
     pdl_trigger();
     const int seq = blockIdx.y, head = blockIdx.x, c = min((int)threadIdx.x, D - 1);
     const int t = p.q_start[seq];                     // written before the step's first kernel
-    if (p.q_start[seq + 1] - t != 1)
+    if (p.q_start[seq + 1] - t != 1) {
+        pdl_wait();
         return;
+    }
     int ranges = p.splits, step = 1;
     size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
     if (p.units > 0) {
         const DecodeUnit u = decode_unit(p, -1, seq);
-        if (u.ranges <= 1)
+        if (u.ranges <= 1) {
+            pdl_wait();
             return;                                   // (the attention kernel has written the row)
+        }
         ranges = u.ranges;
         step = p.nq;
         slot0 = (size_t)u.first_unit * p.nq + head;

@@ -63,3 +63,42 @@ def test_longest_sequences_first(k, ref, seqs, nkv, d):
     assert k.decode_attention_units(seqs, 2 * nkv, nkv, 1, 1024) == (0, int(seqs <= 128))
     assert k.decode_attention_splits(seqs, 2 * nkv, nkv, 1024) == 1
     _check(k, ref, lens, 2 * nkv, nkv, d)
+
+
+# What follows attention in a model is a kernel that starts early and waits for the kernel ahead of it alone: for the merge,
+# which in these steps has nothing to merge (a window or single tokens of at most 128 keys), or for a decode kernel without
+# any single token (0: how many tokens a sequence brings at least is not said).
+@pytest.mark.parametrize("lens,q_lens,window,least", [
+    ([3000, 4096, 2100, 3500] * 2, [1] * 8, 40, 1), ([90, 40, 128, 1] * 4 + [1500], [1] * 16 + [200], None, 1),
+    ([300, 500], [300, 100], None, 0)])
+def test_the_product_behind_reads_finished_rows(k, ref, lens, q_lens, window, least):
+    nq, nkv, d, page = 16, 8, 128, 16
+    pages = sum(-(-n // page) for n in lens)
+    table, positions, seq_of_token, q_start, ctx_len = _paged_setup(lens, q_lens, page, pages, seed=3)
+    q = rnd(sum(q_lens), nq * d, dtype=torch.bfloat16, seed=4)
+    kc = rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=5)
+    vc = rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=6)
+    w = rnd(256, nq * d, dtype=torch.bfloat16, seed=7, scale=0.02)
+    args = (table, q_start, ctx_len, seq_of_token, positions, nq, nkv, d, page, 1 / math.sqrt(d), window, max(q_lens),
+            max(lens), least)
+    out, exp = torch.empty_like(q), torch.empty_like(q)
+    product = torch.empty(q.shape[0], 256, dtype=torch.float32, device="cuda")
+    ref.attention(q, kc, vc, exp, *args)
+    expected = exp.float() @ w.float().t()
+
+    def step():
+        out.fill_(float("nan"))
+        k.attention(q, kc, vc, out, *args)
+        k.linear(out, w, product)
+
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for run in [step] * 10 + [graph.replay] * 20:
+        product.fill_(float("nan"))
+        run()
+        close(out, exp, torch.bfloat16, "attention", rel=1.2e-2)         # (as the other tests of this kernel)
+        close(product, expected, torch.float32, "the product behind", rel=1.5e-2)    # (that of its rows, each 1.2e-2 at most)
+    k.check_error_word()
