@@ -14,11 +14,11 @@
 // depend on the rows beside it, nor on which kernel makes it or how many CTAs share a sum (a cluster of 1, 2, 4 or 8 takes the
 // runs in order).
 //
-// Numbers of x are split times 2^16, so that the last parts of small ones (of all normal numbers) are no smaller than a
-// bfloat16 can be, and sums are 2^16 as large as they should be until the end.  (Those of w are weights, as they are: of one below
-// 2^-109 the last bits are lost.  Both scaled cost prompts 5 to 9 %.)  What is no number or too large for a bfloat16, in x from
-// 2^112 on, has no such parts: its row of x or w is marked.  The outputs of marked rows, and sums that come out infinite, are
-// made by multiply-adds instead.
+// Numbers are split times 2^16, so that the last parts of small ones (of all normal numbers) are no smaller than a
+// bfloat16 can be, and sums are 2^32 as large as they should be until the end.  What is no number, or too large (from 2^112
+// on), has an infinite part and a rest that is no number, so all sums of its row of x or w come out as none.  Sums that do, and
+// sums from 2^96 on, which come out infinite, are made by multiply-adds instead.  (No loop looks for such numbers, which pays for the
+// scaling: 300 rows through the feed-forward of 1,024 x 3,072 75.1 us with rows marked and w not scaled, 70.2 so.)
 //
 // A CTA owns 128 rows of w (the M of the MMA) and up to 128 rows of x (its N).  Eight or sixteen warps bring both from
 // memory (in registers, one block ahead), split them and write the six tiles to one of two stages in shared memory in
@@ -31,8 +31,6 @@
 #define CHIBI_UNIT_ID 18
 #include "common.cuh"
 #include "sm100.cuh"
-
-#include <type_traits>
 
 namespace chibi {
 
@@ -60,14 +58,7 @@ struct F3Params {
 };
 
 template <int NT> constexpr int f3_stage() { return 3 * (F3_W_PLANE + NT * F3_KB * 2); }
-template <int NT> constexpr size_t f3_smem() { return 1024 + 2 * f3_stage<NT>() + 64 + 4 * (F3_ROWS + NT) + 16; }
-
-__device__ __forceinline__ float f3_peer(const void* local, int rank)
-{
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(peer_smem_addr(smem_addr(local), rank)) : "memory");
-    return v;
-}
+template <int NT> constexpr size_t f3_smem() { return 1024 + 2 * f3_stage<NT>() + 64; }
 
 __device__ __forceinline__ float4 f3_peer4(const void* local, int rank)
 {
@@ -119,12 +110,11 @@ __device__ __forceinline__ uint64_t f3_fma2(uint64_t a, uint64_t b, uint64_t c)
     return r;
 }
 constexpr uint64_t F3_ONES = 0x3f8000003f800000ull, F3_MINUS_ONES = 0xbf800000bf800000ull, F3_UP = 0x4780000047800000ull;    // 2^16 twice
-constexpr float F3_DOWN = 0x1p-16f;
-template <bool UP> __device__ __forceinline__ uint64_t f3_scaled(float a, float b)
+constexpr float F3_DOWN = 0x1p-32f;
+__device__ __forceinline__ uint64_t f3_scaled(float a, float b)
 {
     uint64_t r = f3_both(a, b);
-    if (UP)
-        asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(F3_UP));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(F3_UP));
     return r;
 }
 __device__ __forceinline__ uint32_t f3_pair(uint64_t v)
@@ -143,12 +133,10 @@ __device__ __forceinline__ void f3_put(uint32_t at, uint32_t a, uint32_t b)
 {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
 }
-// Writes the three parts of four places, `plane` bytes apart; adds to `none` what is no number if one of them is none, or so
-// large that its leading part is infinite.
-template <bool UP>
-__device__ __forceinline__ void f3_split(float4 v, uint32_t at, uint32_t plane, uint64_t& none)
+// Writes the three parts of four places, `plane` bytes apart.
+__device__ __forceinline__ void f3_split(float4 v, uint32_t at, uint32_t plane)
 {
-    uint64_t x = f3_scaled<UP>(v.x, v.y), y = f3_scaled<UP>(v.z, v.w);
+    uint64_t x = f3_scaled(v.x, v.y), y = f3_scaled(v.z, v.w);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const uint32_t a = f3_pair(x), b = f3_pair(y);
@@ -158,26 +146,6 @@ __device__ __forceinline__ void f3_split(float4 v, uint32_t at, uint32_t plane, 
             y = f3_rest(y, b);
         }
     }
-    none = f3_fma2(x, F3_ONES, f3_fma2(y, F3_ONES, none));
-}
-__device__ __forceinline__ bool f3_none(uint64_t v)
-{
-    const float2 h = f3_halves(v);
-    return !(fabsf(h.x + h.y) < INFINITY);
-}
-// Takes out (as 0) what is no number, or so large that it (UP: 2^16 times it) is infinite as bfloat16; true if there was one.
-template <bool UP>
-__device__ __forceinline__ bool f3_clean(float4& v)
-{
-    bool found = false;
-    auto one = [&](float& x) {
-        if ((__float_as_uint(x) & 0x7fffffffu) >= (UP ? 0x777f8000u : 0x7f7f8000u)) {
-            x = 0.f;
-            found = true;
-        }
-    };
-    one(v.x), one(v.y), one(v.z), one(v.w);
-    return found;
 }
 
 template <int COUNT> __device__ __forceinline__ void f3_tmem_load(uint32_t at, uint32_t (&r)[COUNT])
@@ -203,7 +171,7 @@ template <int COUNT> __device__ __forceinline__ void f3_tmem_store(uint32_t at, 
         tmem_store_32x8(at, r);
 }
 
-// An output of a marked row, by multiply-adds (a rare event, out of line: its registers don't count against the loop).
+// An output by multiply-adds (a rare event, out of line: its registers don't count against the loop).
 __device__ __noinline__ float f3_by_hand(const float* x, const float* w, int K)
 {
     float v = 0.f;
@@ -217,11 +185,12 @@ __global__ void __launch_bounds__(WORKERS == 256 ? 288 : 640, WORKERS == 256 ? 2
 gemm_f32_tc_kernel(const F3Params p)
 {
     pdl_trigger();
-    constexpr int OTHERS = WORKERS == 256 ? 32 : 128, F3_THREADS = OTHERS + WORKERS;
+    constexpr int OTHERS = WORKERS == 256 ? 32 : 128;
     constexpr int STAGE = f3_stage<NT>(), X_PLANE = NT * F3_KB * 2, TMEM = 4 * NT;
     constexpr int SHARES = WORKERS / F3_ROWS, COLS = NT / SHARES;        // threads of a row of w; a thread's rows of x
     constexpr int PIECE = COLS < 16 ? COLS : 16, PIECES = COLS / PIECE;
-    constexpr int PASS = WORKERS / 16, W_EACH = F3_ROWS / PASS, X_EACH = NT >= PASS ? NT / PASS : 1;
+    constexpr int PASS = WORKERS / 16, W_EACH = F3_ROWS / PASS, X_EACH = NT / PASS;
+    static_assert(NT % PASS == 0);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + 2 * STAGE);
@@ -229,7 +198,6 @@ gemm_f32_tc_kernel(const F3Params p)
     uint64_t* const done = bars + 2;             // [2] MMA commit: the stage is read, the accumulator is finished
     uint64_t* const taken = bars + 4;            // [2] workers: the accumulator is read
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
-    int* const marked = reinterpret_cast<int*>(bars + 8);        // [0] any; [1 + row of w], [129 + row of x]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ranks = p.ranks, rank = ranks > 1 ? (int)(blockIdx.x % ranks) : 0;
     const int n0 = (int)(blockIdx.x / ranks) * F3_ROWS, m0 = blockIdx.y * p.cols;
@@ -250,8 +218,6 @@ gemm_f32_tc_kernel(const F3Params p)
         tmem_alloc(tmem_slot, TMEM);
         tmem_relinquish();
     }
-    for (int i = tid; i < 1 + F3_ROWS + NT; i += F3_THREADS)
-        marked[i] = 0;
     // the first weights are asked for in L2 (and read after the wait: the kernel ahead may write them)
     if (tid >= OTHERS && tid < OTHERS + F3_ROWS && n0 + tid - OTHERS < p.N)
         for (int b = 0; b < min(blocks, 4); ++b) {
@@ -334,30 +300,12 @@ gemm_f32_tc_kernel(const F3Params p)
             }
         };
         auto spread = [&](int st) {
-            uint64_t none = 0;
 #pragma unroll
             for (int j = 0; j < W_EACH; ++j)
-                f3_split<false>(wv[j], to + st * STAGE + j * (PASS / 8) * 1024, F3_W_PLANE, none);
-            const bool mine = NT >= PASS || line < NT;
-            if (mine) {
+                f3_split(wv[j], to + st * STAGE + j * (PASS / 8) * 1024, F3_W_PLANE);
 #pragma unroll
-                for (int j = 0; j < X_EACH; ++j)
-                    f3_split<true>(xv[j], to + st * STAGE + 3 * F3_W_PLANE + j * (PASS / 8) * 1024, X_PLANE, none);
-            }
-            if (f3_none(none)) {
-#pragma unroll
-                for (int j = 0; j < W_EACH; ++j)
-                    if (f3_clean<false>(wv[j])) {
-                        f3_split<false>(wv[j], to + st * STAGE + j * (PASS / 8) * 1024, F3_W_PLANE, none);
-                        marked[1 + line + PASS * j] = marked[0] = 1;
-                    }
-#pragma unroll
-                for (int j = 0; j < X_EACH; ++j)
-                    if (mine && f3_clean<true>(xv[j])) {
-                        f3_split<true>(xv[j], to + st * STAGE + 3 * F3_W_PLANE + j * (PASS / 8) * 1024, X_PLANE, none);
-                        marked[1 + F3_ROWS + line + PASS * j] = marked[0] = 1;
-                    }
-            }
+            for (int j = 0; j < X_EACH; ++j)
+                f3_split(xv[j], to + st * STAGE + 3 * F3_W_PLANE + j * (PASS / 8) * 1024, X_PLANE);
         };
         uint64_t run[COLS / 2];
         // Adds block i's accumulator to its run, and a run that is finished to what came before it, in TMEM: by halves, or, where
@@ -422,21 +370,20 @@ gemm_f32_tc_kernel(const F3Params p)
             take(i);
         // ---- the whole sums: of this CTA alone, or of the cluster's through shared memory
         const int kept = ranks >= 4 ? own : 1;                       // sums of a rank
-        float* const sums = reinterpret_cast<float*>(smem);          // [kept][column][row] (the stages are read)
-        auto finish = [&](int m, int n, float v, bool by_hand) {
+        float* const sums = reinterpret_cast<float*>(smem);          // [kept][column][row] (the stages are read: this thread has
+                                                                     // waited for the last products)
+        auto finish = [&](int m, int n, float v) {
             if (m >= p.M || n >= p.N)
                 return;
             v *= F3_DOWN;
-            if (by_hand || !(fabsf(v) < INFINITY))
+            if (!(fabsf(v) < INFINITY))
                 v = f3_by_hand(p.x + (size_t)m * p.x_stride, p.w + (size_t)n * p.w_stride, p.K);
             if (p.residual)
                 v = p.residual[(size_t)m * p.res_stride + n] + v;
             p.out[(size_t)m * p.out_stride + n] = v;
         };
-        asm volatile("barrier.cta.sync.aligned 1, %0;" ::"n"(WORKERS) : "memory");      // (all marks are there; all are through with the stages)
         {
             const int slots = ranks == 1 ? (p.runs > 4 ? 2 : 1) : kept;
-            const bool any = ranks == 1 && marked[0];
             const int row = quarter * 32 + lane;
 #pragma unroll
             for (int c = 0; c < PIECES; ++c) {
@@ -450,8 +397,7 @@ gemm_f32_tc_kernel(const F3Params p)
 #pragma unroll
                     for (int u = 0; u < PIECE; ++u)
                         if (col + u < p.cols)
-                            finish(m0 + col + u, n0 + row, __uint_as_float(a[u]) + (slots > 1 ? __uint_as_float(b[u]) : 0.f),
-                                   any && (marked[1 + row] || marked[1 + F3_ROWS + col + u]));
+                            finish(m0 + col + u, n0 + row, __uint_as_float(a[u]) + (slots > 1 ? __uint_as_float(b[u]) : 0.f));
                 } else {
 #pragma unroll
                     for (int u = 0; u < PIECE; ++u) {
@@ -465,9 +411,6 @@ gemm_f32_tc_kernel(const F3Params p)
         if (ranks > 1) {
             cluster_sync();
             {
-                bool any = false;
-                for (int r = 0; r < ranks; ++r)
-                    any = any || __float_as_int(f3_peer(marked, r)) != 0;
                 // (four rows of w at a time: what bounds this is the number of reads from the other CTAs)
                 const int each = ranks >= 4 ? 1 : 4;                 // runs of a kept sum
                 for (int i = 4 * (rank * WORKERS + tid - OTHERS); i < p.cols * F3_ROWS; i += 4 * ranks * WORKERS) {
@@ -497,15 +440,10 @@ gemm_f32_tc_kernel(const F3Params p)
                         }
                         add(v, w);
                     }
-                    bool by_hand[4] = { false, false, false, false };
-                    if (any)
-                        for (int u = 0; u < 4; ++u)
-                            for (int r = 0; r < ranks; ++r)
-                                by_hand[u] = by_hand[u] || __float_as_int(f3_peer(marked + 1 + row + u, r)) || __float_as_int(f3_peer(marked + 1 + F3_ROWS + col, r));
-                    finish(m0 + col, n0 + row, v.x, by_hand[0]);
-                    finish(m0 + col, n0 + row + 1, v.y, by_hand[1]);
-                    finish(m0 + col, n0 + row + 2, v.z, by_hand[2]);
-                    finish(m0 + col, n0 + row + 3, v.w, by_hand[3]);
+                    finish(m0 + col, n0 + row, v.x);
+                    finish(m0 + col, n0 + row + 1, v.y);
+                    finish(m0 + col, n0 + row + 2, v.z);
+                    finish(m0 + col, n0 + row + 3, v.w);
                 }
             }
             cluster_sync();                                          // nobody leaves while its sums are read
@@ -536,8 +474,6 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
     // sixteen warps take the blocks in turn; eight a run each, so that there is less to put together
     constexpr int XS = 8 * TILES, THREADS = 32 * WARPS, OWN = WARPS < 16 ? F3_RUNS / WARPS : 0;
     extern __shared__ __align__(16) float kept_sums[];       // [block, or turn and run][row of x][row of w]
-    // the last tile in which a row of w, or any, held what is no number (1 + its number); any, rows of x
-    __shared__ int marked[2][17], marked_x[1 + XS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int blocks = (p.K + F3_KB - 1) / F3_KB;
     const int begin = OWN ? min(warp * OWN * p.run_blocks, blocks) : warp, end = OWN ? min((warp + 1) * OWN * p.run_blocks, blocks) : blocks;
@@ -548,11 +484,6 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
         if (n < p.N && k < p.K)
             prefetch_l2(p.w + (size_t)n * p.w_stride + k);
     }
-    if (threadIdx.x < 2 * 17)
-        (&marked[0][0])[threadIdx.x] = 0;
-    if (threadIdx.x < 1 + XS)
-        marked_x[threadIdx.x] = 0;
-    __syncthreads();
     pdl_wait();
 
     float4 wn[2][4], xn[TILES][4];                           // rows g and g + 8 of the tile, row g of every eight of x (if not KEPT)
@@ -595,9 +526,8 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
     uint4* const kept4 = reinterpret_cast<uint4*>(kept_sums + 2 * F3_RUNS * XS * 16);
     uint2* const kept2 = reinterpret_cast<uint2*>(kept4 + blocks * 4 * TILES * 32);
     auto kept_at = [&](int b, int ks, int i) { return ((b * 4 + ks) * TILES + i) * 32 + lane; };
-    auto parts_of = [&](auto up, float4 v, uint32_t (&parts)[3][2], uint64_t& none) {
-        constexpr bool UP = decltype(up)::value;
-        uint64_t x = f3_scaled<UP>(v.x, v.y), y = f3_scaled<UP>(v.z, v.w);
+    auto parts_of = [&](float4 v, uint32_t (&parts)[3][2]) {
+        uint64_t x = f3_scaled(v.x, v.y), y = f3_scaled(v.z, v.w);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             parts[j][0] = f3_pair(x);
@@ -607,7 +537,6 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
                 y = f3_rest(y, parts[j][1]);
             }
         }
-        none = f3_fma2(x, F3_ONES, f3_fma2(y, F3_ONES, none));
     };
     if (begin < end && (int)blockIdx.x < w_tiles) {
         aim(blockIdx.x, begin);
@@ -628,11 +557,8 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
                 }
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
-                    if (f3_clean<true>(v[ks]))
-                        marked_x[1 + 8 * i + g] = marked_x[0] = 1;
-                    uint64_t none = 0;
                     uint32_t parts[3][2];
-                    parts_of(std::true_type(), v[ks], parts, none);
+                    parts_of(v[ks], parts);
                     kept4[kept_at(b, ks, i)] = make_uint4(parts[0][0], parts[0][1], parts[1][0], parts[1][1]);
                     kept2[kept_at(b, ks, i)] = make_uint2(parts[2][0], parts[2][1]);
                 }
@@ -670,28 +596,12 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
                         xf[i][0][0] = a.x, xf[i][0][1] = a.y, xf[i][1][0] = a.z, xf[i][1][1] = a.w, xf[i][2][0] = c.x, xf[i][2][1] = c.y;
                     }
                 }
-                for (bool again = true; again;) {
-                    uint64_t none = 0;
-                    parts_of(std::false_type(), wn[0][ks], low, none);
-                    parts_of(std::false_type(), wn[1][ks], high, none);
-                    if (!KEPT) {
+                parts_of(wn[0][ks], low);
+                parts_of(wn[1][ks], high);
+                if (!KEPT) {
 #pragma unroll
-                        for (int i = 0; i < TILES; ++i)
-                            parts_of(std::true_type(), xn[i][ks], xf[i], none);
-                    }
-                    again = __any_sync(0xffffffffu, f3_none(none));
-                    if (again) {                             // (rare)
-#pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (f3_clean<false>(wn[i][ks]))
-                                marked[turn][1 + g + 8 * i] = marked[turn][0] = 1 + tile;
-                        if (!KEPT) {
-#pragma unroll
-                            for (int i = 0; i < TILES; ++i)
-                                if (f3_clean<true>(xn[i][ks]))
-                                    marked_x[1 + 8 * i + g] = marked_x[0] = 1;
-                        }
-                    }
+                    for (int i = 0; i < TILES; ++i)
+                        parts_of(xn[i][ks], xf[i]);
                 }
                 if (more)
                     fetch(ks);
@@ -769,7 +679,7 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
                 v += half;
             }
             v *= F3_DOWN;
-            if ((marked[turn][0] && marked[turn][1 + o % 16] == 1 + tile) || (marked_x[0] && marked_x[1 + m]) || !(fabsf(v) < INFINITY))
+            if (!(fabsf(v) < INFINITY))
                 v = f3_by_hand(p.x + (size_t)m * p.x_stride, p.w + (size_t)n * p.w_stride, p.K);
             if (p.residual)
                 v = p.residual[(size_t)m * p.res_stride + n] + v;

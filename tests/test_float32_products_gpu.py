@@ -84,3 +84,16 @@ def test_sums_too_large_for_scaled_accumulators(k):
         out = torch.empty(rows, 30, device="cuda")
         k.linear(x[:rows], w, out)
         assert (out == 2.0 ** 126).all()
+
+
+@pytest.mark.parametrize("x_size,w_size", [(1.0, 1e-35), (1.0, 1e-37), (1e30, 1e-37), (1e-20, 1e-17)])
+@pytest.mark.parametrize("rows", [3, 12, 40])
+def test_small_weights_keep_their_bits(k, rows, x_size, w_size):
+    x, w = rnd(rows, 256, seed=5) * x_size, rnd(70, 256, seed=6) * w_size
+    w[:, ::7] += 2.0 ** -126                                 # (the least normal number among them)
+    out = torch.empty(rows, 70, device="cuda")
+    k.linear(x, w, out)
+    exact = x.double() @ w.double().t()
+    # (as above; a number below 2^-126 has parts down to 2^-149, of which 2^-150 is lost at most)
+    lost = 2.0 ** -149 + 2.0 ** -150 * x.double().abs().sum(1, keepdim=True)
+    assert ((out.double() - exact).abs() <= 15 * UNIT * (x.double().abs() @ w.double().abs().t()) + lost).all()
