@@ -804,7 +804,7 @@ __global__ void attn_decode_merge_kernel(const AttnParams p)
     size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
     if (p.units > 0) {
         const DecodeUnit u = decode_unit(p, -1, seq);
-        if (u.ranges <= 1) {
+        if (u.ranges == 1) {                          // (none: no key is visible, and the row becomes zeros here)
             pdl_wait();
             return;                                   // (the attention kernel has written the row)
         }

@@ -102,3 +102,17 @@ def test_the_product_behind_reads_finished_rows(k, ref, lens, q_lens, window, le
         close(out, exp, torch.bfloat16, "attention", rel=1.2e-2)         # (as the other tests of this kernel)
         close(product, expected, torch.float32, "the product behind", rel=1.5e-2)    # (that of its rows, each 1.2e-2 at most)
     k.check_error_word()
+
+
+def test_a_sequence_without_a_key_gives_zeros(k, always):
+    nq, nkv, d, page, lens = 4, 2, 64, 16, [900, 0, 300, 40]
+    splits = k.decode_attention_splits(len(lens), nq, nkv, max(lens))
+    assert splits > 1 and k.decode_attention_units(len(lens), nq, nkv, splits, max(lens))[0] >= len(lens)
+    pages = sum(-(-n // page) for n in lens)
+    table, positions, seq_of_token, q_start, ctx_len = _paged_setup(lens, [1] * 4, page, pages, seed=1)
+    q = rnd(4, nq * d, dtype=torch.bfloat16, seed=2)
+    kc, vc = rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=3), rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=4)
+    out = torch.full_like(q, float("nan"))
+    k.attention(q, kc, vc, out, table, q_start, ctx_len, seq_of_token, positions, nq, nkv, d, page, d ** -0.5, None, 1, max(lens), 1)
+    k.check_error_word()
+    assert (out[1] == 0).all() and torch.isfinite(out).all()
