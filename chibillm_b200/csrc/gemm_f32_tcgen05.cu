@@ -171,18 +171,63 @@ template <int COUNT> __device__ __forceinline__ void f3_tmem_store(uint32_t at, 
         tmem_store_32x8(at, r);
 }
 
-// An output by multiply-adds (a rare event, out of line: its registers don't count against the loop).
-__device__ __noinline__ float f3_by_hand(const float* x, const float* w, int K)
+// Outputs that the tensor cores cannot make (a rare event, out of line: its registers don't count against the loop, if they are not
+// many: four outputs at a time cost a call of few rows 4 of 14 us without any such output), by a whole warp: of lane's `count`
+// ones, (m + u * dm, n + u * dn), those with bit u of `bad`.  The warp reads the rows of one at a time in whole lines; sums are 64-bit, so
+// that their order does not matter.  300 (4) rows of 6,144 x 1,024 without such a row 42 us (14); one row with an infinity 108 (112),
+// one row that is no number 45 (17), all rows 58 (17), a row of w with an infinity 125 (18); by a chain of multiply-adds of one
+// thread each 168 (134), 174 (141), 7,816 (162), 1,495 (39).
+__device__ __noinline__ void f3_by_hand(const F3Params& p, uint32_t bad, int count, int m, int n, int dm, int dn)
 {
-    float v = 0.f;
-    for (int k = 0; k < K; ++k)
-        v = fmaf(x[k], w[k], v);
-    return v;
+    const int lane = threadIdx.x & 31;
+    auto store = [&](int mm, int nn, float v) {
+        p.out[(size_t)mm * p.out_stride + nn] = p.residual ? p.residual[(size_t)mm * p.res_stride + nn] + v : v;
+    };
+    for (int u = 0; u < count; ++u) {
+        const int own_m = m + u * dm, own_n = n + u * dn;
+        bool mine = bad >> u & 1u;
+        if (mine) {
+            // (a row of which nothing is a number is one from its first place on: every lane looks for itself)
+            const float a = p.x[(size_t)own_m * p.x_stride], b = p.w[(size_t)own_n * p.w_stride];
+            if (a != a || b != b) {
+                store(own_m, own_n, NAN);
+                mine = false;
+            }
+        }
+        for (uint32_t left = __ballot_sync(0xffffffffu, mine); left; left &= left - 1) {
+            const int from = __ffs(left) - 1, mm = __shfl_sync(0xffffffffu, own_m, from), nn = __shfl_sync(0xffffffffu, own_n, from);
+            const float* const x = p.x + (size_t)mm * p.x_stride;
+            const float* const w = p.w + (size_t)nn * p.w_stride;
+            double s = 0.0;
+            for (int k0 = 4 * lane; k0 < (p.K + 511) / 512 * 512; k0 += 512) {
+                float4 a[4], b[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int k = k0 + 128 * i;
+                    a[i] = k + 4 <= p.K ? *reinterpret_cast<const float4*>(x + k) : f3_load_end(x, k, p.K);
+                    b[i] = k + 4 <= p.K ? *reinterpret_cast<const float4*>(w + k) : f3_load_end(w, k, p.K);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    s = fma((double)a[i].x, (double)b[i].x, s);
+                    s = fma((double)a[i].y, (double)b[i].y, s);
+                    s = fma((double)a[i].z, (double)b[i].z, s);
+                    s = fma((double)a[i].w, (double)b[i].w, s);
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == from)
+                store(mm, nn, (float)s);
+            __syncwarp();
+        }
+    }
 }
 
 template <int NT, int WORKERS>
 __global__ void __launch_bounds__(WORKERS == 256 ? 288 : 640, WORKERS == 256 ? 2 : 1)
-gemm_f32_tc_kernel(const F3Params p)
+gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
 {
     pdl_trigger();
     constexpr int OTHERS = WORKERS == 256 ? 32 : 128;
@@ -372,15 +417,17 @@ gemm_f32_tc_kernel(const F3Params p)
         const int kept = ranks >= 4 ? own : 1;                       // sums of a rank
         float* const sums = reinterpret_cast<float*>(smem);          // [kept][column][row] (the stages are read: this thread has
                                                                      // waited for the last products)
+        // stores an output; true if it is to be made by hand
         auto finish = [&](int m, int n, float v) {
             if (m >= p.M || n >= p.N)
-                return;
+                return false;
             v *= F3_DOWN;
             if (!(fabsf(v) < INFINITY))
-                v = f3_by_hand(p.x + (size_t)m * p.x_stride, p.w + (size_t)n * p.w_stride, p.K);
+                return true;
             if (p.residual)
                 v = p.residual[(size_t)m * p.res_stride + n] + v;
             p.out[(size_t)m * p.out_stride + n] = v;
+            return false;
         };
         {
             const int slots = ranks == 1 ? (p.runs > 4 ? 2 : 1) : kept;
@@ -394,10 +441,14 @@ gemm_f32_tc_kernel(const F3Params p)
                     f3_tmem_load(lanes + 3 * NT + c * PIECE, b);
                 tmem_load_wait();
                 if (ranks == 1) {
+                    uint32_t bad = 0;
 #pragma unroll
                     for (int u = 0; u < PIECE; ++u)
-                        if (col + u < p.cols)
-                            finish(m0 + col + u, n0 + row, __uint_as_float(a[u]) + (slots > 1 ? __uint_as_float(b[u]) : 0.f));
+                        if (col + u < p.cols
+                            && finish(m0 + col + u, n0 + row, __uint_as_float(a[u]) + (slots > 1 ? __uint_as_float(b[u]) : 0.f)))
+                            bad |= 1u << u;
+                    if (__any_sync(0xffffffffu, bad != 0))
+                        f3_by_hand(p, bad, PIECE, m0 + col, n0 + row, 1, 0);
                 } else {
 #pragma unroll
                     for (int u = 0; u < PIECE; ++u) {
@@ -415,7 +466,7 @@ gemm_f32_tc_kernel(const F3Params p)
                 const int each = ranks >= 4 ? 1 : 4;                 // runs of a kept sum
                 for (int i = 4 * (rank * WORKERS + tid - OTHERS); i < p.cols * F3_ROWS; i += 4 * ranks * WORKERS) {
                     const int col = i / F3_ROWS, row = i % F3_ROWS;
-                    if (m0 + col >= p.M || n0 + row >= p.N)
+                    if (m0 + col >= p.M)                             // (a warp has one column; rows past the end are not stored)
                         continue;
                     float4 s[F3_RUNS];
 #pragma unroll
@@ -440,10 +491,12 @@ gemm_f32_tc_kernel(const F3Params p)
                         }
                         add(v, w);
                     }
-                    finish(m0 + col, n0 + row, v.x);
-                    finish(m0 + col, n0 + row + 1, v.y);
-                    finish(m0 + col, n0 + row + 2, v.z);
-                    finish(m0 + col, n0 + row + 3, v.w);
+                    uint32_t bad = finish(m0 + col, n0 + row, v.x) ? 1u : 0u;
+                    bad |= finish(m0 + col, n0 + row + 1, v.y) ? 2u : 0u;
+                    bad |= finish(m0 + col, n0 + row + 2, v.z) ? 4u : 0u;
+                    bad |= finish(m0 + col, n0 + row + 3, v.w) ? 8u : 0u;
+                    if (__any_sync(0xffffffffu, bad != 0))
+                        f3_by_hand(p, bad, 4, m0 + col, n0 + row, 0, 1);
                 }
             }
             cluster_sync();                                          // nobody leaves while its sums are read
@@ -468,7 +521,7 @@ gemm_f32_tc_kernel(const F3Params p)
 // 7.5, 7.6; 151,936 x 1,024 104, 123, 125 and 106, 106, 107; 6,144 x 1,024 7.0, 8.1, 10.7 and 8.0, 8.1, 8.3.
 template <int TILES, int WARPS, bool KEPT>                   // eights of rows of x; warps; x stays split in shared memory
 __global__ void __launch_bounds__(32 * WARPS, F3_FEW_WARPS / WARPS)
-gemm_f32_few_kernel(const F3Params p, int w_tiles)
+gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
 {
     pdl_trigger();
     // sixteen warps take the blocks in turn; eight a run each, so that there is less to put together
@@ -644,10 +697,8 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
             }
         }
         __syncthreads();
-        for (int o = threadIdx.x; o < XS * 16; o += THREADS) {
+        for (int o = threadIdx.x; o < XS * 16; o += THREADS) {       // (whole warps)
             const int m = o / 16, n = tile * 16 + o % 16;
-            if (m >= p.M || n >= p.N)
-                continue;
             float s[F3_RUNS];
             if (OWN) {
 #pragma unroll
@@ -679,11 +730,11 @@ gemm_f32_few_kernel(const F3Params p, int w_tiles)
                 v += half;
             }
             v *= F3_DOWN;
-            if (!(fabsf(v) < INFINITY))
-                v = f3_by_hand(p.x + (size_t)m * p.x_stride, p.w + (size_t)n * p.w_stride, p.K);
-            if (p.residual)
-                v = p.residual[(size_t)m * p.res_stride + n] + v;
-            p.out[(size_t)m * p.out_stride + n] = v;
+            const bool in = m < p.M && n < p.N, bad = in && !(fabsf(v) < INFINITY);
+            if (in && !bad)
+                p.out[(size_t)m * p.out_stride + n] = p.residual ? p.residual[(size_t)m * p.res_stride + n] + v : v;
+            if (__any_sync(0xffffffffu, bad))
+                f3_by_hand(p, bad ? 1u : 0u, 1, m, n, 0, 0);
         }
         // (the sums of a turn are written again only behind the next turn's barrier; there is one tile to a CTA of sixteen warps, or
         // few)

@@ -97,3 +97,20 @@ def test_small_weights_keep_their_bits(k, rows, x_size, w_size):
     # (as above; a number below 2^-126 has parts down to 2^-149, of which 2^-150 is lost at most)
     lost = 2.0 ** -149 + 2.0 ** -150 * x.double().abs().sum(1, keepdim=True)
     assert ((out.double() - exact).abs() <= 15 * UNIT * (x.double().abs() @ w.double().abs().t()) + lost).all()
+
+
+# (one chain of roundings over K lost 5.8e-7 of the sizes here, 64-bit sums nothing: what is left is the result's rounding)
+@pytest.mark.parametrize("rows", [4, 12, 40, 300])
+def test_large_numbers_are_summed_exactly(k, rows):
+    x, w, residual = rnd(rows, 1028, seed=9)[:, :1027], (rnd(300, 1028, seed=10) * 1e-3)[:, :1027], rnd(rows, 300, seed=11) * 1e33
+    x[rows // 2] *= 1e35
+    w[7] *= 1e37
+    out = residual.clone()
+    k.linear(x, w, out, out)                                 # (added in place)
+    exact, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    large = torch.zeros(rows, 300, dtype=torch.bool, device="cuda")
+    large[rows // 2] = large[:, 7] = True
+    finite, total = exact.abs() < 3e38, exact + residual.double()
+    assert ((out.double() - total).abs() <= 2 * UNIT * (exact.abs() + total.abs()))[large & finite].all()
+    assert ((out.double() - total).abs() <= (15 + 17) * UNIT * size + 2 * UNIT * total.abs())[~large & finite].all()
+    assert torch.isinf(out[exact.abs() > 3.5e38]).all()
