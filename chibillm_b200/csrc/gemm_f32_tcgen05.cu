@@ -833,10 +833,10 @@ CHIBI_API int chibi_gemm_f32(const float* x, const float* w, float* out, const f
     // takes by the row of x.  (Clusters of eight do not fill every SM.)
     const int tiles = (N + F3_ROWS - 1) / F3_ROWS;
     double least = 0.0;
-    for (int parts = (M + 127) / 128; parts <= (M + 15) / 16; ++parts) {
-        const int width = ((M + parts - 1) / parts + 15) / 16 * 16;
-        if ((M + width - 1) / width != parts)
-            continue;
+    for (int width = 128; width >= 16; width -= 16) {
+        const int parts = (M + width - 1) / width;
+        if (((M + parts - 1) / parts + 15) / 16 * 16 != width)
+            continue;                                            // (as many parts of less width are enough)
         for (int r = 1; r <= F3_RUNS; r *= 2) {
             if ((r - 1) * (F3_RUNS / r) >= p.runs)
                 break;                                           // (a CTA without a run)
