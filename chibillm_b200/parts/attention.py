@@ -249,8 +249,9 @@ class PagedAttention(Mixer):
         if decode is None:
             return None
         s = self.spec
-        return (decode(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),) \
-            + (self.runtime.float32_launch_key(ctx, s.head_dim) if self.value_dim == s.head_dim else ())
+        if self.runtime.is_float32:
+            return self.runtime.float32_launch_key(ctx, s.head_dim) if self.value_dim == s.head_dim else ()
+        return (decode(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),)
 
     # ---- run
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, overwrite: bool = False, hold: bool = False):

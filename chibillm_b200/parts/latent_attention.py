@@ -129,8 +129,9 @@ class LatentAttention(Mixer):
         decode = getattr(self.runtime.kernels, "decode_attention_key", None)
         if decode is None:
             return None
-        return (decode(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),) \
-            + self.runtime.float32_launch_key(ctx, self.key_dim)
+        if self.runtime.is_float32:
+            return self.runtime.float32_launch_key(ctx, self.key_dim)
+        return (decode(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, hold: bool = False):
         s, rt = self.spec, self.runtime
