@@ -56,6 +56,12 @@ __device__ __forceinline__ uint64_t af_mul2(uint64_t a, uint64_t b)
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ uint64_t af_add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 // 16 bytes, zeros where `bytes` is 0 (nothing is read then).
 __device__ __forceinline__ void af_copy16(float* dst, const float* src, int bytes)
 {
@@ -124,8 +130,12 @@ __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -IN
 // so: 3 prompts of up to 400 tokens of 16 heads 109 and 38, 4 of up to 600 after 800 of 32 heads 1,235 and 322, 64 tokens after 800
 // of 16 heads 86 and 64, 100 after 4,000 417 and 298, 4 after 800 78 and 59.
 //
-// Numbers that are none: a key or query with one marks its scores, which are then summed by multiply-adds; a value adds
-// itself to the columns of the rows that see it.
+// Queries, keys, values and probabilities are split times 2^16, so that the last parts of small ones (of all normal numbers) are
+// no smaller than a bfloat16 can be; scores and outputs are 2^32 as large as they should be until they are used.  A query or
+// key that is no number, or too large (from 2^112 on), has an infinite part and makes its scores no number; those, and scores from
+// 2^96 on, are summed by multiply-adds.  Such values are marked and taken out, because they would spoil the rows that do not see
+// them: what is no number adds itself to its column of the rows that do, and rows that see a large one, or whose sums are too
+// large, are made by hand.
 constexpr int AT_ROWS = 128, AT_KEYS = 64, AT_WORKERS = 512, AT_THREADS = 128 + AT_WORKERS;
 constexpr int AT_REGS = 96, AT_REGS_FEW = 32, AT_REGS_MANY = 112;    // of a thread at launch, of the first four warps', of the others'
 static_assert(AT_REGS_FEW + 4 * AT_REGS_MANY <= 5 * AT_REGS, "more registers than the block has");
@@ -135,7 +145,7 @@ template <int D> struct AtShape {
     static constexpr int SLICES = D / 64;                        // 64 features are a swizzled line
     static constexpr int Q_PLANE = AT_ROWS * D * 2, KV_PLANE = AT_KEYS * D * 2;
     static constexpr int TILES = 3 * Q_PLANE + 6 * KV_PLANE;
-    static constexpr size_t SHARED = 1024 + TILES + 64 + 4 * (AT_SHARE * AT_ROWS + 20 + AT_ROWS);
+    static constexpr size_t SHARED = 1024 + TILES + 64 + 4 * (3 * AT_SHARE * AT_ROWS + 12);
     static constexpr uint32_t S_COLS = 64 * SLICES;              // TMEM: two buffers of S, three parts of P, O
     static constexpr uint32_t P_AT = 2 * S_COLS, O_AT = P_AT + 96, TMEM = O_AT + D <= 256 ? 256 : 512;
 };
@@ -161,24 +171,13 @@ __device__ __forceinline__ void at_put(uint32_t at, uint32_t a, uint32_t b)
 {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
 }
-// A number whose leading part would be infinite: none (0 and true), or so large that its part is cut off instead of rounded.
-__device__ __noinline__ bool at_odd_parts(float v, uint32_t parts[3])
+constexpr uint64_t AT_UP = 0x4780000047800000ull;                // 2^16 twice
+constexpr float AT_DOWN = 0x1p-32f;
+// Writes the three parts of four numbers, `plane` bytes apart; what the last ones are before they are rounded is no number
+// where one of the four is none or too large.
+__device__ __forceinline__ uint64_t at_split(float4 v, uint32_t at, uint32_t plane)
 {
-    parts[0] = parts[1] = parts[2] = 0;
-    if (!(fabsf(v) < INFINITY))
-        return true;
-    for (int i = 0; i < 3; ++i) {
-        const uint32_t cut = __float_as_uint(v) & 0xffff0000u;
-        parts[i] = cut >> 16;
-        v -= __uint_as_float(cut);
-    }
-    return false;
-}
-// Writes the three parts of four numbers, `plane` bytes apart; adds to `none` what is no number if one of them is none, or so
-// large that its leading part is infinite.
-__device__ __forceinline__ void at_split(float4 v, uint32_t at, uint32_t plane, uint64_t& none)
-{
-    uint64_t x = af_pair(v.x, v.y), y = af_pair(v.z, v.w);
+    uint64_t x = af_mul2(af_pair(v.x, v.y), AT_UP), y = af_mul2(af_pair(v.z, v.w), AT_UP);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         const uint32_t a = at_pair(x), b = at_pair(y);
@@ -188,19 +187,22 @@ __device__ __forceinline__ void at_split(float4 v, uint32_t at, uint32_t plane, 
             y = at_rest(y, b);
         }
     }
-    none = af_fma2(x, 0x3f8000003f800000ull, af_fma2(y, 0x3f8000003f800000ull, none));      // (infinite parts leave no numbers)
+    return af_add2(x, y);
 }
-// The same for numbers among which some are none or very large; true if one is none (its parts are 0 then).
+// The same without what has no parts (2^16 times it is infinite as bfloat16, or it is none); true if there was one.
 __device__ __noinline__ bool at_split_odd(float4 v, uint32_t at, uint32_t plane)
 {
-    uint32_t parts[4][3];
-    bool none = at_odd_parts(v.x, parts[0]);
-    none |= at_odd_parts(v.y, parts[1]);
-    none |= at_odd_parts(v.z, parts[2]);
-    none |= at_odd_parts(v.w, parts[3]);
-    for (int i = 0; i < 3; ++i)
-        at_put(at + i * plane, parts[0][i] | parts[1][i] << 16, parts[2][i] | parts[3][i] << 16);
-    return none;
+    bool found = false;
+    auto one = [&](float& x) {
+        if ((__float_as_uint(x) & 0x7fffffffu) >= 0x777f8000u) {
+            x = 0.f;
+            found = true;
+        }
+    };
+    one(v.x), one(v.y), one(v.z), one(v.w);
+    if (found)
+        at_split(v, at, plane);
+    return found;
 }
 __device__ __forceinline__ bool at_none(uint64_t v)
 {
@@ -209,10 +211,74 @@ __device__ __forceinline__ bool at_none(uint64_t v)
 }
 __device__ __noinline__ float at_dot(const float* a, const float* b, int d)
 {
-    float s = 0.f;
-    for (int i = 0; i < d; ++i)
-        s = fmaf(a[i], b[i], s);
-    return s;
+    float s[4] = { 0.f, 0.f, 0.f, 0.f };
+    for (int i = 0; i < d; i += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + i), y = *reinterpret_cast<const float4*>(b + i);
+        s[0] = fmaf(x.x, y.x, s[0]);
+        s[1] = fmaf(x.y, y.y, s[1]);
+        s[2] = fmaf(x.z, y.z, s[2]);
+        s[3] = fmaf(x.w, y.w, s[3]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+}
+// A thread's part of a row's output (COLS columns, by pieces of four in swizzled places), the scores and the sums of the products
+// anew, in 64 bits what could be too large for 32: exponents against `top`, times `inv` at the end.
+template <int D, bool OPTIONS>
+__device__ __noinline__ void at_row_by_hand(const AttentionF32& p, const int* table, int token, int h, int kv_head, int pos, int first,
+                                            int part, float top, float inv, float* out, int swizzle)
+{
+    constexpr int COLS = D / AT_SHARE, PIECES = COLS / 4;
+    const float* const q = p.q + ((size_t)token * p.nq + h) * D;
+    const float r1 = p.bias_r1 ? p.bias_r1[h] : 0.f, r2 = p.bias_r2 ? p.bias_r2[h] : 0.f, least = top == -INFINITY ? 0.f : top;
+    double sum[COLS];
+    for (int c = 0; c < COLS; ++c)
+        sum[c] = 0.0;
+    for (int key = first; key <= pos; ++key) {
+        const int page = table[key / p.page_size];
+        if (page < 0 || page >= p.num_pages)
+            continue;
+        const size_t at = (size_t)((page * p.nkv + kv_head) * p.page_size + key % p.page_size) * D;
+        const float dot = at_dot(q, p.k_cache + at, D);
+        const double e = expf((OPTIONS ? af_score(p, dot, r1, r2, pos - key) : dot * p.scale) - least);
+        for (int c = 0; c < COLS; ++c)
+            sum[c] = fma(e, (double)p.v_cache[at + part * COLS + c], sum[c]);
+    }
+    for (int c = 0; c < COLS; ++c)
+        reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(out) + (((part * PIECES + c / 4) ^ (swizzle & 7)) << 4))[c & 3] = (float)(sum[c] * inv);
+}
+// A thread's scores that the tensor cores could not make (infinite or no number), by multiply-adds; those of hidden keys stay.
+template <int D, bool OPTIONS>
+__device__ __noinline__ void at_scores_in_memory(const AttentionF32& p, float* s, const int* table, int token, int h, int kv_head, int key0,
+                                                 int first, int pos)
+{
+    const float* const q = p.q + ((size_t)token * p.nq + h) * D;
+    for (int i = 0; i < AT_OWN; ++i) {
+        const int key = key0 + i;
+        if (fabsf(s[i]) < INFINITY || key > pos || key < first)
+            continue;
+        const int page = table[key / p.page_size];
+        if (page < 0 || page >= p.num_pages)
+            continue;
+        const float* const k = p.k_cache + (size_t)((page * p.nkv + kv_head) * p.page_size + key % p.page_size) * D;
+        if (q[0] != q[0] || k[0] != k[0])                        // (a row of which nothing is a number: it is none already)
+            continue;
+        const float dot = at_dot(q, k, D);
+        s[i] = OPTIONS ? dot : dot * p.scale;
+    }
+}
+// (By way of memory: with the registers indexed here, and this call among them, all calls took 4 to 7 % longer.)
+template <int D, bool OPTIONS>
+__device__ __forceinline__ void at_scores_by_hand(const AttentionF32& p, float (&s)[AT_OWN], const int* table, int token, int h, int kv_head,
+                                                  int key0, int first, int pos)
+{
+    float there[AT_OWN];
+#pragma unroll
+    for (int i = 0; i < AT_OWN; ++i)
+        there[i] = s[i];
+    at_scores_in_memory<D, OPTIONS>(p, there, table, token, h, kv_head, key0, first, pos);
+#pragma unroll
+    for (int i = 0; i < AT_OWN; ++i)
+        s[i] = there[i];
 }
 // The warps that share 32 rows.
 __device__ __forceinline__ void at_row_sync(int barrier)
@@ -237,7 +303,7 @@ template <int COUNT> __device__ __forceinline__ void at_tmem_load(uint32_t at, u
 
 template <int D, bool OPTIONS>
 __global__ void __launch_bounds__(AT_THREADS, 1)
-attention_f32_prompt_kernel(const AttentionF32 p)
+attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
 {
     pdl_enter();
     using Shape = AtShape<D>;
@@ -253,12 +319,13 @@ attention_f32_prompt_kernel(const AttentionF32 p)
     uint64_t* const o_done = bars + 3;           // MMA commit
     uint32_t* const tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
     float* const exchange = reinterpret_cast<float*>(bars + 8);          // [4][128]
-    // marks of what holds a number that is none: keys [4][2] and values [4][2] of a block's 64 (block j in place j % 4), any at
-    // all, queries [128]
-    uint32_t* const odd_keys = reinterpret_cast<uint32_t*>(exchange + AT_SHARE * AT_ROWS);
-    uint32_t* const odd_values = odd_keys + 8;
+    // marks of values that have no parts: [4][2], of a block's 64 keys (block j in place j % 4), and whether there are any at all
+    uint32_t* const odd_values = reinterpret_cast<uint32_t*>(exchange + AT_SHARE * AT_ROWS);
     uint32_t* const odd_any = odd_values + 8;
-    int* const odd_row = reinterpret_cast<int*>(odd_any + 4);
+    // [512] of each working thread: the columns that a value which is no number has added itself to; whether a value that is too
+    // large is among what it sees (rare events: in memory they take no registers)
+    uint32_t* const spoiled = odd_any + 4;
+    uint32_t* const large = spoiled + AT_WORKERS;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int seq = blockIdx.z, kv_head = blockIdx.y, G = p.nq / p.nkv;
@@ -285,10 +352,8 @@ attention_f32_prompt_kernel(const AttentionF32 p)
         tmem_alloc(tmem_slot, Shape::TMEM);
         tmem_relinquish();
     }
-    if (tid < AT_ROWS)
-        odd_row[tid] = 0;
-    if (tid < 20)
-        odd_keys[tid] = 0;
+    if (tid < 12)
+        odd_values[tid] = 0;
 
     tcgen05_fence_before();
     __syncthreads();
@@ -387,21 +452,25 @@ attention_f32_prompt_kernel(const AttentionF32 p)
                 v[i] = at >= 0 ? *reinterpret_cast<const float4*>(cache + (size_t)at * D + 4 * quad) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        auto spread = [&](const float4 (&v)[KV_EACH], uint32_t to, uint32_t* flags) {
-            uint64_t none = 0;
+        auto spread = [&](const float4 (&v)[KV_EACH], uint32_t to) {
+            uint64_t last = 0;
 #pragma unroll
             for (int i = 0; i < KV_EACH; ++i)
-                at_split(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE, none);
-            if (at_none(none)) {
+                last = af_add2(at_split(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE), last);
+            return last;
+        };
+        auto spread_values = [&](const float4 (&v)[KV_EACH], uint32_t* flags) {
+            if (at_none(spread(v, v_s))) {
 #pragma unroll
                 for (int i = 0; i < KV_EACH; ++i) {
                     const int r = line + PASS * i;
-                    if (at_split_odd(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE)) {
+                    if (at_split_odd(v[i], v_s + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE)) {
                         atomicOr(&flags[r >> 5], 1u << (r & 31));
                         *odd_any = 1;
                     }
                 }
             }
+            __syncwarp();
         };
         float4 kn[KV_EACH], vn[KV_EACH];
         int page[3], found[2];                                       // pages of blocks j + 1 .. j + 3 (looked up long before they are
@@ -429,16 +498,10 @@ attention_f32_prompt_kernel(const AttentionF32 p)
                                       : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
-            for (int i = 0; i < Q_EACH / 2; ++i) {
-                const int r = line + PASS * (i + half * (Q_EACH / 2));
-                uint64_t none = 0;
-                const uint32_t to = q_s + q_at + (i + half * (Q_EACH / 2)) * (PASS / 8) * 1024;
-                at_split(v[i], to, Shape::Q_PLANE, none);
-                if (at_none(none) && at_split_odd(v[i], to, Shape::Q_PLANE))
-                    odd_row[r] = *odd_any = 1;
-            }
+            for (int i = 0; i < Q_EACH / 2; ++i)
+                at_split(v[i], q_s + q_at + (i + half * (Q_EACH / 2)) * (PASS / 8) * 1024, Shape::Q_PLANE);
         }
-        spread(kn, k_s, odd_keys);
+        spread(kn, k_s);
         fence_proxy_async();
         mbar_arrive(keys_there);
         if (blocks > 1)
@@ -452,7 +515,10 @@ attention_f32_prompt_kernel(const AttentionF32 p)
         const int first = first_visible_key(pos, p.window, p.chunk);
         constexpr int COLS = D / AT_SHARE;
         uint64_t O[COLS / 2];
+        const float down = OPTIONS ? AT_DOWN : p.scale * AT_DOWN;
+        const uint64_t down2 = af_pair(down, down);
         float m = -INFINITY, l = 0.f;
+        spoiled[worker] = large[worker] = 0;
 #pragma unroll
         for (int c = 0; c < COLS / 2; ++c)
             O[c] = 0;
@@ -469,32 +535,44 @@ attention_f32_prompt_kernel(const AttentionF32 p)
 #pragma unroll
             for (int c = 0; c < COLS / 2; ++c)
                 O[c] = af_fma2(O[c], 0x3f8000003f800000ull, af_pair(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])));
-            if (*odd_any)
-                for (int i = 0; i < AT_KEYS; ++i) {
+            if (*odd_any) {
+                uint32_t found = 0;                                  // columns, as in `spoiled`
+                bool too_large = false, left = false;                // (nothing is left to spoil where all are none)
+#pragma unroll
+                for (int c = 0; c < COLS / 2; ++c) {
+                    const float2 o = af_halves(O[c]);
+                    left |= o.x == o.x || o.y == o.y;
+                }
+                for (int i = 0; i < AT_KEYS && left; ++i) {
                     const int key = begin + j * AT_KEYS + i;
                     if ((odd_values[2 * (j & 3) + (i >> 5)] >> (i & 31) & 1) && key <= pos && key >= first) {
                         const float* const v = p.v_cache + key_at(key) + part * COLS;        // (what is marked has been read)
 #pragma unroll
                         for (int c = 0; c < COLS / 2; ++c) {
                             const float x = v[2 * c], y = v[2 * c + 1];
+                            const bool no_x = !(fabsf(x) < INFINITY), no_y = !(fabsf(y) < INFINITY);
                             const float2 o = af_halves(O[c]);
-                            O[c] = af_pair(o.x + (fabsf(x) < INFINITY ? 0.f : x), o.y + (fabsf(y) < INFINITY ? 0.f : y));
+                            O[c] = af_pair(o.x + (no_x ? x : 0.f), o.y + (no_y ? y : 0.f));
+                            found |= (no_x ? 1u : 0u) << (2 * c) | (no_y ? 2u : 0u) << (2 * c);
+                            too_large |= (!no_x && fabsf(x) >= 0x1p111f) || (!no_y && fabsf(y) >= 0x1p111f);
                         }
                     }
                 }
+                spoiled[worker] |= found;
+                large[worker] |= too_large;
+            }
+            __syncwarp();
         };
         for (int j = 0; j < blocks; ++j) {
             const int base = begin + j * AT_KEYS;
             mbar_wait_warp(s_done, j & 1, p.error, 73);
             tcgen05_fence_after();
-            // (places of blocks that all threads are through with: everyone has written keys j)
-            if (worker < 2) {
-                odd_keys[2 * ((j + 2) & 3) + worker] = 0;
+            // (a place of a block that all threads are through with: everyone has written keys j)
+            if (worker < 2)
                 odd_values[2 * ((j + 1) & 3) + worker] = 0;
-            }
             // the next block's scores are made while this one's are worked on
             if (j + 1 < blocks) {
-                spread(kn, k_s, odd_keys + 2 * ((j + 1) & 3));
+                spread(kn, k_s);
                 fence_proxy_async();
                 tcgen05_fence_before();
                 mbar_arrive(keys_there);
@@ -502,36 +580,38 @@ attention_f32_prompt_kernel(const AttentionF32 p)
                     fetch(p.k_cache, found[1], kn);
             }
             float s[AT_OWN];
+            uint64_t none = 0;                                       // (no number, or infinite, if a score is)
             {
                 uint32_t v[Shape::SLICES][AT_OWN];
 #pragma unroll
                 for (int slice = 0; slice < Shape::SLICES; ++slice)
                     at_tmem_load(lanes + (j & 1) * Shape::S_COLS + slice * 64 + part * AT_OWN, v[slice]);
                 tmem_load_wait();
+                uint64_t pairs[AT_OWN / 2];
 #pragma unroll
-                for (int i = 0; i < AT_OWN; ++i) {
-                    s[i] = __uint_as_float(v[0][i]);
+                for (int i = 0; i < AT_OWN / 2; ++i) {
+                    pairs[i] = af_pair(__uint_as_float(v[0][2 * i]), __uint_as_float(v[0][2 * i + 1]));
                     if (Shape::SLICES > 1)
-                        s[i] += __uint_as_float(v[Shape::SLICES - 1][i]);
+                        pairs[i] = af_add2(pairs[i], af_pair(__uint_as_float(v[Shape::SLICES - 1][2 * i]), __uint_as_float(v[Shape::SLICES - 1][2 * i + 1])));
+                    pairs[i] = af_mul2(pairs[i], down2);
+                    if (i % 2)
+                        none = af_fma2(pairs[i - 1], pairs[i], none);
+                    const float2 h = af_halves(pairs[i]);
+                    s[2 * i] = h.x;
+                    s[2 * i + 1] = h.y;
                 }
             }
             const int key0 = base + part * AT_OWN;
-            if (*odd_any) {
-                const uint32_t marked = odd_row[r] ? 0xffffffffu : odd_keys[2 * (j & 3) + part / 2] >> (part & 1) * AT_OWN;
-                for (int i = 0; i < AT_OWN; ++i)
-                    if (marked >> i & 1 && key0 + i <= pos && key0 + i >= first && key_at(key0 + i) >= 0) {
-                        const float dot = at_dot(p.q + ((size_t)(row0 + row / G) * p.nq + h) * D, p.k_cache + key_at(key0 + i), D);
-#pragma unroll
-                        for (int u = 0; u < AT_OWN; ++u)
-                            s[u] = u == i ? dot : s[u];
-                    }
-            }
+            if (at_none(none))
+                at_scores_by_hand<D, OPTIONS>(p, s, table, row0 + row / G, h, kv_head, key0, first, pos);
             // every row sees every key of these?
             const bool whole = __all_sync(0xffffffffu, key0 + AT_OWN - 1 <= pos && key0 >= first);
             float most = -INFINITY;
+            if (OPTIONS) {
 #pragma unroll
-            for (int i = 0; i < AT_OWN; ++i)
-                s[i] = OPTIONS ? af_score(p, s[i], r1, r2, pos - key0 - i) : s[i] * p.scale;
+                for (int i = 0; i < AT_OWN; ++i)
+                    s[i] = af_score(p, s[i], r1, r2, pos - key0 - i);
+            }
             if (!whole) {
 #pragma unroll
                 for (int i = 0; i < AT_OWN; ++i)
@@ -566,7 +646,7 @@ attention_f32_prompt_kernel(const AttentionF32 p)
             uint64_t s2[AT_OWN / 2];
 #pragma unroll
             for (int i = 0; i < AT_OWN / 2; ++i)
-                s2[i] = af_pair(s[2 * i], s[2 * i + 1]);
+                s2[i] = af_mul2(af_pair(s[2 * i], s[2 * i + 1]), AT_UP);
 #pragma unroll
             for (int plane = 0; plane < 3; ++plane) {
                 uint32_t pairs[AT_OWN / 2];
@@ -577,7 +657,7 @@ attention_f32_prompt_kernel(const AttentionF32 p)
                 }
                 tmem_store_32x8(lanes + Shape::P_AT + plane * 32 + part * (AT_OWN / 2), pairs);
             }
-            spread(vn, v_s, odd_values + 2 * (j & 3));
+            spread_values(vn, odd_values + 2 * (j & 3));
             tmem_store_wait();
             fence_proxy_async();
             tcgen05_fence_before();
@@ -596,23 +676,37 @@ attention_f32_prompt_kernel(const AttentionF32 p)
 #pragma unroll
         for (int x = 0; x < AT_SHARE; ++x)
             l += exchange[x * AT_ROWS + r];
+        float top = m;
         if (p.sink) {
-            const float sink = p.sink[h], top = fmaxf(sink, m), keep = af_keep(m, top);
+            const float sink = p.sink[h];
+            top = fmaxf(sink, m);
+            const float keep = af_keep(m, top);
             l = l * keep + af_keep(sink, top);
             const uint64_t keep2 = af_pair(keep, keep);
 #pragma unroll
             for (int c = 0; c < COLS / 2; ++c)
                 O[c] = af_mul2(O[c], keep2);
         }
-        const float inv = l > 0.f ? 1.f / l : 0.f;
+        const float inv = l > 0.f ? 1.f / l : 0.f, inv_down = inv * AT_DOWN;
+        uint32_t none = 0;                                           // columns whose sums are no number, or too large for one
+#pragma unroll
+        for (int c = 0; c < COLS / 2; ++c) {
+            const float2 o = af_halves(O[c]);
+            none |= (fabsf(o.x) < INFINITY ? 0u : 1u) << (2 * c) | (fabsf(o.y) < INFINITY ? 0u : 2u) << (2 * c);
+        }
+        const bool by_hand = l == l && ((none & ~spoiled[worker]) || large[worker]);     // (with a score that is none all of the row is)
         constexpr int CHUNKS = D / 4, SHARE = CHUNKS / AT_SHARE;     // pieces of 16 bytes of a row, and a thread's
         uint8_t* const rows = smem + quarter * 32 * (D * 4);
 #pragma unroll
         for (int c = 0; c < SHARE; ++c) {
             const float2 a = af_halves(O[2 * c]), b = af_halves(O[2 * c + 1]);
             *reinterpret_cast<float4*>(rows + lane * (D * 4) + (((part * SHARE + c) ^ (lane & 7)) << 4)) =
-                make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+                make_float4(a.x * inv_down, a.y * inv_down, b.x * inv_down, b.y * inv_down);
         }
+        if (by_hand)
+            at_row_by_hand<D, OPTIONS>(p, table, row0 + row / G, h, kv_head, pos, first, part, top, inv,
+                                       reinterpret_cast<float*>(rows + lane * (D * 4)), lane);
+        __syncwarp();
         at_row_sync(barrier);
 #pragma unroll 4
         for (int i = part * 32 * SHARE + lane; i < (part + 1) * 32 * SHARE; i += 32) {
@@ -830,7 +924,8 @@ static int attention_f32(const AttentionF32& p, int seqs, int max_q_len, int min
 {
     const int G = p.nq / p.nkv;
     if (max_q_len > 1) {
-        const bool options = p.softcap > 0.f || p.bias_r1;
+        // (a scale whose 2^-32th is no normal number goes the way of the other options)
+        const bool options = p.softcap > 0.f || p.bias_r1 || fabsf(p.scale) < 0x1p-90f;
         const auto kernel = options ? attention_f32_prompt_kernel<D, true> : attention_f32_prompt_kernel<D, false>;
         static bool configured[2] = { false, false };
         if (!configured[options]) {

@@ -96,3 +96,42 @@ def test_values_beyond_the_largest_bfloat16(k, d):
     exact = exact_attention(q, keys, values, table, [T], [T], 1, 1, d, 16, d ** -0.5, None, None, None, None, None)
     assert torch.isfinite(out).all()
     assert float(((out.double() - exact)[:, 1] / exact[:, 1]).abs().max()) <= 2 * 16 * (d / 4 + 16) * UNIT
+
+
+# small and large numbers: last parts down to the least normal number; products, sums of scores and sums of values that a scaled
+# accumulator cannot hold
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("q_size,k_size,v_size", [(1.0, 1.0, 1e-36), (1.0, 1.0, 1e-37), (1e-36, 1e36, 1.0), (1e35, 1e-35, 1.0),
+                                                  (1e-20, 1e20, 1e33), (1.0, 1.0, 1e37)])
+def test_small_and_large_numbers(k, d, q_size, k_size, v_size):
+    nq, nkv, page, q_lens, ctx = 4, 2, 16, [140, 2, 66], [140, 300, 66]
+    pages = [-(-c // page) for c in ctx]
+    table = torch.zeros(3, max(pages), dtype=torch.int32)
+    for s, n in enumerate(pages):
+        table[s, :n] = torch.arange(sum(pages[:s]), sum(pages[:s]) + n)
+    table = table.cuda()
+    keys, values = rnd(sum(pages), nkv, page, d, seed=1) * k_size, rnd(sum(pages), nkv, page, d, seed=2) * v_size
+    q = rnd(sum(q_lens), nq * d, seed=3) * q_size
+    out = _run(k, q, keys, values, table, q_lens, ctx, nq, nkv, d, page)
+    exact = exact_attention(q, keys, values, table, q_lens, ctx, nq, nkv, d, page, d ** -0.5, None, None, None, None, None)
+    # (the bound of test_tiles, times the values' size; a value below 2^-126 loses 2^-150 at most)
+    assert float((out.double() - exact).abs().max()) <= 2 * 6 * 16 * (d / 4 + 16) * UNIT * v_size + 2.0 ** -148
+    # (and no more than multiply-adds, which lost 1.8e-7 and 2.2e-7 of these numbers at every size)
+    relative = float((out.double() - exact).norm() / exact.norm())
+    assert relative <= 2.5e-7, relative
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_large_value_stays_with_the_rows_that_see_it(k, d):
+    T, page, place = 200, 16, 131
+    q, keys, values = rnd(T, d, seed=1), rnd(13, 1, page, d, seed=2), rnd(13, 1, page, d, seed=3)
+    table = torch.arange(13, dtype=torch.int32, device="cuda")[None]
+    clean = _run(k, q, keys, values, table, [T], [T], 1, 1, d, page)
+    values[place // page, 0, place % page, 5] = 1e38
+    values[place // page, 0, place % page, 6] = float("inf")
+    out = _run(k, q, keys, values, table, [T], [T], 1, 1, d, page)
+    exact = exact_attention(q, keys, values, table, [T], [T], 1, 1, d, page, d ** -0.5, None, None, None, None, None)
+    assert torch.equal(out[:place], clean[:place]) and (out[place:, 6] == float("inf")).all()
+    others = [c for c in range(d) if c not in (5, 6)]
+    assert float((out.double() - exact)[place:, others].abs().max()) <= 2 * 6 * 16 * (d / 4 + 16) * UNIT
+    assert float(((out.double() - exact)[place:, 5] / exact[place:, 5]).abs().max()) <= 2 * 16 * (d / 4 + 16) * UNIT
