@@ -66,9 +66,9 @@ struct AttnParams {
     int seqs;                      // decode: all sequences of the step
     int splits;                    // decode: key ranges per sequence
     int units;                     // decode: > 0: key ranges of all sequences together, cut by decode_unit
-    int by_length;                 // decode: the sequences with the most keys start first
     float* scratch_o;              // decode: [S, nq, splits, D], or [units, nq, D]
     float* scratch_ml;             // decode: the same with 2 numbers
+    int2* scratch_plan;            // decode with units: [S] a sequence's first unit and how many it has, if cut by decode_unit
     // decode, optional: q (and the newest key and value) are not in `q` and the caches yet but
     // still the partial sums of the q | k | v product: the kernel adds them up, applies the per-head
     // norm and the rotation itself and appends the new key and value (head size 128 only)
@@ -480,6 +480,32 @@ __device__ __forceinline__ int decode_tiles(const AttnParams& p, int s)
     return (pos + 1 - first_visible_key(pos, p.window, p.chunk) + DEC_TILE - 1) / DEC_TILE;
 }
 
+// The lengths of all sequences (lane i has those of i, i + 32, ...), and whether they are so near to each other (an eighth below
+// the longest on average) that cutting them anew would gain less than it takes: then every sequence has p.splits ranges.
+struct DecodeLengths {
+    int t[DEC_UNIT_SEQS / 32];
+    int most, total;
+    bool equal;
+};
+__device__ __forceinline__ DecodeLengths decode_lengths(const AttnParams& p)
+{
+    constexpr int EACH = DEC_UNIT_SEQS / 32;
+    const int lane = threadIdx.x & 31;
+    DecodeLengths d;
+    int most = 0, total = 0, live = 0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        d.t[i] = 32 * i < p.seqs ? decode_tiles(p, lane + 32 * i) : 0;
+        most = max(most, d.t[i]);
+        total += d.t[i];
+        live += __popc(__ballot_sync(0xffffffffu, d.t[i] > 0));
+    }
+    d.most = __reduce_max_sync(0xffffffffu, most);
+    d.total = __reduce_add_sync(0xffffffffu, total);
+    d.equal = 8 * (live * d.most - d.total) <= live * d.most;
+    return d;
+}
+
 struct DecodeUnit {
     int seq;               // -1: none
     int range, ranges;     // which key range of the sequence, and how many it has
@@ -489,21 +515,13 @@ struct DecodeUnit {
 
 // Cuts the sequences' keys into at most p.units ranges of c tiles (the last of a sequence shorter), c as small as that
 // allows.  Ranges of one length, not so many to every sequence: with as many CTAs as are resident at once the time is that
-// of the longest range.  The lanes try 32 values of c at a time.  `unit` >= 0 asks for that range,
-// else for the ranges of sequence `seq`.
-__device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, int unit, int seq)
+// of the longest range.  The lanes try 32 values of c at a time.
+__device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, const DecodeLengths& d, int unit)
 {
     constexpr int EACH = DEC_UNIT_SEQS / 32;
     const int lane = threadIdx.x & 31;
-    int t[EACH], most = 0, total = 0;
-#pragma unroll
-    for (int i = 0; i < EACH; ++i) {
-        t[i] = 32 * i < p.seqs ? decode_tiles(p, lane + 32 * i) : 0;
-        most = max(most, t[i]);
-        total += t[i];
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    total = __reduce_add_sync(0xffffffffu, total);
+    const int (&t)[EACH] = d.t;
+    const int most = d.most, total = d.total;
     // (at most 32 ranges of a sequence: every one is a partial result for the merge to fetch)
     int low = max(max(DEC_LEAST_TILES, (most + 31) / 32), (total + p.units - 1) / p.units);
     int high = max(low, most);                           // (one range each is no more than p.units)
@@ -544,7 +562,7 @@ __device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, int unit,
             end += lane >= o ? other : 0;
         }
         const int first = before + end - n;
-        const uint32_t mine = __ballot_sync(0xffffffffu, unit >= 0 ? (unit >= first && unit < first + n) : lane + 32 * i == seq);
+        const uint32_t mine = __ballot_sync(0xffffffffu, unit >= first && unit < first + n);
         if (mine) {
             const int l = __ffs(mine) - 1;
             u.seq = 32 * i + l;
@@ -564,9 +582,11 @@ __device__ __forceinline__ int sequence_of_rank(const AttnParams& p, int rank)
 {
     __shared__ __align__(16) int length[DEC_ORDER_SEQS];
     __shared__ int found;
-    const int s = threadIdx.x;
+    const int s = threadIdx.x, tiles = decode_tiles(p, s), tiles0 = decode_tiles(p, 0);
+    if (__syncthreads_and(s >= p.seqs || 8 * abs(tiles - tiles0) <= tiles0))
+        return rank;                                     // (all within an eighth of the first: the order is nothing to them)
     // (distinct, earlier sequences first among equals; -1 is no sequence)
-    const int key = s < p.seqs ? min(decode_tiles(p, s), (1 << 22) - 1) * DEC_ORDER_SEQS + DEC_ORDER_SEQS - 1 - s : -1;
+    const int key = s < p.seqs ? min(tiles, (1 << 22) - 1) * DEC_ORDER_SEQS + DEC_ORDER_SEQS - 1 - s : -1;
     length[s] = key;
     __syncthreads();
     int longer = 0;
@@ -580,6 +600,13 @@ __device__ __forceinline__ int sequence_of_rank(const AttnParams& p, int rank)
     return found;
 }
 
+// How the CTAs share the keys; a kernel each, because the shortest steps pay for code that they jump over (one sequence of 2,048
+// keys, 36 layers: 3.317 ms a step by a kernel of equal shares alone, 3.331 and 3.351 by one with all three).
+constexpr int DEC_SHARES = 0;                // p.splits ranges of every sequence
+constexpr int DEC_UNITS = 1;                 // p.units ranges, cut by the sequences' lengths where these differ
+constexpr int DEC_ORDERED = 2;               // p.splits ranges, the sequences with the most keys first
+
+template <int CUT>
 __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnParams p)
 {
     pdl_trigger();
@@ -591,14 +618,20 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     // before this step's first kernel: the first tiles are on their way while the kernel
     // that writes q and the newest key still runs.
     int seq = blockIdx.z, split = blockIdx.x, ranges = p.splits, unit_tiles = 0;
-    if (p.units > 0) {
-        const DecodeUnit u = decode_unit(p, blockIdx.x, -1);
-        if (u.seq < 0) {
+    if constexpr (CUT == DEC_UNITS) {
+        const DecodeLengths lengths = decode_lengths(p);
+        if (lengths.equal) {
+            seq = blockIdx.x / p.splits;
+            split = blockIdx.x - seq * p.splits;
+        } else {
+            const DecodeUnit u = decode_unit(p, lengths, blockIdx.x);
+            seq = u.seq, split = u.range, ranges = u.ranges, unit_tiles = u.tiles;
+        }
+        if (seq < 0 || seq >= p.seqs) {
             pdl_wait();                               // (every way out waits: the next kernel waits for this one alone)
             return;
         }
-        seq = u.seq, split = u.range, ranges = u.ranges, unit_tiles = u.tiles;
-    } else if (p.by_length) {
+    } else if constexpr (CUT == DEC_ORDERED) {
         seq = sequence_of_rank(p, blockIdx.z);
     }
     const int row_blocks = (p.group + 15) / 16;
@@ -613,7 +646,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
     const int first = first_visible_key(pos, p.window, p.chunk);
     const int key_end = pos + 1;
     const int tiles_total = (key_end - first + DEC_TILE - 1) / DEC_TILE;
-    const int tiles_per_split = unit_tiles > 0 ? unit_tiles : (tiles_total + p.splits - 1) / p.splits;
+    const int tiles_per_split = CUT == DEC_UNITS && unit_tiles > 0 ? unit_tiles : (tiles_total + p.splits - 1) / p.splits;
     const int tile_begin = split * tiles_per_split;
     int tile_end = tile_begin + tiles_per_split;
     if (tile_end > tiles_total)
@@ -759,6 +792,8 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
         }
     }
     __syncthreads();
+    if (CUT == DEC_UNITS && unit_tiles > 0 && split == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        p.scratch_plan[seq] = make_int2(blockIdx.x, ranges);          // (for the merge, which would cut the keys once more)
     for (int idx = threadIdx.x; idx < rows * D; idx += blockDim.x) {
         const int row = idx / D, c = idx - row * D;
         float mmax = -INFINITY;
@@ -778,7 +813,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
             lsum += sink_weight(p.sink, head, mmax);
             p.out[((size_t)t * p.nq + head) * D + c] = __float2bfloat16_rn(lsum > 0.f ? acc / lsum : 0.f);
         } else {
-            const size_t slot = p.units > 0 ? (size_t)blockIdx.x * p.nq + head : ((size_t)seq * p.nq + head) * p.splits + split;
+            const size_t slot = CUT == DEC_UNITS ? (size_t)blockIdx.x * p.nq + head : ((size_t)seq * p.nq + head) * p.splits + split;
             p.scratch_o[slot * D + c] = acc;
             if (c == 0) {
                 p.scratch_ml[slot * 2] = mmax;
@@ -791,6 +826,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
 // Merges the key ranges of one (sequence, head): one block of D threads (whole warps).  Every way out of it waits for the
 // attention kernel: the kernel behind waits for this one alone, and where no sequence has ranges to merge it would otherwise
 // read rows that are not written yet.
+template <bool UNITS>
 __global__ void attn_decode_merge_kernel(const AttnParams p)
 {
     pdl_trigger();
@@ -800,19 +836,22 @@ __global__ void attn_decode_merge_kernel(const AttnParams p)
         pdl_wait();
         return;
     }
-    int ranges = p.splits, step = 1;
+    int ranges = p.splits;
+    const size_t step = UNITS ? p.nq : 1;
     size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
-    if (p.units > 0) {
-        const DecodeUnit u = decode_unit(p, -1, seq);
-        if (u.ranges == 1) {                          // (none: no key is visible, and the row becomes zeros here)
-            pdl_wait();
-            return;                                   // (the attention kernel has written the row)
-        }
-        ranges = u.ranges;
-        step = p.nq;
-        slot0 = (size_t)u.first_unit * p.nq + head;
+    bool planned = false;
+    if constexpr (UNITS) {
+        planned = !decode_lengths(p).equal;
+        slot0 = (size_t)seq * p.splits * p.nq + head;
     }
     pdl_wait();
+    if (UNITS && planned) {
+        const int2 plan = decode_tiles(p, seq) > 0 ? p.scratch_plan[seq] : make_int2(0, 0);
+        if (plan.y == 1)
+            return;                                   // (the attention kernel has written the row)
+        ranges = plan.y;                              // (none: no key is visible, and the row becomes zeros here)
+        slot0 = (size_t)plan.x * p.nq + head;
+    }
     // eight key ranges at a time, all their loads in flight together
     float m_run = -INFINITY, acc = 0.f, lsum = 0.f;
     for (int s0 = 0; s0 < ranges; s0 += 8) {
@@ -820,9 +859,9 @@ __global__ void attn_decode_merge_kernel(const AttnParams p)
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const bool in = s0 + u < ranges;
-            mv[u] = in ? p.scratch_ml[(slot0 + (size_t)(s0 + u) * step) * 2] : -INFINITY;
-            lv[u] = in ? p.scratch_ml[(slot0 + (size_t)(s0 + u) * step) * 2 + 1] : 0.f;
-            ov[u] = in ? p.scratch_o[(slot0 + (size_t)(s0 + u) * step) * D + c] : 0.f;
+            mv[u] = in ? p.scratch_ml[(slot0 + (s0 + u) * step) * 2] : -INFINITY;
+            lv[u] = in ? p.scratch_ml[(slot0 + (s0 + u) * step) * 2 + 1] : 0.f;
+            ov[u] = in ? p.scratch_o[(slot0 + (s0 + u) * step) * D + c] : 0.f;
         }
         float m_new = m_run;
 #pragma unroll
@@ -996,32 +1035,41 @@ using namespace chibi;
 CHIBI_API int chibi_attention_mma_head_dim() { return D; }
 CHIBI_API int chibi_attention_mma_value_dim() { return DV; }
 
-// Scratch floats that a decode launch with these sizes needs.
 // The decode kernels on p's sequences: `splits` key ranges each, or, where `units` is above 0, that many ranges of all
-// sequences together, cut on the device by the sequences' lengths.
+// sequences together (as many as `splits` each, or more), cut on the device by the sequences' lengths where these differ.
 static int launch_decode(AttnParams& p, int seqs, int splits, int units, int by_length, float* scratch,
                          long long scratch_floats, cudaStream_t stream)
 {
-    if (splits < 1 || units < 0 || (units > 0 && (units < seqs || seqs > DEC_UNIT_SEQS)) || (by_length && seqs > DEC_ORDER_SEQS))
+    if (splits < 1 || units < 0 || (units > 0 && (units < seqs * splits || seqs > DEC_UNIT_SEQS)) || (by_length && seqs > DEC_ORDER_SEQS))
         return CHIBI_ERR_ARGUMENT;
     p.seqs = seqs;
     p.splits = splits;
     p.units = units;
-    p.by_length = by_length;
     const bool merge = splits > 1 || units > 0;
     if (merge) {
         const long long parts = (units > 0 ? (long long)units : (long long)seqs * splits) * p.nq;
-        if (!scratch || scratch_floats < parts * (D + 2))
+        if (!scratch || scratch_floats < parts * (D + 2) + (units > 0 ? 2 * seqs : 0))
             return CHIBI_ERR_ARGUMENT;
         p.scratch_o = scratch;
         p.scratch_ml = scratch + (size_t)parts * D;
+        p.scratch_plan = reinterpret_cast<int2*>(scratch + (size_t)parts * (D + 2));      // (D is even: on 8 bytes)
     }
     const int row_blocks = (p.group + 15) / 16;
     const dim3 grid(units > 0 ? units : splits, p.nkv * row_blocks, units > 0 ? 1 : seqs);
-    launch(attn_decode_kernel, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, p);
+    const auto kernel = units > 0 ? attn_decode_kernel<DEC_UNITS> : by_length ? attn_decode_kernel<DEC_ORDERED> : attn_decode_kernel<DEC_SHARES>;
+    static bool configured = false;
+    if (!configured) {
+        for (const auto k : { attn_decode_kernel<DEC_SHARES>, attn_decode_kernel<DEC_UNITS>, attn_decode_kernel<DEC_ORDERED> }) {
+            const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM);
+            if (e != cudaSuccess)
+                return (int)e;
+        }
+        configured = true;
+    }
+    launch(kernel, dim3(grid), dim3(DEC_WARPS * 32), DEC_SMEM, stream, p);
     int st = launch_status();
     if (st == CHIBI_OK && merge) {
-        launch(attn_decode_merge_kernel, dim3(dim3(p.nq, seqs)), dim3((D + 31) / 32 * 32), 0, stream, p);
+        launch(units > 0 ? attn_decode_merge_kernel<true> : attn_decode_merge_kernel<false>, dim3(dim3(p.nq, seqs)), dim3((D + 31) / 32 * 32), 0, stream, p);
         st = launch_status();
     }
     return st;
@@ -1138,9 +1186,7 @@ CHIBI_API int chibi_attention_mma(const void* q, const void* k_cache, const void
     p.tied = k_cache == v_cache ? 1 : 0;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DEC_SMEM);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PRE_SMEM);
+        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PRE_SMEM);
         if (e != cudaSuccess)
             return (int)e;
         configured = true;
@@ -1214,13 +1260,5 @@ CHIBI_API int chibi_attention_decode_fused(const float* partial, int partial_spl
     p.norm_eps = eps;
     p.norm_offset = offset;
     p.append = append;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)DEC_SMEM);
-        if (e != cudaSuccess)
-            return (int)e;
-        configured = true;
-    }
     return launch_decode(p, seqs, splits, units, 0, scratch, scratch_floats, stream);
 }

@@ -107,6 +107,20 @@ class StepContext:
         """Row of the block tables per sequence (its state slot)."""
         return self.state_slots
 
+    def even_contexts(self, window: Optional[int] = None, chunk: Optional[int] = None) -> bool:
+        """Whether the sequences that bring one token see about as many keys each: on average at most an eighth less than
+        the one with the most (the decode attention kernel then shares them out without a look at their lengths)."""
+        key = ("even contexts", window, chunk)
+        even = self.shared.get(key)
+        if even is None:
+            seen = [n for n, q in zip(self.ctx_lens, self.q_lens) if q == 1]
+            if window:
+                seen = [min(n, window) for n in seen]
+            if chunk:
+                seen = [min(n, (n - 1) % chunk + 1) for n in seen]
+            even = self.shared[key] = not seen or 8 * sum(seen) >= 7 * len(seen) * max(seen)
+        return even
+
     @property
     def decode_only(self) -> bool:
         return self.max_q_len == 1

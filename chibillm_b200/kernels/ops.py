@@ -817,7 +817,7 @@ class CudaKernels:
                   window: Optional[int], max_q_len: int, max_ctx_len: int, min_q_len: int = 0,
                   seq_rows: Optional[torch.Tensor] = None, softcap: Optional[float] = None,
                   distance_bias=None, chunk: Optional[int] = None, value_dim: Optional[int] = None,
-                  sink: Optional[torch.Tensor] = None, kv_share: int = 1) -> None:
+                  sink: Optional[torch.Tensor] = None, kv_share: int = 1, even_contexts: bool = False) -> None:
         """Causal attention of every token over its sequence's pages.  bfloat16
         with a head size that is a multiple of 16 runs on the tensor cores (one
         library per head size, compiled when first needed); 32-bit operands with head
@@ -835,7 +835,8 @@ class CudaKernels:
         (slopes, None): slopes[h] * (i - j) is taken off instead.  ``kv_share`` n: n consecutive
         key heads share one value head (the value cache has nkv / n heads).  ``out`` may be
         float32 whatever q's type; these two run prompt portions on the ``mma.sync`` prompt kernel and
-        steps of single tokens on the plain kernel."""
+        steps of single tokens on the plain kernel.  ``even_contexts``: the caller knows that the single tokens' sequences
+        are of about one length (``StepContext.even_contexts``); a matter of time, not of results."""
         _need_cuda(q, k_cache, v_cache, out, block_table, q_start, ctx_len, seq_of_token, positions,
                    seq_rows, sink)
         if sink is not None and (sink.dtype != torch.float32 or sink.numel() != nq or not sink.is_contiguous()):
@@ -883,7 +884,7 @@ class CudaKernels:
         if tensor_cores and not special:
             self._attention_mma(q, k_cache, v_cache, out, block_table, q_start, ctx_len, nq, nkv, d,
                                 page_size, scale, window, max_q_len, max_ctx_len, min_q_len, seq_rows, cap, r1, r2,
-                                chunk, sink)
+                                chunk, sink, even_contexts)
             return
         if not special and q.dtype == torch.float32 and k_cache.dtype == torch.float32 and v_cache.dtype == torch.float32 \
                 and d in self.FLOAT32_HEAD_DIMS:
@@ -965,12 +966,13 @@ class CudaKernels:
 
     def decode_attention_units(self, seqs: int, nq: int, nkv: int, splits: int, max_ctx_len: int) -> Tuple[int, int]:
         """How the decode attention kernel deals with sequences of different lengths (which the host does not know
-        here): (key ranges of all sequences together, or 0; whether the longest sequences start first).  Where
-        ``splits`` ranges each fit the resident CTAs, the same number of CTAs goes to ranges of one length instead, cut
-        on the device (16 sequences of 1,500 to 6,000 keys, 8 kv heads: 64.4 -> 48.2 us; of equal lengths 70.1 and 71.4:
-        the ranges are the same then, and finding them costs a microsecond, so not below 512 keys a range).
+        here; steps that are known to be even don't ask): (key ranges of all sequences together, or 0; whether the longest
+        sequences start first).  Where ``splits`` ranges each fit the resident CTAs, the same number of CTAs goes to ranges of
+        one length instead, cut on the device if the lengths differ (8 kv heads, a replayed graph: 16 sequences of 1,500 to
+        6,000 keys 65.5 -> 51.7 us, 8 38.4 -> 33.3; the look at the lengths costs equal ones 0.4 of 18.6 (8 x 2,048) to 1.2
+        of 70.8 us (16 x 6,000), so not below 512 keys a range).
         Where even one each does not fit, a range costs more than it evens out, and the order does: 64 sequences of
-        1,046 to 4,096 keys 145.5 -> 109.4 us, of equal lengths 179.9 and 180.8.  More sequences than the kernels' searches
+        1,046 to 4,096 keys 143.8 -> 105.9 us, of equal lengths 179.6 and 181.7.  More sequences than the kernels' searches
         take, and contexts too short to be worth them, stay in equal shares and in the batch's order."""
         per_seq = nkv * ((nq // nkv + 15) // 16)
         slots = 2 * self.sm_count
@@ -980,10 +982,10 @@ class CudaKernels:
             return 0, 0
         return min(slots // per_seq, 32 * seqs), 0
 
-    def decode_attention_key(self, seqs: int, nq: int, nkv: int, max_ctx_len: int) -> Tuple[int, int, int]:
+    def decode_attention_key(self, seqs: int, nq: int, nkv: int, max_ctx_len: int, even: bool = False) -> Tuple[int, int, int]:
         """What a captured decode step depends on besides its data."""
         splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
-        return (splits, *self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len))
+        return (splits, *((0, 0) if even else self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)))
 
     def prompt_attention_key_ranges(self, seqs: int, nq: int, nkv: int, max_q_len: int, max_ctx_len: int) -> int:
         """Key ranges per row tile of the tcgen05 prompt attention: 1 unless the step
@@ -997,7 +999,8 @@ class CudaKernels:
 
     def _attention_mma(self, q, k_cache, v_cache, out, block_table, q_start, ctx_len, nq, nkv, d,
                        page_size, scale, window, max_q_len, max_ctx_len, min_q_len, seq_rows,
-                       softcap: float = 0.0, bias_r1=None, bias_r2=None, chunk: int = 0, sink=None) -> None:
+                       softcap: float = 0.0, bias_r1=None, bias_r2=None, chunk: int = 0, sink=None,
+                       even: bool = False) -> None:
         lib = self._attention_libs.get(d)
         if lib is None:
             lib = self._load("chibi_attention_mma", (f"CHIBI_HEAD_DIM={d}",))
@@ -1058,9 +1061,10 @@ class CudaKernels:
         splits, units, by_length, scratch = 1, 0, 0, None
         if mode & 1:
             splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
-            units, by_length = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)
+            if not even:
+                units, by_length = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)
             if splits > 1 or units:
-                scratch = self._scratch((units or seqs * splits) * nq * (d + 2))
+                scratch = self._scratch((units or seqs * splits) * nq * (d + 2) + (2 * seqs if units else 0))
         status = lib.chibi_attention_mma(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0),
             _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv, page_size, k_cache.shape[0], float(scale),
@@ -1076,7 +1080,8 @@ class CudaKernels:
                                       scale: float, window: Optional[int], max_ctx_len: int,
                                       q_norm_w: Optional[torch.Tensor], k_norm_w: Optional[torch.Tensor],
                                       inv_freq: torch.Tensor, rotary_dim: int, eps: float, norm_offset: float,
-                                      append: bool, seq_rows: Optional[torch.Tensor] = None) -> bool:
+                                      append: bool, seq_rows: Optional[torch.Tensor] = None,
+                                      even_contexts: bool = False) -> bool:
         """Decode attention straight from the pending q | k | v product of a step in
         which every sequence brings one token: the attention kernel adds the partial
         sums, applies the per-head norm and the rotation and appends the new key and
@@ -1108,8 +1113,8 @@ class CudaKernels:
             lib = self._load("chibi_attention_mma", (f"CHIBI_HEAD_DIM={d}",))
             lib = self._attention_libs[d] = self._profiled(lib)
         splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
-        units = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)[0]
-        scratch = self._scratch((units or seqs * splits) * nq * (d + 2)) if splits > 1 else None
+        units = 0 if even_contexts else self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)[0]
+        scratch = self._scratch((units or seqs * splits) * nq * (d + 2) + (2 * seqs if units else 0)) if splits > 1 else None
         status = lib.chibi_attention_decode_fused(
             _ptr(pending.partial), pending.splits, width, seqs, _ptr(k_cache), _ptr(v_cache), _ptr(out),
             _ptr(block_table), block_table.stride(0), _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv,

@@ -251,7 +251,7 @@ class PagedAttention(Mixer):
         s = self.spec
         if self.runtime.is_float32:
             return self.runtime.float32_launch_key(ctx, s.head_dim) if self.value_dim == s.head_dim else ()
-        return (decode(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len),)
+        return (decode(ctx.num_seqs, s.num_heads, s.num_kv_heads, ctx.max_ctx_len, ctx.even_contexts(s.window, s.chunk)),)
 
     # ---- run
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, overwrite: bool = False, hold: bool = False):
@@ -297,7 +297,8 @@ class PagedAttention(Mixer):
             if from_partial(pending, cache.keys, cache.values, att, table, ctx.q_start, ctx.ctx_len, nq, nkv, d,
                             cache.page_size, s.scale, s.window, ctx.max_ctx_len, q_norm_w, k_norm_w, fused[0],
                             fused[1], norm.eps if norm is not None else 0.0,
-                            norm.weight_offset if norm is not None else 0.0, writes, ctx.seq_rows):
+                            norm.weight_offset if norm is not None else 0.0, writes, ctx.seq_rows,
+                            ctx.even_contexts(s.window)):
                 return self._output(att, residual, overwrite, hold)
         if fused is None:
             # An encoding the kernels do not know: normalise head by head in
@@ -386,6 +387,8 @@ class PagedAttention(Mixer):
             extra["distance_bias"] = (self.slopes, None)
         if M > 1:
             extra["kv_share"] = M
+        if hasattr(k, "decode_attention_key"):
+            extra["even_contexts"] = ctx.even_contexts(s.window, s.chunk)
         joined = M > 1
         att = ctx.workspace.get("attn.maps" if joined else "attn.out", (T, nq * dv),
                                 torch.float32 if joined else rt.dtype)
@@ -442,6 +445,8 @@ class PagedAttention(Mixer):
             extra["value_dim"] = self.value_dim
         if self.has_sink:
             extra["sink"] = self.sink
+        if hasattr(k, "decode_attention_key"):
+            extra["even_contexts"] = ctx.even_contexts(s.window, s.chunk)
         k.attention(q, cache.keys, cache.values, att, ctx.tables[cache.group], ctx.q_start, ctx.ctx_len,
                     ctx.seq_of_token, ctx.positions, nq, nkv, d, cache.page_size, s.scale,
                     s.window, ctx.max_q_len, ctx.max_ctx_len, ctx.min_q_len, ctx.seq_rows, **extra)

@@ -131,7 +131,7 @@ class LatentAttention(Mixer):
             return None
         if self.runtime.is_float32:
             return self.runtime.float32_launch_key(ctx, self.key_dim)
-        return (decode(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len),)
+        return (decode(ctx.num_seqs, self.spec.num_heads, 1, ctx.max_ctx_len, ctx.even_contexts(self.spec.window)),)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor, ctx, cache, hold: bool = False):
         s, rt = self.spec, self.runtime
@@ -150,6 +150,8 @@ class LatentAttention(Mixer):
             q, gates = self._queries_from_x(x, ctx, cache)
         att = ctx.workspace.get("attn.out", (T, H * kd), rt.dtype)
         extra = {"sink": self.sink} if s.sink else {}
+        if hasattr(k, "decode_attention_key"):
+            extra["even_contexts"] = ctx.even_contexts(s.window)
         k.attention(q, cache.keys, cache.values, att, ctx.tables[cache.group], ctx.q_start, ctx.ctx_len,
                     ctx.seq_of_token, ctx.positions, H, 1, kd, cache.page_size, s.scale, s.window, ctx.max_q_len,
                     ctx.max_ctx_len, ctx.min_q_len, ctx.seq_rows, **extra)

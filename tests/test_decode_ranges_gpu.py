@@ -116,3 +116,20 @@ def test_a_sequence_without_a_key_gives_zeros(k, always):
     k.attention(q, kc, vc, out, table, q_start, ctx_len, seq_of_token, positions, nq, nkv, d, page, d ** -0.5, None, 1, max(lens), 1)
     k.check_error_word()
     assert (out[1] == 0).all() and torch.isfinite(out).all()
+
+
+@pytest.mark.parametrize("lens", [[2100, 2048, 2000, 1900] * 2, [5000, 16, 900, 33, 1200, 2500, 40], [4096] * 40, [4096, 100] * 20])
+def test_a_hint_about_lengths_is_a_matter_of_time(k, ref, lens):
+    nq, nkv, d, page = 16, 8, 128, 16
+    pages = sum(-(-n // page) for n in lens)
+    table, positions, seq_of_token, q_start, ctx_len = _paged_setup(lens, [1] * len(lens), page, pages, seed=1)
+    q = rnd(len(lens), nq * d, dtype=torch.bfloat16, seed=2)
+    kc, vc = rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=3), rnd(pages, nkv, page, d, dtype=torch.bfloat16, seed=4)
+    args = (table, q_start, ctx_len, seq_of_token, positions, nq, nkv, d, page, 1 / math.sqrt(d), None, 1, max(lens), 1)
+    exp = torch.empty_like(q)
+    ref.attention(q, kc, vc, exp, *args)
+    for even in (False, True):
+        out = torch.full_like(q, float("nan"))
+        k.attention(q, kc, vc, out, *args, even_contexts=even)
+        k.check_error_word()
+        close(out, exp, torch.bfloat16, "decode attention", rel=1.2e-2)      # (as the other tests of this kernel)
