@@ -68,7 +68,6 @@ struct AttnParams {
     int units;                     // decode: > 0: key ranges of all sequences together, cut by decode_unit
     float* scratch_o;              // decode: [S, nq, splits, D], or [units, nq, D]
     float* scratch_ml;             // decode: the same with 2 numbers
-    int2* scratch_plan;            // decode with units: [S] a sequence's first unit and how many it has, if cut by decode_unit
     // decode, optional: q (and the newest key and value) are not in `q` and the caches yet but
     // still the partial sums of the q | k | v product: the kernel adds them up, applies the per-head
     // norm and the rotation itself and appends the new key and value (head size 128 only)
@@ -515,8 +514,9 @@ struct DecodeUnit {
 
 // Cuts the sequences' keys into at most p.units ranges of c tiles (the last of a sequence shorter), c as small as that
 // allows.  Ranges of one length, not so many to every sequence: with as many CTAs as are resident at once the time is that
-// of the longest range.  The lanes try 32 values of c at a time.
-__device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, const DecodeLengths& d, int unit)
+// of the longest range.  The lanes try 32 values of c at a time.  `unit` >= 0 asks for that range, else for the ranges of
+// sequence `seq`.
+__device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, const DecodeLengths& d, int unit, int seq)
 {
     constexpr int EACH = DEC_UNIT_SEQS / 32;
     const int lane = threadIdx.x & 31;
@@ -562,7 +562,7 @@ __device__ __forceinline__ DecodeUnit decode_unit(const AttnParams& p, const Dec
             end += lane >= o ? other : 0;
         }
         const int first = before + end - n;
-        const uint32_t mine = __ballot_sync(0xffffffffu, unit >= first && unit < first + n);
+        const uint32_t mine = __ballot_sync(0xffffffffu, unit >= 0 ? (unit >= first && unit < first + n) : lane + 32 * i == seq);
         if (mine) {
             const int l = __ffs(mine) - 1;
             u.seq = 32 * i + l;
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
             seq = blockIdx.x / p.splits;
             split = blockIdx.x - seq * p.splits;
         } else {
-            const DecodeUnit u = decode_unit(p, lengths, blockIdx.x);
+            const DecodeUnit u = decode_unit(p, lengths, blockIdx.x, -1);
             seq = u.seq, split = u.range, ranges = u.ranges, unit_tiles = u.tiles;
         }
         if (seq < 0 || seq >= p.seqs) {
@@ -792,8 +792,6 @@ __global__ void __launch_bounds__(DEC_WARPS * 32) attn_decode_kernel(const AttnP
         }
     }
     __syncthreads();
-    if (CUT == DEC_UNITS && unit_tiles > 0 && split == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-        p.scratch_plan[seq] = make_int2(blockIdx.x, ranges);          // (for the merge, which would cut the keys once more)
     for (int idx = threadIdx.x; idx < rows * D; idx += blockDim.x) {
         const int row = idx / D, c = idx - row * D;
         float mmax = -INFINITY;
@@ -839,19 +837,19 @@ __global__ void attn_decode_merge_kernel(const AttnParams p)
     int ranges = p.splits;
     const size_t step = UNITS ? p.nq : 1;
     size_t slot0 = ((size_t)seq * p.nq + head) * p.splits;
-    bool planned = false;
     if constexpr (UNITS) {
-        planned = !decode_lengths(p).equal;
-        slot0 = (size_t)seq * p.splits * p.nq + head;
+        const DecodeLengths lengths = decode_lengths(p);
+        if (lengths.equal) {
+            slot0 = (size_t)seq * p.splits * p.nq + head;
+        } else {
+            const DecodeUnit u = decode_unit(p, lengths, -1, seq);
+            ranges = u.ranges;
+            slot0 = (size_t)u.first_unit * p.nq + head;
+        }
     }
     pdl_wait();
-    if (UNITS && planned) {
-        const int2 plan = decode_tiles(p, seq) > 0 ? p.scratch_plan[seq] : make_int2(0, 0);
-        if (plan.y == 1)
-            return;                                   // (the attention kernel has written the row)
-        ranges = plan.y;                              // (none: no key is visible, and the row becomes zeros here)
-        slot0 = (size_t)plan.x * p.nq + head;
-    }
+    if (UNITS && ranges == 1)
+        return;                                       // (the attention kernel has written the row; none: no key is visible, zeros)
     // eight key ranges at a time, all their loads in flight together
     float m_run = -INFINITY, acc = 0.f, lsum = 0.f;
     for (int s0 = 0; s0 < ranges; s0 += 8) {
@@ -1048,11 +1046,10 @@ static int launch_decode(AttnParams& p, int seqs, int splits, int units, int by_
     const bool merge = splits > 1 || units > 0;
     if (merge) {
         const long long parts = (units > 0 ? (long long)units : (long long)seqs * splits) * p.nq;
-        if (!scratch || scratch_floats < parts * (D + 2) + (units > 0 ? 2 * seqs : 0))
+        if (!scratch || scratch_floats < parts * (D + 2))
             return CHIBI_ERR_ARGUMENT;
         p.scratch_o = scratch;
         p.scratch_ml = scratch + (size_t)parts * D;
-        p.scratch_plan = reinterpret_cast<int2*>(scratch + (size_t)parts * (D + 2));      // (D is even: on 8 bytes)
     }
     const int row_blocks = (p.group + 15) / 16;
     const dim3 grid(units > 0 ? units : splits, p.nkv * row_blocks, units > 0 ? 1 : seqs);

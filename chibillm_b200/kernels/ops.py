@@ -1064,7 +1064,7 @@ class CudaKernels:
             if not even:
                 units, by_length = self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)
             if splits > 1 or units:
-                scratch = self._scratch((units or seqs * splits) * nq * (d + 2) + (2 * seqs if units else 0))
+                scratch = self._scratch((units or seqs * splits) * nq * (d + 2))
         status = lib.chibi_attention_mma(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), _ptr(block_table), block_table.stride(0),
             _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv, page_size, k_cache.shape[0], float(scale),
@@ -1114,7 +1114,7 @@ class CudaKernels:
             lib = self._attention_libs[d] = self._profiled(lib)
         splits = self.decode_attention_splits(seqs, nq, nkv, max_ctx_len)
         units = 0 if even_contexts else self.decode_attention_units(seqs, nq, nkv, splits, max_ctx_len)[0]
-        scratch = self._scratch((units or seqs * splits) * nq * (d + 2) + (2 * seqs if units else 0)) if splits > 1 else None
+        scratch = self._scratch((units or seqs * splits) * nq * (d + 2)) if splits > 1 else None
         status = lib.chibi_attention_decode_fused(
             _ptr(pending.partial), pending.splits, width, seqs, _ptr(k_cache), _ptr(v_cache), _ptr(out),
             _ptr(block_table), block_table.stride(0), _ptr(seq_rows), _ptr(q_start), _ptr(ctx_len), seqs, nq, nkv,
