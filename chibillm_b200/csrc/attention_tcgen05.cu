@@ -291,7 +291,10 @@ __device__ __forceinline__ void softmax_row(const AttnTcParams& p, QueryRow& w, 
         mx4[u] = fmaxf(mx4[u], __uint_as_float(sv[COLS - 4 + u]));
     float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
     mx *= sl2;                                       // the scale is positive
-    if (pair_any(barrier, mx > w.m + 8.f)) {         // also for the first visible key (m = -inf)
+    tcgen05_fence_before();                          // (the other warp's probabilities are written over these scores)
+    const bool any = pair_any(barrier, mx > w.m + 8.f);      // also for the first visible key (m = -inf)
+    tcgen05_fence_after();
+    if (any) {
         maxima[half * ROWS + thread] = mx;
         pair_sync(barrier);
         mx = fmaxf(mx, maxima[(half ^ 1) * ROWS + thread]);
