@@ -309,6 +309,7 @@ __device__ __forceinline__ void softmax_row(const AttnTcParams& p, QueryRow& w, 
             w.l *= (w.m == -INFINITY) ? 0.f : fast_exp2(w.m - mx);
             w.m = mx;
         }
+        __syncwarp();
     }
     const float base = w.m == -INFINITY ? 0.f : w.m;
     const uint64_t scale2 = pair_of(sl2, sl2), base2 = pair_of(-base, -base);
@@ -546,6 +547,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             if (key0 + KEYS > key_end) {
                 mbar_wait(&v_full[st], (j >> 1) & 1, p.error, 29);
                 clear_values(v_s + st * KV_TILE_BYTES, key_end - key0, half * ROWS + thread);
+                __syncwarp();
             }
             tmem_store_wait();
             tcgen05_fence_before();
@@ -576,6 +578,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     for (int c = 0; c < 8; ++c)
                         reinterpret_cast<uint4*>(dst + c0)[c] = make_uint4(ov[4 * c], ov[4 * c + 1], ov[4 * c + 2], ov[4 * c + 3]);
                 }
+                __syncwarp();
             }
             if (w.live && half == 0) {
                 p.part_ml[slot * 2] = w.m;
@@ -796,6 +799,7 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (key0 + KEYS > key_end) {
                 mbar_wait(&v_full[st], (j >> 1) & 1, p.error, 47);
                 clear_values(v_s + st * KV_TILE_BYTES, key_end - key0, half * ROWS + thread);
+                __syncwarp();
             }
             tmem_store_wait();
             tcgen05_fence_before();
