@@ -7,6 +7,7 @@
 #define CHIBI_UNIT_ID 17
 #include "common.cuh"
 #include "sm100.cuh"
+#include "split_f32.cuh"
 
 namespace chibi {
 
@@ -32,45 +33,6 @@ struct AttentionF32 {
     int* error;
 };
 
-__device__ __forceinline__ uint64_t af_pair(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 af_halves(uint64_t v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t af_fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t af_mul2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t af_add2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-// 16 bytes, zeros where `bytes` is 0 (nothing is read then).
-__device__ __forceinline__ void af_copy16(float* dst, const float* src, int bytes)
-{
-    const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(a), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 __device__ __forceinline__ void af_cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
@@ -88,14 +50,6 @@ __device__ __forceinline__ float af_peer(const float* local, int rank)
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(af_peer_address(local, rank)) : "memory");
     return v;
 }
-__device__ __forceinline__ float4 af_peer4(const float* local, int rank)
-{
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(af_peer_address(local, rank)) : "memory");
-    return v;
-}
-
 // What becomes of a dot product; `distance`: query position - key position.
 __device__ __forceinline__ float af_score(const AttentionF32& p, float dot, float r1, float r2, int distance)
 {
@@ -110,13 +64,12 @@ __device__ __forceinline__ float af_score(const AttentionF32& p, float dot, floa
 __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -INFINITY ? 0.f : expf(m - m_new); }
 
 // ---------------------------------------------------------------- sequences that bring several tokens
-// On the 5th-generation tensor cores.  A 32-bit number is the sum of three bfloat16 numbers (its leading 8 bits, the next
-// 8 of what is left, the last 8, each rounded to nearest), so a product of two is the sum of nine exact products of 8 by
-// 8 bits; the three smallest (below 2^-26 of the whole) are left out, the other six are tcgen05.mma with 32-bit
-// accumulators.  What limits the precision is the accumulator, which the tensor core cuts off instead of rounding: so
-// every sum over 64 features or keys has an accumulator of its own, that takes the five small products first and the
-// large one last, and those sums are added in plain 32-bit arithmetic.  Relative error against 64 bits, 3 prompts of up to
-// 400 tokens: 1.6e-7, by multiply-adds (fma.rn.f32x2) before 2.1e-7.
+// On the 5th-generation tensor cores: numbers are split into three bfloat16 parts (split_f32.cuh), and six of the nine partial
+// products are tcgen05.mma with 32-bit accumulators.  What limits the precision is the accumulator, which the tensor core cuts
+// off instead of rounding: so every sum over 64 features or keys has an accumulator of its own, that takes the five small
+// products first and the large one last, and those sums are added in plain 32-bit arithmetic.  Relative error against 64 bits,
+// 3 prompts of up to 400 tokens: 1.6e-7, by multiply-adds (fma.rn.f32x2) before 2.1e-7 (values of one sign 1.05e-7 and 1.0e-7, for
+// the accumulators are cut off downwards).
 //
 // A CTA owns 128 query rows of one kv head, (token, head of the group) pairs, and walks over the keys in blocks of 64, counted
 // from the sequence's start: what a row gives does not depend on the rows beside it (a key that it does not see has
@@ -127,15 +80,13 @@ __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -IN
 // Bound by the products beside the threads' work: 48 MMAs of 128 x 64 x 16 (shared memory: 48 cycles each) and 24 of
 // 128 x D x 16 (64) a block, 3,900 cycles for heads of 128.  An issuing thread waits while they run (issued by one of the
 // working warps a block took 11,400).  Heads of 128, us by multiply-adds (64 rows a CTA, four CTAs to a row tile's keys) and
-// so: 3 prompts of up to 400 tokens of 16 heads 109 and 38, 4 of up to 600 after 800 of 32 heads 1,235 and 322, 64 tokens after 800
-// of 16 heads 86 and 64, 100 after 4,000 417 and 298, 4 after 800 78 and 59.
+// so: 3 prompts of up to 400 tokens of 16 heads 109 and 38, 4 of 600 after 800 of 32 heads 1,536 and 400, 64 tokens after 800
+// of 16 heads 84 and 80, 100 after 4,000 315 and 308, 4 after 800 82 and 74.
 //
-// Queries, keys, values and probabilities are split times 2^16, so that the last parts of small ones (of all normal numbers) are
-// no smaller than a bfloat16 can be; scores and outputs are 2^32 as large as they should be until they are used.  A query or
-// key that is no number, or too large (from 2^112 on), has an infinite part and makes its scores no number; those, and scores from
-// 2^96 on, are summed by multiply-adds.  Such values are marked and taken out, because they would spoil the rows that do not see
-// them: what is no number adds itself to its column of the rows that do, and rows that see a large one, or whose sums are too
-// large, are made by hand.
+// Scores and outputs are 2^32 as large as they should be until they are used.  A query or key without parts (no number, or from
+// 2^112 on) makes its scores no number; those, and scores from 2^96 on, are summed by multiply-adds.  Such values are marked
+// and taken out, because they would spoil the rows that do not see them: what is no number adds itself to its column of the rows
+// that do, and rows that see a large one, or whose sums are too large, are made by hand.
 constexpr int AT_ROWS = 128, AT_KEYS = 64, AT_WORKERS = 512, AT_THREADS = 128 + AT_WORKERS;
 constexpr int AT_REGS = 96, AT_REGS_FEW = 32, AT_REGS_MANY = 112;    // of a thread at launch, of the first four warps', of the others'
 static_assert(AT_REGS_FEW + 4 * AT_REGS_MANY <= 5 * AT_REGS, "more registers than the block has");
@@ -150,46 +101,8 @@ template <int D> struct AtShape {
     static constexpr uint32_t P_AT = 2 * S_COLS, O_AT = P_AT + 96, TMEM = O_AT + D <= 256 ? 256 : 512;
 };
 
-__device__ __forceinline__ uint32_t at_pair(float a, float b)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
-    return r;
-}
-// What is left of two numbers without their bfloat16 parts (exact).
-__device__ __forceinline__ uint64_t at_rest(uint64_t v, uint32_t pair)
-{
-    const uint64_t parts = af_pair(__uint_as_float(pair << 16), __uint_as_float(pair & 0xffff0000u));
-    return af_fma2(parts, 0xbf800000bf800000ull, v);             // (-1, -1)
-}
-__device__ __forceinline__ uint32_t at_pair(uint64_t v)
-{
-    const float2 h = af_halves(v);
-    return at_pair(h.x, h.y);
-}
-__device__ __forceinline__ void at_put(uint32_t at, uint32_t a, uint32_t b)
-{
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
-}
-constexpr uint64_t AT_UP = 0x4780000047800000ull;                // 2^16 twice
-constexpr float AT_DOWN = 0x1p-32f;
-// Writes the three parts of four numbers, `plane` bytes apart; what the last ones are before they are rounded is no number
-// where one of the four is none or too large.
-__device__ __forceinline__ uint64_t at_split(float4 v, uint32_t at, uint32_t plane)
-{
-    uint64_t x = af_mul2(af_pair(v.x, v.y), AT_UP), y = af_mul2(af_pair(v.z, v.w), AT_UP);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const uint32_t a = at_pair(x), b = at_pair(y);
-        at_put(at + i * plane, a, b);
-        if (i < 2) {
-            x = at_rest(x, a);
-            y = at_rest(y, b);
-        }
-    }
-    return af_add2(x, y);
-}
-// The same without what has no parts (2^16 times it is infinite as bfloat16, or it is none); true if there was one.
+// Writes the parts of four numbers without what has none (2^16 times it is infinite as bfloat16, or it is no number); true if
+// there was one.
 __device__ __noinline__ bool at_split_odd(float4 v, uint32_t at, uint32_t plane)
 {
     bool found = false;
@@ -201,13 +114,8 @@ __device__ __noinline__ bool at_split_odd(float4 v, uint32_t at, uint32_t plane)
     };
     one(v.x), one(v.y), one(v.z), one(v.w);
     if (found)
-        at_split(v, at, plane);
+        split_to_shared(v, at, plane);
     return found;
-}
-__device__ __forceinline__ bool at_none(uint64_t v)
-{
-    const float2 h = af_halves(v);
-    return !(fabsf(h.x + h.y) < INFINITY);
 }
 __device__ __noinline__ float at_dot(const float* a, const float* b, int d)
 {
@@ -456,11 +364,11 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
             uint64_t last = 0;
 #pragma unroll
             for (int i = 0; i < KV_EACH; ++i)
-                last = af_add2(at_split(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE), last);
+                last = pair_add(split_to_shared(v[i], to + kv_at + i * (PASS / 8) * 1024, Shape::KV_PLANE), last);
             return last;
         };
         auto spread_values = [&](const float4 (&v)[KV_EACH], uint32_t* flags) {
-            if (at_none(spread(v, v_s))) {
+            if (pair_is_none(spread(v, v_s))) {
 #pragma unroll
                 for (int i = 0; i < KV_EACH; ++i) {
                     const int r = line + PASS * i;
@@ -499,7 +407,7 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
             }
 #pragma unroll
             for (int i = 0; i < Q_EACH / 2; ++i)
-                at_split(v[i], q_s + q_at + (i + half * (Q_EACH / 2)) * (PASS / 8) * 1024, Shape::Q_PLANE);
+                split_to_shared(v[i], q_s + q_at + (i + half * (Q_EACH / 2)) * (PASS / 8) * 1024, Shape::Q_PLANE);
         }
         spread(kn, k_s);
         fence_proxy_async();
@@ -515,8 +423,8 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
         const int first = first_visible_key(pos, p.window, p.chunk);
         constexpr int COLS = D / AT_SHARE;
         uint64_t O[COLS / 2];
-        const float down = OPTIONS ? AT_DOWN : p.scale * AT_DOWN;
-        const uint64_t down2 = af_pair(down, down);
+        const float down = OPTIONS ? SPLIT_DOWN : p.scale * SPLIT_DOWN;
+        const uint64_t down2 = pair_of(down, down);
         float m = -INFINITY, l = 0.f;
         spoiled[worker] = large[worker] = 0;
 #pragma unroll
@@ -534,13 +442,13 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
             tmem_load_wait();
 #pragma unroll
             for (int c = 0; c < COLS / 2; ++c)
-                O[c] = af_fma2(O[c], 0x3f8000003f800000ull, af_pair(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])));
+                O[c] = pair_fma(O[c], PAIR_ONES, pair_of(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])));
             if (*odd_any) {
                 uint32_t found = 0;                                  // columns, as in `spoiled`
                 bool too_large = false, left = false;                // (nothing is left to spoil where all are none)
 #pragma unroll
                 for (int c = 0; c < COLS / 2; ++c) {
-                    const float2 o = af_halves(O[c]);
+                    const float2 o = halves_of(O[c]);
                     left |= o.x == o.x || o.y == o.y;
                 }
                 for (int i = 0; i < AT_KEYS && left; ++i) {
@@ -551,8 +459,8 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
                         for (int c = 0; c < COLS / 2; ++c) {
                             const float x = v[2 * c], y = v[2 * c + 1];
                             const bool no_x = !(fabsf(x) < INFINITY), no_y = !(fabsf(y) < INFINITY);
-                            const float2 o = af_halves(O[c]);
-                            O[c] = af_pair(o.x + (no_x ? x : 0.f), o.y + (no_y ? y : 0.f));
+                            const float2 o = halves_of(O[c]);
+                            O[c] = pair_of(o.x + (no_x ? x : 0.f), o.y + (no_y ? y : 0.f));
                             found |= (no_x ? 1u : 0u) << (2 * c) | (no_y ? 2u : 0u) << (2 * c);
                             too_large |= (!no_x && fabsf(x) >= 0x1p111f) || (!no_y && fabsf(y) >= 0x1p111f);
                         }
@@ -590,19 +498,19 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
                 uint64_t pairs[AT_OWN / 2];
 #pragma unroll
                 for (int i = 0; i < AT_OWN / 2; ++i) {
-                    pairs[i] = af_pair(__uint_as_float(v[0][2 * i]), __uint_as_float(v[0][2 * i + 1]));
+                    pairs[i] = pair_of(__uint_as_float(v[0][2 * i]), __uint_as_float(v[0][2 * i + 1]));
                     if (Shape::SLICES > 1)
-                        pairs[i] = af_add2(pairs[i], af_pair(__uint_as_float(v[Shape::SLICES - 1][2 * i]), __uint_as_float(v[Shape::SLICES - 1][2 * i + 1])));
-                    pairs[i] = af_mul2(pairs[i], down2);
+                        pairs[i] = pair_add(pairs[i], pair_of(__uint_as_float(v[Shape::SLICES - 1][2 * i]), __uint_as_float(v[Shape::SLICES - 1][2 * i + 1])));
+                    pairs[i] = pair_mul(pairs[i], down2);
                     if (i % 2)
-                        none = af_fma2(pairs[i - 1], pairs[i], none);
-                    const float2 h = af_halves(pairs[i]);
+                        none = pair_fma(pairs[i - 1], pairs[i], none);
+                    const float2 h = halves_of(pairs[i]);
                     s[2 * i] = h.x;
                     s[2 * i + 1] = h.y;
                 }
             }
             const int key0 = base + part * AT_OWN;
-            if (at_none(none))
+            if (pair_is_none(none))
                 at_scores_by_hand<D, OPTIONS>(p, s, table, row0 + row / G, h, kv_head, key0, first, pos);
             // every row sees every key of these?
             const bool whole = __all_sync(0xffffffffu, key0 + AT_OWN - 1 <= pos && key0 >= first);
@@ -639,21 +547,21 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
             l = l * keep + sum;
             if (j > 0)
                 add_output(j - 1);
-            const uint64_t keep2 = af_pair(keep, keep);
+            const uint64_t keep2 = pair_of(keep, keep);
 #pragma unroll
             for (int c = 0; c < COLS / 2; ++c)
-                O[c] = af_mul2(O[c], keep2);
+                O[c] = pair_mul(O[c], keep2);
             uint64_t s2[AT_OWN / 2];
 #pragma unroll
             for (int i = 0; i < AT_OWN / 2; ++i)
-                s2[i] = af_mul2(af_pair(s[2 * i], s[2 * i + 1]), AT_UP);
+                s2[i] = pair_mul(pair_of(s[2 * i], s[2 * i + 1]), SPLIT_UP);
 #pragma unroll
             for (int plane = 0; plane < 3; ++plane) {
                 uint32_t pairs[AT_OWN / 2];
 #pragma unroll
                 for (int i = 0; i < AT_OWN / 2; ++i) {
-                    pairs[i] = at_pair(s2[i]);
-                    s2[i] = at_rest(s2[i], pairs[i]);
+                    pairs[i] = bf16_pair(s2[i]);
+                    s2[i] = without_bf16_pair(s2[i], pairs[i]);
                 }
                 tmem_store_32x8(lanes + Shape::P_AT + plane * 32 + part * (AT_OWN / 2), pairs);
             }
@@ -682,16 +590,16 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
             top = fmaxf(sink, m);
             const float keep = af_keep(m, top);
             l = l * keep + af_keep(sink, top);
-            const uint64_t keep2 = af_pair(keep, keep);
+            const uint64_t keep2 = pair_of(keep, keep);
 #pragma unroll
             for (int c = 0; c < COLS / 2; ++c)
-                O[c] = af_mul2(O[c], keep2);
+                O[c] = pair_mul(O[c], keep2);
         }
-        const float inv = l > 0.f ? 1.f / l : 0.f, inv_down = inv * AT_DOWN;
+        const float inv = l > 0.f ? 1.f / l : 0.f, inv_down = inv * SPLIT_DOWN;
         uint32_t none = 0;                                           // columns whose sums are no number, or too large for one
 #pragma unroll
         for (int c = 0; c < COLS / 2; ++c) {
-            const float2 o = af_halves(O[c]);
+            const float2 o = halves_of(O[c]);
             none |= (fabsf(o.x) < INFINITY ? 0u : 1u) << (2 * c) | (fabsf(o.y) < INFINITY ? 0u : 2u) << (2 * c);
         }
         const bool by_hand = l == l && ((none & ~spoiled[worker]) || large[worker]);     // (with a score that is none all of the row is)
@@ -699,7 +607,7 @@ attention_f32_prompt_kernel(const __grid_constant__ AttentionF32 p)
         uint8_t* const rows = smem + quarter * 32 * (D * 4);
 #pragma unroll
         for (int c = 0; c < SHARE; ++c) {
-            const float2 a = af_halves(O[2 * c]), b = af_halves(O[2 * c + 1]);
+            const float2 a = halves_of(O[2 * c]), b = halves_of(O[2 * c + 1]);
             *reinterpret_cast<float4*>(rows + lane * (D * 4) + (((part * SHARE + c) ^ (lane & 7)) << 4)) =
                 make_float4(a.x * inv_down, a.y * inv_down, b.x * inv_down, b.y * inv_down);
         }
@@ -802,10 +710,10 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
                 uint64_t d0 = 0, d1 = 0;
 #pragma unroll
                 for (int i = 0; i < N; ++i) {
-                    d0 = af_fma2(q[g][i][0], k[i].x, d0);
-                    d1 = af_fma2(q[g][i][1], k[i].y, d1);
+                    d0 = pair_fma(q[g][i][0], k[i].x, d0);
+                    d1 = pair_fma(q[g][i][1], k[i].y, d1);
                 }
-                const float2 a = af_halves(d0), b = af_halves(d1);
+                const float2 a = halves_of(d0), b = halves_of(d1);
                 float dot = (a.x + a.y) + (b.x + b.y);
 #pragma unroll
                 for (int x = 4; x > 0; x >>= 1)
@@ -814,13 +722,13 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
                     const float s = af_score(p, dot, r1[g], r2[g], pos - u);
                     const float m_new = fmaxf(m[g], s);
                     const float keep = af_keep(m[g], m_new), e = s == -INFINITY ? 0.f : expf(s - m_new);
-                    const uint64_t k2 = af_pair(keep, keep), e2 = af_pair(e, e);
+                    const uint64_t k2 = pair_of(keep, keep), e2 = pair_of(e, e);
                     l[g] = l[g] * keep + e;
                     m[g] = m_new;
 #pragma unroll
                     for (int i = 0; i < N; ++i) {
-                        o[g][i][0] = af_fma2(e2, v[i].x, af_mul2(o[g][i][0], k2));
-                        o[g][i][1] = af_fma2(e2, v[i].y, af_mul2(o[g][i][1], k2));
+                        o[g][i][0] = pair_fma(e2, v[i].x, pair_mul(o[g][i][0], k2));
+                        o[g][i][1] = pair_fma(e2, v[i].y, pair_mul(o[g][i][1], k2));
                     }
                 }
             }
@@ -846,7 +754,7 @@ attention_f32_token_kernel(const AttentionF32 p, int ranks, int head_blocks)
         for (int i = 0; i < N; ++i)
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                float2 a = af_halves(o[g][i][x]);
+                float2 a = halves_of(o[g][i][x]);
                 a.x *= keep;
                 a.y *= keep;
                 a.x += __shfl_xor_sync(0xffffffffu, a.x, 8);

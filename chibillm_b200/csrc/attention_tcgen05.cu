@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "sm100.cuh"
 #include "attention_tc.cuh"
+#include "split_f32.cuh"
 #include "tensor_map.cuh"
 
 #ifndef CHIBI_HEAD_DIM
@@ -71,32 +72,6 @@ __device__ __forceinline__ float max3(float a, float b, float c)
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// Two 32-bit numbers in one register pair.
-__device__ __forceinline__ uint64_t pair_of(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 halves_of(uint64_t v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t pair_add(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // The output accumulator's columns of this thread *= f, in TMEM (a rare event: piece by piece, so that it takes few registers).
 __device__ __forceinline__ void rescale_output_row(uint32_t o_addr, float f)
 {

@@ -1,11 +1,10 @@
 // out[M, N] = x[M, K] * w[N, K]^T (+ residual[M, N]), all 32-bit, on the 5th-generation tensor cores.
 //
-// A 32-bit number is the sum of three bfloat16 numbers (its leading 8 bits, the next 8 of what is left, and the last 8;
-// each rounded to nearest), so a product of two is the sum of nine exact products of 8 by 8 bits.  The three
-// smallest of them (below 2^-26 of the whole) are left out, the other six are tcgen05.mma with 32-bit accumulators.
-// What limits the precision is the accumulator, which the tensor core cuts off instead of rounding: so a block of 64 places
-// has an accumulator of its own, that takes the five small products of all its places first and the large one last (four
-// roundings at the size of the sum), and the blocks are added up in plain 32-bit arithmetic.  Relative error against 64 bits
+// Numbers are split into three bfloat16 parts (split_f32.cuh), and six of the nine partial products are tcgen05.mma with
+// 32-bit accumulators.  What limits the precision is the accumulator, which the tensor core cuts off instead of rounding:
+// so a block of 64 places has an accumulator of its own, that takes the five small products of all its places first and the
+// large one last (four roundings at the size of the sum), and the blocks are added up in plain 32-bit arithmetic.  Relative
+// error against 64 bits
 // (2-norm, normal numbers, K = 64 / 128 / 1,024 / 3,072 / 12,300): 7.9e-8 / 8.3e-8 / 9.6e-8 / 1.0e-7 / 1.3e-7; by multiply-adds
 // (fma.rn.f32x2) before 1.1e-7 / 1.5e-7 / 1.6e-7 / 1.9e-7 / 3.6e-7.
 //
@@ -14,11 +13,10 @@
 // depend on the rows beside it, nor on which kernel makes it or how many CTAs share a sum (a cluster of 1, 2, 4 or 8 takes the
 // runs in order).
 //
-// Numbers are split times 2^16, so that the last parts of small ones (of all normal numbers) are no smaller than a
-// bfloat16 can be, and sums are 2^32 as large as they should be until the end.  What is no number, or too large (from 2^112
-// on), has an infinite part and a rest that is no number, so all sums of its row of x or w come out as none.  Sums that do, and
-// sums from 2^96 on, which come out infinite, are made by multiply-adds instead.  (No loop looks for such numbers, which pays for the
-// scaling: 300 rows through the feed-forward of 1,024 x 3,072 75.1 us with rows marked and w not scaled, 70.2 so.)
+// Sums are 2^32 as large as they should be until the end.  What has no parts (no number, or from 2^112 on) makes all sums of its row
+// of x or w come out as no number.  Sums that do, and sums from 2^96 on, which come out infinite, are made by hand instead.
+// (No loop looks for such numbers, which pays for the scaling: 300 rows through the feed-forward of 1,024 x 3,072 75.1 us with
+// rows marked and w not scaled, 70.2 so.)
 //
 // A CTA owns 128 rows of w (the M of the MMA) and up to 128 rows of x (its N).  Eight or sixteen warps bring both from
 // memory (in registers, one block ahead), split them and write the six tiles to one of two stages in shared memory in
@@ -31,6 +29,7 @@
 #define CHIBI_UNIT_ID 18
 #include "common.cuh"
 #include "sm100.cuh"
+#include "split_f32.cuh"
 
 namespace chibi {
 
@@ -88,64 +87,6 @@ __device__ __forceinline__ float4 f3_load_end(const float* row, int k, int K)
     if (k + 3 < K)
         v.w = row[k + 3];
     return v;
-}
-
-// The three bfloat16 parts of 32-bit numbers, two at a time.
-__device__ __forceinline__ uint64_t f3_both(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 f3_halves(uint64_t v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ uint64_t f3_fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-constexpr uint64_t F3_ONES = 0x3f8000003f800000ull, F3_MINUS_ONES = 0xbf800000bf800000ull, F3_UP = 0x4780000047800000ull;    // 2^16 twice
-constexpr float F3_DOWN = 0x1p-32f;
-__device__ __forceinline__ uint64_t f3_scaled(float a, float b)
-{
-    uint64_t r = f3_both(a, b);
-    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(F3_UP));
-    return r;
-}
-__device__ __forceinline__ uint32_t f3_pair(uint64_t v)
-{
-    const float2 h = f3_halves(v);
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(h.y), "f"(h.x));
-    return r;
-}
-// What is left of two numbers without their bfloat16 parts (exact).
-__device__ __forceinline__ uint64_t f3_rest(uint64_t v, uint32_t pair)
-{
-    return f3_fma2(f3_both(__uint_as_float(pair << 16), __uint_as_float(pair & 0xffff0000u)), F3_MINUS_ONES, v);
-}
-__device__ __forceinline__ void f3_put(uint32_t at, uint32_t a, uint32_t b)
-{
-    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(a), "r"(b) : "memory");
-}
-// Writes the three parts of four places, `plane` bytes apart.
-__device__ __forceinline__ void f3_split(float4 v, uint32_t at, uint32_t plane)
-{
-    uint64_t x = f3_scaled(v.x, v.y), y = f3_scaled(v.z, v.w);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const uint32_t a = f3_pair(x), b = f3_pair(y);
-        f3_put(at + i * plane, a, b);
-        if (i < 2) {
-            x = f3_rest(x, a);
-            y = f3_rest(y, b);
-        }
-    }
 }
 
 template <int COUNT> __device__ __forceinline__ void f3_tmem_load(uint32_t at, uint32_t (&r)[COUNT])
@@ -347,10 +288,10 @@ gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
         auto spread = [&](int st) {
 #pragma unroll
             for (int j = 0; j < W_EACH; ++j)
-                f3_split(wv[j], to + st * STAGE + j * (PASS / 8) * 1024, F3_W_PLANE);
+                split_to_shared(wv[j], to + st * STAGE + j * (PASS / 8) * 1024, F3_W_PLANE);
 #pragma unroll
             for (int j = 0; j < X_EACH; ++j)
-                f3_split(xv[j], to + st * STAGE + 3 * F3_W_PLANE + j * (PASS / 8) * 1024, X_PLANE);
+                split_to_shared(xv[j], to + st * STAGE + 3 * F3_W_PLANE + j * (PASS / 8) * 1024, X_PLANE);
         };
         uint64_t run[COLS / 2];
         // Adds block i's accumulator to its run, and a run that is finished to what came before it, in TMEM: by halves, or, where
@@ -371,7 +312,7 @@ gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
                 tmem_load_wait();
 #pragma unroll
                 for (int u = 0; u < PIECE / 2; ++u)
-                    run[c * PIECE / 2 + u] = f3_fma2(run[c * PIECE / 2 + u], F3_ONES, f3_both(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1])));
+                    run[c * PIECE / 2 + u] = pair_fma(run[c * PIECE / 2 + u], PAIR_ONES, pair_of(__uint_as_float(v[2 * u]), __uint_as_float(v[2 * u + 1])));
             }
             tcgen05_fence_before();
             mbar_arrive(&taken[st]);
@@ -388,7 +329,7 @@ gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
                     }
 #pragma unroll
                     for (int u = 0; u < PIECE / 2; ++u) {
-                        const float2 h = f3_halves(run[c * PIECE / 2 + u]);
+                        const float2 h = halves_of(run[c * PIECE / 2 + u]);
                         v[2 * u] = __float_as_uint(joins ? __uint_as_float(v[2 * u]) + h.x : h.x);
                         v[2 * u + 1] = __float_as_uint(joins ? __uint_as_float(v[2 * u + 1]) + h.y : h.y);
                     }
@@ -421,7 +362,7 @@ gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
         auto finish = [&](int m, int n, float v) {
             if (m >= p.M || n >= p.N)
                 return false;
-            v *= F3_DOWN;
+            v *= SPLIT_DOWN;
             if (!(fabsf(v) < INFINITY))
                 return true;
             if (p.residual)
@@ -579,18 +520,6 @@ gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
     uint4* const kept4 = reinterpret_cast<uint4*>(kept_sums + 2 * F3_RUNS * XS * 16);
     uint2* const kept2 = reinterpret_cast<uint2*>(kept4 + blocks * 4 * TILES * 32);
     auto kept_at = [&](int b, int ks, int i) { return ((b * 4 + ks) * TILES + i) * 32 + lane; };
-    auto parts_of = [&](float4 v, uint32_t (&parts)[3][2]) {
-        uint64_t x = f3_scaled(v.x, v.y), y = f3_scaled(v.z, v.w);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            parts[j][0] = f3_pair(x);
-            parts[j][1] = f3_pair(y);
-            if (j < 2) {
-                x = f3_rest(x, parts[j][0]);
-                y = f3_rest(y, parts[j][1]);
-            }
-        }
-    };
     if (begin < end && (int)blockIdx.x < w_tiles) {
         aim(blockIdx.x, begin);
 #pragma unroll
@@ -611,7 +540,7 @@ gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     uint32_t parts[3][2];
-                    parts_of(v[ks], parts);
+                    split_parts(v[ks], parts);
                     kept4[kept_at(b, ks, i)] = make_uint4(parts[0][0], parts[0][1], parts[1][0], parts[1][1]);
                     kept2[kept_at(b, ks, i)] = make_uint2(parts[2][0], parts[2][1]);
                 }
@@ -649,12 +578,12 @@ gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
                         xf[i][0][0] = a.x, xf[i][0][1] = a.y, xf[i][1][0] = a.z, xf[i][1][1] = a.w, xf[i][2][0] = c.x, xf[i][2][1] = c.y;
                     }
                 }
-                parts_of(wn[0][ks], low);
-                parts_of(wn[1][ks], high);
+                split_parts(wn[0][ks], low);
+                split_parts(wn[1][ks], high);
                 if (!KEPT) {
 #pragma unroll
                     for (int i = 0; i < TILES; ++i)
-                        parts_of(xn[i][ks], xf[i]);
+                        split_parts(xn[i][ks], xf[i]);
                 }
                 if (more)
                     fetch(ks);
@@ -729,7 +658,7 @@ gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
                         half += s[r];
                 v += half;
             }
-            v *= F3_DOWN;
+            v *= SPLIT_DOWN;
             const bool in = m < p.M && n < p.N, bad = in && !(fabsf(v) < INFINITY);
             if (in && !bad)
                 p.out[(size_t)m * p.out_stride + n] = p.residual ? p.residual[(size_t)m * p.res_stride + n] + v : v;
