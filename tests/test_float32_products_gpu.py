@@ -114,3 +114,19 @@ def test_large_numbers_are_summed_exactly(k, rows):
     assert ((out.double() - total).abs() <= 2 * UNIT * (exact.abs() + total.abs()))[large & finite].all()
     assert ((out.double() - total).abs() <= (15 + 17) * UNIT * size + 2 * UNIT * total.abs())[~large & finite].all()
     assert torch.isinf(out[exact.abs() > 3.5e38]).all()
+
+
+# Operands of one sign: what the accumulators cut off does not cancel.  Of a block of 64 places four roundings, each of at most a
+# unit of what is there (2 UNIT), the first three smaller; then the sums of blocks, runs and halves.  On average less: 2-norm
+# 9.3e-8, 0.84e-7 of it one-sided, at every K; by multiply-adds 4.4e-8 to 9.2e-8.
+@pytest.mark.parametrize("rows", [8, 12, 64])
+@pytest.mark.parametrize("K", [64, 1024, 12288])
+def test_operands_of_one_sign(k, rows, K):
+    x, w = rnd(rows, K, seed=7).abs(), rnd(300, K, seed=8).abs()
+    out = torch.empty(rows, 300, device="cuda")
+    k.linear(x, w, out)
+    exact = x.double() @ w.double().t()
+    error = (out.double() - exact) / exact
+    # (a sum of n blocks, each with its own error, has the average of theirs and the roundings of the sums in between)
+    assert float(error.abs().max()) <= (2 * 5 + 1 + -(-K // 64)) * UNIT
+    assert float(error.square().mean().sqrt()) <= 2 * UNIT and -2 * UNIT <= float(error.mean()) <= 0
