@@ -80,8 +80,9 @@ __device__ __forceinline__ float af_keep(float m, float m_new) { return m == -IN
 // Bound by the products beside the threads' work: 48 MMAs of 128 x 64 x 16 (shared memory: 48 cycles each) and 24 of
 // 128 x D x 16 (64) a block, 3,900 cycles for heads of 128.  An issuing thread waits while they run (issued by one of the
 // working warps a block took 11,400).  Heads of 128, us by multiply-adds (64 rows a CTA, four CTAs to a row tile's keys) and
-// so: 3 prompts of up to 400 tokens of 16 heads 109 and 38, 4 of 600 after 800 of 32 heads 1,536 and 400, 64 tokens after 800
-// of 16 heads 84 and 80, 100 after 4,000 315 and 308, 4 after 800 82 and 74.
+// so: with keys and values that are not in
+// L2: 3 prompts of up to 400 tokens of 16 heads 104 and 45 (in L2 109 and 37), 4 of 600 after 800 of 32 heads 1,536 and 383, 64 tokens
+// after 800 of 16 heads 84 and 76, 100 after 4,000 315 and 285, 4 after 800 82 and 70; 2,000 tokens, heads of 64, 393 and 145.
 //
 // Scores and outputs are 2^32 as large as they should be until they are used.  A query or key without parts (no number, or from
 // 2^112 on) makes its scores no number; those, and scores from 2^96 on, are summed by multiply-adds.  Such values are marked

@@ -25,8 +25,9 @@
 // the swizzled K-major layout; a warp of its own issues the MMAs (an issuing thread waits while they run); and while they
 // do, the others read the accumulator of the block before, in one of two buffers in TMEM, and add it up.  Bound by that work
 // beside 24 MMAs a block (64 cycles each with 128 columns, and shared memory as long); tiles of 64 x 64 by multiply-adds were
-// bound by their reads of shared memory.  Us by multiply-adds and so: 300 rows of 6,144 x 1,024 134 and 35, of 12,288 x 2,048
-// 447 and 122, 1,200 rows 1,563 and 440 (134 TFLOP/s, 6 times as many products), 64 rows of 1,024 x 3,072 26 and 15.5.
+// bound by their reads of shared memory.  Us by multiply-adds and so, in a replayed graph, weights in turn that L2 does not
+// hold: 300 rows of 6,144 x 1,024 134 and 34, of 12,288 x 2,048 449 and 120, 1,200 rows 1,564 and 429 (141 TFLOP/s, 6 times as many
+// products), 64 rows of 1,024 x 3,072 26 and 14.4.
 #define CHIBI_UNIT gemm_f32_tcgen05
 #define CHIBI_UNIT_ID 18
 #include "common.cuh"
@@ -460,8 +461,10 @@ gemm_f32_tc_kernel(const __grid_constant__ F3Params p)
 // 16 x 64 numbers (eight pieces of 16 bytes a lane, a row's 64 bytes by four lanes; the places of a fragment are taken as they
 // lie), splits sixteen places, asks for the next block's in their stead and multiplies; a block's or a run's sums go to shared
 // memory, where they are put together in order.  Bound by the weights' way from memory, with many of them by mma.sync's rate.  Us by
-// multiply-adds and so, one / four / eight rows: 4,096 x 1,024 5.8, 6.4, 7.8 and 5.7, 5.8, 5.8; 1,024 x 3,072 7.1, 8.1, 10.1 and 7.5,
-// 7.5, 7.6; 151,936 x 1,024 104, 123, 125 and 106, 106, 107; 6,144 x 1,024 7.0, 8.1, 10.7 and 8.0, 8.1, 8.3.
+// multiply-adds and so, one / four / eight / sixteen rows, in a replayed graph, weights in turn that L2 does not hold (the same
+// weights again, where they fit: 0.3 to 2 less): 4,096 x 1,024 5.8, 6.4, 7.8, 11.3 and 5.7, 5.7, 5.8, 8.6; 1,024 x 3,072 7.1, 8.1, 10.1, 13.7
+// and 7.0, 7.1, 7.3, 10.9; 6,144 x 1,024 7.2, 8.3, 10.9, 16.1 and 8.1, 8.0, 8.1, 13.0; 2,048 x 6,144 12.7, 14.1, 18.4, 25.6 and 13.3, 13.7, 14.2,
+// 20.9; 151,936 x 1,024 107, 131, 137, 176 and 103, 115, 116, 177.
 template <int TILES, int WARPS, bool KEPT>                   // eights of rows of x; warps; x stays split in shared memory
 __global__ void __launch_bounds__(32 * WARPS, F3_FEW_WARPS / WARPS)
 gemm_f32_few_kernel(const __grid_constant__ F3Params p, int w_tiles)
@@ -691,9 +694,9 @@ static int f3_few(const F3Params& p, size_t shared, cudaStream_t stream)
 }
 
 // Which form of it, by how many tiles of 16 rows of w there are: one CTA of sixteen warps an SM where every tile has one at once
-// (1,024 x 2,048, eight rows, 5.6 us; eight warps 6.5), or two rounds and a half do (6,144 x 1,024 8.2 and 9.4); eight warps
-// where two to an SM have one round (4,096 x 1,024 5.8 and 6.1) or many (12,288 x 2,048 23.4 and 26.5); from eight
-// tiles an SM on, x is split once and kept (151,936 x 1,024 107 and 119; 12,288 x 2,048 30.7).
+// (1,024 x 2,048, eight rows, 5.0 us; eight warps 6.0), or two rounds and a half do (6,144 x 1,024 7.6 and 8.2); eight warps
+// where two to an SM have one round (4,096 x 1,024 5.1 and 5.6) or many (12,288 x 2,048 21.0 and 24.0); from eight
+// tiles an SM on, x is split once and kept (151,936 x 1,024 103 and 114; 12,288 x 2,048 29.0).
 template <int TILES>
 static int f3_few_rows(const F3Params& p, int form, cudaStream_t stream)
 {
@@ -755,7 +758,7 @@ CHIBI_API int chibi_gemm_f32(const float* x, const float* w, float* out, const f
     p.run_blocks = (blocks + F3_RUNS - 1) / F3_RUNS;
     p.runs = (blocks + p.run_blocks - 1) / p.run_blocks;
     // To 16 rows the kernel for few; but mma.sync does 16 x 8 x 16 products in 32 cycles of a quarter of an SM, and with
-    // 9 to 16 rows and many rows of w that is what bounds it (151,936 x 1,024: 232 us and 180 here, 8 rows 107).
+    // 9 to 16 rows and many rows of w that is what bounds it (151,936 x 1,024: 232 us and 176 here, 8 rows 107).
     const int sms = device_sm_count();
     if (cols <= 0 && (M <= 8 || (M <= 16 && (N + 15) / 16 < F3_FEW_MANY * sms)))
         return M <= 8 ? f3_few_rows<1>(p, -cols, stream) : f3_few_rows<2>(p, -cols, stream);

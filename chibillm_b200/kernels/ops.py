@@ -821,7 +821,8 @@ class CudaKernels:
         """Causal attention of every token over its sequence's pages.  bfloat16
         with a head size that is a multiple of 16 runs on the tensor cores (one
         library per head size, compiled when first needed); 32-bit operands with head
-        sizes 64 and 128 run kernels of their own (32-bit arithmetic throughout);
+        sizes 64 and 128 run kernels of their own (prompts as products of three bfloat16 parts
+        with 32-bit sums, single tokens by 32-bit multiply-adds);
         everything else runs the plain kernel.  ``softcap`` c: a scaled score
         s becomes c * tanh(s / c).  ``distance_bias`` (r1, r2), float32 [nq] each:
         r1[h] * ln(1 + r2[h] * (i - j)) is taken off the score of query i and key j.
