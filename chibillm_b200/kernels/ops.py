@@ -969,11 +969,11 @@ class CudaKernels:
         """How the decode attention kernel deals with sequences of different lengths (which the host does not know
         here; steps that are known to be even don't ask): (key ranges of all sequences together, or 0; whether the longest
         sequences start first).  Where ``splits`` ranges each fit the resident CTAs, the same number of CTAs goes to ranges of
-        one length instead, cut on the device if the lengths differ (8 kv heads, a replayed graph: 16 sequences of 1,500 to
-        6,000 keys 65.5 -> 51.7 us, 8 38.4 -> 33.3; the look at the lengths costs equal ones 0.4 of 18.6 (8 x 2,048) to 1.2
-        of 70.8 us (16 x 6,000), so not below 512 keys a range).
+        one length instead, cut on the device if the lengths differ (8 kv heads, a replayed graph: 16 sequences of 1,622 to
+        6,000 keys 65.5 -> 52.5 us, 8 of 2,660 to 6,000 38.4 -> 33.5; the look at the lengths costs equal ones 0.8 of 18.6 us (8 x
+        2,048) to 2.4 of 70.8 (16 x 6,000), so not below 512 keys a range).
         Where even one each does not fit, a range costs more than it evens out, and the order does: 64 sequences of
-        1,046 to 4,096 keys 143.8 -> 105.9 us, of equal lengths 179.6 and 181.7.  More sequences than the kernels' searches
+        1,041 to 4,096 keys 143.8 -> 105.6 us, of equal lengths 179.6 and 180.9.  More sequences than the kernels' searches
         take, and contexts too short to be worth them, stay in equal shares and in the batch's order."""
         per_seq = nkv * ((nq // nkv + 15) // 16)
         slots = 2 * self.sm_count
